@@ -149,10 +149,6 @@ struct eddy_ctx {
     bool exact_all;
   };
   std::map<int, ThrSet> thr_cache;
-  // changed-node records per network that units of sets of g genes needed
-  // beyond the default (kept across sets and eddy_clear_sets): later
-  // batches start there
-  std::map<int, int> kmax_hint;
   int lg_shift = 0;
   bool lg_ready = false;
   int lg_n = -1;  // sample count the fixed-point lgamma table was built for
@@ -253,7 +249,7 @@ int prepare_sets(eddy_ctx *ctx, const std::vector<int> &ids) {
     if (rc) return rc;
   }
   auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-  std::vector<size_t> ov(ns), opr(ns), ovt(ns), opl(ns), ova(ns), oct(ns);
+  std::vector<size_t> ov(ns), opr(ns), oco(ns), opl(ns), ova(ns), oct(ns);
   size_t o = 0;
   for (int k = 0; k < ns; k++) {
     const int g = (int)ctx->sets[ids[k]].genes.size();
@@ -273,8 +269,8 @@ int prepare_sets(eddy_ctx *ctx, const std::vector<int> &ids) {
   for (int k = 0; k < ns; k++) {
     const int g = (int)ctx->sets[ids[k]].genes.size(), c = g * (g - 1) / 2;
     o = al(o);
-    ovt[k] = o;
-    o += (size_t)st_stride(g) * n + 16;
+    oco[k] = o;
+    o += sizeof(uint32_t) * (size_t)g * code_words(n);
     o = al(o);
     opl[k] = o;  // planes, then their word-major copy
     o += 2 * sizeof(uint64_t) * (size_t)g * 3 * W;
@@ -315,7 +311,7 @@ int prepare_sets(eddy_ctx *ctx, const std::vector<int> &ids) {
     for (int k = 0; k < ns; k++) {
       const int g = (int)ctx->sets[ids[k]].genes.size(), c = g * (g - 1) / 2;
       CK(launch_prep((const int8_t *)(db + ov[k]), g, n, W, c, (uint64_t *)(db + opl[k]),
-                     (uint64_t *)(db + ova[k]), (uint16_t *)(db + oct[k]), (int8_t *)(db + ovt[k]),
+                     (uint64_t *)(db + ova[k]), (uint16_t *)(db + oct[k]), (uint32_t *)(db + oco[k]),
                      ctx->stream));
       ctx->launches += 2 + (c > 0);
     }
@@ -358,7 +354,8 @@ int prepare_sets(eddy_ctx *ctx, const std::vector<int> &ids) {
     sd.planesT = sd.planes + (size_t)sh.g * 3 * W;
     sd.valid = (const uint64_t *)(db + ova[k]);
     sd.vals = (const int8_t *)(db + ov[k]);
-    sd.valsT = (const int8_t *)(db + ovt[k]);
+    sd.codes = (const uint32_t *)(db + oco[k]);
+    sd.n16 = code_words(n);
     sd.ctot = (const uint16_t *)(db + oct[k]);
     sd.prior = (const uint8_t *)(db + opr[k]);
     sd.lg = ctx->d_lg.as<int64_t>();
@@ -633,12 +630,11 @@ struct UnitRef {
 // Runs the units `units` (in job order: a job's units are consecutive) as
 // one batch: the sets' data resident, the set table, labellings, decisions,
 // networks, normalisation and JS, one synchronisation.  Units whose status
-// asks for a re-run go to *again (need: the records they want; collision:
-// a hash collision was found); *queue_full: the general-path queue
+// asks for a re-run (a hash collision) go to *again; *queue_full: the general-path queue
 // overflowed (nothing was stored: the batch must be decided another way).
-int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> &units, int kmax,
-              bool popc_batch, std::vector<UnitRef> *again, int *need, bool *collision,
-              bool *queue_full, float *t_pairs, float *t_units) {
+int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> &units,
+              bool popc_batch, std::vector<UnitRef> *again, bool *collision, bool *queue_full,
+              float *t_pairs, float *t_units) {
   const int Bt = (int)units.size(), W = ctx->W, n = ctx->samples, S = n + 2;
   // slots: the jobs of the batch, in order
   std::vector<int> slot_job, ids;
@@ -672,7 +668,7 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
     b.nb = nb;
     b.dm0 = (long long)dmw;
     dmw += dmask_words(nb, b.sd.c);
-    b.unit_bytes = (long long)unit_scratch_bytes(b.sd.c, S, kmax);
+    b.unit_bytes = (long long)unit_scratch_bytes(b.sd.c, S);
     b.sc0 = (long long)scb;
     scb += (size_t)nb * b.unit_bytes;
     bp.gmax = std::max(bp.gmax, b.sd.g);
@@ -743,8 +739,8 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   BatchDev bd{};
   bd.B = Bt;
   bd.nsets = ns;
-  bd.kmax = kmax;
-  bd.key_walk = getenv("EDDY_KEY_WALK") ? 1 : 0;
+  bd.memo_max = kMemoMax;
+  if (const char *em = getenv("EDDY_MEMO_MAX")) bd.memo_max = std::max(0, std::min(kMemoMax, atoi(em)));
   bd.sets = ctx->d_sets.as<BatchSet>();
   bd.uslot = ctx->d_uslot.as<int32_t>();
   bd.masks = ctx->d_masks.as<uint64_t>();
@@ -811,7 +807,7 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
     // everything a replay bakes in: the sets, their state, the batch shape
     // and every buffer address
     std::vector<uintptr_t> key = {(uintptr_t)ctx->prep_gen, (uintptr_t)ctx->salt,
-                                  (uintptr_t)Bt, (uintptr_t)kmax, (uintptr_t)v,
+                                  (uintptr_t)Bt, (uintptr_t)v,
                                   (uintptr_t)ctx->o.seed, (uintptr_t)ctx->d_masks.p,
                                   (uintptr_t)ctx->d_dmask.p, (uintptr_t)ctx->d_scratch.p,
                                   (uintptr_t)ctx->d_js.p, (uintptr_t)ctx->d_U.p,
@@ -821,7 +817,7 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
                                   (uintptr_t)ctx->d_stats.p, (uintptr_t)ctx->d_afp8.p,
                                   (uintptr_t)ctx->d_Y.p, (uintptr_t)ctx->d_err.p,
                                   (uintptr_t)ctx->d_mask0.p, (uintptr_t)ctx->stream,
-                                  (uintptr_t)bp.sets[0].sd.exact_all, (uintptr_t)bd.key_walk};
+                                  (uintptr_t)bp.sets[0].sd.exact_all, (uintptr_t)bd.memo_max};
     for (int k = 0; k < ns; k++) {
       key.push_back((uintptr_t)ids[k]);
       key.push_back((uintptr_t)bp.sets[k].nb);
@@ -935,10 +931,7 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   }
   for (int i = 0; i < Bt; i++) {
     Job &J = jobs[units[i].job];
-    if (hst[i] & kUnitKmaxOverflow) {
-      *need = std::max(*need, (int)(hst[i] >> 16));
-      again->push_back(units[i]);
-    } else if (hst[i] & kUnitHashCollision) {
+    if (hst[i] & kUnitHashCollision) {
       *collision = true;
       again->push_back(units[i]);
     } else {
@@ -949,7 +942,7 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   // detailed outputs of the kept units that finished
   for (int q = 0; q < nk; q++) {
     const int i = kept[q];
-    if (hst[i] & (kUnitKmaxOverflow | kUnitHashCollision)) continue;
+    if (hst[i] & kUnitHashCollision) continue;
     Job &J = jobs[units[i].job];
     KeepOut *K = J.keep;
     const int g = ctx->res_sd[uslot[i]].g, GW = (g + 31) / 32, Uk = hU[i];
@@ -996,30 +989,13 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
 int run_jobs(eddy_ctx *ctx, std::vector<Job> &jobs) {
   if (jobs.empty()) return EDDY_OK;
   const int n = ctx->samples, S = n + 2, W = ctx->W;
-  int gmax = 0, cmax = 1, total = 0;
+  int cmax = 1, total = 0;
   size_t per_unit_max = 1;
-  // kmax: changed-node records per network (records are written only for
-  // changed nodes, so room for more costs memory, not time).  64 covers the
-  // networks of most sets; at 200 genes with ~3% of the pair tests within
-  // 20% of the threshold, about one unit in eight of a context's first
-  // batch needs more and is re-run, and the per-size hint gives later
-  // batches that room.  EDDY_KMAX lowers it, to test those re-runs.
-  const char *ek = getenv("EDDY_KMAX");
-  int kmax = 1;
   for (const Job &J : jobs) {
     const int g = (int)ctx->sets[J.set_id].genes.size(), c = g * (g - 1) / 2;
-    gmax = std::max(gmax, g);
     cmax = std::max(cmax, c);
     total += J.n_units;
-    int k = std::min(g + 1, 64);
-    auto it = ctx->kmax_hint.find(g);
-    if (it != ctx->kmax_hint.end()) k = std::max(k, std::min(g + 1, it->second));
-    kmax = std::max(kmax, k);
-  }
-  if (ek) kmax = std::max(1, std::min(16, atoi(ek)));
-  for (const Job &J : jobs) {
-    const int g = (int)ctx->sets[J.set_id].genes.size(), c = g * (g - 1) / 2;
-    per_unit_max = std::max(per_unit_max, unit_scratch_bytes(c, S, kmax) + 4 * (size_t)c + 8 * W + 64);
+    per_unit_max = std::max(per_unit_max, unit_scratch_bytes(c, S) + 4 * (size_t)c + 8 * W + 64);
   }
   // batch size: bounded by memory (masks, decisions and scratch, up to 16 GB),
   // by 16384 units (the general-path queue holds unit indices below 2^15)
@@ -1041,32 +1017,18 @@ int run_jobs(eddy_ctx *ctx, std::vector<Job> &jobs) {
   float t_pairs = 0, t_units = 0;
   for (int b0 = 0; b0 < total; b0 += Bmax) {
     std::vector<UnitRef> todo(all.begin() + b0, all.begin() + std::min(total, b0 + Bmax));
-    int kmax_run = kmax;
     bool popc_batch = false;
     for (int attempt = 0; attempt < 4 && !todo.empty(); attempt++) {
       std::vector<UnitRef> again;
-      int need = 0;
       bool collision = false, queue_full = false;
-      int rc = run_batch(ctx, jobs, todo, kmax_run, popc_batch, &again, &need, &collision,
-                         &queue_full, &t_pairs, &t_units);
+      int rc = run_batch(ctx, jobs, todo, popc_batch, &again, &collision, &queue_full, &t_pairs,
+                         &t_units);
       if (rc) return rc;
       if (queue_full) {
         // a large share of tables near a threshold: decide this batch with
         // the popcount kernel
         popc_batch = true;
         continue;
-      }
-      if (need) {
-        // the re-run holds every record these units need (their networks do
-        // not change); sets of this size start with a quarter more later
-        const int want = std::max(need, kmax_run + 1);
-        kmax_run = std::min(gmax + 1, (want + 7) / 8 * 8);
-        if (!ek)
-          for (const UnitRef &r : again) {
-            const int g = (int)ctx->sets[jobs[r.job].set_id].genes.size();
-            int &hint = ctx->kmax_hint[g];
-            hint = std::max(hint, std::min(g + 1, (want + want / 4 + 7) / 8 * 8));
-          }
       }
       if (collision) ctx->salt = ctx->salt * 6364136223846793005ull + 1442695040888963407ull;
       todo.swap(again);

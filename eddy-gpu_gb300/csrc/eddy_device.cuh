@@ -446,44 +446,41 @@ __device__ __forceinline__ uint32_t pair_mask(const int *t, int prior, const Set
 // --------------------------------------------------- capped parent lists
 // Generates the parent list of node t (ascending gene index) of the network
 // "full network of class k with the pair tables of sample sigma removed":
-// row bits of the full network XOR the flips that sigma's cells trigger.
+// row bits of the full network XOR the flips that sigma's cells trigger
+// (sigma < 0: the full network's).
 struct ListGen {
-  const uint32_t *row;   // GW words, bit j = edge (t, j), j < t
-  const uint32_t *phi;   // flip entries (p << 9 | flipbits), sorted by p
-  const uint16_t *pcol;  // column of each flip entry
-  const int8_t *stsig;   // states (0..3) of all genes at sample sigma, or null
-  int fi, fe, w, GW, strow;
+  const uint32_t *row;  // GW words, bit j = edge (t, j), j < t
+  const uint2 *ent;     // kept flip entries of the row: [fi, fe), by column
+  const uint32_t *cw;   // packed states at sigma's word, or null
+  int fi, fe, w, GW, n16, sh, a4;
   uint32_t word;
 
   __device__ __forceinline__ uint32_t flipword(int ww) {
     uint32_t m = 0;
-    if (stsig == nullptr || strow > 2) {
-      return 0;
-    }
+    if (cw == nullptr) return 0;
     const int hi = 32 * (ww + 1);
     while (fi < fe) {
-      int col = pcol[fi];
+      const uint2 en = ent[fi];
+      const int col = en.x & 511;
       if (col >= hi) break;
-      int sc = stsig[col];
-      if (sc <= 2) {
-        uint32_t bits = phi[fi] & 0x1FFu;
-        if ((bits >> (strow * 3 + sc)) & 1u) m |= 1u << (col - 32 * ww);
-      }
+      const int b = (cw[(size_t)col * n16] >> sh) & 3;
+      m |= ((en.y >> (a4 + b)) & 1u) << (col - 32 * ww);
       fi++;
     }
     return m;
   }
-  __device__ __forceinline__ void init(const uint32_t *row_, int GW_, const uint32_t *phi_,
-                                       const uint16_t *pcol_, int fi_, int fe_,
-                                       const int8_t *stsig_, int strow_) {
+  __device__ __forceinline__ void init(const uint32_t *row_, int GW_, const uint2 *ent_, int fi_,
+                                       int fe_, const uint32_t *codes, int n16_, int t,
+                                       int sigma) {
     row = row_;
     GW = GW_;
-    phi = phi_;
-    pcol = pcol_;
+    ent = ent_;
     fi = fi_;
     fe = fe_;
-    stsig = stsig_;
-    strow = strow_;
+    n16 = n16_;
+    cw = sigma >= 0 ? codes + (sigma >> 4) : nullptr;
+    sh = 2 * (sigma & 15);
+    a4 = sigma >= 0 ? 4 * (int)((cw[(size_t)t * n16] >> sh) & 3u) : 0;
     w = 0;
     word = (GW > 0) ? (row[0] ^ flipword(0)) : 0u;
   }

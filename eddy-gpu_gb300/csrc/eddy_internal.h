@@ -16,9 +16,6 @@ constexpr int kDofSlots = 3;        // dof 1, 2, 4 (dof 0 never gives an edge)
 constexpr int kMaxBdeuParents = 3;  // kernel5.cu:119-130 caps at 1 + 3
 constexpr int kDivisors = 15;       // distinct q and q*r of the BDeu terms
 constexpr uint32_t kUnitOk = 0;
-constexpr uint32_t kUnitKmaxOverflow = 1u;   // more changed nodes than kmax;
-                                             // bits 16-31 then hold the most
-                                             // changed nodes of its networks
 constexpr uint32_t kUnitHashCollision = 2u;  // equal hash, unequal networks
 constexpr uint32_t kUnitBadShape = 4u;
 
@@ -48,8 +45,9 @@ struct SetDev {
   const uint64_t *planesT; // [W][g][3] the same planes word-major (follows planes)
   const uint64_t *valid;  // [W] all-sample mask
   const int8_t *vals;     // [g][n]  -1/0/1, 2 = any other value
-  const int8_t *valsT;    // [n][st_stride(g)] states 0-3 (st_of) of the same,
-                          // sample-major, rows padded with 3 to 16 bytes
+  const uint32_t *codes;  // [g][n16] states 0-3 (st_of) of the same, two bits
+                          // each, 16 samples a word
+  int n16;                // code_words(n)
   const uint16_t *ctot;   // [c][9]  permutation-invariant full-sample table
   const uint8_t *prior;   // [c]     prior bit of pair p
   const int64_t *lg;      // [kDivisors][n+1] fixed-point lgamma(m+4/d)-lgamma(4/d)
@@ -69,9 +67,8 @@ struct SetDev {
 #else
 #define EDDY_HD
 #endif
-// Row stride of the sample-major state matrix: genes rounded up to 16, so
-// that every row starts on a 16-byte boundary.
-EDDY_HD constexpr int st_stride(int g) { return (g + 15) & ~15; }
+// 32-bit words of a gene's packed states (two bits a sample).
+EDDY_HD constexpr int code_words(int n) { return (n + 15) >> 4; }
 EDDY_HD constexpr int chunk_words(int c) { return ((c + 31) / 32 + 31) / 32; }
 // u32 words of one set's decision masks and chunk bitmaps for nb units
 EDDY_HD constexpr size_t dmask_words(int nb, int c) {
@@ -119,9 +116,8 @@ __device__ __forceinline__ void mark_chunk(uint32_t *ucb, int p) {
 struct BatchDev {
   int B;                       // units in the batch
   int nsets;                   // sets in the batch
-  int kmax;                    // changed-node records per network
-  int key_walk;                // 1: the key table from a walk over the unique
-                               // networks' records (EDDY_KEY_WALK, a test switch)
+  int memo_max;                // most entries of a row whose lists are formed
+                               // per subset of them (EDDY_MEMO_MAX lowers it)
   const BatchSet *sets;        // [nsets]
   const int32_t *uslot;        // [B] set of each unit (index into sets)
   const uint64_t *masks;       // [B][W] class-1 sample mask per unit

@@ -10,14 +10,14 @@
 //                       leave-one-out decision mask per class: the reference's
 //                       run2/run2Scalable (kernel1.cu:389-477) over all S
 //                       networks collapsed to <= 10 distinct tables per class.
-//   k_units             one block per unit: full networks, flip lists,
-//                       per-network capped parent lists as deltas
+//   k_units             one block per unit: full networks, flip lists, the
+//                       capped parent lists that left-out samples change
 //                       (kernel2.cu:114-142, kernel3.cu:134-165), network
 //                       hashing and first-occurrence dedup with exact
 //                       verification (kernel4.cu:72-84, main.cu:1060-1121),
 //                       BDeu over the unique networks in fixed point
-//                       (kernel5.cu:237-257), normalisation and JS
-//                       (main.cu:1293-1428).
+//                       (kernel5.cu:237-257).
+//   k_js                normalisation and JS (main.cu:1293-1428).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -56,14 +56,17 @@ __global__ void k_planes(const int8_t *vals, int g, int n, int W, uint64_t *plan
   if (i == 0) valid[w] = v;
 }
 
-// Sample-major states: valsT[s][i] = st_of(vals[i][s]), rows of
-// st_stride(g) bytes padded with state 3 (no value).
-__global__ void k_transpose(const int8_t *vals, int g, int n, int8_t *valsT) {
-  const int gp = st_stride(g);
+// Packed states: codes[i][s / 16] holds st_of(vals[i][s]) of sample s in
+// bits 2 (s mod 16), 3 past the last sample.
+__global__ void k_codes(const int8_t *vals, int g, int n, uint32_t *codes) {
+  const int n16 = code_words(n);
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= gp * n) return;
-  const int s = idx / gp, i = idx % gp;
-  valsT[idx] = (int8_t)(i < g ? st_of(vals[(size_t)i * n + s]) : 3);
+  if (idx >= g * n16) return;
+  const int i = idx / n16, s0 = 16 * (idx % n16);
+  uint32_t x = 0;
+  for (int q = 0; q < 16; q++)
+    x |= (uint32_t)(s0 + q < n ? st_of(vals[(size_t)i * n + s0 + q]) : 3) << (2 * q);
+  codes[idx] = x;
 }
 
 __global__ void k_ctot(const uint64_t *planes, int g, int W, int c, uint16_t *ctot) {
@@ -256,47 +259,31 @@ __global__ void __launch_bounds__(128) k_pairs(const BatchSet *__restrict__ sets
 }
 
 // ------------------------------------------------------------ k_units
-// Open-addressing table: key -> smallest value inserted with it.  `empty`
-// marks a free slot (no real key equals it); probing stops after `probes`
-// slots (an insert that finds no place returns false).
-struct MinTable {
-  unsigned long long *key;
-  int *val;
-  unsigned mask;
-  unsigned long long empty;
-  unsigned probes;
-  __device__ bool insert_min(unsigned long long k, int v) const {
-    unsigned slot = (unsigned)(mix64(k) & mask);
-    for (unsigned i = 0; i < probes; i++, slot = (slot + 1) & mask) {
-      const unsigned long long prev = atomicCAS(&key[slot], empty, k);
-      if (prev == empty || prev == k) {
-        atomicMin(&val[slot], v);
-        return true;
-      }
-    }
-    return false;
-  }
-  // value of a key that was inserted
-  __device__ int get(unsigned long long k) const {
-    unsigned slot = (unsigned)(mix64(k) & mask);
-    while (key[slot] != k) slot = (slot + 1) & mask;
-    return val[slot];
-  }
-};
-// slots of the shared-memory tables (in the BDeu work region, idle then)
-constexpr int kSmSlots = 512;
-constexpr unsigned kSmProbes = 64;
-
-struct UnitLayout {
-  size_t phi[2], pcol[2], rec, htk, htv, dist, uid, urep, sig;
-  size_t skey, sbits, srep, hsk, hsv, wl, ksc, memo, total;
-  int HT, rec_words;  // rec_words: 64-bit words per network record
-};
-// Rows with at most kMemoE kept flip entries have their capped list under
-// every non-empty subset of those entries tabulated once per unit:
-// [2 g rows][kMemoSub subsets][2 words] (record entry or ~0 when the list
-// is the full network's, and the list's hash).
-constexpr int kMemoE = 6, kMemoSub = (1 << kMemoE) - 1;
+// Kept flip entries of the two full networks' rows, one uint2 each:
+//   x = column (9 bits) | node << 9 | position in its row << 18 (3 bits)
+//       | last of its row << 21
+//   y = cells: bit 4a + b set when the entry fires for a left-out sample of
+//       states a (node) and b (column), no bit for a missing value (3);
+//       bits 16-31: the row's first variant (memo rows)
+__device__ __forceinline__ uint32_t cells16(uint32_t fb) {
+  return (fb & 7u) | (((fb >> 3) & 7u) << 4) | (((fb >> 6) & 7u) << 8);
+}
+// A row with at most E <= kMemoE kept entries (and no more subsets of them
+// than its class has samples) is a memo row: its capped list under every
+// non-empty subset of its entries (a variant) is formed once per unit.  The
+// other rows' lists are formed per left-out sample.  E is lowered until the
+// unit's variants fit unit_variants(g), which rows of up to five entries
+// always do.
+constexpr int kMemoE = 8;
+__host__ __device__ constexpr int unit_variants(int g) { return 62 * g + 64; }
+// slots of the table of the lists formed per sample (in the unit's scratch)
+__host__ __device__ constexpr int big_slots(int g) {
+  int s = 256;
+  while (s < 16 * g && s < 8192) s <<= 1;
+  return s;
+}
+// network table: slots held in shared memory (larger ones in the scratch)
+constexpr int kSmSlots = 4096;
 // genes of a set of c pairs (c = g (g - 1) / 2, so 1 + 8 c = (2 g - 1)^2)
 __host__ __device__ inline int genes_of_pairs(int c) {
   int r = (int)sqrt((double)(1 + 8 * (long long)c));
@@ -305,76 +292,68 @@ __host__ __device__ inline int genes_of_pairs(int c) {
   return (r + 1) / 2;
 }
 
-__host__ __device__ inline UnitLayout unit_layout(int c, int S, int kmax) {
+struct UnitLayout {
+  size_t phi[2], ent, ment, mdh, msc, vcan, sel, hs, dist, sig, urep, wl, vrep, ubits, htab;
+  size_t bkey, bsc, bpos, total;
+};
+__host__ __device__ inline UnitLayout unit_layout(int c, int S) {
   UnitLayout L;
   size_t o = 0;
-  auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-  for (int k = 0; k < 2; k++) {
-    L.phi[k] = o;
-    o = al(o + sizeof(uint32_t) * (size_t)(c > 0 ? c : 1));
-    L.pcol[k] = o;
-    o = al(o + sizeof(uint16_t) * (size_t)(c > 0 ? c : 1));
-  }
-  L.rec_words = 2 + kmax;  // [H, nchg | flags, chg...]
-  L.rec = o;
-  o = al(o + sizeof(uint64_t) * (size_t)L.rec_words * S);
-  int HT = 1;
-  while (HT < 2 * S) HT <<= 1;
-  L.HT = HT;
-  L.htk = o;
-  o = al(o + sizeof(uint64_t) * (size_t)HT);
-  L.htv = o;
-  o = al(o + sizeof(int32_t) * (size_t)HT);
-  L.dist = o;
-  o = al(o + sizeof(int64_t) * 2 * (size_t)S);
-  L.uid = o;
-  o = al(o + sizeof(int32_t) * (size_t)S);
-  L.urep = o;
-  o = al(o + sizeof(int32_t) * (size_t)S);
-  L.sig = o;  // class-1 samples then class-2 samples, in index order
-  o = al(o + sizeof(int32_t) * (size_t)S);
-  L.skey = o;  // per network: signature key (0 = no flip entry triggered)
-  o = al(o + sizeof(uint64_t) * (size_t)S);
-  L.sbits = o;  // per network: triggered entries as a bitset (<= 64 entries)
-  o = al(o + sizeof(uint64_t) * (size_t)S);
-  L.srep = o;  // per network: first network with the same signature
-  o = al(o + sizeof(int32_t) * (size_t)S);
-  L.hsk = o;  // signature hash table
-  o = al(o + sizeof(uint64_t) * (size_t)HT);
-  L.hsv = o;
-  o = al(o + sizeof(int32_t) * (size_t)HT);
-  L.wl = o;  // work list of networks
-  o = al(o + sizeof(int32_t) * (size_t)S);
-  L.ksc = o;  // scores of the distinct changed-node keys: [HT][2 classes]
-  o = al(o + 2 * sizeof(int64_t) * (size_t)HT);
-  L.memo = o;  // per-row capped lists under each subset of the row's entries
-  o = al(o + 2 * sizeof(uint64_t) * kMemoSub * 2 * (size_t)genes_of_pairs(c));
+  auto take = [&](size_t bytes) {
+    const size_t at = o;
+    o = (o + bytes + 255) & ~(size_t)255;
+    return at;
+  };
+  const size_t cc = c > 0 ? c : 1;
+  const int g = genes_of_pairs(c);
+  const size_t nv = unit_variants(g), nb = big_slots(g);
+  L.dist = take(sizeof(int64_t) * 2 * (size_t)S);
+  L.hs = take(sizeof(uint64_t) * (size_t)S);    // per network: hash, ~0 = its class's full one
+  L.sig = take(sizeof(int32_t) * (size_t)S);    // class-1 samples then class-2 samples
+  L.urep = take(sizeof(int32_t) * (size_t)S);   // unique networks in order
+  L.wl = take(sizeof(int32_t) * (size_t)S);     // networks merged by hash, to verify
+  L.vrep = take(sizeof(int32_t) * (size_t)S);   // and what they were merged with
+  L.ubits = take(sizeof(uint32_t) * (size_t)((S + 31) / 32));
+  int ht = 1;
+  while (ht < 2 * (S + 2)) ht <<= 1;
+  L.htab = take(ht > kSmSlots ? sizeof(int32_t) * (size_t)ht : 0);
+  L.ment = take(sizeof(uint64_t) * nv);         // variants: key (or ~0: the full list)
+  L.mdh = take(sizeof(uint64_t) * nv);          // hash less the full list's
+  L.msc = take(2 * sizeof(int64_t) * nv);       // scores less the full list's, both classes
+  L.vcan = take(sizeof(uint16_t) * nv);         // first variant of the row with the same key
+  L.sel = take(sizeof(uint16_t) * nv);          // the variants to score
+  L.bkey = take(sizeof(uint64_t) * nb);
+  L.bsc = take(2 * sizeof(int64_t) * nb);
+  L.bpos = take(sizeof(int32_t) * nb);
+  for (int k = 0; k < 2; k++) L.phi[k] = take(sizeof(uint32_t) * cc);
+  L.ent = take(2 * sizeof(uint2) * cc);
   L.total = o;
   return L;
 }
 
-size_t unit_scratch_bytes(int c, int S, int kmax) { return unit_layout(c, S, kmax).total; }
+size_t unit_scratch_bytes(int c, int S) { return unit_layout(c, S).total; }
 
 // Block-wide exclusive scan (blockDim multiple of 32, <= 1024).
-__device__ __forceinline__ int block_scan(int v, int &total, int *sbuf) {
+template <class T>
+__device__ __forceinline__ T block_scan(T v, T &total, T *sbuf) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  int x = v;
+  T x = v;
   for (int o = 1; o < 32; o <<= 1) {
-    int y = __shfl_up_sync(0xffffffffu, x, o);
+    T y = __shfl_up_sync(0xffffffffu, x, o);
     if (lane >= o) x += y;
   }
   if (lane == 31) sbuf[warp] = x;
   __syncthreads();
   if (warp == 0) {
-    int t = (lane < nw) ? sbuf[lane] : 0;
+    T t = (lane < nw) ? sbuf[lane] : (T)0;
     for (int o = 1; o < 32; o <<= 1) {
-      int y = __shfl_up_sync(0xffffffffu, t, o);
+      T y = __shfl_up_sync(0xffffffffu, t, o);
       if (lane >= o) t += y;
     }
     sbuf[lane] = t;
   }
   __syncthreads();
-  int excl = x - v + (warp ? sbuf[warp - 1] : 0);
+  const T excl = x - v + (warp ? sbuf[warp - 1] : (T)0);
   total = sbuf[nw - 1];
   __syncthreads();
   return excl;
@@ -383,31 +362,33 @@ __device__ __forceinline__ int block_scan(int v, int &total, int *sbuf) {
 struct UnitSmem {
   // fixed part; variable arrays follow in dynamic shared memory
   SetDev sd;    // the unit's set (copied from the batch's set table)
-  unsigned long long HF[2];
-  long long base[2][2];  // [data class][full network of class]
-  int nphi[2];
-  int ndab;
-  int nrphi[2];
-  int tfull;    // a shared-memory table ran out of probes
-  int nent[2];  // flip entries per class
-  int nwl;      // work-list length
+  unsigned long long HF[2];  // hashes of the two full networks
+  long long base[2][2];      // [data class][full network of class]
+  int ndab;     // nodes whose full lists differ between the classes
+  int split[2]; // class 2's first memo entry, first variant
+  int nbig[2];  // rows formed per sample, per class
   int firstB0;  // first class-2 network equal to the class-2 full network
-  int firstE2;  // first class-2 network with an empty signature (S - 1: none)
-  int ncand;    // candidates for unique networks
-  int maxchg;   // most changed nodes of a network past kmax (0: none)
-  int nlg;      // keys of merged-row lists logged by the records
-  int scan[32];
+  int nchg;     // networks that differ from their class's full network
+  int nver;     // networks merged by hash
+  int nsel;     // variants to score
+  int any;
   unsigned status;
-  int U;
-  double red_d[32];
-  long long red_l[32];
+  int scan[32];
+  unsigned long long scan64[32];
 };
 
 // BDeu work items (node scores) processed per round
 constexpr int kItems = 512;
-// the task prefix array (2 kItems + 1 ints) also holds the memo offsets of
-// the 2g rows of a unit, g <= 512 (the library's gene-set limit)
-static_assert(2 * 512 <= 2 * kItems + 1, "memo offsets do not fit the task prefix array");
+// the BDeu item arrays (keys, scores, task prefix) in one region that also
+// holds the variants' hashes while the networks are hashed (kSmVar of them)
+// and then the network table
+constexpr int kSmVar = 2048;
+constexpr size_t kWorkBytes = sizeof(unsigned long long) * kItems + 2 * sizeof(long long) * kItems +
+                              sizeof(int) * (2 * kItems + 4);
+static_assert(kSmVar * sizeof(unsigned long long) <= kWorkBytes && kSmSlots * sizeof(int) <= kWorkBytes,
+              "work region");
+// kept flip entries a unit holds in shared memory (more go to its scratch)
+constexpr int kEntCache = 1280;
 
 struct UnitPtrs {
   uint64_t *mA, *mB;      // [W]
@@ -415,79 +396,59 @@ struct UnitPtrs {
   uint32_t *rows;         // [2][g][GW]
   uint16_t *cnt3;         // [2][g][3] state counts per class
   uint16_t *fcnt;         // [2][g] capped count of full networks
+  int16_t *fend;          // [2][g] column of the mp-th parent (0x7FFF: fewer)
   uint16_t *fps;          // [2][g][3] first three parents
   unsigned long long *fh; // [2][g] node hash of full networks
   int *phs, *phe;         // [2][g] flip-entry range per row
-  uint16_t *dab;          // [g] nodes whose full lists differ between classes
-  uint16_t *rphi;         // [2][g] rows that hold flip entries, per class
-  int8_t *stsig;          // [nwarps][g] states at sigma
+  int *moff;              // [2][g] variants of the rows before
+  int *nst;               // [2][g] scratch of the compaction
+  uint16_t *big;          // [2][g] rows formed per sample, per class
+  uint8_t *need;          // [g] 1 = full lists differ, 2 = scores needed
+  uint32_t *used;         // [unit_variants / 32] variants some network uses
   unsigned long long *itk;   // [kItems] node-score items: t | np << 14 | parents
   long long *acc;            // [kItems][2] their scores per class
   int *tq;                   // [2 kItems + 1] task prefix per (item, class)
   int8_t *dmap;              // [96] divisor map (copy of the constant one)
   long long *fsc;            // [2 full][2 data][g] base node scores
-  uint32_t *ephi;            // [kEntCache] the kept flip entries, compacted
-  uint16_t *epcol;           // [kEntCache] their columns
+  uint2 *ent;                // [kEntCache] the kept flip entries
+  size_t bytes;
 };
-// flip entries a unit keeps in shared memory (more stay in its scratch)
-constexpr int kEntCache = 1536;
-// slots of the shared table of distinct changed-node keys, which takes the
-// place of the flip-entry cache (ephi, then epcol) once the records are made
-constexpr int kKeyT = 1024;
-static_assert(kKeyT * sizeof(unsigned long long) <=
-                  kEntCache * (sizeof(uint32_t) + sizeof(uint16_t)),
-              "key table larger than the flip-entry cache");
-
-__host__ __device__ inline size_t unit_smem_bytes(int g, int W, int GW, int nwarps) {
-  size_t o = sizeof(UnitSmem);
-  auto al = [](size_t x) { return (x + 15) & ~(size_t)15; };
-  o = al(o) + 2 * sizeof(uint64_t) * W;
-  o = al(o) + 2 * sizeof(int) * W;
-  o = al(o) + 2 * sizeof(uint32_t) * (size_t)g * GW;
-  o = al(o) + 2 * 3 * sizeof(uint16_t) * g;
-  o = al(o) + 2 * sizeof(uint16_t) * g;
-  o = al(o) + 2 * 3 * sizeof(uint16_t) * g;
-  o = al(o) + 2 * sizeof(unsigned long long) * g;
-  o = al(o) + 4 * sizeof(int) * g;
-  o = al(o) + sizeof(uint16_t) * g;
-  o = al(o) + 2 * sizeof(uint16_t) * g;
-  o = al(o) + (size_t)nwarps * st_stride(g);
-  o = al(o) + sizeof(unsigned long long) * kItems;
-  o = al(o) + 2 * sizeof(long long) * kItems;
-  o = al(o) + sizeof(int) * (2 * kItems + 1);
-  o = al(o) + 96;
-  o = al(o) + 4 * sizeof(long long) * g;
-  o = al(o) + sizeof(uint32_t) * kEntCache;
-  o = al(o) + sizeof(uint16_t) * kEntCache;
-  return al(o);
-}
-
-size_t unit_smem_size(int g, int W, int nwarps) { return unit_smem_bytes(g, W, (g + 31) / 32, nwarps); }
-
-__device__ inline UnitPtrs carve(char *base, int g, int W, int GW, int nwarps) {
+__host__ __device__ inline UnitPtrs carve(char *base, int g, int W, int GW) {
   UnitPtrs P;
   size_t o = sizeof(UnitSmem);
-  auto al = [](size_t x) { return (x + 15) & ~(size_t)15; };
-  o = al(o); P.mA = (uint64_t *)(base + o); P.mB = P.mA + W; o += 2 * sizeof(uint64_t) * W;
-  o = al(o); P.pcA = (int *)(base + o); P.pcB = P.pcA + W; o += 2 * sizeof(int) * W;
-  o = al(o); P.rows = (uint32_t *)(base + o); o += 2 * sizeof(uint32_t) * (size_t)g * GW;
-  o = al(o); P.cnt3 = (uint16_t *)(base + o); o += 2 * 3 * sizeof(uint16_t) * g;
-  o = al(o); P.fcnt = (uint16_t *)(base + o); o += 2 * sizeof(uint16_t) * g;
-  o = al(o); P.fps = (uint16_t *)(base + o); o += 2 * 3 * sizeof(uint16_t) * g;
-  o = al(o); P.fh = (unsigned long long *)(base + o); o += 2 * sizeof(unsigned long long) * g;
-  o = al(o); P.phs = (int *)(base + o); P.phe = P.phs + 2 * g; o += 4 * sizeof(int) * g;
-  o = al(o); P.dab = (uint16_t *)(base + o); o += sizeof(uint16_t) * g;
-  o = al(o); P.rphi = (uint16_t *)(base + o); o += 2 * sizeof(uint16_t) * g;
-  o = al(o); P.stsig = (int8_t *)(base + o); o += (size_t)nwarps * st_stride(g);
-  o = al(o); P.itk = (unsigned long long *)(base + o); o += sizeof(unsigned long long) * kItems;
-  o = al(o); P.acc = (long long *)(base + o); o += 2 * sizeof(long long) * kItems;
-  o = al(o); P.tq = (int *)(base + o); o += sizeof(int) * (2 * kItems + 1);
-  o = al(o); P.dmap = (int8_t *)(base + o); o += 96;
-  o = al(o); P.fsc = (long long *)(base + o); o += 4 * sizeof(long long) * g;
-  o = al(o); P.ephi = (uint32_t *)(base + o); o += sizeof(uint32_t) * kEntCache;
-  o = al(o); P.epcol = (uint16_t *)(base + o);
+  auto take = [&](size_t bytes) {
+    o = (o + 15) & ~(size_t)15;
+    char *p = base + o;
+    o += bytes;
+    return p;
+  };
+  P.mA = (uint64_t *)take(2 * sizeof(uint64_t) * W);
+  P.mB = P.mA + W;
+  P.pcA = (int *)take(2 * sizeof(int) * W);
+  P.pcB = P.pcA + W;
+  P.rows = (uint32_t *)take(2 * sizeof(uint32_t) * (size_t)g * GW);
+  P.cnt3 = (uint16_t *)take(2 * 3 * sizeof(uint16_t) * g);
+  P.fcnt = (uint16_t *)take(2 * sizeof(uint16_t) * g);
+  P.fend = (int16_t *)take(2 * sizeof(int16_t) * g);
+  P.fps = (uint16_t *)take(2 * 3 * sizeof(uint16_t) * g);
+  P.fh = (unsigned long long *)take(2 * sizeof(unsigned long long) * g);
+  P.phs = (int *)take(4 * sizeof(int) * g);
+  P.phe = P.phs + 2 * g;
+  P.moff = (int *)take(2 * sizeof(int) * g);
+  P.nst = (int *)take(2 * sizeof(int) * g);
+  P.big = (uint16_t *)take(2 * sizeof(uint16_t) * g);
+  P.need = (uint8_t *)take(g);
+  P.used = (uint32_t *)take(sizeof(uint32_t) * ((unit_variants(g) + 31) / 32));
+  P.itk = (unsigned long long *)take(kWorkBytes);
+  P.acc = (long long *)(P.itk + kItems);
+  P.tq = (int *)(P.acc + 2 * kItems);
+  P.dmap = (int8_t *)take(96);
+  P.fsc = (long long *)take(4 * sizeof(long long) * g);
+  P.ent = (uint2 *)take(sizeof(uint2) * kEntCache);
+  P.bytes = (o + 15) & ~(size_t)15;
   return P;
 }
+static size_t unit_smem_bytes(int g, int W) { return carve(nullptr, g, W, (g + 31) / 32).bytes; }
 
 // Network s of a unit: class k (0 = class 1, 1 = class 2) and left-out
 // sample sigma (-1 for the two full networks), kernel1.cu:85-88, 412-416.
@@ -500,33 +461,18 @@ __device__ __forceinline__ void net_of(int s, const SetDev &sd, const int *sig, 
   sigma = sig[s - 1];
 }
 
-// The states of every gene at sample sigma (3 for all when sigma < 0) into a
-// warp's row of st_stride(g) bytes (16-byte aligned), 16 bytes per lane.
-__device__ __forceinline__ void load_stsig(const SetDev &sd, int sigma, int8_t *dst, int lane) {
-  const int nv = st_stride(sd.g) / 16;
-  const uint4 *src = reinterpret_cast<const uint4 *>(sd.valsT + (size_t)(sigma >= 0 ? sigma : 0) * st_stride(sd.g));
-  uint4 *d = reinterpret_cast<uint4 *>(dst);
-  for (int i = lane; i < nv; i += 32)
-    d[i] = sigma >= 0 ? __ldg(src + i) : make_uint4(0x03030303u, 0x03030303u, 0x03030303u, 0x03030303u);
-  __syncwarp();
-}
-
 __device__ __forceinline__ void gen_for(ListGen &G, const SetDev &sd, const UnitPtrs &P,
-                                        const uint32_t *phi, const uint16_t *pcol, int k, int t,
-                                        const int8_t *st) {
-  const int GW = sd.GW;
-  const int strow = st ? st[t] : 3;
-  G.init(P.rows + ((size_t)k * sd.g + t) * GW, GW, phi, pcol, P.phs[k * sd.g + t],
-         P.phe[k * sd.g + t], st, strow);
+                                        const uint2 *ent, int k, int t, int sigma) {
+  const int i = k * sd.g + t;
+  G.init(P.rows + (size_t)i * sd.GW, sd.GW, ent, P.phs[i], P.phe[i], sd.codes, sd.n16, t, sigma);
 }
 
 // Exact comparison of the capped lists of node t in two networks.
-__device__ bool lists_equal(const SetDev &sd, const UnitPtrs &P, const uint32_t *const *phi,
-                            const uint16_t *const *pcol, int t, int k1, const int8_t *st1, int k2,
-                            const int8_t *st2) {
+__device__ __noinline__ bool lists_equal(const SetDev &sd, const UnitPtrs &P, const uint2 *ent, int t,
+                                         int k1, int sigma1, int k2, int sigma2) {
   ListGen a, b;
-  gen_for(a, sd, P, phi[k1], pcol[k1], k1, t, st1);
-  gen_for(b, sd, P, phi[k2], pcol[k2], k2, t, st2);
+  gen_for(a, sd, P, ent, k1, t, sigma1);
+  gen_for(b, sd, P, ent, k2, t, sigma2);
   for (int i = 0; i < sd.mp; i++) {
     int x = a.next(), y = b.next();
     if (x != y) return false;
@@ -535,12 +481,58 @@ __device__ bool lists_equal(const SetDev &sd, const UnitPtrs &P, const uint32_t 
   return true;
 }
 
+// A capped list's key: node, count of the first three parents, the parents.
+__device__ __forceinline__ unsigned long long list_key(int t, int cnt, const int *ps) {
+  return (unsigned long long)t | ((unsigned long long)(cnt < 3 ? cnt : 3) << 14) |
+         ((unsigned long long)(ps[0] & 0xFFFF) << 16) |
+         ((unsigned long long)(ps[1] & 0xFFFF) << 32) | ((unsigned long long)(ps[2] & 0xFFFF) << 48);
+}
+
+// The list of row i = (k, t) for left-out sample sigma, when it differs
+// from the full network's: its key and hash (false: the full list).  The
+// lists differ exactly when the first column that a triggered entry
+// toggles is not past the full list's end (an edge taken out there was in
+// the list; one put in there belongs to it).
+__device__ __noinline__ bool sample_list(const SetDev &sd, const UnitPtrs &P, const uint2 *ent, int k,
+                                         int t, int sigma, unsigned long long &key,
+                                         unsigned long long &hash) {
+  const int i = k * sd.g + t;
+  const uint32_t *cw = sd.codes + (sigma >> 4);
+  const int sh = 2 * (sigma & 15);
+  const int a4 = 4 * ((cw[(size_t)t * sd.n16] >> sh) & 3);
+  int first = 0x7FFFFFFF;
+  for (int e = P.phs[i]; e < P.phe[i]; e++) {
+    const uint2 en = ent[e];
+    const int col = en.x & 511;
+    const int b = (cw[(size_t)col * sd.n16] >> sh) & 3;
+    if ((en.y >> (a4 + b)) & 1u) {
+      first = col;
+      break;
+    }
+  }
+  if (first > P.fend[i]) return false;
+  ListGen G;
+  gen_for(G, sd, P, ent, k, t, sigma);
+  uint64_t h = node_hash_init(sd.salt, t);
+  int cnt = 0, ps[3] = {0xFFFF, 0xFFFF, 0xFFFF};
+  while (cnt < sd.mp) {
+    const int j = G.next();
+    if (j < 0) break;
+    if (cnt < 3) ps[cnt] = j;
+    h = node_hash_step(h, j);
+    cnt++;
+  }
+  key = list_key(t, cnt, ps);
+  hash = h;
+  return true;
+}
 
 // Node scores of `n` items, kItems per round, as a flat task list over the
 // block: task (item, class, parent configuration j).  get(i) -> the item's
-// key (t | np << 14 | p0 << 16 | p1 << 32 | p2 << 48; np = 0 or a key of ~0
-// = nothing to score); emit(i, class-1 score, class-2 score).  Fixed-point
-// terms are summed with atomics: exact, in any order.
+// key (t | np << 14 | p0 << 16 | p1 << 32 | p2 << 48; ~0 = nothing to
+// score); emit(i, key, class-1 score, class-2 score).  Fixed-point terms are
+// summed with atomics: exact, in any order.  Nodes without parents are
+// scored from the state counts.
 template <class Get, class Emit>
 __device__ void bdeu_items(const SetDev &sd, const UnitPtrs &P, int *scan, int n, Get get,
                            Emit emit) {
@@ -555,7 +547,9 @@ __device__ void bdeu_items(const SetDev &sd, const UnitPtrs &P, int *scan, int n
                 p2 = (int)((key >> 48) & 0xFFFF);
       for (int cls = 0; cls < 2; cls++) {
         P.tq[2 * i + cls] = np ? bdeu_tasks(P.cnt3 + 3 * g * cls, np, p0, p1, p2) : 0;
-        P.acc[2 * i + cls] = 0;
+        P.acc[2 * i + cls] = (key != ~0ull && np == 0)
+                                 ? bdeu_score0(sd, (int)(key & 0x3FFF), P.cnt3 + 3 * g * cls)
+                                 : 0;
       }
     }
     __syncthreads();
@@ -603,17 +597,47 @@ __device__ void bdeu_items(const SetDev &sd, const UnitPtrs &P, int *scan, int n
         atomicAdd((unsigned long long *)&P.acc[seg], (unsigned long long)term);
     }
     __syncthreads();
-    for (int i = tid; i < m; i += nt) emit(b0 + i, P.acc[2 * i], P.acc[2 * i + 1]);
+    for (int i = tid; i < m; i += nt) emit(b0 + i, P.itk[i], P.acc[2 * i], P.acc[2 * i + 1]);
     __syncthreads();
   }
 }
 
+// Both classes' scores of one key by one thread.
+__device__ __noinline__ void key_scores(const SetDev &sd, const UnitPtrs &P, unsigned long long key,
+                                        long long *s) {
+  const int t = (int)(key & 0x3FFF), np = (int)((key >> 14) & 3);
+  const int p0 = (int)((key >> 16) & 0xFFFF), p1 = (int)((key >> 32) & 0xFFFF),
+            p2 = (int)((key >> 48) & 0xFFFF);
+  for (int cls = 0; cls < 2; cls++) {
+    const uint16_t *cnt3 = P.cnt3 + 3 * sd.g * cls;
+    if (np == 0) {
+      s[cls] = bdeu_score0(sd, t, cnt3);
+      continue;
+    }
+    const int q = bdeu_tasks(cnt3, np, p0, p1, p2);
+    s[cls] = 0;
+    for (int j = 0; j < q; j++)
+      s[cls] += bdeu_config_term(sd, t, np, p0, p1, p2, cls ? P.mB : P.mA, cnt3, j, P.dmap);
+  }
+}
 
-
+// One block per unit.  A left-out sample changes only rows whose flip
+// entries it triggers, and both a network's hash and its score are sums over
+// rows, so nothing is kept per network but those sums: a lane takes one
+// left-out sample and walks its class's entries (the same for the whole
+// warp), adding the hash, and later the scores, of each row's variant.  The
+// walk reads two state bits per entry and sample, coalesced, where a warp
+// per network that lists its changed nodes waits on chains of its own.
+// Measured against that form: 10000 units of 200 genes x 1000 samples near
+// the threshold 44.0 -> 20.0 ms, 301 units of 387 x 600 35.0 -> 5.3 ms (its
+// table of changed nodes had no room for their ~1500 distinct lists), 90410
+// units that mostly have no entry 9.3 -> 3.0 ms.  Bound by issue and latency
+// in P1 and the node scores now.
 __global__ void __launch_bounds__(256, 3) k_units(const __grid_constant__ BatchDev bd) {
   extern __shared__ __align__(16) char smraw[];
   UnitSmem &SM = *reinterpret_cast<UnitSmem *>(smraw);
   const int nw = blockDim.x >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tid = threadIdx.x, nt = blockDim.x;
   const int u = blockIdx.x;
   // the unit's set: its descriptor into shared memory, its slices of the
   // batch's masks and scratch
@@ -624,39 +648,43 @@ __global__ void __launch_bounds__(256, 3) k_units(const __grid_constant__ BatchD
   {
     const int *src = reinterpret_cast<const int *>(&bs.sd);
     int *dst = reinterpret_cast<int *>(&SM.sd);
-    for (int i = threadIdx.x; i < (int)(sizeof(SetDev) / sizeof(int)); i += blockDim.x) dst[i] = src[i];
+    for (int i = tid; i < (int)(sizeof(SetDev) / sizeof(int)); i += nt) dst[i] = src[i];
   }
+  if (tid == 0) SM.any = 0;
   __syncthreads();
   const SetDev &sd = SM.sd;
-  const int g = sd.g, W = sd.W, GW = sd.GW, S = sd.S, c = sd.c;
-  UnitPtrs P = carve(smraw, g, W, GW, nw);
-  const UnitLayout L = unit_layout(c, S, bd.kmax);
+  const int g = sd.g, W = sd.W, GW = sd.GW, S = sd.S, c = sd.c, nA = sd.nA, nB = sd.nB;
+  const int keep = bd.keep_slot ? bd.keep_slot[u] : -1;
   uint32_t *ucb = bd.dmask + bs_dm0 + (size_t)bs_nb * c + (size_t)ul * chunk_words(c);
-  uint32_t *phi[2] = {(uint32_t *)(scr + L.phi[0]), (uint32_t *)(scr + L.phi[1])};
-  uint16_t *pcol[2] = {(uint16_t *)(scr + L.pcol[0]), (uint16_t *)(scr + L.pcol[1])};
-  unsigned long long *rec = (unsigned long long *)(scr + L.rec);
-  unsigned long long *htk = (unsigned long long *)(scr + L.htk);
-  int *htv = (int *)(scr + L.htv);
-  long long *dist = (long long *)(scr + L.dist);
-  int *uid = (int *)(scr + L.uid);
-  int *urep = (int *)(scr + L.urep);
-  int *sig = (int *)(scr + L.sig);
-  unsigned long long *skey = (unsigned long long *)(scr + L.skey);
-  unsigned long long *sbits = (unsigned long long *)(scr + L.sbits);
-  int *srep = (int *)(scr + L.srep);
-  unsigned long long *hsk = (unsigned long long *)(scr + L.hsk);
-  int *hsv = (int *)(scr + L.hsv);
-  int *wl = (int *)(scr + L.wl);
   uint32_t *dm = bd.dmask + bs_dm0 + (size_t)ul * c;
-  const int tid = threadIdx.x, nt = blockDim.x;
+  // a unit without a nonzero mask has empty networks only: one unique
+  // network, no JS
+  for (int i = tid; i < chunk_words(c); i += nt)
+    if (ucb[i]) SM.any = 1;
+  __syncthreads();
+  if (!SM.any && keep < 0) {
+    if (tid == 0) {
+      bd.U[u] = 1;
+      bd.status[u] = 0u;
+      if (bd.stats) atomicAdd(&bd.stats[4 * (size_t)bd.uslot[u] + 3], (unsigned long long)(S - 1));
+    }
+    return;
+  }
+  const UnitPtrs P = carve(smraw, g, W, GW);
+  const UnitLayout L = unit_layout(c, S);
+  uint32_t *phi[2] = {(uint32_t *)(scr + L.phi[0]), (uint32_t *)(scr + L.phi[1])};
+  long long *dist = (long long *)(scr + L.dist);
+  int *sig = (int *)(scr + L.sig);
 
-  // ---- P0: masks, state counts, selection prefixes, init
+  // ---- P0: init
   if (tid == 0) {
     SM.HF[0] = SM.HF[1] = 0;
-    SM.nphi[0] = SM.nphi[1] = 0;
     SM.ndab = 0;
     SM.status = 0;
-    SM.maxchg = 0;
+    SM.nbig[0] = SM.nbig[1] = 0;
+    SM.firstB0 = S - 1;
+    SM.nchg = SM.nver = SM.nsel = 0;
+    SM.split[0] = SM.split[1] = 0;
     for (int a = 0; a < 2; a++)
       for (int b = 0; b < 2; b++) SM.base[a][b] = 0;
   }
@@ -670,55 +698,13 @@ __global__ void __launch_bounds__(256, 3) k_units(const __grid_constant__ BatchD
   for (int i = tid; i < 4 * g; i += nt) P.phs[i] = (i < 2 * g) ? 0x7fffffff : 0;
   for (int i = tid; i < 82; i += nt) P.dmap[i] = c_dmap[i];
   __syncthreads();
-  // state counts per class from the word-major planes: a warp's loads of a
-  // word are 32 consecutive planes
-  for (int i = tid; i < g * 3; i += nt) {
-    const uint64_t *pl = sd.planesT + i;
-    int a = 0, b = 0;
-    for (int w = 0; w < W; w++) {
-      const uint64_t x = pl[(size_t)w * 3 * g];
-      a += __popcll(x & P.mA[w]);
-      b += __popcll(x & P.mB[w]);
-    }
-    P.cnt3[i] = (uint16_t)a;
-    P.cnt3[3 * g + i] = (uint16_t)b;
-  }
-  if (warp == 0) {
-    for (int cls = 0; cls < 2; cls++) {
-      const uint64_t *m = cls ? P.mB : P.mA;
-      int *pc = cls ? P.pcB : P.pcA;
-      int run = 0;
-      for (int w0 = 0; w0 < W; w0 += 32) {
-        int w = w0 + lane;
-        int v = (w < W) ? __popcll(m[w]) : 0;
-        int x = v;
-        for (int o = 1; o < 32; o <<= 1) {
-          int y = __shfl_up_sync(0xffffffffu, x, o);
-          if (lane >= o) x += y;
-        }
-        if (w < W) pc[w] = run + x - v;
-        run += __shfl_sync(0xffffffffu, x, 31);
-      }
-    }
-  }
-
-  __syncthreads();
-  // sample lists of both classes in index order (network -> left-out
-  // sample): thread per sample bit
-  for (int i = tid; i < 64 * W; i += nt) {
-    const int w = i >> 6, bit = i & 63;
-    const uint64_t below64 = (bit ? (~0ull >> (64 - bit)) : 0ull);
-    const uint64_t a = P.mA[w], b = P.mB[w];
-    if ((a >> bit) & 1ull) sig[P.pcA[w] + __popcll(a & below64)] = i;
-    else if ((b >> bit) & 1ull) sig[sd.nA + P.pcB[w] + __popcll(b & below64)] = i;
-  }
 
   // ---- P1: full-network rows and flip lists, from the 32-pair chunks that
   // hold a nonzero mask (the decision kernel's bitmap; the other chunks are
   // all zero).  Each nonzero mask word read is set back to zero.  Warp w
   // owns the rows whose pairs start in [w c/nw, (w+1) c/nw) and walks its
   // flagged chunks in pair order, four loads at a time.  Edge bits go into
-  // the row bitsets; the flip entries land, in pair
+  // the row bitsets; the flip entries (column, cells << 16) land, in pair
   // order, in the warp's own segment of the list (which starts at its first
   // pair); a row's entry range is the min / max position of its entries
   // (rows without entries keep start > end).
@@ -757,8 +743,7 @@ __global__ void __launch_bounds__(256, 3) k_units(const __grid_constant__ BatchD
         const int wpos = cls ? wpos1 : wpos0;
         const int pos = wpos + __popc(bal & below);
         if (flag) {
-          phi[cls][pos] = ((uint32_t)p << 9) | fb;
-          pcol[cls][pos] = (uint16_t)j;
+          phi[cls][pos] = (uint32_t)j | (cells16(fb) << 16);
           atomicMin(&P.phs[cls * g + t], pos);
           atomicMax(&P.phe[cls * g + t], pos + 1);
         }
@@ -796,9 +781,7 @@ __global__ void __launch_bounds__(256, 3) k_units(const __grid_constant__ BatchD
   }
   __syncthreads();
   // every warp has read the unit's chunk bitmap: zero it for the next batch
-  {
-    for (int i = tid; i < chunk_words(c); i += nt) ucb[i] = 0u;
-  }
+  for (int i = tid; i < chunk_words(c); i += nt) ucb[i] = 0u;
 
   // ---- P1b: only flip entries that can change a capped list are kept.
   // Node t's capped list is its first mp parents.  If R of the row's
@@ -808,6 +791,7 @@ __global__ void __launch_bounds__(256, 3) k_units(const __grid_constant__ BatchD
   // there: entries at later columns change no list and no network, and are
   // dropped (networks that differ only in them are the same network).  A
   // row's entries are contiguous and in column order.
+  int kept = 0;
   for (int i = tid; i < 2 * g; i += nt) {
     const int e0 = P.phs[i], e1 = P.phe[i];
     if (e0 >= e1) continue;
@@ -815,7 +799,7 @@ __global__ void __launch_bounds__(256, 3) k_units(const __grid_constant__ BatchD
     const uint32_t *row = P.rows + (size_t)i * GW;
     int R = 0;
     for (int e = e0; e < e1; e++) {
-      const int j = pcol[k][e];
+      const int j = phi[k][e] & 0xFFFF;
       R += (row[j >> 5] >> (j & 31)) & 1u;
     }
     int need = sd.mp + R, reach = t;  // t: every column of the row
@@ -830,90 +814,103 @@ __global__ void __launch_bounds__(256, 3) k_units(const __grid_constant__ BatchD
       need -= pc;
     }
     int e = e0;
-    while (e < e1 && pcol[k][e] <= reach) e++;
+    while (e < e1 && (int)(phi[k][e] & 0xFFFF) <= reach) e++;
     if (e == e0) {
       P.phs[i] = 0x7fffffff;
       P.phe[i] = 0;
     } else {
       P.phe[i] = e;
     }
+    kept += e - e0;
   }
-  __syncthreads();
-  // ---- P1c: the kept entries, when they fit, compacted into shared memory
-  // (rows in (class, node) order), where every later phase reads them
-  bool compacted = false;
-  {
-    int kept = 0;
-    for (int i0 = 0; i0 < 2 * g; i0 += nt) {
-      const int i = i0 + tid;
-      const int cnt = (i < 2 * g && P.phs[i] < P.phe[i]) ? P.phe[i] - P.phs[i] : 0;
-      int total;
-      block_scan(cnt, total, SM.scan);
-      kept += total;
-    }
-    if (kept <= kEntCache) {
-      int running = 0;
+  const bool entries = __syncthreads_or(kept) != 0;
+
+  // ---- P1c: the kept entries compacted: memo rows' in (class, node)
+  // order, then the other rows', in shared memory when they fit.  moff is
+  // the variants of the rows before (a variant's row is the last one whose
+  // moff is not past it).
+  const uint2 *ent = P.ent;
+  int nmemo = 0, nvar = 0, E = bd.memo_max;
+  auto memo_row = [&](int i, int e) {
+    return e >= 1 && e <= E && (1 << e) <= (i < g ? nA : nB) + 8;
+  };
+  if (entries) {
+    unsigned long long running;
+    // packed: memo entries, other entries << 20, variants << 40
+    while (true) {
+      running = 0ull;
       for (int i0 = 0; i0 < 2 * g; i0 += nt) {
         const int i = i0 + tid;
-        const int e0 = i < 2 * g ? P.phs[i] : 0, e1 = i < 2 * g ? P.phe[i] : 0;
-        const int cnt = e0 < e1 ? e1 - e0 : 0;
-        int total;
-        const int off = running + block_scan(cnt, total, SM.scan);
-        if (cnt) {
-          const int k = i / g;
-          for (int q = 0; q < cnt; q++) {
-            P.ephi[off + q] = phi[k][e0 + q];
-            P.epcol[off + q] = pcol[k][e0 + q];
+        const int e = (i < 2 * g && P.phs[i] < P.phe[i]) ? P.phe[i] - P.phs[i] : 0;
+        const bool mr = memo_row(i, e);
+        const unsigned long long v =
+            mr ? (unsigned long long)e | ((unsigned long long)((1 << e) - 1) << 40)
+               : (unsigned long long)e << 20;
+        unsigned long long total;
+        const unsigned long long off = running + block_scan(v, total, SM.scan64);
+        if (i < 2 * g) {
+          P.moff[i] = (int)(off >> 40);
+          P.nst[i] = mr ? (int)(off & 0xFFFFF) : (int)((off >> 20) & 0xFFFFF);
+          if (i == g) {
+            SM.split[0] = (int)(off & 0xFFFFF);
+            SM.split[1] = (int)(off >> 40);
           }
-          P.phs[i] = off;
-          P.phe[i] = off + cnt;
         }
         running += total;
       }
-      phi[0] = phi[1] = P.ephi;
-      pcol[0] = pcol[1] = P.epcol;
-      compacted = true;
+      nvar = (int)(running >> 40);
+      if (nvar <= unit_variants(g) || E <= 0) break;
+      E--;
       __syncthreads();
     }
-  }
-
-  // rows holding flip entries, ascending, per class, and entry totals
-  if (tid == 0) SM.nent[0] = SM.nent[1] = 0;
-  for (int k = 0; k < 2; k++) {
-    int running = 0;
-    for (int t0 = 0; t0 < g; t0 += nt) {
-      const int t = t0 + tid;
-      const int ne = (t < g) ? P.phe[k * g + t] - P.phs[k * g + t] : 0;
-      int total;
-      const int off = block_scan(ne > 0 ? 1 : 0, total, SM.scan);
-      if (ne > 0) {
-        P.rphi[k * g + running + off] = (uint16_t)t;
-        atomicAdd(&SM.nent[k], ne);
+    nmemo = (int)(running & 0xFFFFF);
+    const int nbig = (int)((running >> 20) & 0xFFFFF);
+    uint2 *dst = nmemo + nbig <= kEntCache ? P.ent : (uint2 *)(scr + L.ent);
+    ent = dst;
+    __syncthreads();
+    for (int i = tid; i < 2 * g; i += nt) {
+      const int e0 = P.phs[i], e1 = P.phe[i];
+      if (e0 >= e1) {
+        P.phs[i] = P.phe[i] = 0;
+        continue;
       }
-      running += total;
+      const int k = i / g, t = i - k * g, e = e1 - e0;
+      const bool mr = memo_row(i, e);
+      const int at = P.nst[i] + (mr ? 0 : nmemo);
+      for (int q = 0; q < e; q++) {
+        const uint32_t x = phi[k][e0 + q];
+        dst[at + q] = make_uint2((x & 0xFFFFu) | ((uint32_t)t << 9) | ((uint32_t)(q & 7) << 18) |
+                                     (q + 1 == e ? 1u << 21 : 0u),
+                                 (x >> 16) | ((uint32_t)(mr ? P.moff[i] : 0) << 16));
+      }
+      P.phs[i] = at;
+      P.phe[i] = at + e;
+      if (!mr) P.big[k * g + atomicAdd(&SM.nbig[k], 1)] = (uint16_t)t;
     }
-    if (tid == 0) SM.nrphi[k] = running;
+  } else {
+    for (int i = tid; i < 2 * g; i += nt) P.phs[i] = P.phe[i] = 0;
   }
+  for (int i = tid; i < (nvar + 31) / 32; i += nt) P.used[i] = 0u;
   __syncthreads();
 
   // ---- P2: capped lists of the two full networks; their hashes summed per
   // warp, then one atomic per warp and class
   unsigned long long hsum[2] = {0ull, 0ull};
   for (int i = tid; i < 2 * g; i += nt) {
-    const int k = i / g, t = i % g;
-    ListGen G;
-    gen_for(G, sd, P, phi[k], pcol[k], k, t, nullptr);
+    const int k = i >= g ? 1 : 0, t = i - k * g;
+    const uint32_t *row = P.rows + (size_t)i * GW;
     uint64_t h = node_hash_init(sd.salt, t);
-    int cnt = 0;
+    int cnt = 0, last = -1;
     int ps[3] = {0xFFFF, 0xFFFF, 0xFFFF};
-    while (cnt < sd.mp) {
-      int j = G.next();
-      if (j < 0) break;
-      if (cnt < 3) ps[cnt] = j;
-      h = node_hash_step(h, j);
-      cnt++;
-    }
+    for (int w = 0; w < GW && cnt < sd.mp; w++)
+      for (uint32_t x = row[w]; x && cnt < sd.mp; x &= x - 1) {
+        last = 32 * w + __ffs(x) - 1;
+        if (cnt < 3) ps[cnt] = last;
+        h = node_hash_step(h, last);
+        cnt++;
+      }
     P.fcnt[i] = (uint16_t)cnt;
+    P.fend[i] = (int16_t)(cnt < sd.mp ? 0x7FFF : last);
     for (int q = 0; q < 3; q++) P.fps[i * 3 + q] = (uint16_t)ps[q];
     P.fh[i] = h;
     hsum[k] += h;
@@ -927,683 +924,359 @@ __global__ void __launch_bounds__(256, 3) k_units(const __grid_constant__ BatchD
     atomicAdd(&SM.HF[1], hsum[1]);
   }
   __syncthreads();
-  for (int t = tid; t < g; t += nt) {
-    if (!lists_equal(sd, P, phi, pcol, t, 0, nullptr, 1, nullptr)) {
-      int idx = atomicAdd(&SM.ndab, 1);
-      P.dab[idx] = (uint16_t)t;
+  // nodes whose capped lists differ between the full networks
+  {
+    int nd = 0;
+    for (int t = tid; t < g; t += nt) {
+      const uint32_t *ra = P.rows + (size_t)t * GW, *rb = P.rows + (size_t)(g + t) * GW;
+      bool same = P.fcnt[t] == P.fcnt[g + t];
+      int left = P.fcnt[t];
+      for (int w = 0; same && w < GW && left > 0; w++) {
+        // the words agree up to the column of the last one in the list
+        const uint32_t x = ra[w] ^ rb[w];
+        uint32_t m = ra[w];
+        const int pc = __popc(m);
+        if (pc >= left) {
+          for (int q = 1; q < left; q++) m &= m - 1;
+          same = (x & ((m & -m) | ((m & -m) - 1u))) == 0u;
+          left = 0;
+        } else {
+          same = x == 0u;
+          left -= pc;
+        }
+      }
+      P.need[t] = same ? 0 : 1;
+      nd += same ? 0 : 1;
     }
+    if (nd) atomicAdd(&SM.ndab, nd);
   }
-  __syncthreads();
 
-  // ---- P3: networks grouped by signature.  The network of left-out sample
-  // sigma is its class's full network with the pair tables of sigma's cells
-  // removed, i.e. the full rows XOR the flip entries that sigma triggers (entry
-  // (t, j, fb) fires when fb holds the bit of sigma's states at t and j).
-  // Samples that trigger the same entries have equal networks, so lists are
-  // generated once per distinct signature.  Signature = additive hash of the
-  // triggered entry ordinals (salted per class; never 0 when non-empty), with
-  // the exact bitset alongside when the class has <= 64 entries.
-  const unsigned long long ksalt0 = mix64(sd.salt ^ 0x243F6A8885A308D3ull);
-  const unsigned long long ksalt1 = mix64(sd.salt ^ 0x13198A2E03707344ull);
-  const int n = sd.n;
-  const int HTs = L.HT;
-  auto class_of = [&](int s) -> int { return (s == 0) ? 0 : (s == S - 1) ? 1 : (s <= sd.nA ? 0 : 1); };
-  // triggered entries of sample sigma in class k: hash (0 when none) and bits
-  auto signature = [&](int k, int sigma, unsigned long long &bits) -> unsigned long long {
-    const int nrk = SM.nrphi[k];
-    const bool exact = SM.nent[k] <= 64;
-    const unsigned long long ks = k ? ksalt1 : ksalt0;
-    const uint32_t *ph = phi[k];
-    const uint16_t *pc = pcol[k];
-    unsigned long long key = 0;
-    bits = 0;
-    int ord = 0, any = 0;
-    for (int r = 0; r < nrk; r++) {
-      const int t = P.rphi[k * g + r];
-      const int e0 = P.phs[k * g + t], e1 = P.phe[k * g + t];
-      const int a = st_of(sd.vals[(size_t)t * n + sigma]);
-      if (a <= 2) {
-        for (int e = e0; e < e1; e++) {
-          const int b = st_of(sd.vals[(size_t)pc[e] * n + sigma]);
-          if (b <= 2 && ((ph[e] >> (3 * a + b)) & 1u)) {
-            const int o = ord + (e - e0);
-            key += mix64(ks + (unsigned long long)o);
-            if (exact) bits |= 1ull << o;
-            any = 1;
-          }
+  // ---- the variants of the memo rows: key (node, first three parents)
+  // and hash of each list that differs from the full one
+  unsigned long long *ment = (unsigned long long *)(scr + L.ment);
+  unsigned long long *mdh = nvar <= kSmVar ? P.itk : (unsigned long long *)(scr + L.mdh);
+  for (int v = tid; v < nvar; v += nt) {
+    int lo = 0, hi = 2 * g - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (P.moff[mid] <= v) lo = mid;
+      else hi = mid - 1;
+    }
+    const int i = lo, k = i >= g ? 1 : 0, t = i - k * g;
+    const int sub = v - P.moff[i] + 1;
+    const int e0 = P.phs[i], e1 = P.phe[i];
+    unsigned long long key = ~0ull, dh = 0ull;
+    if ((int)(ent[e0 + __ffs(sub) - 1].x & 511u) <= P.fend[i]) {
+      const uint32_t *row = P.rows + (size_t)i * GW;
+      uint64_t h = node_hash_init(sd.salt, t);
+      int cnt = 0, ps[3] = {0xFFFF, 0xFFFF, 0xFFFF};
+      int e = e0, col = ent[e0].x & 511;
+      for (int w = 0; w < GW && cnt < sd.mp; w++) {
+        uint32_t x = row[w];
+        while (e < e1 && (col >> 5) == w) {
+          if ((sub >> (e - e0)) & 1) x ^= 1u << (col & 31);
+          if (++e < e1) col = ent[e].x & 511;
+        }
+        for (; x && cnt < sd.mp; x &= x - 1) {
+          const int j = 32 * w + __ffs(x) - 1;
+          if (cnt < 3) ps[cnt] = j;
+          h = node_hash_step(h, j);
+          cnt++;
         }
       }
-      ord += e1 - e0;
+      key = list_key(t, cnt, ps);
+      dh = h - P.fh[i];
+      // two lists of a node with one hash: another salt
+      if (dh == 0ull) atomicOr(&SM.status, kUnitHashCollision);
     }
-    return any ? (key | 1ull) : 0ull;
-  };
-  // The same from the trigger bitsets: entry o of class k fires for sample
-  // sigma when bit sigma of trig[(koff + o) W ..] is set.  Until the BDeu
-  // phase, the task prefix (tq) holds the entries by ordinal and the base
-  // score array (fsc) the bitsets.
-  uint32_t *ent = (uint32_t *)P.tq;
-  uint64_t *trig = (uint64_t *)P.fsc;
-  auto signature_t = [&](int k, int sigma, unsigned long long &bits) -> unsigned long long {
-    const int ne = SM.nent[k];
-    const bool exact = ne <= 64;
-    const unsigned long long ks = k ? ksalt1 : ksalt0;
-    const uint64_t *T = trig + (size_t)(k ? SM.nent[0] : 0) * W + (sigma >> 6);
-    const int sh = sigma & 63;
-    unsigned long long key = 0;
-    bits = 0;
-    int any = 0;
-    for (int o = 0; o < ne; o++) {
-      if ((T[(size_t)o * W] >> sh) & 1ull) {
-        key += mix64(ks + (unsigned long long)o);
-        if (exact) bits |= 1ull << o;
-        any = 1;
-      }
-    }
-    return any ? (key | 1ull) : 0ull;
-  };
-  // Trigger bitsets, when they fit: entries by ordinal (rows in order, then
-  // entries in position order, as signature() counts them), then per entry
-  // and sample word the OR over the set bits (a, b) of fb of
-  // plane(t, a) & plane(j, b), read 64 samples at a time.
-  const int ne0 = SM.nent[0], ne1 = SM.nent[1];
-  const bool tbits = ne0 + ne1 <= 2 * kItems + 1 && (ne0 + ne1) * W <= 4 * g;
-  if (tbits) {
-    for (int k = 0; k < 2; k++) {
-      const int nrk = SM.nrphi[k];
-      int running = k ? ne0 : 0;
-      for (int r0 = 0; r0 < nrk; r0 += nt) {
-        const int r = r0 + tid;
-        int t = 0, e0 = 0, cnt = 0;
-        if (r < nrk) {
-          t = P.rphi[k * g + r];
-          e0 = P.phs[k * g + t];
-          cnt = P.phe[k * g + t] - e0;
+    ment[v] = key;
+    mdh[v] = dh;
+  }
+  // sample lists of both classes in index order (network -> left-out
+  // sample)
+  if (warp == 0) {
+    for (int cls = 0; cls < 2; cls++) {
+      const uint64_t *m = cls ? P.mB : P.mA;
+      int *pc = cls ? P.pcB : P.pcA;
+      int run = 0;
+      for (int w0 = 0; w0 < W; w0 += 32) {
+        int w = w0 + lane;
+        int v = (w < W) ? __popcll(m[w]) : 0;
+        int x = v;
+        for (int o = 1; o < 32; o <<= 1) {
+          int y = __shfl_up_sync(0xffffffffu, x, o);
+          if (lane >= o) x += y;
         }
-        int total;
-        const int off = block_scan(cnt, total, SM.scan);
-        for (int i = 0; i < cnt; i++)
-          ent[running + off + i] = (uint32_t)t | ((uint32_t)pcol[k][e0 + i] << 9) |
-                                     ((phi[k][e0 + i] & 0x1FFu) << 18);
-        running += total;
+        if (w < W) pc[w] = run + x - v;
+        run += __shfl_sync(0xffffffffu, x, 31);
       }
     }
-    __syncthreads();
-    for (int idx = tid; idx < (ne0 + ne1) * W; idx += nt) {
-      const int o = idx / W, w = idx - o * W;
-      const uint32_t en = ent[o];
-      const uint32_t fb = en >> 18;
-      const uint64_t *pt = sd.planes + (size_t)(en & 0x1FFu) * 3 * W + w;
-      const uint64_t *pj = sd.planes + (size_t)((en >> 9) & 0x1FFu) * 3 * W + w;
-      const uint64_t t0 = pt[0], t1 = pt[W], t2 = pt[2 * W];
-      const uint64_t j0 = pj[0], j1 = pj[W], j2 = pj[2 * W];
-      uint64_t x = 0;
-      if (fb & 0x001u) x |= t0 & j0;
-      if (fb & 0x002u) x |= t0 & j1;
-      if (fb & 0x004u) x |= t0 & j2;
-      if (fb & 0x008u) x |= t1 & j0;
-      if (fb & 0x010u) x |= t1 & j1;
-      if (fb & 0x020u) x |= t1 & j2;
-      if (fb & 0x040u) x |= t2 & j0;
-      if (fb & 0x080u) x |= t2 & j1;
-      if (fb & 0x100u) x |= t2 & j2;
-      trig[idx] = x;
-    }
   }
-  // Tables (key -> smallest network index) in shared memory first; a unit
-  // whose keys do not fit there within kSmProbes probes uses its global
-  // table of HT slots instead (initialised only then).
-  unsigned long long *smk = P.itk;
-  int *smv = (int *)P.acc;
-  auto table_init = [&](unsigned long long *k, int *v, int slots, unsigned long long empty) {
-    for (int i = tid; i < slots; i += nt) {
-      k[i] = empty;
-      v[i] = 0x7fffffff;
-    }
-  };
-  const MinTable sig_sm{smk, smv, kSmSlots - 1, 0ull, kSmProbes};
-  const MinTable sig_gl{hsk, hsv, (unsigned)HTs - 1, 0ull, (unsigned)HTs};
-  table_init(smk, smv, kSmSlots, 0ull);
-  if (tid == 0) {
-    skey[0] = skey[S - 1] = 0ull;
-    sbits[0] = sbits[S - 1] = 0ull;
-    srep[0] = 0;
-    srep[S - 1] = S - 1;
-    SM.tfull = 0;
-    SM.firstE2 = S - 1;
-  }
+  const int nbigs = SM.nbig[0] + SM.nbig[1];
+  const int KB = big_slots(g);
+  unsigned long long *bkey = (unsigned long long *)(scr + L.bkey);
+  if (nbigs)
+    for (int i = tid; i < KB; i += nt) bkey[i] = ~0ull;
   __syncthreads();
-  for (int s = 1 + tid; s < S - 1; s += nt) {
-    unsigned long long bits;
-    const unsigned long long key = tbits ? signature_t(class_of(s), sig[s - 1], bits)
-                                         : signature(class_of(s), sig[s - 1], bits);
-    skey[s] = key;
-    sbits[s] = bits;
-    if (key && !sig_sm.insert_min(key, s)) SM.tfull = 1;
-    if (!key && s > sd.nA) atomicMin(&SM.firstE2, s);
-  }
-  if (tid == 0) SM.nwl = 0;
-  __syncthreads();
-  const bool sig_global = SM.tfull != 0;
-  if (sig_global) {
-    table_init(hsk, hsv, HTs, 0ull);
-    __syncthreads();
-    for (int s = 1 + tid; s < S - 1; s += nt)
-      if (skey[s]) sig_gl.insert_min(skey[s], s);
+  const bool networks = entries || keep >= 0;
+  if (networks) {
+    for (int i = tid; i < 64 * W; i += nt) {
+      const int w = i >> 6, bit = i & 63;
+      const uint64_t below64 = (bit ? (~0ull >> (64 - bit)) : 0ull);
+      const uint64_t a = P.mA[w], b = P.mB[w];
+      if ((a >> bit) & 1ull) sig[P.pcA[w] + __popcll(a & below64)] = i;
+      else if ((b >> bit) & 1ull) sig[nA + P.pcB[w] + __popcll(b & below64)] = i;
+    }
     __syncthreads();
   }
-  const MinTable &sig_tab = sig_global ? sig_gl : sig_sm;
-  // representatives, the work list of distinct signatures, and an exact check
-  // that every network shares its representative's triggered entries
-  for (int s = 1 + tid; s < S - 1; s += nt) {
-    const unsigned long long key = skey[s];
-    int rep = s;
-    if (key) {
-      rep = sig_tab.get(key);
-      if (rep == s) {
-        wl[atomicAdd(&SM.nwl, 1)] = s;
-      } else {
-        const int k = class_of(s);
-        bool ok = (class_of(rep) == k);
-        if (ok && SM.nent[k] <= 64) {
-          ok = (sbits[s] == sbits[rep]);
-        } else if (ok) {
-          // more than 64 entries: compare the triggered sets entry by entry
-          const int sa = sig[s - 1], sb = sig[rep - 1];
-          const int nrk = SM.nrphi[k];
-          for (int r = 0; ok && r < nrk; r++) {
-            const int t = P.rphi[k * g + r];
-            const int aa = st_of(sd.vals[(size_t)t * n + sa]), ab = st_of(sd.vals[(size_t)t * n + sb]);
-            for (int e = P.phs[k * g + t]; ok && e < P.phe[k * g + t]; e++) {
-              const int j = pcol[k][e];
-              const int ba = st_of(sd.vals[(size_t)j * n + sa]), bb = st_of(sd.vals[(size_t)j * n + sb]);
-              const bool fa = aa <= 2 && ba <= 2 && ((phi[k][e] >> (3 * aa + ba)) & 1u);
-              const bool fbb = ab <= 2 && bb <= 2 && ((phi[k][e] >> (3 * ab + bb)) & 1u);
-              ok = (fa == fbb);
-            }
-          }
-        }
-        if (!ok) atomicOr(&SM.status, kUnitHashCollision);
-      }
-    }
-    srep[s] = rep;
-  }
-  if (tid == 0) {
-    unsigned long long *R0 = rec;
-    unsigned long long *R1 = rec + (size_t)(S - 1) * L.rec_words;
-    R0[0] = SM.HF[0];
-    R0[1] = 0;
-    R1[0] = SM.HF[1];
-    R1[1] = 0;
-  }
-  __syncthreads();
-  // the capped list of each row with 1..kMemoE kept entries under every
-  // non-empty subset of them (the entries a left-out sample triggers):
-  // the record entry (t, first three parents) when it differs from the
-  // full network's list, and its hash; one thread per (row, subset).
-  // Packed by row: row i's 2^e - 1 lists from moff[i] on (the task prefix
-  // array is free from the signatures until the BDeu phase), so the lists
-  // the records read lie close together.
-  unsigned long long *memo = (unsigned long long *)(scr + L.memo);
-  int *moff = P.tq;
-  uint32_t *used = (uint32_t *)P.fsc;
+
   // a changed node's key (node, first three parents) unless it equals the
   // full network's: the items scored in the BDeu phase
   auto differs = [&](int k, unsigned long long e) -> bool {
     const int t = (int)(e & 0x3FFF), np = (int)((e >> 14) & 3);
-    const int fnp = P.fcnt[k * g + t] < 3 ? P.fcnt[k * g + t] : 3;
+    const int i = k * g + t, fnp = P.fcnt[i] < 3 ? P.fcnt[i] : 3;
     if (np != fnp) return true;
     for (int q = 0; q < np; q++)
-      if ((int)((e >> (16 + 16 * q)) & 0xFFFF) != (int)P.fps[(k * g + t) * 3 + q]) return true;
+      if ((int)((e >> (16 + 16 * q)) & 0xFFFF) != (int)P.fps[i * 3 + q]) return true;
     return false;
   };
-  {
-    int running = 0;
-    for (int i0 = 0; i0 < 2 * g; i0 += nt) {
-      const int i = i0 + tid;
-      int sz = 0;
-      if (i < 2 * g) {
-        const int e = P.phe[i] - P.phs[i];
-        sz = (e >= 1 && e <= kMemoE) ? (1 << e) - 1 : 0;
-      }
-      int total;
-      const int off = block_scan(sz, total, SM.scan);
-      if (i < 2 * g) moff[i] = running + off;
-      running += total;
+  // slot of a key in the table of lists formed per sample (-1: no room)
+  constexpr int kProbes = 32;
+  auto big_slot = [&](unsigned long long key, bool insert) -> int {
+    unsigned slot = (unsigned)(mix64(key) & (KB - 1));
+    for (int pr = 0; pr < kProbes; pr++, slot = (slot + 1u) & (KB - 1)) {
+      // a slot only ever goes from empty to its final key
+      unsigned long long cur = insert ? *(volatile unsigned long long *)&bkey[slot] : bkey[slot];
+      if (insert && cur == ~0ull) cur = atomicCAS(&bkey[slot], ~0ull, key);
+      if (cur == key || (insert && cur == ~0ull)) return (int)slot;
+      if (cur == ~0ull) return -1;
     }
-    // the lists the records use, one bit each (the base score array is
-    // free until the BDeu phase: 32 g bytes >= 2 g kMemoSub bits)
-    for (int w = tid; w < (running + 31) / 32; w += nt) used[w] = 0u;
-    if (tid == 0) SM.nlg = 0;
-    __syncthreads();
-  }
-  for (int task = tid; task < 2 * g * kMemoSub; task += nt) {
-    const int i = task / kMemoSub, msub = task - i * kMemoSub + 1;
-    const int e0 = P.phs[i], e1 = P.phe[i];
-    if (e0 >= e1 || e1 - e0 > kMemoE || msub >= (1 << (e1 - e0))) continue;
-    const int k = i / g, t = i - k * g;
-    const uint32_t *row = P.rows + (size_t)i * GW;
-    ListGen Go;
-    gen_for(Go, sd, P, phi[k], pcol[k], k, t, nullptr);
-    uint64_t h = node_hash_init(sd.salt, t);
-    int cnt = 0, ps[3] = {0xFFFF, 0xFFFF, 0xFFFF};
-    bool diff = false;
-    for (int w = 0; w < GW && cnt < sd.mp; w++) {
-      uint32_t x = row[w];
-      for (int q = 0; q < e1 - e0; q++) {
-        const int j = pcol[k][e0 + q];
-        if (((msub >> q) & 1) && (j >> 5) == w) x ^= 1u << (j & 31);
-      }
-      while (x && cnt < sd.mp) {
-        const int j = 32 * w + __ffs(x) - 1;
-        x &= x - 1;
-        if (Go.next() != j) diff = true;
-        if (cnt < 3) ps[cnt] = j;
-        h = node_hash_step(h, j);
-        cnt++;
-      }
-    }
-    // a shorter list than the full network's differs too
-    if (cnt < sd.mp && Go.next() >= 0) diff = true;
-    unsigned long long *M = memo + ((size_t)moff[i] + (msub - 1)) * 2;
-    M[0] = diff ? ((unsigned long long)t | ((unsigned long long)(cnt < 3 ? cnt : 3) << 14) |
-                   ((unsigned long long)(ps[0] & 0xFFFF) << 16) |
-                   ((unsigned long long)(ps[1] & 0xFFFF) << 32) |
-                   ((unsigned long long)(ps[2] & 0xFFFF) << 48))
-                : ~0ull;
-    M[1] = h;
-  }
-  __syncthreads();
-
-  // one record per distinct signature: changed nodes (capped list differs
-  // from the full network's) with their lists, and the network hash.  A
-  // warp per network.  A first pass over the rows holding entries finds
-  // the rows whose entries the left-out sample triggers (shared memory
-  // only) and lists them (row | subset << 16, or a merged-row mark) in the
-  // warp's part of the BDeu item arrays, idle from the signatures until the
-  // dedup; a second pass looks up (or merges) the listed rows' lists 32 at
-  // a time, so a network's memo loads are in flight together.
-  constexpr int kMergedRow = 0x8000;  // a row with more than kMemoE entries
-  int8_t *myst = P.stsig + (size_t)warp * st_stride(g);
-  uint32_t *lsts = reinterpret_cast<uint32_t *>(P.itk);  // P.acc follows P.itk
-  const int lcap = (int)((reinterpret_cast<uint32_t *>(P.acc + 2 * kItems) - lsts) / nw) & ~31;
-  uint32_t *lst = lsts + (size_t)warp * lcap;
-  const int nwl = SM.nwl;
-  for (int wi = warp; wi < nwl; wi += nw) {
-    const int s = wl[wi];
-    const int k = class_of(s);
-    const int sigma = sig[s - 1];
-    unsigned long long *R = rec + (size_t)s * L.rec_words;
-    const int nrk = SM.nrphi[k];
-    load_stsig(sd, sigma, myst, lane);
-    unsigned long long dh = 0;
-    int nchg = 0, nl = 0;
-    auto flush = [&]() {
-      __syncwarp();
-      for (int l0 = 0; l0 < nl; l0 += 32) {
-        const int l = l0 + lane;
-        bool changed = false;
-        unsigned long long hn = 0, ent = 0;
-        int t = 0;
-        if (l < nl) {
-          const uint32_t le = lst[l];
-          t = (int)(le & 0xFFFFu);
-          const int sub = (int)(le >> 16);
-          if (sub != kMergedRow) {
-            const int mi = moff[k * g + t] + sub - 1;
-            const unsigned long long *M = memo + (size_t)mi * 2;
-            if (M[0] != ~0ull) {
-              changed = true;
-              ent = M[0];
-              hn = M[1];
-              if (!((used[mi >> 5] >> (mi & 31)) & 1u)) atomicOr(&used[mi >> 5], 1u << (mi & 31));
-            }
-          } else {
-            ListGen Gn, Go;
-            gen_for(Gn, sd, P, phi[k], pcol[k], k, t, myst);
-            gen_for(Go, sd, P, phi[k], pcol[k], k, t, nullptr);
-            uint64_t h = node_hash_init(sd.salt, t);
-            int cnt = 0, ps[3] = {0xFFFF, 0xFFFF, 0xFFFF};
-            bool diff = false;
-            for (int i = 0; i < sd.mp; i++) {
-              int x = Gn.next(), y = Go.next();
-              if (x != y) diff = true;
-              if (x < 0) break;
-              if (cnt < 3) ps[cnt] = x;
-              h = node_hash_step(h, x);
-              cnt++;
-            }
-            if (diff) {
-              changed = true;
-              hn = h;
-              ent = (unsigned long long)t | ((unsigned long long)(cnt < 3 ? cnt : 3) << 14) |
-                    ((unsigned long long)(ps[0] & 0xFFFF) << 16) |
-                    ((unsigned long long)(ps[1] & 0xFFFF) << 32) |
-                    ((unsigned long long)(ps[2] & 0xFFFF) << 48);
-              if (differs(k, ent)) {
-                // logged in the signature table's keys (free from here on)
-                const int ix = atomicAdd(&SM.nlg, 1);
-                if (ix < HTs) hsk[ix] = ent;
-              }
-            }
-          }
-        }
-        const unsigned bal = __ballot_sync(0xffffffffu, changed);
-        if (changed) {
-          const int pos = nchg + __popc(bal & ((1u << lane) - 1u));
-          dh += hn - P.fh[k * g + t];
-          if (pos < bd.kmax) R[2 + pos] = ent;
-        }
-        nchg += __popc(bal);
-      }
-      nl = 0;
-      __syncwarp();
-    };
-    for (int t0 = 0; t0 < nrk; t0 += 32) {
-      const int t = (t0 + lane < nrk) ? (int)P.rphi[k * g + t0 + lane] : -1;
-      int sub = 0;
-      if (t >= 0 && myst[t] <= 2) {
-        // the entries of row t that sample sigma triggers
-        const int sr = myst[t] * 3;
-        const int e0 = P.phs[k * g + t], e1 = P.phe[k * g + t];
-        if (e1 - e0 <= kMemoE) {
-          for (int q = 0; q < e1 - e0; q++) {
-            const int sc = myst[pcol[k][e0 + q]];
-            if (sc <= 2 && (((phi[k][e0 + q] & 0x1FFu) >> (sr + sc)) & 1u)) sub |= 1 << q;
-          }
-        } else {
-          bool flips = false;
-          for (int i = e0; i < e1 && !flips; i++) {
-            const int sc = myst[pcol[k][i]];
-            flips = sc <= 2 && (((phi[k][i] & 0x1FFu) >> (sr + sc)) & 1u);
-          }
-          if (flips) sub = kMergedRow;
-        }
-      }
-      const unsigned bal = __ballot_sync(0xffffffffu, sub != 0);
-      if (sub) lst[nl + __popc(bal & ((1u << lane) - 1u))] = (uint32_t)t | ((uint32_t)sub << 16);
-      nl += __popc(bal);
-      if (nl > lcap - 32) flush();
-    }
-    flush();
-    for (int o = 16; o > 0; o >>= 1) dh += __shfl_down_sync(0xffffffffu, dh, o);
-    if (lane == 0) {
-      R[0] = SM.HF[k] + dh;
-      R[1] = (unsigned long long)nchg;
-      if (nchg > bd.kmax) {
-        atomicOr(&SM.status, kUnitKmaxOverflow);
-        atomicMax(&SM.maxchg, nchg);
-      }
-    }
-  }
-  __syncthreads();
-  if (SM.status & kUnitKmaxOverflow) {
-    if (tid == 0) {
-      // bits 16-31: the records the unit needs (the host re-runs it with
-      // room for them)
-      bd.status[u] = SM.status | ((unsigned)min(SM.maxchg, 0xFFFF) << 16);
-      bd.js[u] = __longlong_as_double(0x7ff8000000000000ll);
-      bd.U[u] = -1;
-    }
-    return;
-  }
-  // record of any network: the full network's for an empty signature, else
-  // its signature representative's
-  auto rec_of = [&](int s) -> const unsigned long long * {
-    const int r = (s == 0 || s == S - 1) ? s : (skey[s] == 0 ? (class_of(s) ? S - 1 : 0) : srep[s]);
-    return rec + (size_t)r * L.rec_words;
+    return -1;
   };
+  // fn(variant) for every memo row whose entries sample sg triggers, in
+  // class k: a flat walk over the class's entries, four at a time
+  auto walk = [&](int k, int sg, auto &&fn) {
+    const uint32_t *cw = sd.codes + (sg >> 4);
+    const int sh = 2 * (sg & 15), n16 = sd.n16;
+    const int e0 = k ? SM.split[0] : 0, e1 = k ? nmemo : SM.split[0];
+    int sub = 0;
+    for (int e = e0; e < e1; e += 4) {
+      uint2 en[4];
+      uint32_t a[4], b[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) en[q] = ent[e + q < e1 ? e + q : e1 - 1];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        a[q] = __ldg(cw + ((en[q].x >> 9) & 511u) * n16);
+        b[q] = __ldg(cw + (en[q].x & 511u) * n16);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        if (e + q >= e1) break;
+        const uint32_t cell = ((a[q] >> sh) & 3u) * 4u + ((b[q] >> sh) & 3u);
+        sub |= (int)(((en[q].y >> cell) & 1u) << ((en[q].x >> 18) & 7u));
+        if (en[q].x >> 21) {
+          if (sub) fn((int)(en[q].y >> 16) + sub - 1);
+          sub = 0;
+        }
+      }
+    }
+  };
+  const int nch0 = (nA + 31) >> 5, nch = nch0 + ((nB + 31) >> 5);
 
-  // ---- P4: first-occurrence dedup.  Networks without changed nodes are
-  // their class's full network: class-1 ones duplicate network 0, class-2
-  // ones the first class-2 network without changes (firstB0).  Every other
-  // network shares its signature representative's network, and that
-  // representative comes first.  So the unique networks are the candidates
-  // -- network 0, firstB0 and the signature representatives with changes --
-  // that are the first occurrence of their network hash; only they go into
-  // the table, and only they are looked up.
-  const int HT = L.HT;
-  const int nrep = SM.nwl;  // signature representatives in wl
-  // firstB0: the first class-2 network with an empty signature, or a class-2
-  // representative (its group's first network) whose record has no changes
-  if (tid == 0) {
-    SM.firstB0 = SM.firstE2;
-    SM.ncand = 2;
-  }
-  __syncthreads();
-  for (int i = tid; i < nrep; i += nt) {
-    const int s = wl[i];
-    if (s > sd.nA && rec[(size_t)s * L.rec_words + 1] == 0) atomicMin(&SM.firstB0, s);
+  // ---- P3: every network's hash: its class's full network's, plus the
+  // hash difference of each row the left-out sample changes.  A lane per
+  // sample, a warp per 32 samples of one class.
+  unsigned long long *hs = (unsigned long long *)(scr + L.hs);
+  auto as_key = [](unsigned long long h) { return h == ~0ull ? ~1ull : h; };
+  if (entries) {
+    for (int ch = warp; ch < nch; ch += nw) {
+      const int k = ch >= nch0 ? 1 : 0, i = 32 * (k ? ch - nch0 : ch) + lane;
+      const int nk = k ? nB : nA;
+      const bool live = i < nk;
+      const int s = 1 + (k ? nA : 0) + (live ? i : nk - 1);
+      const int sg = sig[s - 1];
+      unsigned long long dh = 0ull;
+      bool chg = false;
+      walk(k, sg, [&](int v) {
+        const unsigned long long d = mdh[v];
+        if (d) {
+          dh += d;
+          chg = true;
+          if (!((P.used[v >> 5] >> (v & 31)) & 1u)) atomicOr(&P.used[v >> 5], 1u << (v & 31));
+        }
+      });
+      for (int r = 0; r < SM.nbig[k]; r++) {
+        const int t = P.big[k * g + r];
+        unsigned long long key, h;
+        if (!sample_list(sd, P, ent, k, t, sg, key, h)) continue;
+        const unsigned long long d = h - P.fh[k * g + t];
+        if (d == 0ull) atomicOr(&SM.status, kUnitHashCollision);
+        dh += d;
+        chg = true;
+        if (differs(k, key)) big_slot(key, true);
+      }
+      if (live) hs[s] = chg ? as_key(SM.HF[k] + dh) : ~0ull;
+      const unsigned nc = __ballot_sync(0xffffffffu, live && chg);
+      const int first0 = __reduce_min_sync(0xffffffffu, (k && live && !chg) ? s : S - 1);
+      if (lane == 0) {
+        if (nc) atomicAdd(&SM.nchg, __popc(nc));
+        if (first0 < S - 1) atomicMin(&SM.firstB0, first0);
+      }
+    }
+  } else if (tid == 0) {
+    SM.firstB0 = nA + 1;  // the first class-2 network
   }
   __syncthreads();
   const int firstB0 = SM.firstB0;
-  // candidates (in the per-network id array, no longer needed per network)
-  int *cand = uid;
-  if (tid == 0) {
-    cand[0] = 0;
-    cand[1] = firstB0;
-  }
-  for (int i = tid; i < nrep; i += nt) {
-    const int s = wl[i];
-    if (rec[(size_t)s * L.rec_words + 1] != 0) cand[atomicAdd(&SM.ncand, 1)] = s;
-  }
-  // network table: shared memory first (the signature table is done with),
-  // the global one when the candidates do not fit
-  const MinTable net_sm{smk, smv, kSmSlots - 1, ~0ull, kSmProbes};
-  const MinTable net_gl{htk, htv, (unsigned)HT - 1, ~0ull, (unsigned)HT};
-  auto net_key = [&](int s) -> unsigned long long {
-    unsigned long long key = rec_of(s)[0];
-    return key == ~0ull ? key ^ 1ull : key;
-  };
-  table_init(smk, smv, kSmSlots, ~0ull);
-  if (tid == 0) SM.tfull = 0;
-  __syncthreads();
-  const int m = SM.ncand;
-  for (int i = tid; i < m; i += nt)
-    if (!net_sm.insert_min(net_key(cand[i]), cand[i])) SM.tfull = 1;
-  // bitmap of the unique networks over the network ids, and the merged
-  // candidates with their representatives (both in the signature-bitset
-  // scratch, free after the signature phase)
-  uint32_t *ubits = (uint32_t *)sbits;
-  const int nbw = (S + 31) >> 5;
-  int *vrep = (int *)sbits + nbw;
-  for (int i = tid; i < nbw; i += nt) ubits[i] = 0u;
-  if (tid == 0) SM.nwl = 0;
-  __syncthreads();
-  const bool net_global = SM.tfull != 0;
-  if (net_global) {
-    table_init(htk, htv, HT, ~0ull);
+
+  // ---- P4: first-occurrence dedup.  Networks without changed nodes are
+  // their class's full network: class-1 ones duplicate network 0, class-2
+  // ones the first of them (firstB0).  So the unique networks are the
+  // candidates -- network 0, firstB0 and the changed networks -- that are
+  // the first occurrence of their hash: a table of network ids, compared by
+  // hash, keeps the smallest id of each.
+  int *urep = (int *)(scr + L.urep);
+  int *wl = (int *)(scr + L.wl), *vrep = (int *)(scr + L.vrep);
+  int U;
+  if (SM.nchg == 0) {
+    U = SM.ndab ? 2 : 1;
+    if (tid == 0) {
+      urep[0] = 0;
+      if (U == 2) urep[1] = firstB0;
+    }
     __syncthreads();
-    for (int i = tid; i < m; i += nt) net_gl.insert_min(net_key(cand[i]), cand[i]);
+  } else {
+    int slots = 64;
+    while (slots < 2 * (SM.nchg + 2)) slots <<= 1;
+    int *tab = slots <= kSmSlots ? (int *)P.itk : (int *)(scr + L.htab);
+    const unsigned tmask = (unsigned)slots - 1u;
+    uint32_t *ubits = (uint32_t *)(scr + L.ubits);
+    const int nbw = (S + 31) >> 5;
+    for (int i = tid; i < slots; i += nt) tab[i] = -1;
+    for (int i = tid; i < nbw; i += nt) ubits[i] = 0u;
+    if (tid == 0) {
+      hs[0] = as_key(SM.HF[0]);
+      hs[firstB0] = as_key(SM.HF[1]);
+      if (firstB0 != S - 1) hs[S - 1] = ~0ull;
+    }
     __syncthreads();
-  }
-  const MinTable &net_tab = net_global ? net_gl : net_sm;
-  for (int i = tid; i < m; i += nt) {
-    const int c = cand[i];
-    const int r = net_tab.get(net_key(c));
-    if (r == c) {
-      atomicOr(&ubits[c >> 5], 1u << (c & 31));
-    } else {
-      // merged by hash: checked list by list below
-      const int k = atomicAdd(&SM.nwl, 1);
-      wl[k] = c;
-      vrep[k] = r;
-    }
-  }
-  __syncthreads();
-  // unique networks in network order: the set bits before each one
-  int running = 0;
-  for (int w0 = 0; w0 < nbw; w0 += nt) {
-    const int w = w0 + tid;
-    const uint32_t word = w < nbw ? ubits[w] : 0u;
-    int total;
-    const int off = block_scan(__popc(word), total, SM.scan);
-    for (uint32_t x = word; x; x &= x - 1) {
-      const int b = __ffs(x) - 1;
-      urep[running + off + __popc(word & ((1u << b) - 1u))] = 32 * w + b;
-    }
-    running += total;
-  }
-  if (tid == 0) SM.U = running;
-  __syncthreads();
-  const int U = SM.U;
-  // exact check of every hash merge (warp per merged network)
-  const int nver = SM.nwl;
-  for (int wi = warp; wi < nver; wi += nw) {
-    const int s = wl[wi];
-    const int r = vrep[wi];
-    int ks, ss, kr, sr;
-    net_of(s, sd, sig, ks, ss);
-    net_of(r, sd, sig, kr, sr);
-    const unsigned long long *Rs = rec_of(s);
-    const unsigned long long *Rr = rec_of(r);
-    const int ns = (int)Rs[1], nr = (int)Rr[1];
-    // both are their class's full network: equal by construction
-    if (ks == kr && ns == 0 && nr == 0) continue;
-    bool ok = true;
-    // states at the left-out sample of s, shared by the warp
-    load_stsig(sd, ss, myst, lane);
-    if (ks == kr) {
-      if (ns != nr) ok = false;
-      // every changed node of s must be changed in r
-      for (int i = lane; ok && i < ns; i += 32) {
-        int t = (int)(Rs[2 + i] & 0x3FFF);
-        bool found = false;
-        for (int j = 0; j < nr; j++)
-          if ((int)(Rr[2 + j] & 0x3FFF) == t) { found = true; break; }
-        if (!found) ok = false;
-      }
-      ok = __all_sync(0xffffffffu, ok);
-    }
-    // node-by-node list comparison: s's lists from the shared states, r's
-    // lists with the states of r's left-out sample read from global memory
-    if (ok) {
-      // nodes to compare: changed of s, changed of r, and DAB when classes differ
-      const int nd = (ks != kr) ? SM.ndab : 0;
-      const int total = ns + nr + nd;
-      for (int i = lane; i < total; i += 32) {
-        int t;
-        if (i < ns) t = (int)(Rs[2 + i] & 0x3FFF);
-        else if (i < ns + nr) t = (int)(Rr[2 + (i - ns)] & 0x3FFF);
-        else t = P.dab[i - ns - nr];
-        ListGen a;
-        gen_for(a, sd, P, phi[ks], pcol[ks], ks, t, ss >= 0 ? myst : nullptr);
-        const int GWl = sd.GW;
-        const int8_t *rT = sd.valsT + (size_t)(sr >= 0 ? sr : 0) * st_stride(sd.g);
-        const int strow_r = (sr >= 0) ? rT[t] : 3;
-        const uint32_t *rowr = P.rows + ((size_t)kr * g + t) * GWl;
-        int fi = P.phs[kr * g + t], fe = P.phe[kr * g + t];
-        int w = 0;
-        auto flipw = [&](int ww) -> uint32_t {
-          uint32_t mm = 0;
-          if (sr < 0 || strow_r > 2) return 0u;
-          const int hi = 32 * (ww + 1);
-          while (fi < fe) {
-            int col = pcol[kr][fi];
-            if (col >= hi) break;
-            int sc = rT[col];
-            if (sc <= 2 && ((phi[kr][fi] & 0x1FFu) >> (strow_r * 3 + sc)) & 1u) mm |= 1u << (col - 32 * ww);
-            fi++;
-          }
-          return mm;
-        };
-        uint32_t word = GWl > 0 ? (rowr[0] ^ flipw(0)) : 0u;
-        auto nextb = [&]() -> int {
-          while (true) {
-            if (word) {
-              int j = __ffs(word) - 1;
-              word &= word - 1;
-              return 32 * w + j;
-            }
-            if (++w >= GWl) return -1;
-            word = rowr[w] ^ flipw(w);
-          }
-        };
-        for (int q = 0; q < sd.mp; q++) {
-          int x = a.next(), y = nextb();
-          if (x != y) { ok = false; break; }
-          if (x < 0) break;
+    for (int s = tid; s < S; s += nt) {
+      const unsigned long long key = hs[s];
+      if (key == ~0ull) continue;
+      for (unsigned slot = (unsigned)(mix64(key) & tmask);; slot = (slot + 1u) & tmask) {
+        int cur = *(volatile int *)&tab[slot];
+        if (cur < 0) {
+          cur = atomicCAS(&tab[slot], -1, s);
+          if (cur < 0) break;
+        }
+        if (hs[cur] == key) {
+          atomicMin(&tab[slot], s);
+          break;
         }
       }
-      ok = __all_sync(0xffffffffu, ok);
     }
-    if (!ok && lane == 0) atomicOr(&SM.status, kUnitHashCollision);
-    __syncwarp();
-  }
-  __syncthreads();
-  if (bd.stats && tid == 0)
-    atomicAdd(&bd.stats[4 * (size_t)bd.uslot[u] + 3], (unsigned long long)(S - U));
-
-  // ---- Keys of the changed nodes' lists.  The leave-one-out networks of a
-  // unit share most of their changed nodes' lists (one flip near a
-  // threshold changes the same node in every network whose left-out sample
-  // triggers it), so the items hold few distinct keys (node, first three
-  // parents): ~240 among ~24000 items per unit when nearly every pair sits
-  // near the threshold.  Each distinct key is scored once, in a
-  // shared-memory table of KT slots (in the flip-entry cache, which no phase
-  // reads from here on), and every item adds its key's score.  The keys are
-  // the memo lists the records used and the logged merged-row lists; when
-  // more were logged than the log holds, the items are walked instead.  A
-  // key that finds no slot within kKeyProbes probes: every item is scored
-  // on its own.
-  constexpr int kKeyProbes = 64;
-  const int KT = HT < kKeyT ? HT : kKeyT;  // slot-indexed scores fit ksc ([HT][2])
-  unsigned long long *kt = (unsigned long long *)P.ephi;
-  const unsigned kmask = (unsigned)KT - 1u;
-  if (compacted && bd.keep_slot && bd.keep_slot[u] >= 0) {
-    // the detailed outputs still read the flip entries: back to the
-    // unit's scratch, each class's (nent[k] <= c) to its own arrays, the
-    // class-2 row ranges shifted to start at 0
-    const int ne0 = SM.nent[0], ne = ne0 + SM.nent[1];
-    for (int k = 0; k < 2; k++) {
-      uint32_t *gphi = (uint32_t *)(scr + L.phi[k]);
-      uint16_t *gpcol = (uint16_t *)(scr + L.pcol[k]);
-      const int e0 = k ? ne0 : 0, e1 = k ? ne : ne0;
-      for (int i = e0 + tid; i < e1; i += nt) {
-        gphi[i - e0] = P.ephi[i];
-        gpcol[i - e0] = P.epcol[i];
+    __syncthreads();
+    for (int s = tid; s < S; s += nt) {
+      const unsigned long long key = hs[s];
+      if (key == ~0ull) continue;
+      unsigned slot = (unsigned)(mix64(key) & tmask);
+      int r = tab[slot];
+      while (hs[r] != key) r = tab[slot = (slot + 1u) & tmask];
+      if (r == s) {
+        atomicOr(&ubits[s >> 5], 1u << (s & 31));
+      } else {
+        // merged by hash: checked list by list below
+        const int q = atomicAdd(&SM.nver, 1);
+        wl[q] = s;
+        vrep[q] = r;
       }
-      phi[k] = gphi;
-      pcol[k] = gpcol;
     }
-    for (int t = tid; t < g; t += nt)
-      if (P.phs[g + t] < P.phe[g + t]) {
-        P.phs[g + t] -= ne0;
-        P.phe[g + t] -= ne0;
+    __syncthreads();
+    // unique networks in network order: the set bits before each one
+    int running = 0;
+    for (int w0 = 0; w0 < nbw; w0 += nt) {
+      const int w = w0 + tid;
+      const uint32_t word = w < nbw ? ubits[w] : 0u;
+      int total;
+      const int off = block_scan(__popc(word), total, SM.scan);
+      int at = running + off;
+      for (uint32_t x = word; x; x &= x - 1) urep[at++] = 32 * w + __ffs(x) - 1;
+      running += total;
+    }
+    U = running;
+    __syncthreads();
+    // exact check of every hash merge, a warp per merged network: in one
+    // class, the rows' triggered entries agree, or else their lists do; in
+    // two, the lists of all nodes
+    const int nver = SM.nver;
+    for (int wi = warp; wi < nver; wi += nw) {
+      const int s = wl[wi], r = vrep[wi];
+      int ks, ss, kr, sr;
+      net_of(s, sd, sig, ks, ss);
+      net_of(r, sd, sig, kr, sr);
+      // a network without changes is compared as its class's full network
+      if (s == firstB0) ss = -1;
+      if (r == firstB0) sr = -1;
+      bool ok = true;
+      if (ks == kr && ss >= 0 && sr >= 0) {
+        const uint32_t *ca = sd.codes + (ss >> 4), *cb = sd.codes + (sr >> 4);
+        const int ha = 2 * (ss & 15), hb = 2 * (sr & 15), n16 = sd.n16;
+        for (int t = lane; ok && t < g; t += 32) {
+          const int i = ks * g + t, e0 = P.phs[i], e1 = P.phe[i];
+          if (e0 >= e1) continue;
+          const uint32_t a = 4u * ((ca[(size_t)t * n16] >> ha) & 3u);
+          const uint32_t b = 4u * ((cb[(size_t)t * n16] >> hb) & 3u);
+          bool same = true;
+          for (int e = e0; same && e < e1; e++) {
+            const uint2 en = ent[e];
+            const uint32_t x = (ca[(size_t)(en.x & 511u) * n16] >> ha) & 3u;
+            const uint32_t y = (cb[(size_t)(en.x & 511u) * n16] >> hb) & 3u;
+            same = (((en.y >> (a + x)) ^ (en.y >> (b + y))) & 1u) == 0u;
+          }
+          if (!same) ok = lists_equal(sd, P, ent, t, ks, ss, kr, sr);
+        }
+      } else if (ks != kr && ss < 0 && sr < 0) {
+        ok = SM.ndab == 0;  // the two full networks
+      } else {
+        for (int t = lane; ok && t < g; t += 32) ok = lists_equal(sd, P, ent, t, ks, ss, kr, sr);
       }
+      if (!ok) atomicOr(&SM.status, kUnitHashCollision);
+    }
     __syncthreads();
   }
-  for (int i = tid; i < KT; i += nt) kt[i] = ~0ull;
-  if (tid == 0) SM.tfull = 0;
-  __syncthreads();
-  auto insert_key = [&](unsigned long long rc) {
-    unsigned slot = (unsigned)(mix64(rc) & kmask);
-    for (int pr = 0; pr < kKeyProbes; pr++, slot = (slot + 1u) & kmask) {
-      // a slot only ever goes from empty to its final key: a read first,
-      // the atomic only on an empty slot
-      unsigned long long cur = kt[slot];
-      if (cur == ~0ull) cur = atomicCAS(&kt[slot], ~0ull, rc);
-      if (cur == ~0ull || cur == rc) return;
-    }
-    SM.tfull = 1;
-  };
-  const bool keys_logged = !bd.key_walk && SM.nlg <= HTs;
-  if (keys_logged) {
-    for (int task = tid; task < 2 * g * kMemoSub; task += nt) {
-      const int i = task / kMemoSub, q = task - i * kMemoSub;
-      const int e = P.phe[i] - P.phs[i];
-      if (e < 1 || e > kMemoE || q >= (1 << e) - 1) continue;
-      const int mi = moff[i] + q;
-      if (!((used[mi >> 5] >> (mi & 31)) & 1u)) continue;
-      const unsigned long long ent = memo[(size_t)mi * 2];
-      if (differs(i / g, ent)) insert_key(ent);
-    }
-    for (int x = tid; x < SM.nlg; x += nt) insert_key(hsk[x]);
+  if (tid == 0) {
+    bd.U[u] = SM.status ? -1 : U;
+    bd.status[u] = SM.status;
+    if (bd.stats) atomicAdd(&bd.stats[4 * (size_t)bd.uslot[u] + 3], (unsigned long long)(S - U));
   }
-  __syncthreads();
+  // one network has no JS (the range of its scores is empty), whatever its
+  // score is
+  if ((U == 1 && keep < 0) || SM.status) return;
 
-  // ---- P5: BDeu.  Base node scores of the two full networks: nodes
-  // without parents from the state counts, the others as flat tasks; a
-  // class-2 node whose capped parents equal the class-1 one copies its score.
+  // ---- P5: BDeu.  The JS takes only differences of the networks' scores,
+  // so the nodes that every network scores alike are left out (unless the
+  // scores themselves are kept): needed are the nodes whose full lists
+  // differ between the classes and those of rows with entries.
+  for (int i = tid; i < g * 3; i += nt) {
+    // state counts per class from the word-major planes: a warp's loads of
+    // a word are 32 consecutive planes
+    const uint64_t *pl = sd.planesT + i;
+    int a = 0, b = 0;
+    for (int w = 0; w < W; w++) {
+      const uint64_t x = pl[(size_t)w * 3 * g];
+      a += __popcll(x & P.mA[w]);
+      b += __popcll(x & P.mB[w]);
+    }
+    P.cnt3[i] = (uint16_t)a;
+    P.cnt3[3 * g + i] = (uint16_t)b;
+  }
+  for (int t = tid; t < g; t += nt)
+    if (keep >= 0 || P.need[t] || P.phs[t] < P.phe[t] || P.phs[g + t] < P.phe[g + t]) P.need[t] |= 2;
+  for (int i = tid; i < 4 * g; i += nt) P.fsc[i] = 0;
+  __syncthreads();
+  // base scores of the needed nodes in the two full networks; a class-2
+  // node whose first parents equal the class-1 one's copies its scores
   auto same_as_class1 = [&](int t) -> bool {
     const int a = P.fcnt[t] < 3 ? P.fcnt[t] : 3, b = P.fcnt[g + t] < 3 ? P.fcnt[g + t] : 3;
     if (a != b) return false;
@@ -1611,193 +1284,145 @@ __global__ void __launch_bounds__(256, 3) k_units(const __grid_constant__ BatchD
       if (P.fps[t * 3 + q] != P.fps[(g + t) * 3 + q]) return false;
     return true;
   };
-  for (int i = tid; i < 2 * g; i += nt) {
-    if (P.fcnt[i] != 0) continue;
-    const int k = i / g, t = i % g;
-    P.fsc[(k * 2 + 0) * g + t] = bdeu_score0(sd, t, P.cnt3);
-    P.fsc[(k * 2 + 1) * g + t] = bdeu_score0(sd, t, P.cnt3 + 3 * g);
-  }
   bdeu_items(
       sd, P, SM.scan, 2 * g,
       [&](int i) -> unsigned long long {
-        const int k = i / g, t = i % g;
-        if (P.fcnt[i] == 0 || (k == 1 && same_as_class1(t))) return ~0ull;
-        const int np = P.fcnt[i] < 3 ? P.fcnt[i] : 3;
-        return (unsigned long long)t | ((unsigned long long)np << 14) |
-               ((unsigned long long)P.fps[i * 3] << 16) |
-               ((unsigned long long)P.fps[i * 3 + 1] << 32) |
-               ((unsigned long long)P.fps[i * 3 + 2] << 48);
+        const int k = i >= g ? 1 : 0, t = i - k * g;
+        if (!(P.need[t] & 2) || (k == 1 && same_as_class1(t))) return ~0ull;
+        const int ps[3] = {P.fps[i * 3], P.fps[i * 3 + 1], P.fps[i * 3 + 2]};
+        return list_key(t, P.fcnt[i], ps);
       },
-      [&](int i, long long s1, long long s2) {
-        const int k = i / g, t = i % g;
-        if (P.fcnt[i] == 0 || (k == 1 && same_as_class1(t))) return;
+      [&](int i, unsigned long long key, long long s1, long long s2) {
+        if (key == ~0ull) return;
+        const int k = i >= g ? 1 : 0, t = i - k * g;
         P.fsc[(k * 2 + 0) * g + t] = s1;
         P.fsc[(k * 2 + 1) * g + t] = s2;
       });
   for (int t = tid; t < g; t += nt)
-    if (P.fcnt[g + t] != 0 && same_as_class1(t)) {
+    if ((P.need[t] & 2) && same_as_class1(t)) {
       P.fsc[(1 * 2 + 0) * g + t] = P.fsc[(0 * 2 + 0) * g + t];
       P.fsc[(1 * 2 + 1) * g + t] = P.fsc[(0 * 2 + 1) * g + t];
     }
   __syncthreads();
-  for (int i = tid; i < 4; i += nt) {
-    const int k = i / 2, cls = i % 2;
+  if (warp < 4) {
+    // warp 2 k + cls: the sum of full network k's scores over class cls
     long long s = 0;
-    for (int t = 0; t < g; t++) s += P.fsc[(k * 2 + cls) * g + t];
-    SM.base[cls][k] = s;
+    for (int t = lane; t < g; t += 32) s += P.fsc[warp * g + t];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) SM.base[warp & 1][warp >> 1] = s;
+  }
+  // the used variants' distinct keys within each row, and the keys of the
+  // lists formed per sample, scored once each
+  longlong2 *msc = (longlong2 *)(scr + L.msc);
+  longlong2 *bsc = (longlong2 *)(scr + L.bsc);
+  uint16_t *vcan = (uint16_t *)(scr + L.vcan), *sel = (uint16_t *)(scr + L.sel);
+  const int vsplit = SM.split[1];
+  auto is_used = [&](int v) { return ((P.used[v >> 5] >> (v & 31)) & 1u) != 0u; };
+  if (SM.nchg) {
+    for (int v = tid; v < nvar; v += nt) {
+      if (!is_used(v)) continue;
+      const unsigned long long key = ment[v];
+      if (!differs(v >= vsplit ? 1 : 0, key)) {
+        msc[v] = make_longlong2(0, 0);
+        vcan[v] = (uint16_t)v;
+        continue;
+      }
+      // the row's first used variant with this key (a key names its node)
+      int can = v;
+      for (int w = v - 1; w >= 0 && can - w < 256; w--) {
+        const unsigned long long kw = ment[w];
+        if (kw != ~0ull && (kw & 0x3FFF) != (key & 0x3FFF)) break;
+        if (w < vsplit && v >= vsplit) break;
+        if (kw == key && is_used(w)) can = w;
+      }
+      vcan[v] = (uint16_t)can;
+      if (can == v) sel[atomicAdd(&SM.nsel, 1)] = (uint16_t)v;
+    }
+    int *bpos = (int *)(scr + L.bpos);
+    int nbk = 0;
+    if (nbigs) {
+      for (int i0 = 0; i0 < KB; i0 += nt) {
+        const bool has = i0 + tid < KB && bkey[i0 + tid] != ~0ull;
+        int total;
+        const int off = block_scan(has ? 1 : 0, total, SM.scan);
+        if (has) bpos[nbk + off] = i0 + tid;
+        nbk += total;
+      }
+    }
+    __syncthreads();
+    const int nsel = SM.nsel;
+    bdeu_items(
+        sd, P, SM.scan, nsel + nbk,
+        [&](int i) -> unsigned long long { return i < nsel ? ment[sel[i]] : bkey[bpos[i - nsel]]; },
+        [&](int i, unsigned long long key, long long s1, long long s2) {
+          if (i < nsel) {
+            const int v = sel[i], k = v >= vsplit ? 1 : 0, t = (int)(key & 0x3FFF);
+            msc[v] = make_longlong2(s1 - P.fsc[(k * 2 + 0) * g + t], s2 - P.fsc[(k * 2 + 1) * g + t]);
+          } else {
+            bsc[bpos[i - nsel]] = make_longlong2(s1, s2);
+          }
+        });
+    for (int v = tid; v < nvar; v += nt)
+      if (is_used(v) && vcan[v] != v) msc[v] = msc[vcan[v]];
   }
   __syncthreads();
-  // unique networks: base of their class + deltas of the changed nodes whose
-  // capped list (first three parents) differs from the full network's; the
-  // changed nodes of all unique networks form one flat item list
-  // (prefix over the networks in wl)
-  for (int uu = tid; uu < U; uu += nt) {
-    int k, sigma;
-    net_of(urep[uu], sd, sig, k, sigma);
-    dist[uu] = SM.base[0][k];
-    dist[S + uu] = SM.base[1][k];
-  }
+  // unique networks: base of their class plus the variants' differences, a
+  // lane per network, a warp per 32 networks of one class
   {
-    int running = 0;
-    for (int u0 = 0; u0 < U; u0 += nt) {
-      const int uu = u0 + tid;
-      const int v = uu < U ? (int)rec_of(urep[uu])[1] : 0;
-      int total;
-      const int off = block_scan(v, total, SM.scan);
-      if (uu < U) wl[uu] = running + off;
-      running += total;
-    }
-    if (tid == 0) SM.nwl = running;
-    __syncthreads();
-  }
-  const int nchg_all = SM.nwl;
-  // item e -> (unique network, changed-node record)
-  auto item_of = [&](int e, int &uu, int &k, unsigned long long &rec) {
-    int lo = 0, hi = U - 1;
+    int lo = 0, hi = U;  // the class-1 networks among the unique ones
     while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (wl[mid] <= e) lo = mid;
-      else hi = mid - 1;
+      const int mid = (lo + hi) >> 1;
+      if (urep[mid] <= nA) lo = mid + 1;
+      else hi = mid;
     }
-    uu = lo;
-    int sigma;
-    const int s = urep[uu];
-    net_of(s, sd, sig, k, sigma);
-    rec = rec_of(s)[2 + (e - wl[uu])];
-  };
-  // the score delta of item e, given its key's scores in both classes
-  auto add_delta = [&](int uu, int k, unsigned long long rec, long long s1, long long s2) {
-    const int t = (int)(rec & 0x3FFF), np = (int)((rec >> 14) & 3);
-    if (np == 0) {
-      s1 = bdeu_score0(sd, t, P.cnt3);
-      s2 = bdeu_score0(sd, t, P.cnt3 + 3 * g);
-    }
-    atomicAdd((unsigned long long *)&dist[uu],
-              (unsigned long long)(s1 - P.fsc[(k * 2 + 0) * g + t]));
-    atomicAdd((unsigned long long *)&dist[S + uu],
-              (unsigned long long)(s2 - P.fsc[(k * 2 + 1) * g + t]));
-  };
-  // the items of unique network uu whose list differs from the full
-  // network's, in record order, read four records at a time
-  auto for_items = [&](int uu, auto &&fn) {
-    constexpr int kRecBatch = 4;
-    const unsigned long long *R = rec_of(urep[uu]);
-    const int nrec = (int)R[1];
-    const int k = class_of(urep[uu]);
-    for (int e0 = 0; e0 < nrec; e0 += kRecBatch) {
-      unsigned long long rb[kRecBatch];
-#pragma unroll
-      for (int q = 0; q < kRecBatch; q++) rb[q] = e0 + q < nrec ? R[2 + e0 + q] : ~0ull;
-#pragma unroll
-      for (int q = 0; q < kRecBatch; q++)
-        if (rb[q] != ~0ull && differs(k, rb[q])) fn(k, rb[q]);
-    }
-  };
-  int *kpos = htv;  // key list index -> slot
-  unsigned long long *klist = hsk;
-  long long *ksc = (long long *)(scr + L.ksc);
-  if (!keys_logged) {
-    // a thread per unique network inserts its items' keys
-    for (int uu = tid; uu < U; uu += nt)
-      for_items(uu, [&](int, unsigned long long rc) { insert_key(rc); });
-    __syncthreads();
-  }
-  if (!SM.tfull) {
-    // the keys in slot order: key list and slot -> list index
-    int nk = 0;
-    for (int i0 = 0; i0 < KT; i0 += nt) {
-      const int i = i0 + tid;
-      const unsigned long long key = i < KT ? kt[i] : ~0ull;
-      const bool has = key != ~0ull;
-      int total;
-      const int off = block_scan(has ? 1 : 0, total, SM.scan);
-      if (has) {
-        kpos[nk + off] = i;
-        klist[nk + off] = key;
+    const int U1 = lo, uc0 = (U1 + 31) >> 5, uc = uc0 + ((U - U1 + 31) >> 5);
+    for (int ch = warp; ch < uc; ch += nw) {
+      const int k = ch >= uc0 ? 1 : 0;
+      const int uu = 32 * (k ? ch - uc0 : ch) + (k ? U1 : 0) + lane;
+      const bool live = uu < (k ? U : U1);
+      const int s = live ? urep[uu] : 0;
+      long long d1 = SM.base[0][k], d2 = SM.base[1][k];
+      const bool plain = !live || s == 0 || s == firstB0;
+      if (!__all_sync(0xffffffffu, plain)) {
+        const int sg = sig[plain ? (k ? nA : 0) : s - 1];
+        long long x1 = 0, x2 = 0;
+        walk(k, sg, [&](int v) {
+          if (!is_used(v)) return;
+          const longlong2 x = msc[v];
+          x1 += x.x;
+          x2 += x.y;
+        });
+        for (int r = 0; !plain && r < SM.nbig[k]; r++) {
+          const int t = P.big[k * g + r];
+          unsigned long long key, h;
+          if (!sample_list(sd, P, ent, k, t, sg, key, h) || !differs(k, key)) continue;
+          const int slot = big_slot(key, false);
+          long long sc[2];
+          if (slot >= 0) {
+            sc[0] = bsc[slot].x;
+            sc[1] = bsc[slot].y;
+          } else {
+            key_scores(sd, P, key, sc);  // the table had no room
+          }
+          x1 += sc[0] - P.fsc[(k * 2 + 0) * g + t];
+          x2 += sc[1] - P.fsc[(k * 2 + 1) * g + t];
+        }
+        if (!plain) {
+          d1 += x1;
+          d2 += x2;
+        }
       }
-      nk += total;
+      if (live) {
+        dist[uu] = d1;
+        dist[S + uu] = d2;
+      }
     }
-    __syncthreads();
-    bdeu_items(
-        sd, P, SM.scan, nk, [&](int i) -> unsigned long long { return klist[i]; },
-        [&](int i, long long s1, long long s2) {
-          ksc[2 * kpos[i]] = s1;
-          ksc[2 * kpos[i] + 1] = s2;
-        });
-    __syncthreads();
-    // each network's deltas summed by its thread (exact integer sums)
-    for (int uu = tid; uu < U; uu += nt) {
-      long long d1 = 0, d2 = 0;
-      for_items(uu, [&](int k, unsigned long long rc) {
-        unsigned slot = (unsigned)(mix64(rc) & kmask);
-        int pr = 0;
-        while (kt[slot] != rc && ++pr < kKeyProbes) slot = (slot + 1u) & kmask;
-        if (pr >= kKeyProbes) {  // not found: cannot happen; the unit is re-run
-          atomicOr(&SM.status, kUnitHashCollision);
-          return;
-        }
-        const int t = (int)(rc & 0x3FFF), np = (int)((rc >> 14) & 3);
-        long long s1 = ksc[2 * slot], s2 = ksc[2 * slot + 1];
-        if (np == 0) {
-          s1 = bdeu_score0(sd, t, P.cnt3);
-          s2 = bdeu_score0(sd, t, P.cnt3 + 3 * g);
-        }
-        d1 += s1 - P.fsc[(k * 2 + 0) * g + t];
-        d2 += s2 - P.fsc[(k * 2 + 1) * g + t];
-      });
-      dist[uu] += d1;
-      dist[S + uu] += d2;
-    }
-    __syncthreads();  // every network's score is complete before it is read
-  } else {
-    bdeu_items(
-        sd, P, SM.scan, nchg_all,
-        [&](int e) -> unsigned long long {
-          int uu, k;
-          unsigned long long rec;
-          item_of(e, uu, k, rec);
-          if (!differs(k, rec)) return ~0ull;
-          return rec;  // t | np << 14 | parents: the item key format
-        },
-        [&](int e, long long s1, long long s2) {
-          int uu, k;
-          unsigned long long rec;
-          item_of(e, uu, k, rec);
-          if (!differs(k, rec)) return;
-          add_delta(uu, k, rec, s1, s2);
-        });
   }
 
-  // ---- P6: unique count and status; the normalisation and JS follow in
-  // k_js (up to 32 units per warp) from the fixed-point scores in dist
-  const int keep = bd.keep_slot ? bd.keep_slot[u] : -1;
-  if (tid == 0) {
-    bd.U[u] = U;
-    bd.status[u] = SM.status;
-  }
-
-  // ---- P7: detailed outputs of kept units
+  // ---- P6: detailed outputs of kept units (the normalisation and JS
+  // follow in k_js from the fixed-point scores in dist)
   if (keep >= 0) {
+    __syncthreads();
     const int mpk = bd.mpk;
     const double fx = ldexp(1.0, -sd.lg_shift);
     for (int uu = tid; uu < U; uu += nt) {
@@ -1815,10 +1440,9 @@ __global__ void __launch_bounds__(256, 3) k_units(const __grid_constant__ BatchD
       const int s = urep[uu];
       int k, sigma;
       net_of(s, sd, sig, k, sigma);
-      load_stsig(sd, sigma, myst, lane);
       for (int t = lane; t < g; t += 32) {
         ListGen G;
-        gen_for(G, sd, P, phi[k], pcol[k], k, t, sigma >= 0 ? myst : nullptr);
+        gen_for(G, sd, P, ent, k, t, sigma);
         int cnt = 0;
         while (cnt < sd.mp) {
           int j = G.next();
@@ -1828,7 +1452,6 @@ __global__ void __launch_bounds__(256, 3) k_units(const __grid_constant__ BatchD
         }
         bd.out_cnt[((size_t)keep * S + uu) * bd.keep_g + t] = cnt;
       }
-      __syncwarp();
     }
   }
 }
@@ -1860,20 +1483,21 @@ __global__ void __launch_bounds__(32 * kJsWarps) k_js(const __grid_constant__ Ba
   const int u0 = (blockIdx.x * kJsWarps + warp) * upw, u = u0 + lane;
   const bool mine = lane < upw && u < bd.B;
   const int Ur = mine ? bd.U[u] : 0;
-  const int U = Ur > 0 ? Ur : 0;
+  const int keep = (Ur > 0 && bd.keep_slot) ? bd.keep_slot[u] : -1;
+  // one network: no JS, and no likelihoods unless they are kept
+  const int U = Ur > 1 || (Ur == 1 && keep >= 0) ? Ur : 0;
   const int S = bd.sets[0].sd.S;  // n + 2, the same for every set of a batch
   // this lane's unit's scores (its set's slice of the scratch), shared with
   // the warp through shuffles
   unsigned long long dptr = 0ull;
   if (mine) {
     const BatchSet &bs = bd.sets[bd.uslot[u]];
-    const UnitLayout L = unit_layout(bs.sd.c, S, bd.kmax);
+    const UnitLayout L = unit_layout(bs.sd.c, S);
     dptr = (unsigned long long)(bd.scratch + bs.sc0 + (size_t)(u - bs.u0) * bs.unit_bytes + L.dist);
   }
   auto dist_of = [&](int o) {
     return (long long *)__shfl_sync(0xffffffffu, dptr, o);
   };
-  const int keep = (U > 0 && bd.keep_slot) ? bd.keep_slot[u] : -1;
   // the warp's units as prefix intervals of the flattened list
   int incl = U;
 #pragma unroll
@@ -2033,15 +1657,17 @@ __global__ void __launch_bounds__(32 * kJsWarps) k_js(const __grid_constant__ Ba
     double js = acc[warp][2][lane] / log(2.0);
     if (h0 == l0 || h1 == l1) js = __longlong_as_double(0x7ff8000000000000ll);
     bd.js[u] = js;
+  } else if (mine) {
+    bd.js[u] = __longlong_as_double(0x7ff8000000000000ll);
   }
 }
 
 // ------------------------------------------------------------ launchers
 cudaError_t launch_prep(const int8_t *vals, int g, int n, int W, int c, uint64_t *planes,
-                        uint64_t *valid, uint16_t *ctot, int8_t *valsT, cudaStream_t st) {
+                        uint64_t *valid, uint16_t *ctot, uint32_t *codes, cudaStream_t st) {
   int tot = g * W;
   k_planes<<<(tot + 127) / 128, 128, 0, st>>>(vals, g, n, W, planes, valid);
-  k_transpose<<<(st_stride(g) * n + 255) / 256, 256, 0, st>>>(vals, g, n, valsT);
+  k_codes<<<(g * code_words(n) + 127) / 128, 128, 0, st>>>(vals, g, n, codes);
   if (c > 0) k_ctot<<<(c + 127) / 128, 128, 0, st>>>(planes, g, W, c, ctot);
   return cudaGetLastError();
 }
@@ -2074,7 +1700,7 @@ cudaError_t launch_pairs(const BatchSet *sets, const int32_t *uslot, const uint6
 cudaError_t launch_units(const BatchDev &bd, int gmax, int W, cudaStream_t st, cudaEvent_t ev_mid,
                          bool ev_external) {
   const int threads = 256;
-  size_t smem = unit_smem_bytes(gmax, W, (gmax + 31) / 32, threads / 32);
+  const size_t smem = unit_smem_bytes(gmax, W);
   cudaError_t e = cudaFuncSetAttribute(k_units, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   k_units<<<bd.B, threads, smem, st>>>(bd);

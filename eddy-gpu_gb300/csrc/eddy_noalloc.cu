@@ -38,14 +38,13 @@ constexpr int kNAMaxGenes = 64;
 constexpr int kNAMaxSamples = 2048;
 constexpr int kNAPairs = kNAMaxGenes * (kNAMaxGenes - 1) / 2;
 constexpr int kNAW = kNAMaxSamples / 64;
-constexpr int kNAKmax = kNAMaxGenes + 1;  // a network changes at most g nodes
 
 __host__ __device__ constexpr size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // region sizes at the maximum shape
 constexpr size_t kOffVals = 0;
-constexpr size_t kOffValsT = kOffVals + al256((size_t)kNAMaxGenes * kNAMaxSamples);
-constexpr size_t kOffPlanes = kOffValsT + al256((size_t)st_stride(kNAMaxGenes) * kNAMaxSamples);
+constexpr size_t kOffCodes = kOffVals + al256((size_t)kNAMaxGenes * kNAMaxSamples);
+constexpr size_t kOffPlanes = kOffCodes + al256(4ull * kNAMaxGenes * code_words(kNAMaxSamples));
 constexpr size_t kOffValid = kOffPlanes + al256(2 * 8ull * kNAMaxGenes * 3 * kNAW);  // + word-major
 constexpr size_t kOffCtot = kOffValid + al256(8ull * kNAW);
 constexpr size_t kOffPrior = kOffCtot + al256(2ull * 9 * kNAPairs);
@@ -60,7 +59,7 @@ constexpr size_t kOffUnit = kOffSlot + 256;
 }  // namespace
 
 // size of the per-unit scratch at the maximum shape (computed at set-up)
-size_t unit_scratch_bytes(int c, int S, int kmax);
+size_t unit_scratch_bytes(int c, int S);
 
 namespace {
 constexpr size_t kNoAllocBytes = kOffUnit + (2u << 20);  // unit scratch <= 2 MB (checked)
@@ -107,7 +106,7 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
   if (g < 2 || n < 2 || opts->max_parents < 1) return EDDY_ERR_ARG;
   if (g > kNAMaxGenes || n > kNAMaxSamples) return EDDY_ERR_CAPACITY;
   const int c = g * (g - 1) / 2, W = (n + 63) / 64, S = n + 2;
-  if (unit_scratch_bytes(c, S, kNAKmax) > (2u << 20)) return EDDY_ERR_CAPACITY;
+  if (unit_scratch_bytes(c, S) > (2u << 20)) return EDDY_ERR_CAPACITY;
   int nA = 0;
   for (int s = 0; s < n; s++) {
     if (labels[s] > 1) return EDDY_ERR_ARG;
@@ -152,7 +151,7 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
     return bail(EDDY_ERR_CUDA);
   if (launch_prep((const int8_t *)(base + kOffVals), g, n, W, c, (uint64_t *)(base + kOffPlanes),
                   (uint64_t *)(base + kOffValid), (uint16_t *)(base + kOffCtot),
-                  (int8_t *)(base + kOffValsT), st) != cudaSuccess)
+                  (uint32_t *)(base + kOffCodes), st) != cudaSuccess)
     return bail(EDDY_ERR_CUDA);
 
   SetDev sd{};
@@ -173,7 +172,8 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
   sd.planesT = sd.planes + (size_t)g * 3 * W;
   sd.valid = (const uint64_t *)(base + kOffValid);
   sd.vals = (const int8_t *)(base + kOffVals);
-  sd.valsT = (const int8_t *)(base + kOffValsT);
+  sd.codes = (const uint32_t *)(base + kOffCodes);
+  sd.n16 = code_words(n);
   sd.ctot = (const uint16_t *)(base + kOffCtot);
   sd.prior = (const uint8_t *)(base + kOffPrior);
   sd.lg = (const int64_t *)(base + kOffLg);
@@ -195,7 +195,7 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
     BatchSet bs{};
     bs.sd = sd;
     bs.nb = 1;
-    bs.unit_bytes = (long long)unit_scratch_bytes(c, S, kNAKmax);
+    bs.unit_bytes = (long long)unit_scratch_bytes(c, S);
     // decisions (the unit kernel zeroes the masks it reads, so every attempt
     // decides again), from masks and a chunk bitmap that start at zero
     if (cudaMemcpyAsync(base + kOffSets, &bs, sizeof bs, cudaMemcpyHostToDevice, st) != cudaSuccess ||
@@ -206,7 +206,7 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
     BatchDev bd{};
     bd.B = 1;
     bd.nsets = 1;
-    bd.kmax = kNAKmax;
+    bd.memo_max = kMemoMax;
     bd.sets = d_sets;
     bd.uslot = d_slot;
     bd.masks = (const uint64_t *)(base + kOffMask);
