@@ -397,6 +397,113 @@ __device__ __forceinline__ unsigned quick_zero_f2(const f32x2 *o, float chiA) {
   return ((okx && f2_x(L) < f2_x(Rr)) ? 1u : 0u) | ((oky && f2_y(L) < f2_y(Rr)) ? 2u : 0u);
 }
 
+// The ten decisions of both classes' tables of a pair at once (lane x =
+// class 1, y = class 2), from the exact float counts o[9] and the margins R
+// and C: chi^2 = N (Q - 1), Q = sum_ij o_ij^2 / (R_i C_j), and with one
+// sample of cell (a, b) taken out
+//   Q' = Q + d_b K_b + e_a (S_a + d_b o_ab^2) - (2 o_ab - 1) / ((C_b - 1) (R_a - 1)),
+// S_a = sum_j o_aj^2 / C_j, K_b = sum_i o_ib^2 / R_i, d_b = 1 / (C_b (C_b - 1)),
+// e_a = 1 / (R_a (R_a - 1)), chi'^2 = (N - 1)(Q' - 1): five operations a
+// table on packed FP32 pairs, where evaluating each table anew takes about a
+// hundred.  Every term of Q' but the last is positive and built from exact
+// integers with at most 16 roundings of 2^-24 (a reciprocal approximation
+// counts two), and the last is below 0.4 where this applies, so |error of
+// Q'| < 24 2^-24 Q' = 1.5e-6 Q', i.e. 1.5e-6 (N + chi^2) in chi^2; the
+// thresholds are moved inward by twice that.  Applies to quick_zero's
+// tables: every margin >= 2, 32 <= N <= 4096, every expected count >= 5
+// before and after (dof 4, no Yates correction, unchanged support).  A
+// class whose decisions are not all certain, or whose chi^2 comes near the
+// AS 147 underflow, is left to the general path: its bit of the result.
+// mask: the certain classes' ten bits (class 1 from bit 0, class 2 from 16).
+__device__ __forceinline__ f32x2 f2_rcp(f32x2 v) {
+  return f2_pack(rcp_approx(f2_x(v)), rcp_approx(f2_y(v)));
+}
+__device__ __forceinline__ f32x2 f2_dup(float v) { return f2_pack(v, v); }
+__device__ __forceinline__ unsigned loo_f2(const f32x2 *o, const f32x2 *R, const f32x2 *C, f32x2 N,
+                                           const Thr &T, bool exact_all, uint32_t &mask) {
+  const f32x2 one = f2_dup(1.f);
+  const float rmx = fminf(f2_x(R[0]), fminf(f2_x(R[1]), f2_x(R[2])));
+  const float rmy = fminf(f2_y(R[0]), fminf(f2_y(R[1]), f2_y(R[2])));
+  const float cmx = fminf(f2_x(C[0]), fminf(f2_x(C[1]), f2_x(C[2])));
+  const float cmy = fminf(f2_y(C[0]), fminf(f2_y(C[1]), f2_y(C[2])));
+  const float Nx = f2_x(N), Ny = f2_y(N);
+  const bool okx = !exact_all && rmx >= 2.f && cmx >= 2.f && Nx >= 32.f && Nx <= 4096.f &&
+                   (rmx - 1.f) * (cmx - 1.f) >= 5.f * (Nx - 1.f) && rmx * cmx >= 5.f * Nx;
+  const bool oky = !exact_all && rmy >= 2.f && cmy >= 2.f && Ny >= 32.f && Ny <= 4096.f &&
+                   (rmy - 1.f) * (cmy - 1.f) >= 5.f * (Ny - 1.f) && rmy * cmy >= 5.f * Ny;
+  f32x2 iR[3], iR1[3], eR[3], iC[3], iC1[3], eC[3];
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    const f32x2 r1 = f2_sub(R[a], one), c1 = f2_sub(C[a], one);
+    eR[a] = f2_rcp(f2_mul(R[a], r1));
+    iR[a] = f2_mul(eR[a], r1);
+    iR1[a] = f2_mul(eR[a], R[a]);
+    eC[a] = f2_rcp(f2_mul(C[a], c1));
+    iC[a] = f2_mul(eC[a], c1);
+    iC1[a] = f2_mul(eC[a], C[a]);
+  }
+  f32x2 p[9], S[3], Qb[3];
+#pragma unroll
+  for (int k = 0; k < 9; k++) p[k] = f2_mul(o[k], o[k]);
+#pragma unroll
+  for (int a = 0; a < 3; a++)
+    S[a] = f2_fma(p[3 * a + 2], iC[2], f2_fma(p[3 * a + 1], iC[1], f2_mul(p[3 * a], iC[0])));
+  const f32x2 Q = f2_fma(S[2], iR[2], f2_fma(S[1], iR[1], f2_mul(S[0], iR[0])));
+#pragma unroll
+  for (int b = 0; b < 3; b++) {
+    const f32x2 K = f2_fma(p[6 + b], iR[2], f2_fma(p[3 + b], iR[1], f2_mul(p[b], iR[0])));
+    Qb[b] = f2_fma(eC[b], K, Q);
+  }
+  // thresholds on Q (N) and Q' (N - 1)
+  const f32x2 mB = f2_fma(f2_add(N, f2_dup(T.chiB)), f2_dup(3e-6f), f2_dup(T.chiB));
+  const f32x2 mA = f2_fma(f2_add(N, f2_dup(T.chiA)), f2_dup(-3e-6f), f2_dup(T.chiA));
+  const f32x2 mK = f2_fma(f2_add(N, f2_dup(T.kLo)), f2_dup(-3e-6f), f2_dup(T.kLo));
+  const f32x2 rN = f2_rcp(N), rN1 = f2_rcp(f2_sub(N, one));
+  const f32x2 qB = f2_fma(mB, rN, one), qA = f2_fma(mA, rN, one), qK = f2_fma(mK, rN, one);
+  const f32x2 qB1 = f2_fma(mB, rN1, one), qA1 = f2_fma(mA, rN1, one);
+  // the sign of threshold - Q' is the decision: shifted in, cell 8 first,
+  // the full table last (bit 0)
+  unsigned bx = 0, by = 0, ax = 0, ay = 0;
+  float hx = f2_x(Q), hy = f2_y(Q), lx = f2_x(o[0]), ly = f2_y(o[0]);
+  auto put = [&](f32x2 q, f32x2 tB, f32x2 tA) {
+    const f32x2 dB = f2_sub(tB, q), dA = f2_sub(tA, q);
+    bx = __funnelshift_l(__float_as_uint(f2_x(dB)), bx, 1);
+    by = __funnelshift_l(__float_as_uint(f2_y(dB)), by, 1);
+    ax = __funnelshift_l(__float_as_uint(f2_x(dA)), ax, 1);
+    ay = __funnelshift_l(__float_as_uint(f2_y(dA)), ay, 1);
+  };
+#pragma unroll
+  for (int k = 8; k >= 0; k--) {
+    const int a = k / 3, b = k % 3;
+    const f32x2 Sab = f2_fma(p[k], eC[b], S[a]);
+    const f32x2 w = f2_mul(iC1[b], iR1[a]);
+    const f32x2 q = f2_fma(f2_fma(o[k], f2_dup(-2.f), one), w, f2_fma(eR[a], Sab, Qb[b]));
+    put(q, qB1, qA1);
+    hx = fmaxf(hx, f2_x(q));
+    hy = fmaxf(hy, f2_y(q));
+    lx = fminf(lx, f2_x(o[k]));
+    ly = fminf(ly, f2_y(o[k]));
+  }
+  put(Q, qB, qA);
+  // an empty cell has no sample to take out: its slot shares the full
+  // table's decision
+  if (lx == 0.f || ly == 0.f) {
+    unsigned zx = 0, zy = 0;
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+      zx |= (f2_x(o[k]) == 0.f ? 2u : 0u) << k;
+      zy |= (f2_y(o[k]) == 0.f ? 2u : 0u) << k;
+    }
+    bx = (bx & ~zx) | ((bx & 1u) ? zx : 0u);
+    by = (by & ~zy) | ((by & 1u) ? zy : 0u);
+    ax = (ax & ~zx) | ((ax & 1u) ? zx : 0u);
+    ay = (ay & ~zy) | ((ay & 1u) ? zy : 0u);
+  }
+  const bool sx = okx && ax == bx && hx < f2_x(qK), sy = oky && ay == by && hy < f2_y(qK);
+  mask = (sx ? bx : 0u) | (sy ? by << 16 : 0u);
+  return (sx ? 0u : 1u) | (sy ? 0u : 2u);
+}
+
 // The general path: full-table decision, the Minkowski leave-one-out filter
 // and, when that cannot settle them, the nine cell-removed tables one by one.
 // Counts by value and not inlined: it runs for a small share of the tables.

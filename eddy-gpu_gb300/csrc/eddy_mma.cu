@@ -8,10 +8,16 @@
 // accumulation in TMEM, exact for counts < 2^24.  This replaces the S x c x n
 // tally loops of the reference's run2/run2Scalable (kernel1.cu:76-336);
 // class 2 = full-sample table - class 1.  The epilogue reads the counts out
-// of TMEM and settles, in the same kernel, every table whose ten
-// leave-one-out variants provably hold no edge; the others are queued for
-// k_general, which sets the bits of the 10-bit decision masks of both
-// classes (kernel1.cu:121-203, 419-431) in a buffer that starts at zero.
+// of TMEM and decides there: first the bound that settles a table whose ten
+// leave-one-out variants provably hold no edge, then, for the pairs of which
+// some lane needs them, all ten decisions of both classes (loo_f2).  It
+// stores the 10-bit decision masks (kernel1.cu:121-203, 419-431) into a
+// buffer that starts at zero; only tables within the FP32 error of a
+// threshold, with Yates' correction or with an empty row or column go
+// through a queue to k_general.  (With every table past the bound queued,
+// 24 bytes each, 10000 units of 200 genes x 1000 samples near the threshold
+// spent 8.3 ms in this kernel, bound by the queue's stores, and 20.8 ms in
+// k_general; now 5.3 and 0.25 ms, bound by the epilogue's issue slots.)
 //
 // When every value of the set is -1/0/1 (kCore), a table's margins are the
 // two genes' own class counts, which a small kernel counts per unit: the
@@ -184,6 +190,18 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t *r) {
         "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t *r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld9(uint32_t taddr, uint32_t *r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
+                 "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r[8]) : "r"(taddr + 8));
+}
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -276,24 +294,6 @@ __device__ __forceinline__ unsigned core_zero_f2(const f32x2 *o, const CoreGene 
   const f32x2 Rr = f2_mul(f2_pack(chiA, chiA), qD);
   return ((okx && f2_x(L) < f2_x(Rr)) ? 1u : 0u) | ((oky && f2_y(L) < f2_y(Rr)) ? 2u : 0u);
 }
-// The class-1 table of pair q of a group as integers, for the queue: the
-// four counted cells from TMEM and the five derived from the row gene's and
-// the column gene's class-1 counts wr, wc and the class-1 size n1.
-__device__ __forceinline__ void core_table(const uint32_t *r, int q, uint32_t wr, uint32_t wc,
-                                           int n1, int *t) {
-  t[0] = (int)__uint_as_float(r[4 * q]);
-  t[1] = (int)__uint_as_float(r[4 * q + 1]);
-  t[3] = (int)__uint_as_float(r[4 * q + 2]);
-  t[4] = (int)__uint_as_float(r[4 * q + 3]);
-  const int r0 = (int)(wr & 0xFFFFu), r1 = (int)(wr >> 16);
-  const int c0 = (int)(wc & 0xFFFFu), c1 = (int)(wc >> 16);
-  t[2] = r0 - t[0] - t[1];
-  t[5] = r1 - t[3] - t[4];
-  t[6] = c0 - t[0] - t[3];
-  t[7] = c1 - t[1] - t[4];
-  t[8] = (n1 - r0 - r1) - t[6] - t[7];
-}
-
 }  // namespace
 
 // Tile t of a batch's launch: its set k (sets ordered by tile0), column
@@ -337,8 +337,8 @@ template <int kStages, int kEpi, int kGroups, bool kCore>
 __global__ void __maxnreg__(max_regs<kEpi>())
     k_pairs_mma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                 const BatchSet *__restrict__ sets, int nsets, const float *__restrict__ ctotf,
-                int nk, int ntot, unsigned long long *stats, unsigned *err, unsigned *gqueue,
-                unsigned qcap, const uint32_t *__restrict__ margc,
+                int nk, int ntot, uint32_t *dmask, unsigned long long *stats, unsigned *err,
+                unsigned *gqueue, unsigned qcap, const uint32_t *__restrict__ margc,
                 const float4 *__restrict__ gcnt, const uint32_t *__restrict__ gtab) {
   constexpr int kTN = 32 * kGroups;
   constexpr int kPPG = kCore ? kCorePairs : kPairsPerGroup;  // pairs per column group
@@ -570,7 +570,7 @@ __global__ void __maxnreg__(max_regs<kEpi>())
         // the group's 32 TMEM columns (the 4-cell layout reads them in two
         // halves in pass 1, and again in full for pass 2)
         const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * kTN + grp * 32);
-        uint32_t r[32];
+        uint32_t r[kCore ? 1 : 32];
         if constexpr (!kCore) {
           tmem_ld32(taddr, r);
           tmem_ld_wait();
@@ -646,64 +646,99 @@ __global__ void __maxnreg__(max_regs<kEpi>())
         qmask &= vmask;
         ntab += (unsigned)__popc(vmask);
         nfilt += (unsigned)__popc(vmask & ~qmask);
-        // pass 2 (rare): the flagged tables into the launch's queue, one
-        // atomic per warp: counts, class, prior, pair and unit
-        if (__any_sync(0xffffffffu, qmask != 0u)) {
-          const unsigned cnt = (unsigned)__popc(qmask);
-          unsigned incl = cnt;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-          }
-          unsigned qbase = 0;
-          if (lane == 31) qbase = atomicAdd(gqueue, incl);
-          unsigned idx = __shfl_sync(0xffffffffu, qbase, 31) + incl - cnt;
+        // pass 2: the ten decisions of the flagged tables, a pair at a time
+        // (the pairs that some lane flagged).  Certain masks go straight to
+        // the unit's decision masks; the rest into the launch's queue.
+        const uint32_t wmask = __reduce_or_sync(0xffffffffu, qmask);
+        if (wmask == 0u) continue;
+        uint32_t marks = 0u;  // chunks of the group's pairs with a nonzero mask
+        const int pg = kCore ? crow * (crow - 1) / 2 + ccol0 : p0;
+        uint32_t *udm = ulive ? unit_dmask(dmask, bs, u) : nullptr;
+#pragma unroll 1
+        for (int q = 0; q < kPPG; q++) {
+          if (((wmask >> (2 * q)) & 3u) == 0u) continue;
+          __syncwarp();
+          // pair index (row-major over the lower triangle)
+          const int p = pg + q;
+          f32x2 o[9], R[3], C[3], Nq;
+          int prior;
           if constexpr (kCore) {
-            tmem_ld32(taddr, r);
+            uint32_t rq[4];
+            tmem_ld4(taddr + 4 * q, rq);
+            const uint32_t *mc = margc + bs.mg0;
+            const int Bp = bs.mblocks * kTM, col = ccol0 + q;
+            CoreGene Rg, Cg;
+            core_gene(Rg, wcur[kCorePairs], gc4[crow], N);
+            core_gene(Cg, mc[(size_t)col * Bp + ul], gc4[col], N);
             tmem_ld_wait();
+            core_cells(rq, reinterpret_cast<const float4 *>(gct)[q], Rg, Cg, o);
+            R[0] = Rg.M0, R[1] = Rg.M1, R[2] = Rg.M2;
+            C[0] = Cg.M0, C[1] = Cg.M1, C[2] = Cg.M2;
+            Nq = N;
+            prior = (int)((__float_as_uint(gct[32]) >> q) & 1u);
+          } else {
+            uint32_t rq[9];
+            tmem_ld9(taddr + 9 * q, rq);
+            const float *f = gct + q * 12;
+            tmem_ld_wait();
+#pragma unroll
+            for (int k = 0; k < 9; k++) {
+              const float a = __uint_as_float(rq[k]);
+              o[k] = f2_pack(a, f[k] - a);
+            }
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+              R[a] = f2_add(f2_add(o[3 * a], o[3 * a + 1]), o[3 * a + 2]);
+              C[a] = f2_add(f2_add(o[a], o[3 + a]), o[6 + a]);
+            }
+            Nq = f2_add(f2_add(R[0], R[1]), R[2]);
+            prior = f[9] != 0.f ? 1 : 0;
           }
+          const uint32_t want = (qmask >> (2 * q)) & 3u;
+          uint32_t m = 0u;
+          const uint32_t unc = want & loo_f2(o, R, C, Nq, sd.thr[prior][2], sd.exact_all != 0, m);
+          if (!(want & 1u)) m &= 0xFFFF0000u;
+          if (!(want & 2u)) m &= 0xFFFFu;
+          // a class whose ten tables agree is settled at once
+          nfilt += (want & ~unc & 1u) && ((m & 0x3FFu) == 0u || (m & 0x3FFu) == 0x3FFu);
+          nfilt += (want & ~unc & 2u) && ((m >> 16) == 0u || (m >> 16) == 0x3FFu);
+          if (m) {
+            udm[p] = m;  // this warp alone holds the unit's pair
+            marks |= 1u << ((p >> 5) - (pg >> 5));
+          }
+          // the warp's uncertain tables into the queue, one atomic: counts,
+          // class, prior, pair and unit
+          const unsigned b0 = __ballot_sync(0xffffffffu, unc & 1u);
+          const unsigned b1 = __ballot_sync(0xffffffffu, (unc & 2u) != 0u);
+          if ((b0 | b1) == 0u) continue;
+          unsigned qbase = 0;
+          if (lane == 0) qbase = atomicAdd(gqueue, (unsigned)(__popc(b0) + __popc(b1)));
+          qbase = __shfl_sync(0xffffffffu, qbase, 0);
 #pragma unroll
-          for (int q = 0; q < kPPG; q++) {
-            if (((qmask >> (2 * q)) & 3u) == 0u) continue;
-            // pair index (row-major over the lower triangle)
-            const int p = kCore ? crow * (crow - 1) / 2 + ccol0 + q : p0 + q;
-            // the class-1 table and the full-sample table, as integers
-            int t1[9], tf[9], prior;
-            if constexpr (kCore) {
-              prior = (int)((__float_as_uint(gct[32]) >> q) & 1u);
-              core_table(r, q, wcur[kCorePairs], wcur[q], (int)f2_x(N), t1);
+          for (int cls = 0; cls < 2; cls++) {
+            if (!((unc >> cls) & 1u)) continue;
+            const unsigned below = (1u << lane) - 1u;
+            const unsigned idx = cls ? qbase + __popc(b0) + __popc(b1 & below) : qbase + __popc(b0 & below);
+            uint32_t t[9];
 #pragma unroll
-              for (int k = 0; k < 9; k++) tf[k] = (int)sd.ctot[(size_t)p * 9 + k];
+            for (int k = 0; k < 9; k++) t[k] = (uint32_t)(cls ? f2_y(o[k]) : f2_x(o[k]));
+            if (idx < qcap) {
+              unsigned *it = qitems + (size_t)idx * kQWords;
+              it[0] = t[0] | (t[1] << 16);
+              it[1] = t[2] | (t[3] << 16);
+              it[2] = t[4] | (t[5] << 16);
+              it[3] = t[6] | (t[7] << 16);
+              it[4] = t[8] | ((uint32_t)cls << 16) | ((uint32_t)prior << 17);
+              it[5] = (uint32_t)p | ((uint32_t)u << 17);  // pair < 2^17, batch unit < 2^15
             } else {
-              const float *f = gct + q * 12;
-              prior = (f[9] != 0.f) ? 1 : 0;
-#pragma unroll
-              for (int k = 0; k < 9; k++) {
-                t1[k] = (int)__uint_as_float(r[9 * q + k]);
-                tf[k] = (int)f[k];
-              }
-            }
-#pragma unroll
-            for (int cls = 0; cls < 2; cls++) {
-              if (!((qmask >> (2 * q + cls)) & 1u)) continue;
-              uint32_t o[9];
-#pragma unroll
-              for (int k = 0; k < 9; k++) o[k] = (uint32_t)(cls ? tf[k] - t1[k] : t1[k]);
-              if (idx < qcap) {
-                unsigned *it = qitems + (size_t)idx * kQWords;
-                it[0] = o[0] | (o[1] << 16);
-                it[1] = o[2] | (o[3] << 16);
-                it[2] = o[4] | (o[5] << 16);
-                it[3] = o[6] | (o[7] << 16);
-                it[4] = o[8] | ((uint32_t)cls << 16) | ((uint32_t)prior << 17);
-                it[5] = (uint32_t)p | ((uint32_t)u << 17);  // pair < 2^17, batch unit < 2^15
-              } else {
-                atomicOr(err, 2u);
-              }
-              idx++;
+              atomicOr(err, 2u);
             }
           }
+        }
+        if (marks) {
+          uint32_t *ucb = unit_chunks(dmask, bs, u);
+          mark_chunk(ucb, (marks & 1u) ? pg : (pg | 31) + 1);
+          if (marks == 3u) mark_chunk(ucb, (pg | 31) + 1);
         }
       }
       // the slot (accumulator and table buffer) is free again
@@ -1299,7 +1334,7 @@ static cudaError_t launch_variant(const BatchSet *sets, int nsets, const MmaPlan
   if (e != cudaSuccess) return e;
   const int grid = plan.ntot < sms ? plan.ntot : sms;
   kern<<<grid, 32 * (2 + kEpi), smem, st>>>(ma, mb, sets, nsets, ctotf, np / kKC, plan.ntot,
-                                            stats, err, gqueue, qcap, margc, gcnt, gtab);
+                                            dmask, stats, err, gqueue, qcap, margc, gcnt, gtab);
   return cudaGetLastError();
 }
 
