@@ -63,7 +63,7 @@ def load_peaks():
 
 
 def algorithmic_bytes(g, n, mp, U):
-    """Per-unit algorithmic bytes of the network stages (k_units + k_js:
+    """Per-unit algorithmic bytes of the network stages (k_units:
     network assembly, dedup, BDeu, normalisation and JS) when each stage reads
     its inputs and writes its outputs once through HBM: the S x c edge bits
     of the S leave-one-out networks read, S x g x mp 16-bit parent entries and
@@ -297,7 +297,7 @@ def run_multiset(args, rank, world, local):
             "wall_units_per_s": units / wall, "units": units, "sets": len(sids),
             "sets_per_s": len(sids) / (ms / 1e3), "ms": ms, "launches": t["launches"],
             "stage_ms": {"k_operands+k_pairs_mma": t["ms_gemm"], "k_general+k_exact": t["ms_decide"],
-                         "k_units": t["ms_networks"], "k_js": t["ms_js"]},
+                         "k_units": t["ms_networks"]},
             "sets_stopped_at_iteration0": stop0,
             "sets_with_all_iterations": sum(1 for it in iters if it == R),
             "per_set_value": units / (ms_per_set / 1e3),
@@ -534,7 +534,7 @@ def run_ours(args, rank, world, local):
             "gpu_launches": acc["launches"],
             "stage_ms": {"k_operands+k_pairs_mma": acc["ms_gemm"],
                          "k_general+k_exact": acc["ms_decide"], "k_units": acc["ms_networks"],
-                         "k_js": acc["ms_js"], "steps": args.steps},
+                         "steps": args.steps},
             "roofline": roofline,
             "kernels": {"k_pairs_mma": k1, "k_units": k2},
             "clocks": clk.summary(),

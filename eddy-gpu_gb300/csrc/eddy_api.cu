@@ -116,9 +116,9 @@ struct eddy_ctx {
   std::vector<SetHost> sets;
   cudaStream_t stream = nullptr;
   // batch boundaries: 0 before the decisions, 4 after the contraction, 1
-  // after the decisions, 5 after the networks, 2 after the JS; 2 and 3 also
-  // time the autotuner's choices
-  cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+  // after the decisions, 2 after the networks and the JS; 2 and 3 also time
+  // the autotuner's choices
+  cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   GlibcRand rng{1};
   std::vector<uint8_t> seen;
   std::vector<int> order;
@@ -156,7 +156,7 @@ struct eddy_ctx {
   // timing of the last run
   double ms_total = 0, ms_pairs = 0, ms_units = 0;
   // the same split by kernel: operands + contraction, general + exact
-  // decisions, networks, normalisation + JS
+  // decisions, networks with normalisation and JS; the last is 0
   double ms_stage[4] = {0, 0, 0, 0};
   long long launches = 0;
   uint64_t salt = 0x5EED5EEDull;
@@ -788,9 +788,9 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
       if (rc) return rc;
     }
     CK(record(ctx->ev[1], capturing));
-    CK(launch_units(bd, bp.gmax, W, ctx->stream, ctx->ev[5], capturing));
+    CK(launch_units(bd, bp.gmax, W, ctx->stream));
     CK(record(ctx->ev[2], capturing));
-    ctx->launches += 2;  // networks, then normalisation and JS
+    ctx->launches += 1;  // networks, normalisation and JS
     return EDDY_OK;
   };
   ctx->dmask_clean = nullptr;  // until the batch is seen to finish
@@ -860,9 +860,9 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
                                   layout_core(v), ns == 1 ? bp.sets[0].sd.g : 0, ctx->ev[4],
                                   true));
           cap_ck(record(ctx->ev[1], true));
-          cap_ck(launch_units(bd, bp.gmax, W, ctx->stream, ctx->ev[5], true));
+          cap_ck(launch_units(bd, bp.gmax, W, ctx->stream));
           cap_ck(record(ctx->ev[2], true));
-          ctx->launches += 1 + mma_launches() + 2;
+          ctx->launches += 1 + mma_launches() + 1;
         }
         cudaGraph_t graph = nullptr;
         const cudaError_t ce = cudaStreamEndCapture(ctx->stream, &graph);
@@ -917,8 +917,8 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   *t_pairs += a;
   *t_units += bms;
   {
-    const int cut[5] = {0, 4, 1, 5, 2};
-    for (int q = 0; q < 4; q++) {
+    const int cut[4] = {0, 4, 1, 2};
+    for (int q = 0; q < 3; q++) {
       float m = 0;
       if (cudaEventElapsedTime(&m, ctx->ev[cut[q]], ctx->ev[cut[q + 1]]) == cudaSuccess)
         ctx->ms_stage[q] += m;

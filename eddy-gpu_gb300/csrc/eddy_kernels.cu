@@ -16,8 +16,8 @@
 //                       hashing and first-occurrence dedup with exact
 //                       verification (kernel4.cu:72-84, main.cu:1060-1121),
 //                       BDeu over the unique networks in fixed point
-//                       (kernel5.cu:237-257).
-//   k_js                normalisation and JS (main.cu:1293-1428).
+//                       (kernel5.cu:237-257), normalisation and JS
+//                       (main.cu:1293-1428).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -268,13 +268,12 @@ __global__ void __launch_bounds__(128) k_pairs(const BatchSet *__restrict__ sets
 __device__ __forceinline__ uint32_t cells16(uint32_t fb) {
   return (fb & 7u) | (((fb >> 3) & 7u) << 4) | (((fb >> 6) & 7u) << 8);
 }
-// A row with at most E <= kMemoE kept entries (and no more subsets of them
+// A row with at most E <= BatchDev::memo_max kept entries (and no more subsets of them
 // than its class has samples) is a memo row: its capped list under every
 // non-empty subset of its entries (a variant) is formed once per unit.  The
 // other rows' lists are formed per left-out sample.  E is lowered until the
 // unit's variants fit unit_variants(g), which rows of up to five entries
 // always do.
-constexpr int kMemoE = 8;
 __host__ __device__ constexpr int unit_variants(int g) { return 62 * g + 64; }
 // slots of the table of the lists formed per sample (in the unit's scratch)
 __host__ __device__ constexpr int big_slots(int g) {
@@ -375,6 +374,8 @@ struct UnitSmem {
   unsigned status;
   int scan[32];
   unsigned long long scan64[32];
+  long long red[6][32];
+  double redd[3][32];
 };
 
 // BDeu work items (node scores) processed per round
@@ -621,6 +622,134 @@ __device__ __noinline__ void key_scores(const SetDev &sd, const UnitPtrs &P, uns
   }
 }
 
+// Normalisation (main.cu:1302-1404) and JS (main.cu:1406-1428) of a unit
+// from its unique networks' node-summed fixed-point scores dist[U], dist[S
+// + U]: per class min, max and mean of the scores (exact integers),
+// likelihoods exp((d - mean) 10 / (max - min)) normalised to sum 1, then the
+// two KL terms of kool() (routines.cu:42-60), zeros skipped, in FP64.  The
+// exponentials replace the scores in dist.  Sums are formed in a fixed
+// order: a thread's networks in turn, then a tree over the warp, then the
+// warps in turn.  pl, ql: the kept normalised likelihoods, or null.
+//
+// Inside k_units rather than after it: FP64 is slow on this part (about two
+// operations a cycle and SM, ~128 cycles to a dependent one), and here its
+// waits pass under the other blocks' integer work.  As a kernel of its own,
+// a warp per unit or more units a warp, it took 6.0 ms for 10000 units of
+// 1000 networks, 18.4 ms for 75000 of 400 and 68 us for one unit of 300.
+static __device__ __noinline__ double unit_js(long long *dist, int S, int U, UnitSmem &SM, double *pl,
+                                              double *ql) {
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
+  // the warps that hold networks, and the lanes of a warp that do (the sums
+  // over the others' zeros are left out: each costs a dependent FP64 add)
+  const int nw = min(nt >> 5, (U + 31) >> 5), lanes = min(U, 32);
+  long long mn0 = LLONG_MAX, mx0 = LLONG_MIN, mn1 = LLONG_MAX, mx1 = LLONG_MIN;
+  unsigned long long s0 = 0, s1 = 0;  // modulo 2^64
+  for (int uu = tid; uu < U; uu += nt) {
+    const long long a = dist[uu], b = dist[S + uu];
+    mn0 = min(mn0, a);
+    mx0 = max(mx0, a);
+    mn1 = min(mn1, b);
+    mx1 = max(mx1, b);
+    s0 += (unsigned long long)a;
+    s1 += (unsigned long long)b;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    mn0 = min(mn0, (long long)__shfl_xor_sync(0xffffffffu, mn0, o));
+    mx0 = max(mx0, (long long)__shfl_xor_sync(0xffffffffu, mx0, o));
+    mn1 = min(mn1, (long long)__shfl_xor_sync(0xffffffffu, mn1, o));
+    mx1 = max(mx1, (long long)__shfl_xor_sync(0xffffffffu, mx1, o));
+    s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+  }
+  if (lane == 0) {
+    SM.red[0][warp] = mn0;
+    SM.red[1][warp] = mx0;
+    SM.red[2][warp] = mn1;
+    SM.red[3][warp] = mx1;
+    SM.red[4][warp] = (long long)s0;
+    SM.red[5][warp] = (long long)s1;
+  }
+  __syncthreads();
+  mn0 = mn1 = LLONG_MAX;
+  mx0 = mx1 = LLONG_MIN;
+  s0 = s1 = 0;
+  for (int w = 0; w < nw; w++) {
+    mn0 = min(mn0, SM.red[0][w]);
+    mx0 = max(mx0, SM.red[1][w]);
+    mn1 = min(mn1, SM.red[2][w]);
+    mx1 = max(mx1, SM.red[3][w]);
+    s0 += (unsigned long long)SM.red[4][w];
+    s1 += (unsigned long long)SM.red[5][w];
+  }
+  // one score for all networks in a class: no JS
+  if ((mn0 == mx0 || mn1 == mx1) && !pl) return __longlong_as_double(0x7ff8000000000000ll);
+  // the sums of the scores less the smallest: exact
+  s0 -= (unsigned long long)U * (unsigned long long)mn0;
+  s1 -= (unsigned long long)U * (unsigned long long)mn1;
+  const double m0 = (double)(long long)s0 / (double)U, m1 = (double)(long long)s1 / (double)U;
+  const double sA = 10.0 / (double)(mx0 - mn0), sB = 10.0 / (double)(mx1 - mn1);
+  // equal exponents in both classes throughout (two networks ranked alike,
+  // above all): equal likelihoods, every term of the JS is log(1)
+  if (U <= 32 && !pl) {
+    bool differ = false;
+    if (tid < U)
+      differ = ((double)(dist[tid] - mn0) - m0) * sA != ((double)(dist[S + tid] - mn1) - m1) * sB;
+    if (!__syncthreads_or(differ)) return 0.0;
+  }
+  double za = 0.0, zb = 0.0;
+  for (int uu = tid; uu < U; uu += nt) {
+    const double ea = exp(((double)(dist[uu] - mn0) - m0) * sA);
+    const double eb = exp(((double)(dist[S + uu] - mn1) - m1) * sB);
+    dist[uu] = __double_as_longlong(ea);
+    dist[S + uu] = __double_as_longlong(eb);
+    za += ea;
+    zb += eb;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    if (o < lanes) {
+      za += __shfl_xor_sync(0xffffffffu, za, o);
+      zb += __shfl_xor_sync(0xffffffffu, zb, o);
+    }
+  if (lane == 0) {
+    SM.redd[0][warp] = za;
+    SM.redd[1][warp] = zb;
+  }
+  __syncthreads();
+  za = SM.redd[0][0];
+  zb = SM.redd[1][0];
+  for (int w = 1; w < nw; w++) {
+    za += SM.redd[0][w];
+    zb += SM.redd[1][w];
+  }
+  double t = 0.0;
+  for (int uu = tid; uu < U; uu += nt) {
+    const double Pu = __longlong_as_double(dist[uu]) / za;
+    const double Qu = __longlong_as_double(dist[S + uu]) / zb;
+    const double M = (Pu + Qu) / 2;
+    if (M != 0) {
+      double x = 0.0;
+      if (Pu != 0) x += 0.5 * (Pu * log(Pu / M));
+      if (Qu != 0) x += 0.5 * (Qu * log(Qu / M));
+      t += x;
+    }
+    if (pl) {
+      pl[uu] = Pu;
+      ql[uu] = Qu;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    if (o < lanes) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane == 0) SM.redd[2][warp] = t;
+  __syncthreads();
+  t = SM.redd[2][0];
+  for (int w = 1; w < nw; w++) t += SM.redd[2][w];
+  if (mn0 == mx0 || mn1 == mx1) return __longlong_as_double(0x7ff8000000000000ll);
+  return t / log(2.0);
+}
+
 // One block per unit.  A left-out sample changes only rows whose flip
 // entries it triggers, and both a network's hash and its score are sums over
 // rows, so nothing is kept per network but those sums: a lane takes one
@@ -633,7 +762,7 @@ __device__ __noinline__ void key_scores(const SetDev &sd, const UnitPtrs &P, uns
 // table of changed nodes had no room for their ~1500 distinct lists), 90410
 // units that mostly have no entry 9.3 -> 3.0 ms.  Bound by issue and latency
 // in P1 and the node scores now.
-__global__ void __launch_bounds__(256, 3) k_units(const __grid_constant__ BatchDev bd) {
+__global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
   extern __shared__ __align__(16) char smraw[];
   UnitSmem &SM = *reinterpret_cast<UnitSmem *>(smraw);
   const int nw = blockDim.x >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -664,6 +793,7 @@ __global__ void __launch_bounds__(256, 3) k_units(const __grid_constant__ BatchD
   __syncthreads();
   if (!SM.any && keep < 0) {
     if (tid == 0) {
+      bd.js[u] = __longlong_as_double(0x7ff8000000000000ll);
       bd.U[u] = 1;
       bd.status[u] = 0u;
       if (bd.stats) atomicAdd(&bd.stats[4 * (size_t)bd.uslot[u] + 3], (unsigned long long)(S - 1));
@@ -1206,11 +1336,11 @@ __global__ void __launch_bounds__(256, 3) k_units(const __grid_constant__ BatchD
     }
     U = running;
     __syncthreads();
-    // exact check of every hash merge, a warp per merged network: in one
-    // class, the rows' triggered entries agree, or else their lists do; in
+    // exact check of every hash merge, a lane per merged network: in one
+    // class the rows' triggered entries agree, or else their lists do; in
     // two, the lists of all nodes
     const int nver = SM.nver;
-    for (int wi = warp; wi < nver; wi += nw) {
+    for (int wi = tid; wi < nver; wi += nt) {
       const int s = wl[wi], r = vrep[wi];
       int ks, ss, kr, sr;
       net_of(s, sd, sig, ks, ss);
@@ -1222,30 +1352,35 @@ __global__ void __launch_bounds__(256, 3) k_units(const __grid_constant__ BatchD
       if (ks == kr && ss >= 0 && sr >= 0) {
         const uint32_t *ca = sd.codes + (ss >> 4), *cb = sd.codes + (sr >> 4);
         const int ha = 2 * (ss & 15), hb = 2 * (sr & 15), n16 = sd.n16;
-        for (int t = lane; ok && t < g; t += 32) {
-          const int i = ks * g + t, e0 = P.phs[i], e1 = P.phe[i];
-          if (e0 >= e1) continue;
-          const uint32_t a = 4u * ((ca[(size_t)t * n16] >> ha) & 3u);
-          const uint32_t b = 4u * ((cb[(size_t)t * n16] >> hb) & 3u);
-          bool same = true;
-          for (int e = e0; same && e < e1; e++) {
-            const uint2 en = ent[e];
-            const uint32_t x = (ca[(size_t)(en.x & 511u) * n16] >> ha) & 3u;
-            const uint32_t y = (cb[(size_t)(en.x & 511u) * n16] >> hb) & 3u;
-            same = (((en.y >> (a + x)) ^ (en.y >> (b + y))) & 1u) == 0u;
-          }
-          if (!same) ok = lists_equal(sd, P, ent, t, ks, ss, kr, sr);
+        auto agree = [&](uint2 en) {
+          const uint32_t t = (en.x >> 9) & 511u, j = en.x & 511u;
+          const uint32_t a = 4u * ((ca[t * n16] >> ha) & 3u) + ((ca[j * n16] >> ha) & 3u);
+          const uint32_t b = 4u * ((cb[t * n16] >> hb) & 3u) + ((cb[j * n16] >> hb) & 3u);
+          return (((en.y >> a) ^ (en.y >> b)) & 1u) == 0u;
+        };
+        auto row = [&](int t) { return lists_equal(sd, P, ent, t, ks, ss, kr, sr); };
+        // the class's memo entries in a flat walk (a row that disagrees is
+        // compared once: the walk goes on behind it), then the other rows
+        const int e1 = ks ? nmemo : SM.split[0];
+        for (int e = ks ? SM.split[0] : 0; ok && e < e1; e++) {
+          const uint2 en = ent[e];
+          if (agree(en)) continue;
+          const int t = (en.x >> 9) & 511;
+          ok = row(t);
+          e = P.phe[ks * g + t] - 1;
         }
+        for (int q = 0; ok && q < SM.nbig[ks]; q++) ok = row(P.big[ks * g + q]);
       } else if (ks != kr && ss < 0 && sr < 0) {
         ok = SM.ndab == 0;  // the two full networks
       } else {
-        for (int t = lane; ok && t < g; t += 32) ok = lists_equal(sd, P, ent, t, ks, ss, kr, sr);
+        for (int t = 0; ok && t < g; t++) ok = lists_equal(sd, P, ent, t, ks, ss, kr, sr);
       }
       if (!ok) atomicOr(&SM.status, kUnitHashCollision);
     }
     __syncthreads();
   }
   if (tid == 0) {
+    bd.js[u] = __longlong_as_double(0x7ff8000000000000ll);
     bd.U[u] = SM.status ? -1 : U;
     bd.status[u] = SM.status;
     if (bd.stats) atomicAdd(&bd.stats[4 * (size_t)bd.uslot[u] + 3], (unsigned long long)(S - U));
@@ -1419,10 +1554,9 @@ __global__ void __launch_bounds__(256, 3) k_units(const __grid_constant__ BatchD
     }
   }
 
-  // ---- P6: detailed outputs of kept units (the normalisation and JS
-  // follow in k_js from the fixed-point scores in dist)
+  __syncthreads();
+  // ---- P6: detailed outputs of kept units
   if (keep >= 0) {
-    __syncthreads();
     const int mpk = bd.mpk;
     const double fx = ldexp(1.0, -sd.lg_shift);
     for (int uu = tid; uu < U; uu += nt) {
@@ -1453,213 +1587,14 @@ __global__ void __launch_bounds__(256, 3) k_units(const __grid_constant__ BatchD
         bd.out_cnt[((size_t)keep * S + uu) * bd.keep_g + t] = cnt;
       }
     }
+    __syncthreads();
   }
-}
 
-// Normalisation (main.cu:1302-1404) and JS (main.cu:1406-1428) of every
-// unit of a batch from the node-summed fixed-point scores k_units left in
-// the unit's scratch: per class min, max and mean of the scores,
-// likelihoods exp((d - mean) 10 / (max - min)) normalised to sum 1, then the
-// two KL terms of kool() (routines.cu:42-60), zeros skipped, in FP64.  A
-// unit k_units gave up on (U < 0) is left as it is.
-//
-// One warp per upw <= 32 units.  Lane l < upw holds unit upw w + l's
-// minimum, maximum and mean (an exact integer sum); the warp then walks the
-// units' unique networks as one flattened list, 32 at a time, so that every
-// lane runs an FP64 exponential or logarithm whatever the units' sizes
-// (units have ~8 unique networks, and FP64 is slow on this part: one warp
-// per unit leaves three lanes in four idle).  upw is chosen so that the
-// grid still covers the GPU (one unit per warp for small batches).  A
-// unit's sums are formed in a fixed order: a segmented tree sum within each
-// 32-network pass, the passes added in turn.  Between the two passes a
-// network's exponentials replace its scores in the unit's dist array (the
-// scores are not read after this kernel).
-constexpr int kJsWarps = 8;
-__global__ void __launch_bounds__(32 * kJsWarps) k_js(const __grid_constant__ BatchDev bd, int upw) {
-  __shared__ int pre[kJsWarps][33];
-  __shared__ double acc[kJsWarps][3][32];
-  __shared__ long long red[kJsWarps][6][32];  // per unit: min, max (class 1, 2), sums
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int u0 = (blockIdx.x * kJsWarps + warp) * upw, u = u0 + lane;
-  const bool mine = lane < upw && u < bd.B;
-  const int Ur = mine ? bd.U[u] : 0;
-  const int keep = (Ur > 0 && bd.keep_slot) ? bd.keep_slot[u] : -1;
-  // one network: no JS, and no likelihoods unless they are kept
-  const int U = Ur > 1 || (Ur == 1 && keep >= 0) ? Ur : 0;
-  const int S = bd.sets[0].sd.S;  // n + 2, the same for every set of a batch
-  // this lane's unit's scores (its set's slice of the scratch), shared with
-  // the warp through shuffles
-  unsigned long long dptr = 0ull;
-  if (mine) {
-    const BatchSet &bs = bd.sets[bd.uslot[u]];
-    const UnitLayout L = unit_layout(bs.sd.c, S);
-    dptr = (unsigned long long)(bd.scratch + bs.sc0 + (size_t)(u - bs.u0) * bs.unit_bytes + L.dist);
-  }
-  auto dist_of = [&](int o) {
-    return (long long *)__shfl_sync(0xffffffffu, dptr, o);
-  };
-  // the warp's units as prefix intervals of the flattened list
-  int incl = U;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
-  }
-  pre[warp][lane] = incl - U;
-  if (lane == 31) pre[warp][32] = incl;
-  acc[warp][0][lane] = acc[warp][1][lane] = acc[warp][2][lane] = 0.0;
-  red[warp][0][lane] = red[warp][2][lane] = LLONG_MAX;
-  red[warp][1][lane] = red[warp][3][lane] = LLONG_MIN;
-  red[warp][4][lane] = red[warp][5][lane] = 0;
-  __syncwarp();
-  const int total = pre[warp][32];
-  // owner of network i: the last unit whose interval starts at or before i
-  auto owner = [&](int i) {
-    int lo = 0, hi = 31;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (pre[warp][mid] <= i) lo = mid;
-      else hi = mid - 1;
-    }
-    return lo;
-  };
-  // the run's last live lane: the one after it has another owner or is dead
-  auto run_end = [&](int o, bool live) {
-    const int on = __shfl_down_sync(0xffffffffu, o, 1);
-    const bool nlive = __shfl_down_sync(0xffffffffu, live ? 1 : 0, 1) != 0;
-    return live && (lane == 31 || on != o || !nlive);
-  };
-  // v combined (op) over this lane's run of equal owners, ending at the
-  // run's last lane
-  auto seg_scan = [&](long long v, int o, auto op) {
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const long long y = __shfl_up_sync(0xffffffffu, v, d);
-      const int oy = __shfl_up_sync(0xffffffffu, o, d);
-      if (lane >= d && oy == o) v = op(v, y);
-    }
-    return v;
-  };
-  auto mn = [](long long a, long long b) { return a < b ? a : b; };
-  auto mx = [](long long a, long long b) { return a > b ? a : b; };
-  auto ad = [](long long a, long long b) { return a + b; };
-  // pass 0: each unit's smallest and largest score per class, then the sum
-  // of the scores less the smallest (exact integers), over the flattened list
-  for (int i0 = 0; i0 < total; i0 += 32) {
-    const int i = i0 + lane;
-    const bool live = i < total;
-    const int o = live ? owner(i) : 31;
-    const long long *d = dist_of(o);
-    long long a = LLONG_MAX, b = LLONG_MAX;
-    if (live) {
-      const int uu = i - pre[warp][o];
-      a = d[uu];
-      b = d[S + uu];
-    }
-    const long long a0 = seg_scan(a, o, mn), a1 = seg_scan(live ? a : LLONG_MIN, o, mx);
-    const long long b0 = seg_scan(b, o, mn), b1 = seg_scan(live ? b : LLONG_MIN, o, mx);
-    if (run_end(o, live)) {
-      red[warp][0][o] = mn(red[warp][0][o], a0);
-      red[warp][1][o] = mx(red[warp][1][o], a1);
-      red[warp][2][o] = mn(red[warp][2][o], b0);
-      red[warp][3][o] = mx(red[warp][3][o], b1);
-    }
-    __syncwarp();
-  }
-  const long long l0 = red[warp][0][lane], h0 = red[warp][1][lane];
-  const long long l1 = red[warp][2][lane], h1 = red[warp][3][lane];
-  for (int i0 = 0; i0 < total; i0 += 32) {
-    const int i = i0 + lane;
-    const bool live = i < total;
-    const int o = live ? owner(i) : 31;
-    const long long *d = dist_of(o);
-    const long long ol0 = __shfl_sync(0xffffffffu, l0, o), ol1 = __shfl_sync(0xffffffffu, l1, o);
-    long long a = 0, b = 0;
-    if (live) {
-      const int uu = i - pre[warp][o];
-      a = d[uu] - ol0;
-      b = d[S + uu] - ol1;
-    }
-    const long long qa = seg_scan(a, o, ad), qb = seg_scan(b, o, ad);
-    if (run_end(o, live)) {
-      red[warp][4][o] += qa;
-      red[warp][5][o] += qb;
-    }
-    __syncwarp();
-  }
-  double m0 = 0.0, m1 = 0.0, sA = 0.0, sB = 0.0;
-  if (U > 0) {
-    m0 = (double)red[warp][4][lane] / (double)U;
-    m1 = (double)red[warp][5][lane] / (double)U;
-    sA = 10.0 / (double)(h0 - l0);
-    sB = 10.0 / (double)(h1 - l1);
-  }
-  // sum of v over this lane's run of equal owners, added to dst[owner] by
-  // the run's last live lane
-  auto seg_add = [&](double v, int o, bool live, double *dst) {
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const double y = __shfl_up_sync(0xffffffffu, v, d);
-      const int oy = __shfl_up_sync(0xffffffffu, o, d);
-      if (lane >= d && oy == o) v += y;
-    }
-    const int on = __shfl_down_sync(0xffffffffu, o, 1);
-    const bool nlive = __shfl_down_sync(0xffffffffu, live ? 1 : 0, 1) != 0;
-    if (live && (lane == 31 || on != o || !nlive)) dst[o] += v;
-  };
-  // pass 1: the likelihoods, summed per unit and class
-  for (int i0 = 0; i0 < total; i0 += 32) {
-    const int i = i0 + lane;
-    const bool live = i < total;
-    const int o = live ? owner(i) : 31;
-    const long long ol0 = __shfl_sync(0xffffffffu, l0, o), ol1 = __shfl_sync(0xffffffffu, l1, o);
-    const double om0 = __shfl_sync(0xffffffffu, m0, o), om1 = __shfl_sync(0xffffffffu, m1, o);
-    const double osA = __shfl_sync(0xffffffffu, sA, o), osB = __shfl_sync(0xffffffffu, sB, o);
-    long long *d = dist_of(o);
-    double ea = 0.0, eb = 0.0;
-    if (live) {
-      const int uu = i - pre[warp][o];
-      ea = exp(((double)(d[uu] - ol0) - om0) * osA);
-      eb = exp(((double)(d[S + uu] - ol1) - om1) * osB);
-      d[uu] = __double_as_longlong(ea);
-      d[S + uu] = __double_as_longlong(eb);
-    }
-    seg_add(ea, o, live, acc[warp][0]);
-    seg_add(eb, o, live, acc[warp][1]);
-  }
-  __syncwarp();
-  // pass 2: the normalised likelihoods and the two KL terms
-  for (int i0 = 0; i0 < total; i0 += 32) {
-    const int i = i0 + lane;
-    const bool live = i < total;
-    const int o = live ? owner(i) : 31;
-    const int okeep = __shfl_sync(0xffffffffu, keep, o);
-    const long long *d = dist_of(o);
-    double t = 0.0;
-    if (live) {
-      const int uu = i - pre[warp][o];
-      const double Pu = __longlong_as_double(d[uu]) / acc[warp][0][o];
-      const double Qu = __longlong_as_double(d[S + uu]) / acc[warp][1][o];
-      const double M = (Pu + Qu) / 2;
-      if (M != 0) {
-        if (Pu != 0) t += 0.5 * (Pu * log(Pu / M));
-        if (Qu != 0) t += 0.5 * (Qu * log(Qu / M));
-      }
-      if (okeep >= 0) {
-        bd.out_lval[((size_t)okeep * 2 + 0) * S + uu] = Pu;
-        bd.out_lval[((size_t)okeep * 2 + 1) * S + uu] = Qu;
-      }
-    }
-    seg_add(t, o, live, acc[warp][2]);
-  }
-  __syncwarp();
-  if (U > 0) {
-    double js = acc[warp][2][lane] / log(2.0);
-    if (h0 == l0 || h1 == l1) js = __longlong_as_double(0x7ff8000000000000ll);
-    bd.js[u] = js;
-  } else if (mine) {
-    bd.js[u] = __longlong_as_double(0x7ff8000000000000ll);
-  }
+  // ---- P7: normalisation and JS
+  double *pl = keep >= 0 ? bd.out_lval + ((size_t)keep * 2 + 0) * S : nullptr;
+  double *ql = keep >= 0 ? bd.out_lval + ((size_t)keep * 2 + 1) * S : nullptr;
+  const double js = unit_js(dist, S, U, SM, pl, ql);
+  if (tid == 0) bd.js[u] = js;
 }
 
 // ------------------------------------------------------------ launchers
@@ -1697,32 +1632,11 @@ cudaError_t launch_pairs(const BatchSet *sets, const int32_t *uslot, const uint6
   return cudaGetLastError();
 }
 
-cudaError_t launch_units(const BatchDev &bd, int gmax, int W, cudaStream_t st, cudaEvent_t ev_mid,
-                         bool ev_external) {
-  const int threads = 256;
+cudaError_t launch_units(const BatchDev &bd, int gmax, int W, cudaStream_t st) {
   const size_t smem = unit_smem_bytes(gmax, W);
   cudaError_t e = cudaFuncSetAttribute(k_units, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k_units<<<bd.B, threads, smem, st>>>(bd);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  if (ev_mid) {
-    e = ev_external ? cudaEventRecordWithFlags(ev_mid, st, cudaEventRecordExternal)
-                    : cudaEventRecord(ev_mid, st);
-    if (e != cudaSuccess) return e;
-  }
-  // units per warp: as many as keep about eight warps per SM busy (the SM
-  // count read once, thread-safely, from the current device)
-  static const int sms = [] {
-    int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 1)
-      v = 148;
-    return v;
-  }();
-  const int upw = std::max(1, std::min(32, bd.B / (sms * kJsWarps)));
-  const int warps = (bd.B + upw - 1) / upw;
-  k_js<<<(warps + kJsWarps - 1) / kJsWarps, 32 * kJsWarps, 0, st>>>(bd, upw);
+  k_units<<<bd.B, 256, smem, st>>>(bd);
   return cudaGetLastError();
 }
 
