@@ -271,6 +271,34 @@ bool beta_pddn(const double *js, int R, double &alpha, double &beta, double &pdd
 }
 
 // ------------------------------------------------------------ BDeu table
+namespace {
+// an unevaluated sum of two doubles, |lo| <= ulp(hi) / 2
+struct Two {
+  double hi, lo;
+};
+Two two_sum(double a, double b) {
+  const double s = a + b, t = s - a;
+  return {s, (a - (s - t)) + (b - t)};
+}
+Two add(Two x, Two y) {
+  const Two s = two_sum(x.hi, y.hi);
+  return two_sum(s.hi, s.lo + x.lo + y.lo);
+}
+Two two_of(long double v) {
+  const double hi = (double)v;
+  return {hi, (double)(v - hi)};
+}
+}  // namespace
+
+// LG(D)[m] = lgamma(m + a) - lgamma(a) = sum of log(a + i) over i < m, a =
+// 4 / D, in pairs of doubles.  The first two logarithms of a divisor come
+// from logl (once per process); each further one adds log1p(1 / (a + i)) =
+// 2 atanh(z), z = 1 / (2 (a + i) + 1) = D / (8 + (2 i + 1) D), whose series
+// 2 (z + z^3 / 3 + ...) needs few terms: z is kept as a pair, the terms from
+// z^3 on, at most z^2 / 3 < 1/26 of z, in double.  The error of a sum of n
+// is below n 2^-58, under 1% of the fixed-point step at n = 1000 (2^-40).
+// lgammal, entry by entry, took 1.1 us each where long double has no
+// hardware (16 ms for a table of 1000 samples); this takes ~20 ns.
 void bdeu_table_into(int n, int64_t *lg, int &shift, int8_t dmap[82]) {
   static const int D[kDivisors] = {1, 2, 3, 4, 6, 8, 9, 12, 16, 18, 24, 27, 36, 54, 81};
   memset(dmap, -1, 82);
@@ -279,12 +307,50 @@ void bdeu_table_into(int n, int64_t *lg, int &shift, int8_t dmap[82]) {
   const double bound = 5.0 * 512.0 * (double)lgamma((double)n + 5.0) + 1.0;
   shift = (int)floor(log2(4.0e18 / bound));
   if (shift > 44) shift = 44;
-  const long double scale = ldexpl(1.0L, shift);
+  struct First {
+    Two log_a[kDivisors], log_a1[kDivisors];
+    First() {
+      for (int i = 0; i < kDivisors; i++) {
+        const long double d = logl((long double)D[i]);
+        log_a[i] = two_of(logl(4.0L) - d);
+        log_a1[i] = two_of(logl(4.0L + (long double)D[i]) - d);
+      }
+    }
+  };
+  static const First first;
+  constexpr int kTerms = 21;
+  static const struct Inv {
+    double v[kTerms];
+    Inv() {
+      for (int k = 0; k < kTerms; k++) v[k] = 1.0 / (2 * k + 3);
+    }
+  } inv;
+  const double scale = ldexp(1.0, shift);
   for (int i = 0; i < kDivisors; i++) {
-    const long double a = 4.0L / (long double)D[i];
-    const long double la = lgammal(a);
-    for (int m = 0; m <= n; m++)
-      lg[(size_t)i * (n + 1) + m] = (int64_t)llroundl((lgammal((long double)m + a) - la) * scale);
+    int64_t *out = lg + (size_t)i * (n + 1);
+    const double d = (double)D[i];
+    Two sum = {0.0, 0.0}, l = first.log_a1[i];
+    out[0] = 0;
+    for (int m = 1; m <= n; m++) {
+      // sum += log(a + m - 1)
+      if (m == 1) {
+        sum = add(sum, first.log_a[i]);
+      } else {
+        sum = add(sum, l);
+        // l = log(a + m): z from a + (m - 1)
+        const double den = 8.0 + (2.0 * (m - 1) + 1.0) * d;
+        const double z = d / den, zl = std::fma(-z, den, d) / den, z2 = z * z;
+        // terms past the last are below 2^-60 of z
+        const int last = z2 < 0x1p-12 ? 4 : z2 < 0x1p-7 ? 8 : z2 < 0x1p-4 ? 12 : kTerms - 1;
+        double t = inv.v[last];
+        for (int k = last - 1; k >= 0; k--) t = t * z2 + inv.v[k];
+        const Two p = two_sum(2.0 * z, 2.0 * (zl + z * z2 * t));
+        l = add(l, p);
+      }
+      // the sum scaled (exactly) and rounded to the nearest integer
+      const double hi = sum.hi * scale, lo = sum.lo * scale, r = nearbyint(hi);
+      out[m] = (int64_t)r + (int64_t)llround((hi - r) + lo);
+    }
   }
 }
 

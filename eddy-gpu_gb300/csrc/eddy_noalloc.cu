@@ -41,20 +41,25 @@ constexpr int kNAW = kNAMaxSamples / 64;
 
 __host__ __device__ constexpr size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// region sizes at the maximum shape
-constexpr size_t kOffVals = 0;
-constexpr size_t kOffCodes = kOffVals + al256((size_t)kNAMaxGenes * kNAMaxSamples);
+// region sizes at the maximum shape.  The regions a call uploads come first,
+// the mask, the set table, the unit's slot (0), the prior bits, the BDeu
+// table and behind it the values (as much of the two as the call has), and
+// go up in one copy from a host buffer of the same layout: a copy from
+// pageable memory costs tens of microseconds however small it is.
+constexpr size_t kOffMask = 0;
+constexpr size_t kOffSets = kOffMask + al256(8ull * kNAW);
+constexpr size_t kOffSlot = kOffSets + al256(sizeof(BatchSet));
+constexpr size_t kOffPrior = kOffSlot + 256;
+constexpr size_t kOffLg = kOffPrior + al256((size_t)kNAPairs);
+constexpr size_t off_vals(int n) { return kOffLg + al256(8ull * kDivisors * (n + 1)); }
+constexpr size_t kUploadBytes = off_vals(kNAMaxSamples) + al256((size_t)kNAMaxGenes * kNAMaxSamples);
+constexpr size_t kOffCodes = kUploadBytes;
 constexpr size_t kOffPlanes = kOffCodes + al256(4ull * kNAMaxGenes * code_words(kNAMaxSamples));
 constexpr size_t kOffValid = kOffPlanes + al256(2 * 8ull * kNAMaxGenes * 3 * kNAW);  // + word-major
 constexpr size_t kOffCtot = kOffValid + al256(8ull * kNAW);
-constexpr size_t kOffPrior = kOffCtot + al256(2ull * 9 * kNAPairs);
-constexpr size_t kOffMask = kOffPrior + al256((size_t)kNAPairs);
-constexpr size_t kOffLg = kOffMask + al256(8ull * kNAW);
-constexpr size_t kOffDmask = kOffLg + al256(8ull * kDivisors * (kNAMaxSamples + 1));
+constexpr size_t kOffDmask = kOffCtot + al256(2ull * 9 * kNAPairs);
 constexpr size_t kOffOut = kOffDmask + al256(dmask_bytes(1, kNAPairs));  // js, U, status
-constexpr size_t kOffSets = kOffOut + 256;  // the one-set table and the unit's slot (0)
-constexpr size_t kOffSlot = kOffSets + al256(sizeof(BatchSet));
-constexpr size_t kOffUnit = kOffSlot + 256;
+constexpr size_t kOffUnit = kOffOut + 256;
 
 }  // namespace
 
@@ -73,8 +78,10 @@ DevSlot g_slots[64];
 // One call at a time per process: the device array and these host staging
 // buffers are shared by every call.
 std::mutex g_call;
-int64_t g_lg_host[kDivisors * (kNAMaxSamples + 1)];
-int8_t g_vals_host[kNAMaxGenes * kNAMaxSamples];
+alignas(256) unsigned char g_upload[kUploadBytes];
+// sample count and scale of the BDeu table in g_upload (it depends on the
+// sample count alone, so calls of one count form it once)
+int g_lg_n = -1, g_lg_shift = 0;
 
 // Once per device, with that device current: the array's device address
 // and the BDeu divisor map in constant memory (the map is the same for
@@ -86,7 +93,8 @@ int setup_device(int dev, unsigned char **out) {
     if (cudaGetSymbolAddress(&p, g_noalloc) != cudaSuccess || p == nullptr) return EDDY_ERR_CUDA;
     int shift = 0;
     int8_t dmap[82];
-    bdeu_table_into(1, g_lg_host, shift, dmap);
+    int64_t two[2 * kDivisors];
+    bdeu_table_into(1, two, shift, dmap);
     if (set_divisor_map(dmap) != cudaSuccess) return EDDY_ERR_CUDA;
     g_slots[dev].ptr = (unsigned char *)p;
   }
@@ -121,19 +129,23 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
 
-  // host-side staging in fixed-size stack/static buffers (no heap)
-  uint64_t mask[kNAW];
+  // host-side staging in fixed-size static buffers (no heap)
+  uint64_t *mask = (uint64_t *)(g_upload + kOffMask);
   for (int w = 0; w < W; w++) mask[w] = 0;
   for (int s = 0; s < n; s++)
     if (labels[s] == 0) mask[s >> 6] |= 1ull << (s & 63);
-  uint8_t pbits[kNAPairs];
+  memset(g_upload + kOffSlot, 0, sizeof(int32_t));
+  uint8_t *pbits = g_upload + kOffPrior;
   for (int r = 1, p = 0; r < g; r++)
     for (int col = 0; col < r; col++, p++) pbits[p] = (prior && prior[(size_t)r * g + col] == 1) ? 1 : 0;
-  int8_t *v8 = g_vals_host;
+  int8_t *v8 = (int8_t *)(g_upload + off_vals(n));
   for (size_t i = 0; i < (size_t)g * n; i++) v8[i] = (vals[i] >= -1 && vals[i] <= 1) ? vals[i] : 2;
-  int shift = 0;
-  int8_t dmap[82];
-  bdeu_table_into(n, g_lg_host, shift, dmap);
+  if (g_lg_n != n) {
+    int8_t dmap[82];
+    g_lg_n = -1;
+    bdeu_table_into(n, (int64_t *)(g_upload + kOffLg), g_lg_shift, dmap);
+    g_lg_n = n;
+  }
   // From the first enqueue on, an error return first waits for this call's
   // work on the stream (ignoring that wait's own status): the lock must not
   // be released while copies or kernels of this call may still use the
@@ -142,18 +154,6 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
     cudaStreamSynchronize(st);
     return code;
   };
-  if (cudaMemcpyAsync(base + kOffLg, g_lg_host, 8ull * kDivisors * (n + 1), cudaMemcpyHostToDevice,
-                      st) != cudaSuccess)
-    return bail(EDDY_ERR_CUDA);
-  if (cudaMemcpyAsync(base + kOffVals, v8, (size_t)g * n, cudaMemcpyHostToDevice, st) != cudaSuccess ||
-      cudaMemcpyAsync(base + kOffMask, mask, 8ull * W, cudaMemcpyHostToDevice, st) != cudaSuccess ||
-      cudaMemcpyAsync(base + kOffPrior, pbits, (size_t)c, cudaMemcpyHostToDevice, st) != cudaSuccess)
-    return bail(EDDY_ERR_CUDA);
-  if (launch_prep((const int8_t *)(base + kOffVals), g, n, W, c, (uint64_t *)(base + kOffPlanes),
-                  (uint64_t *)(base + kOffValid), (uint16_t *)(base + kOffCtot),
-                  (uint32_t *)(base + kOffCodes), st) != cudaSuccess)
-    return bail(EDDY_ERR_CUDA);
-
   SetDev sd{};
   sd.g = g;
   sd.n = n;
@@ -171,35 +171,42 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
   sd.planes = (const uint64_t *)(base + kOffPlanes);
   sd.planesT = sd.planes + (size_t)g * 3 * W;
   sd.valid = (const uint64_t *)(base + kOffValid);
-  sd.vals = (const int8_t *)(base + kOffVals);
+  sd.vals = (const int8_t *)(base + off_vals(n));
   sd.codes = (const uint32_t *)(base + kOffCodes);
   sd.n16 = code_words(n);
   sd.ctot = (const uint16_t *)(base + kOffCtot);
   sd.prior = (const uint8_t *)(base + kOffPrior);
   sd.lg = (const int64_t *)(base + kOffLg);
   sd.lg_stride = n + 1;
-  sd.lg_shift = shift;
+  sd.lg_shift = g_lg_shift;
 
   double *d_js = (double *)(base + kOffOut);
   int32_t *d_U = (int32_t *)(base + kOffOut + 8);
   uint32_t *d_status = (uint32_t *)(base + kOffOut + 12);
   const BatchSet *d_sets = (const BatchSet *)(base + kOffSets);
   const int32_t *d_slot = (const int32_t *)(base + kOffSlot);
-  if (cudaMemsetAsync(base + kOffSlot, 0, sizeof(int32_t), st) != cudaSuccess)
-    return bail(EDDY_ERR_CUDA);
   uint64_t salt = 0x5EED5EEDull;
   for (int attempt = 0; attempt < 4; attempt++) {
     sd.salt = salt;
     // the batch's set table: this one set, its unit 0, its masks and
-    // scratch at the start of their regions (a host copy on the stack)
+    // scratch at the start of their regions
     BatchSet bs{};
     bs.sd = sd;
     bs.nb = 1;
     bs.unit_bytes = (long long)unit_scratch_bytes(c, S);
-    // decisions (the unit kernel zeroes the masks it reads, so every attempt
-    // decides again), from masks and a chunk bitmap that start at zero
-    if (cudaMemcpyAsync(base + kOffSets, &bs, sizeof bs, cudaMemcpyHostToDevice, st) != cudaSuccess ||
-        cudaMemsetAsync(base + kOffDmask, 0, dmask_bytes(1, c), st) != cudaSuccess ||
+    memcpy(g_upload + kOffSets, &bs, sizeof bs);
+    // the inputs, the first time; then decisions (the unit kernel zeroes the
+    // masks it reads, so every attempt decides again), from masks and a chunk
+    // bitmap that start at zero
+    const size_t up = attempt == 0 ? off_vals(n) + (size_t)g * n : kOffSlot;
+    if (cudaMemcpyAsync(base, g_upload, up, cudaMemcpyHostToDevice, st) != cudaSuccess)
+      return bail(EDDY_ERR_CUDA);
+    if (attempt == 0 &&
+        launch_prep((const int8_t *)(base + off_vals(n)), g, n, W, c, (uint64_t *)(base + kOffPlanes),
+                    (uint64_t *)(base + kOffValid), (uint16_t *)(base + kOffCtot),
+                    (uint32_t *)(base + kOffCodes), st) != cudaSuccess)
+      return bail(EDDY_ERR_CUDA);
+    if (cudaMemsetAsync(base + kOffDmask, 0, dmask_bytes(1, c), st) != cudaSuccess ||
         launch_pairs(d_sets, d_slot, (const uint64_t *)(base + kOffMask),
                      (uint32_t *)(base + kOffDmask), 1, W, c, nullptr, st) != cudaSuccess)
       return bail(EDDY_ERR_CUDA);
@@ -221,7 +228,7 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
     unsigned char out[16];
     if (cudaMemcpyAsync(out, base + kOffOut, 16, cudaMemcpyDeviceToHost, st) != cudaSuccess)
       return bail(EDDY_ERR_CUDA);
-    if (cudaStreamSynchronize(st) != cudaSuccess) return EDDY_ERR_CUDA;
+    if (cudaStreamSynchronize(st) != cudaSuccess) return bail(EDDY_ERR_CUDA);
     uint32_t status;
     memcpy(js, out, 8);
     memcpy(unique, out + 8, 4);
