@@ -87,7 +87,7 @@ struct DevBuf {
 
 struct SetHost {
   std::vector<int32_t> genes;
-  std::vector<uint8_t> prior;  // g*g or empty
+  std::vector<uint8_t> prior;  // bit per pair (row-major lower triangle), or empty
   std::vector<uint8_t> labels; // external labellings R x n
   int R_ext = 0;
   bool done = false;
@@ -123,9 +123,10 @@ struct eddy_ctx {
   std::vector<uint8_t> seen;
   std::vector<int> order;
   // device data: the fixed-point lgamma table, the resident sets' inputs
-  // (one arena), the unpermuted labelling's mask; per batch: masks,
+  // (one arena), the unpermuted labelling's mask, the matrix; per batch: masks,
   // decisions, per-unit scratch, results, the set table and unit slots
-  DevBuf d_lg, d_setdata, d_mask0;
+  DevBuf d_lg, d_setdata, d_mask0, d_mat;
+  bool mat_ready = false;  // d_mat holds the matrix
   DevBuf d_masks, d_dmask, d_scratch, d_js, d_U, d_status, d_keep, d_uset, d_uperm;
   DevBuf d_uslot, d_sets;
   DevBuf d_oids, d_ocnt, d_opar, d_odist, d_olval, d_orows, d_stats;
@@ -135,7 +136,7 @@ struct eddy_ctx {
   void *dmask_clean = nullptr;
   PinnedBuf h_stage;          // per-batch uploads: unit sets, permutations, slots, set table
   PinnedBuf h_res;            // per-batch results
-  PinnedBuf h_vals;           // the resident sets' values and prior bits on their way in
+  PinnedBuf h_vals;           // the resident sets' table, rows and prior bits on their way in
   int sms = 148;
   // autotuned contingency-kernel choice (layout and tile shape) per (n,
   // power of two of the pair count); tuned_variant: the last one used (-1 =
@@ -214,7 +215,7 @@ Shape shape_of(const eddy_ctx *ctx, int set_id) {
   sh.c = sh.g * (sh.g - 1) / 2;
   const char *pl = getenv("EDDY_PAIR_LAYOUT");
   bool full = true;
-  for (int v : S.genes) full = full && ctx->gene_full[v];
+  for (int v : S.genes) full = full && v < ctx->genes && ctx->gene_full[v];
   sh.core = (full && !(pl && strcmp(pl, "full") == 0)) ? 1 : 0;
   return sh;
 }
@@ -234,13 +235,14 @@ int ensure_lg(eddy_ctx *ctx) {
   return EDDY_OK;
 }
 
-// Makes the sets `ids` resident, in this slot order: their values (gene
-// rows gathered from the matrix), prior bits, state planes, sample-major
-// values and full-sample tables in one device arena, laid out array by
-// array (all sets' values, then all prior bits, ...), so that the host
-// staging goes up in two copies.  The arena is rebuilt only when the list
-// changes; the descriptors are re-derived every call (they also carry the
-// run's switches).
+// Makes the sets `ids` resident, in this slot order: their prior bits, state
+// planes, packed states and full-sample tables in one device arena.  One
+// copy takes up the preparation table, the genes' rows and the prior bits.
+// The planes are formed from the whole matrix, which goes up once per
+// eddy_load_matrix, or, while the sets hold less than half as many genes as
+// it has rows, from their own rows gathered into the same copy.  The arena is
+// rebuilt only when the list changes; the descriptors are re-derived every
+// call (they also carry the run's switches).
 int prepare_sets(eddy_ctx *ctx, const std::vector<int> &ids) {
   const int n = ctx->samples, W = ctx->W, ns = (int)ids.size();
   CK(cudaSetDevice(ctx->o.device));
@@ -249,72 +251,79 @@ int prepare_sets(eddy_ctx *ctx, const std::vector<int> &ids) {
     if (rc) return rc;
   }
   auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-  std::vector<size_t> ov(ns), opr(ns), oco(ns), opl(ns), ova(ns), oct(ns);
-  size_t o = 0;
+  std::vector<size_t> opr(ns), oco(ns), opl(ns), oct(ns);
+  size_t genes = 0, o = al(sizeof(PrepSet) * (size_t)ns);
   for (int k = 0; k < ns; k++) {
-    const int g = (int)ctx->sets[ids[k]].genes.size();
-    if (g > 512) return fail(ctx, EDDY_ERR_CAPACITY, "gene set %d has %d genes (> 512)", ids[k], g);
-    ov[k] = o;
-    o += (size_t)g * n;
+    const size_t g = ctx->sets[ids[k]].genes.size();
+    // (a matrix loaded after the set was added may have fewer rows)
+    for (int v : ctx->sets[ids[k]].genes)
+      if (v >= ctx->genes) return fail(ctx, EDDY_ERR_ARG, "gene index %d out of range", v);
+    if (g > 512) return fail(ctx, EDDY_ERR_CAPACITY, "gene set %d has %d genes (> 512)", ids[k], (int)g);
+    genes += g;
   }
-  const size_t vals_bytes = o;
-  o = al(o);
-  const size_t pr0 = o;
+  const size_t orows = o;
+  o = al(o + sizeof(int32_t) * genes);
   for (int k = 0; k < ns; k++) {
-    const int g = (int)ctx->sets[ids[k]].genes.size(), c = g * (g - 1) / 2;
+    const size_t g = ctx->sets[ids[k]].genes.size(), c = g * (g - 1) / 2;
     opr[k] = o;
-    o += (size_t)(c > 0 ? c : 1);
+    o += c > 0 ? c : 1;
   }
-  const size_t prior_bytes = o - pr0;
+  o = al(o);
+  const bool changed = ids != ctx->res_ids;
+  const bool gather = changed && !ctx->mat_ready && 2 * genes <= (size_t)ctx->genes;
+  const size_t ovals = o, upload = gather ? o + genes * (size_t)n : o;
+  // (the offsets of a list do not depend on how its rows went up)
+  o = al(o + (2 * genes <= (size_t)ctx->genes ? genes * (size_t)n : 0));
+  const size_t ovalid = o;
+  o = al(o + sizeof(uint64_t) * W);
   for (int k = 0; k < ns; k++) {
-    const int g = (int)ctx->sets[ids[k]].genes.size(), c = g * (g - 1) / 2;
-    o = al(o);
+    const size_t g = ctx->sets[ids[k]].genes.size(), c = g * (g - 1) / 2;
     oco[k] = o;
-    o += sizeof(uint32_t) * (size_t)g * code_words(n);
-    o = al(o);
+    o = al(o + sizeof(uint32_t) * g * code_words(n));
     opl[k] = o;  // planes, then their word-major copy
-    o += 2 * sizeof(uint64_t) * (size_t)g * 3 * W;
-    o = al(o);
-    ova[k] = o;
-    o += sizeof(uint64_t) * W;
-    o = al(o);
+    o = al(o + 2 * sizeof(uint64_t) * g * 3 * W);
     oct[k] = o;
-    o += sizeof(uint16_t) * 9 * (size_t)(c > 0 ? c : 1);
+    o = al(o + sizeof(uint16_t) * 9 * (c > 0 ? c : 1));
   }
-  const size_t total = al(o);
-  if (ids != ctx->res_ids) {
+  const size_t total = o;
+  if (changed) {
     ctx->res_ids.clear();
     ctx->y_ready = false;
     // (the previous batch's copies out of the staging finished at its
     // synchronisation)
-    CK(ctx->h_vals.ensure(al(vals_bytes) + prior_bytes + 16));
-    int8_t *hv = ctx->h_vals.as<int8_t>();
-    uint8_t *hp = ctx->h_vals.as<uint8_t>(al(vals_bytes));
+    CK(ctx->h_vals.ensure(upload));
+    CK(ctx->d_setdata.ensure(total));
+    uint8_t *hb = ctx->h_vals.as<uint8_t>(), *db = ctx->d_setdata.as<uint8_t>();
+    PrepSet *ps = ctx->h_vals.as<PrepSet>();
+    int32_t *rows = ctx->h_vals.as<int32_t>(orows);
+    int gene0 = 0, pblk0 = 0;
     for (int k = 0; k < ns; k++) {
       const SetHost &S = ctx->sets[ids[k]];
-      const int g = (int)S.genes.size();
-      for (int i = 0; i < g; i++)
-        memcpy(hv + ov[k] + (size_t)i * n, ctx->data.data() + (size_t)S.genes[i] * n, n);
-      uint8_t *pb = hp + (opr[k] - pr0);
-      const int c = g * (g - 1) / 2;
-      memset(pb, 0, (size_t)(c > 0 ? c : 1));
-      if (!S.prior.empty()) {
-        int p = 0;
-        for (int r = 1; r < g; r++)
-          for (int col = 0; col < r; col++, p++) pb[p] = S.prior[(size_t)r * g + col] == 1 ? 1 : 0;
-      }
+      const int g = (int)S.genes.size(), c = g * (g - 1) / 2;
+      ps[k] = PrepSet{(uint64_t *)(db + opl[k]), (uint32_t *)(db + oco[k]), (uint16_t *)(db + oct[k]),
+                      g, c, gene0, pblk0};
+      if (gather)
+        for (int i = 0; i < g; i++)
+          memcpy(hb + ovals + (size_t)(gene0 + i) * n, ctx->data.data() + (size_t)S.genes[i] * n, n);
+      else if (g)
+        memcpy(rows + gene0, S.genes.data(), sizeof(int32_t) * (size_t)g);
+      if (S.prior.empty()) memset(hb + opr[k], 0, (size_t)(c > 0 ? c : 1));
+      else memcpy(hb + opr[k], S.prior.data(), (size_t)c);
+      gene0 += g;
+      pblk0 += prep_pair_blocks(c);
     }
-    CK(ctx->d_setdata.ensure(total));
-    uint8_t *db = ctx->d_setdata.as<uint8_t>();
-    CK(cudaMemcpyAsync(db, hv, vals_bytes, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(db + pr0, hp, prior_bytes, cudaMemcpyHostToDevice, ctx->stream));
-    for (int k = 0; k < ns; k++) {
-      const int g = (int)ctx->sets[ids[k]].genes.size(), c = g * (g - 1) / 2;
-      CK(launch_prep((const int8_t *)(db + ov[k]), g, n, W, c, (uint64_t *)(db + opl[k]),
-                     (uint64_t *)(db + ova[k]), (uint16_t *)(db + oct[k]), (uint32_t *)(db + oco[k]),
-                     ctx->stream));
-      ctx->launches += 2 + (c > 0);
+    if (!gather && !ctx->mat_ready) {
+      CK(ctx->d_mat.ensure(ctx->data.size()));
+      CK(cudaMemcpyAsync(ctx->d_mat.p, ctx->data.data(), ctx->data.size(), cudaMemcpyHostToDevice,
+                         ctx->stream));
+      ctx->mat_ready = true;
     }
+    CK(cudaMemcpyAsync(db, hb, upload, cudaMemcpyHostToDevice, ctx->stream));
+    CK(launch_prep((const PrepSet *)db, ns, gene0, pblk0,
+                   gather ? (const int8_t *)(db + ovals) : ctx->d_mat.as<int8_t>(),
+                   gather ? nullptr : (const int32_t *)(db + orows), n, W, (uint64_t *)(db + ovalid),
+                   ctx->stream));
+    ctx->launches += (gene0 > 0) + (pblk0 > 0);
     ctx->res_ids = ids;
     ctx->prep_gen++;
   }
@@ -352,8 +361,7 @@ int prepare_sets(eddy_ctx *ctx, const std::vector<int> &ids) {
     sd.core = sh.core;
     sd.planes = (const uint64_t *)(db + opl[k]);
     sd.planesT = sd.planes + (size_t)sh.g * 3 * W;
-    sd.valid = (const uint64_t *)(db + ova[k]);
-    sd.vals = (const int8_t *)(db + ov[k]);
+    sd.valid = (const uint64_t *)(db + ovalid);
     sd.codes = (const uint32_t *)(db + oco[k]);
     sd.n16 = code_words(n);
     sd.ctot = (const uint16_t *)(db + oct[k]);
@@ -392,6 +400,24 @@ bool use_popc() {
 // in one pass: the tensor-core epilogue and its general path would settle
 // nothing and list ten FP64 decisions per table.
 bool use_popc(const SetDev &sd) { return use_popc() || sd.exact_all; }
+// Batches for the popcount kernel.  The contraction computes 128 rows per
+// set however few units it has, and a set's operand Y (0.6-10 KB a pair) is
+// built first; the popcount kernel's time is its units'.  Measured, units at
+// which they meet: 20 (200 genes x 1000 samples, 387 x 600), 45 (137 x 777),
+// 64 (91 x 451 with missing values, whose tables cost 2.25 times the
+// popcounts) and 400 (40 x 400) with the operand resident, about 5e6 pair
+// words a batch; 10 to 25 units a set when a batch's sets fill the GPU (500
+// sets' iteration 0: 33.9 -> 20.9 ms a sweep).  Batches of 512 units and more
+// of one set time the contraction's shapes.  EDDY_PAIRS_KERNEL=mma, a pinned
+// shape or queue keeps the contraction.
+constexpr int kFewUnits = 16;
+constexpr double kFewPairWords = 5e6;
+bool few_units(int units, int nsets, double pair_words) {
+  const char *e = getenv("EDDY_PAIRS_KERNEL");
+  if ((e && strcmp(e, "mma") == 0) || getenv("EDDY_MMA_VARIANT") || getenv("EDDY_GENERAL_QUEUE_CAP"))
+    return false;
+  return units <= kFewUnits * nsets || (units < 512 && pair_words <= kFewPairWords);
+}
 
 // Contingency-kernel choices for a batch: tile shape v % mma_variants(), in
 // the 4-cell layout when v >= mma_variants() and in the 9-cell layout
@@ -439,11 +465,13 @@ int pick_variant(eddy_ctx *ctx, const Shape &sh, int B) {
   return 3 % nv;
 }
 
-// The resident sets' Y arena in a layout (built once per resident list and
-// layout): each slot's column groups from its grp0, its genes from its gc0.
-int prepare_y(eddy_ctx *ctx, bool core) {
+// The layout of the resident sets' Y arena: each slot's column groups from
+// its grp0, its genes from its gc0.  The arena is built once per resident
+// list and layout, by build_y below.
+int layout_y(eddy_ctx *ctx, bool core) {
   if (ctx->y_ready && ctx->y_core == (core ? 1 : 0)) return EDDY_OK;
   const int ns = (int)ctx->res_sd.size();
+  ctx->y_ready = false;
   ctx->y_grp0.assign(ns, 0);
   ctx->y_gc0.assign(ns, 0);
   int G = 0, genes = 0;
@@ -455,12 +483,6 @@ int prepare_y(eddy_ctx *ctx, bool core) {
   }
   CK(ctx->d_Y.ensure(mma_y_bytes(G, genes, ctx->samples)));
   ctx->y = YArena{ctx->d_Y.as<uint8_t>(), G, genes, ctx->samples};
-  for (int k = 0; k < ns; k++) {
-    if (ctx->res_sd[k].c == 0) continue;
-    CK(launch_build_y(ctx->res_sd[k], core, ctx->y, ctx->y_grp0[k], ctx->y_gc0[k], ctx->stream));
-    ctx->launches += mma_build_launches(ctx->res_sd[k]);
-  }
-  ctx->y_ready = true;
   ctx->y_core = core ? 1 : 0;
   return EDDY_OK;
 }
@@ -512,6 +534,16 @@ int upload_table(eddy_ctx *ctx, const BatchPlan &bp, size_t off) {
   return EDDY_OK;
 }
 
+// The Y arena of the resident sets, from the uploaded set table (planned).
+int build_y(eddy_ctx *ctx, const BatchPlan &bp, bool core) {
+  if (ctx->y_ready) return EDDY_OK;
+  CK(launch_build_y(ctx->d_sets.as<BatchSet>(), (int)bp.sets.size(), core, ctx->y, ctx->W,
+                    ctx->stream));
+  ctx->launches += 1;
+  ctx->y_ready = true;
+  return EDDY_OK;
+}
+
 // Decisions of a batch: the popcount kernel, or the tensor-core path in the
 // variant picked (tuning it on this batch when it is the first of its shape
 // with >= 512 units: every choice is timed once, same results, the fastest
@@ -536,7 +568,7 @@ int launch_pairs_any(eddy_ctx *ctx, BatchPlan &bp, const uint64_t *masks, uint32
       if (rc) return rc;
     }
     CK(launch_pairs(ctx->d_sets.as<BatchSet>(), ctx->d_uslot.as<int32_t>(), masks, dmask, bp.B,
-                    ctx->W, bp.cmax, stats, ctx->stream));
+                    ctx->W, bp.gmax, stats, ctx->stream));
     CK(mark());
     ctx->launches += 1;
     return EDDY_OK;
@@ -548,13 +580,15 @@ int launch_pairs_any(eddy_ctx *ctx, BatchPlan &bp, const uint64_t *masks, uint32
   const int g_single = ns == 1 ? bp.sets[0].sd.g : 0;
   auto run = [&](int v, unsigned long long *st, cudaEvent_t evm) -> int {
     {
-      int rc = prepare_y(ctx, layout_core(v));
+      int rc = layout_y(ctx, layout_core(v));
       if (rc) return rc;
     }
     const MmaPlan mp = plan_mma(ctx, bp, v);
     CK(ctx->d_afp8.ensure(mma_a_bytes(mp, ctx->samples, layout_core(v))));
     {
       int rc = upload_table(ctx, bp, toff);
+      if (rc) return rc;
+      rc = build_y(ctx, bp, layout_core(v));
       if (rc) return rc;
     }
     CK(launch_pairs_mma(ctx->d_sets.as<BatchSet>(), ns, mp, masks, ctx->d_uslot.as<int32_t>(),
@@ -676,6 +710,11 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
     bp.fp64 = bp.fp64 && use_popc(b.sd);
   }
   const bool masks_host = jobs[units[0].job].masks_host != nullptr;
+  {
+    double words = 0;
+    for (const BatchSet &b : bp.sets) words += (b.sd.core ? 1.0 : 2.25) * b.nb * (double)b.sd.c * W;
+    popc_batch = popc_batch || few_units(Bt, ns, words);
+  }
   // kept units: unit 0 of a keeping job
   std::vector<int> kept;  // batch indices of kept units
   std::vector<int32_t> keep_slot(Bt, -1);
@@ -798,7 +837,7 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
     // the table of the tuned shape, uploaded outside the graph
     const int v = pick_variant(ctx, sh0, Bt);
     {
-      int rc = prepare_y(ctx, layout_core(v));
+      int rc = layout_y(ctx, layout_core(v));
       if (rc) return rc;
     }
     const MmaPlan mp = plan_mma(ctx, bp, v);
@@ -833,6 +872,8 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
       // graph, before its launch
       {
         int rc = upload_table(ctx, bp, o_tab);
+        if (rc) return rc;
+        rc = build_y(ctx, bp, layout_core(v));
         if (rc) return rc;
       }
       CK(cudaMemsetAsync(ctx->d_err.p, 0, sizeof(unsigned), ctx->stream));
@@ -1150,7 +1191,7 @@ int eddy_ctx_destroy(eddy_ctx *ctx) {
   if (!ctx) return EDDY_ERR_ARG;
   cudaSetDevice(ctx->o.device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-  DevBuf *bufs[] = {&ctx->d_lg, &ctx->d_setdata, &ctx->d_mask0, &ctx->d_masks, &ctx->d_dmask,
+  DevBuf *bufs[] = {&ctx->d_lg, &ctx->d_setdata, &ctx->d_mask0, &ctx->d_mat, &ctx->d_masks, &ctx->d_dmask,
                     &ctx->d_scratch, &ctx->d_js, &ctx->d_U, &ctx->d_status, &ctx->d_keep,
                     &ctx->d_uset, &ctx->d_uperm, &ctx->d_uslot, &ctx->d_sets, &ctx->d_oids,
                     &ctx->d_ocnt, &ctx->d_opar, &ctx->d_odist, &ctx->d_olval, &ctx->d_orows,
@@ -1200,6 +1241,7 @@ int eddy_load_matrix(eddy_ctx *ctx, const int8_t *data, int genes, int samples,
     ctx->gene_full[i] = bad ? 0 : 1;
   }
   ctx->labels0.assign(class_of_sample, class_of_sample + samples);
+  ctx->mat_ready = false;
   ctx->res_ids.clear();
   ctx->res_sd.clear();
   ctx->y_ready = false;
@@ -1220,7 +1262,12 @@ int eddy_add_set(eddy_ctx *ctx, const int32_t *gene_idx, int g, const uint8_t *p
   S.genes.assign(gene_idx, gene_idx + g);
   for (int v : S.genes)
     if (v < 0 || v >= ctx->genes) return fail(ctx, EDDY_ERR_ARG, "gene index %d out of range", v);
-  if (prior) S.prior.assign(prior, prior + (size_t)g * g);
+  if (prior && g > 1) {
+    S.prior.resize((size_t)g * (g - 1) / 2);
+    uint8_t *pb = S.prior.data();
+    for (int r = 1; r < g; pb += r, r++)
+      for (int col = 0; col < r; col++) pb[col] = prior[(size_t)r * g + col] == 1;
+  }
   ctx->sets.push_back(std::move(S));
   if (set_id) *set_id = (int)ctx->sets.size() - 1;
   return EDDY_OK;

@@ -44,9 +44,8 @@ struct SetDev {
   const uint64_t *planes; // [g][3][W]  bit s of plane (i, a) = (x_i(s) == a-1)
   const uint64_t *planesT; // [W][g][3] the same planes word-major (follows planes)
   const uint64_t *valid;  // [W] all-sample mask
-  const int8_t *vals;     // [g][n]  -1/0/1, 2 = any other value
-  const uint32_t *codes;  // [g][n16] states 0-3 (st_of) of the same, two bits
-                          // each, 16 samples a word
+  const uint32_t *codes;  // [g][n16] states 0-3 (st_of), two bits each, 16
+                          // samples a word
   int n16;                // code_words(n)
   const uint16_t *ctot;   // [c][9]  permutation-invariant full-sample table
   const uint8_t *prior;   // [c]     prior bit of pair p
@@ -54,6 +53,15 @@ struct SetDev {
   int lg_stride;          // n+1
   int lg_shift;           // fixed-point scale 2^lg_shift
   uint64_t salt;          // network hash salt
+};
+
+// One set of a preparation: where its arrays go, its first gene among the
+// genes of all the sets and its first block of 128 pairs among theirs.
+struct PrepSet {
+  uint64_t *planes;  // and the word-major copy behind them
+  uint32_t *codes;
+  uint16_t *ctot;
+  int g, c, gene0, pblk0;
 };
 
 // Decision masks of a batch, per set: [nb][c] u32 (class 1 in bits 0-9,

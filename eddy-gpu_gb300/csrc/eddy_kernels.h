@@ -9,15 +9,18 @@
 namespace eddy {
 size_t unit_scratch_bytes(int c, int S);
 constexpr int kMemoMax = 8;  // BatchDev::memo_max unless lowered
-cudaError_t launch_prep(const int8_t *vals, int g, int n, int W, int c, uint64_t *planes,
-                        uint64_t *valid, uint16_t *ctot, uint32_t *codes, cudaStream_t st);
+// State planes, packed states and full-sample tables of the sets of a table
+// on the device (genes and pair_blocks: of all of them).
+cudaError_t launch_prep(const PrepSet *sets, int ns, int genes, int pair_blocks, const int8_t *vals,
+                        const int32_t *rows, int n, int W, uint64_t *valid, cudaStream_t st);
+constexpr int prep_pair_blocks(int c) { return (c + 127) / 128; }
 cudaError_t launch_counter_masks(int n, int nA, int W, uint64_t seed, const int32_t *unit_set,
                                  const int32_t *unit_perm, const uint64_t *mask0, uint64_t *masks,
                                  int B, cudaStream_t st);
 // Popcount contingency and decision kernel for a batch (sets: its device
-// set table, uslot: each unit's set; cmax: the largest pair count).
+// set table, uslot: each unit's set; gmax: the largest set).
 cudaError_t launch_pairs(const BatchSet *sets, const int32_t *uslot, const uint64_t *masks,
-                         uint32_t *dmask, int B, int W, int cmax, unsigned long long *stats,
+                         uint32_t *dmask, int B, int W, int gmax, unsigned long long *stats,
                          cudaStream_t st);
 // Network, BDeu and JS kernel of a batch (gmax: the largest set).
 cudaError_t launch_units(const BatchDev &bd, int gmax, int W, cudaStream_t st);

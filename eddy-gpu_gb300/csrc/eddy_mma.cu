@@ -929,33 +929,15 @@ __device__ __forceinline__ void store_e4m3_16(uint8_t *dst, uint32_t bits) {
   memcpy(&o, v, 16);
   *reinterpret_cast<uint4 *>(dst) = o;
 }
-// samples [16 ch, 16 ch + 16) of plane(row, a) & plane(col, b)
-__device__ __forceinline__ uint32_t pair_bits16(const uint64_t *planes, int W, int row, int a,
-                                                int col, int b, int ch) {
-  const int s0 = ch * 16, w = s0 >> 6, sh = s0 & 63;
-  if (w >= W) return 0u;
-  const uint64_t x = planes[((size_t)row * 3 + a) * W + w] & planes[((size_t)col * 3 + b) * W + w];
-  return (uint32_t)(x >> sh) & 0xFFFFu;
-}
-
-// 9-cell Y: row (group*32 + q*9 + 3a + b), q < 3 = indicator over the
-// samples of pair group*3 + q having (x_row = a-1, x_col = b-1); rows 27..31
-// of each group and out-of-range pairs are zero.  A tile of any variant is
-// a run of whole groups.  Work item = one 16-sample chunk of one row.
-__device__ __forceinline__ void build_y_chunk(const uint64_t *planes, int W, int c, int n_pad,
-                                              long long idx, uint8_t *Y) {
-  const int chunks = n_pad / 16;
-  const int rr = (int)(idx / chunks), ch = (int)(idx % chunks);
-  const int grp = rr / 32, r32 = rr % 32;
-  const int q = r32 / 9, cell = r32 % 9;
-  const int p = grp * kPairsPerGroup + q;
-  uint32_t bits = 0;
-  if (r32 < kPairsPerGroup * 9 && p < c) {
-    int row, col;
-    pair_rc(p, row, col);
-    bits = pair_bits16(planes, W, row, cell / 3, col, cell % 3, ch);
+// One row of Y for a warp: the indicator over the samples of plane rows x & y
+// (null: a zero row), lanes over its 16-sample chunks.
+__device__ __forceinline__ void build_y_row(const uint64_t *x, const uint64_t *y, int W, int n_pad,
+                                            uint8_t *Y) {
+  for (int ch = threadIdx.x & 31; ch < n_pad / 16; ch += 32) {
+    const int w = ch >> 2;
+    const uint64_t v = x && w < W ? x[w] & y[w] : 0ull;
+    store_e4m3_16(Y + ch * 16, (uint32_t)(v >> (16 * (ch & 3))) & 0xFFFFu);
   }
-  store_e4m3_16(Y + (size_t)rr * n_pad + ch * 16, bits);
 }
 
 // 9-cell full-sample tables as FP32 for the epilogue: pair p -> 12 floats
@@ -996,20 +978,6 @@ __device__ __forceinline__ uint32_t core_group_entry(int k, int g) {
   return ((uint32_t)lo << 16) | (uint32_t)(8 * (k - core_groups_before(lo)));
 }
 
-// 4-cell Y: row (group*32 + 4q + 2a + b) = indicator over the samples of
-// pair q of the group having (x_row = a-1, x_col = b-1), a, b in {0, 1};
-// padding pairs are zero.
-__device__ __forceinline__ void build_y_core_chunk(const uint64_t *planes, int g, int W, int n_pad,
-                                                   long long idx, uint8_t *Y) {
-  const int chunks = n_pad / 16;
-  const int rr = (int)(idx / chunks), ch = (int)(idx % chunks);
-  const uint32_t e = core_group_entry(rr / 32, g);
-  const int row = (int)(e >> 16), col = (int)(e & 0xFFFFu) + (rr % 32) / 4;
-  uint32_t bits = 0;
-  if (row != 0xFFFF && col < row) bits = pair_bits16(planes, W, row, (rr >> 1) & 1, col, rr & 1, ch);
-  store_e4m3_16(Y + (size_t)rr * n_pad + ch * 16, bits);
-}
-
 // 4-cell full-sample tables, one group: 8 float4 of the counted cells (0, 1,
 // 3, 4 of the nine; zero for padding pairs), then the prior bits of the
 // group's pairs and three zero words (144 bytes).
@@ -1040,40 +1008,72 @@ __device__ __forceinline__ void gene_counts(const uint64_t *planes, int W, int i
   out[i] = make_float4((float)cnt[0], (float)cnt[1], (float)cnt[2], 0.f);
 }
 
-// The per-set operands in one launch of 128-thread blocks: blocks [0, b[0])
-// build Y, [b[0], b[1]) the FP32 tables and, in the 4-cell layout,
-// [b[1], b[2]) the group table and [b[2], b[3]) the genes' counts.
+__host__ __device__ inline int ngroups_of(const SetDev &sd, bool core) {
+  return core ? core_groups_before(sd.g) : (sd.c + kPairsPerGroup - 1) / kPairsPerGroup;
+}
+__host__ __device__ inline int ngroups_pad_of(const SetDev &sd, bool core) {
+  const int g = ngroups_of(sd, core);
+  return (g > 0 ? (g + kGroupPad - 1) / kGroupPad : 1) * kGroupPad;
+}
+
+// The operands of all the sets of a batch in one launch, a block per column
+// group (set k's from its grp0): the group's 32 rows of Y, its FP32 tables
+// and, in the 4-cell layout, its entry of the group table and its share of
+// the genes' counts.  9-cell rows: q*9 + 3a + b, q < 3 = pair group*3 + q with
+// (x_row = a-1, x_col = b-1), rows 27..31 zero; 4-cell rows: 4q + 2a + b, a, b
+// in {0, 1}.  A warp takes whole rows, so a row's genes are found once and
+// its stores are coalesced (found per 16 bytes, with a 64-bit division and a
+// square root each, the same 12 GB of 500 sets took 11.9 ms).
 struct SetupArgs {
-  const uint64_t *planes;
-  const uint16_t *ctot;
-  const uint8_t *prior;
-  int g, W, c, n_pad, ngroups, core;
-  int b[4];
+  const BatchSet *sets;
+  int nsets, W, n_pad, core;
   uint8_t *Y;
   float *ctf;
   uint32_t *gtab;
   float4 *gcnt;
 };
 __global__ void __launch_bounds__(128) k_setup(const __grid_constant__ SetupArgs a) {
-  const int blk = blockIdx.x;
-  if (blk < a.b[0]) {
-    const long long idx = (long long)blk * 128 + threadIdx.x;
-    if (idx >= (long long)a.ngroups * 32 * (a.n_pad / 16)) return;
-    if (a.core) build_y_core_chunk(a.planes, a.g, a.W, a.n_pad, idx, a.Y);
-    else build_y_chunk(a.planes, a.W, a.c, a.n_pad, idx, a.Y);
-  } else if (blk < a.b[1]) {
-    const int i = (blk - a.b[0]) * 128 + threadIdx.x;
+  int lo = 0, hi = a.nsets - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (a.sets[mid].grp0 <= (int)blockIdx.x) lo = mid;
+    else hi = mid - 1;
+  }
+  const BatchSet &bs = a.sets[lo];
+  const SetDev &sd = bs.sd;
+  const int grp = (int)blockIdx.x - bs.grp0, ng = ngroups_pad_of(sd, a.core != 0);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = a.W;
+  uint8_t *Y = a.Y + (size_t)blockIdx.x * 32 * a.n_pad;
+  float *ctf = a.ctf + (size_t)bs.grp0 * (kGroupCtBytes / 4);
+  const uint32_t e = a.core ? core_group_entry(grp, sd.g) : 0u;
+  for (int r = warp; r < 32; r += 4) {
+    int row = 0xFFFF, col = 0, x = 0, y = 0;
     if (a.core) {
-      if (i < a.ngroups) ctot_core_group(a.ctot, a.prior, a.g, i, a.ctf);
-    } else if (i < a.ngroups * kPairsPerGroup) {
-      ctot_f_pair(a.ctot, a.prior, a.c, i, a.ctf);
+      row = (int)(e >> 16);
+      col = (int)(e & 0xFFFFu) + r / 4;
+      x = (r >> 1) & 1;
+      y = r & 1;
+      if (col >= row) row = 0xFFFF;
+    } else {
+      const int p = grp * kPairsPerGroup + r / 9;
+      if (r < kPairsPerGroup * 9 && p < sd.c) pair_rc(p, row, col);
+      x = (r % 9) / 3;
+      y = r % 3;
     }
-  } else if (blk < a.b[2]) {
-    const int k = (blk - a.b[1]) * 128 + threadIdx.x;
-    if (k < a.ngroups) a.gtab[k] = core_group_entry(k, a.g);
-  } else if (blk < a.b[3]) {
-    const int i = (blk - a.b[2]) * 128 + threadIdx.x;
-    if (i < a.g) gene_counts(a.planes, a.W, i, a.gcnt);
+    const bool live = row != 0xFFFF;
+    build_y_row(live ? sd.planes + ((size_t)row * 3 + x) * W : nullptr,
+                sd.planes + ((size_t)col * 3 + y) * W, W, a.n_pad, Y + (size_t)r * a.n_pad);
+  }
+  if (a.core) {
+    if (threadIdx.x == 0) {
+      ctot_core_group(sd.ctot, sd.prior, sd.g, grp, ctf);
+      a.gtab[blockIdx.x] = e;
+    }
+    // genes grp, grp + ng, ...
+    if (threadIdx.x == 32)
+      for (int i = grp; i < sd.g; i += ng) gene_counts(sd.planes, W, i, a.gcnt + bs.gc0);
+  } else if (lane == 0 && warp < kPairsPerGroup) {
+    ctot_f_pair(sd.ctot, sd.prior, sd.c, grp * kPairsPerGroup + warp, ctf);
   }
 }
 
@@ -1184,14 +1184,8 @@ static bool make_map(CUtensorMap *m, void *ptr, int cols, int rows, int box_rows
            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// pair groups of a set, and that count padded for every variant
-static int ngroups_of(const SetDev &sd, bool core) {
-  return core ? core_groups_before(sd.g) : (sd.c + kPairsPerGroup - 1) / kPairsPerGroup;
-}
-int mma_ngroups_pad(const SetDev &sd, bool core) {
-  const int g = ngroups_of(sd, core);
-  return (g > 0 ? (g + kGroupPad - 1) / kGroupPad : 1) * kGroupPad;
-}
+// pair groups of a set, padded for every variant
+int mma_ngroups_pad(const SetDev &sd, bool core) { return ngroups_pad_of(sd, core); }
 int mma_npad(int n) { return (n + kKC - 1) / kKC * kKC; }
 // The Y arena: the operand Y (G x 32 rows of n_pad samples), the FP32
 // full-sample tables (a multiple of 128 bytes in, kGroupCtBytes per group),
@@ -1275,36 +1269,22 @@ MmaPlan mma_plan(BatchSet *sets, int nsets, int variant, bool core) {
   return p;
 }
 
-cudaError_t launch_build_y(const SetDev &sd, bool core, const YArena &y, int grp0, int gc0,
+cudaError_t launch_build_y(const BatchSet *sets, int nsets, bool core, const YArena &y, int W,
                            cudaStream_t st) {
-  const int ng = mma_ngroups_pad(sd, core), np = mma_npad(sd.n);
-  const long long work = (long long)ng * 32 * (np / 16);
+  if (y.G <= 0) return cudaSuccess;
   SetupArgs a{};
-  a.planes = sd.planes;
-  a.ctot = sd.ctot;
-  a.prior = sd.prior;
-  a.g = sd.g;
-  a.W = sd.W;
-  a.c = sd.c;
-  a.n_pad = np;
-  a.ngroups = ng;
+  a.sets = sets;
+  a.nsets = nsets;
+  a.W = W;
+  a.n_pad = mma_npad(y.n);
   a.core = core ? 1 : 0;
-  a.Y = y.base + (size_t)grp0 * 32 * np;
-  a.ctf = reinterpret_cast<float *>(y.base + y_ct_offset(y)) + (size_t)grp0 * (kGroupCtBytes / 4);
-  a.b[0] = (int)((work + 127) / 128);
-  a.b[1] = a.b[0] + (core ? (ng + 127) / 128 : (ng * kPairsPerGroup + 127) / 128);
-  a.b[2] = a.b[1];
-  a.b[3] = a.b[1];
-  if (core) {
-    a.gtab = reinterpret_cast<uint32_t *>(y.base + y_gt_offset(y)) + grp0;
-    a.gcnt = reinterpret_cast<float4 *>(y.base + y_gc_offset(y)) + gc0;
-    a.b[2] = a.b[1] + (ng + 127) / 128;
-    a.b[3] = a.b[2] + (sd.g + 127) / 128;
-  }
-  k_setup<<<a.b[3], 128, 0, st>>>(a);
+  a.Y = y.base;
+  a.ctf = reinterpret_cast<float *>(y.base + y_ct_offset(y));
+  a.gtab = reinterpret_cast<uint32_t *>(y.base + y_gt_offset(y));
+  a.gcnt = reinterpret_cast<float4 *>(y.base + y_gc_offset(y));
+  k_setup<<<y.G, 128, 0, st>>>(a);
   return cudaGetLastError();
 }
-int mma_build_launches(const SetDev &) { return 1; }
 
 template <int kStages, int kEpi, int kGroups, bool kCore>
 static cudaError_t launch_variant(const BatchSet *sets, int nsets, const MmaPlan &plan,

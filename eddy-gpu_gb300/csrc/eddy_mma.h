@@ -21,12 +21,13 @@ struct YArena {
   int G, genes, n;
 };
 size_t mma_y_bytes(int G, int genes, int n);
-// Builds one set's slice of the arena: its pair-cell indicator operand Y,
-// the FP32 copy of its full-sample tables the epilogue reads and (4-cell
-// layout) its group table and genes' full-sample state counts.
-cudaError_t launch_build_y(const SetDev &sd, bool core, const YArena &y, int grp0, int gc0,
+// Builds the slices of the arena of a batch's sets in one launch: their
+// pair-cell indicator operand Y, the FP32 copy of their full-sample tables the
+// epilogue reads and (4-cell layout) their group table and genes'
+// full-sample state counts.  sets: the device set table (grp0 and gc0
+// filled in).
+cudaError_t launch_build_y(const BatchSet *sets, int nsets, bool core, const YArena &y, int W,
                            cudaStream_t st);
-int mma_build_launches(const SetDev &sd);
 
 // The contingency plan of a batch for a tile shape (variant) and layout:
 // fills each set's mb0, mblocks, tile0, ntn, marg_b0 and mg0; the totals

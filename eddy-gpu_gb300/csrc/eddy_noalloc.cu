@@ -42,13 +42,14 @@ constexpr int kNAW = kNAMaxSamples / 64;
 __host__ __device__ constexpr size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // region sizes at the maximum shape.  The regions a call uploads come first,
-// the mask, the set table, the unit's slot (0), the prior bits, the BDeu
+// the mask, the set tables, the unit's slot (0), the prior bits, the BDeu
 // table and behind it the values (as much of the two as the call has), and
 // go up in one copy from a host buffer of the same layout: a copy from
 // pageable memory costs tens of microseconds however small it is.
 constexpr size_t kOffMask = 0;
 constexpr size_t kOffSets = kOffMask + al256(8ull * kNAW);
-constexpr size_t kOffSlot = kOffSets + al256(sizeof(BatchSet));
+constexpr size_t kOffPrep = kOffSets + al256(sizeof(BatchSet));
+constexpr size_t kOffSlot = kOffPrep + 256;
 constexpr size_t kOffPrior = kOffSlot + 256;
 constexpr size_t kOffLg = kOffPrior + al256((size_t)kNAPairs);
 constexpr size_t off_vals(int n) { return kOffLg + al256(8ull * kDivisors * (n + 1)); }
@@ -139,7 +140,12 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
   for (int r = 1, p = 0; r < g; r++)
     for (int col = 0; col < r; col++, p++) pbits[p] = (prior && prior[(size_t)r * g + col] == 1) ? 1 : 0;
   int8_t *v8 = (int8_t *)(g_upload + off_vals(n));
-  for (size_t i = 0; i < (size_t)g * n; i++) v8[i] = (vals[i] >= -1 && vals[i] <= 1) ? vals[i] : 2;
+  bool core = true;
+  for (size_t i = 0; i < (size_t)g * n; i++) {
+    const bool in = vals[i] >= -1 && vals[i] <= 1;
+    v8[i] = in ? vals[i] : 2;
+    core &= in;
+  }
   if (g_lg_n != n) {
     int8_t dmap[82];
     g_lg_n = -1;
@@ -165,13 +171,13 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
   sd.mp = opts->max_parents;
   sd.GW = (g + 31) / 32;
   sd.bonf = opts->bonferroni ? 1 : 0;
+  sd.core = core ? 1 : 0;
   sd.alpha_edge = opts->alpha_edge;
   sd.alpha_edge_prior = opts->alpha_edge_prior;
   sd.exact_all = compute_thresholds(sd.alpha_edge, sd.alpha_edge_prior, g, sd.bonf, sd.thr) ? 1 : 0;
   sd.planes = (const uint64_t *)(base + kOffPlanes);
   sd.planesT = sd.planes + (size_t)g * 3 * W;
   sd.valid = (const uint64_t *)(base + kOffValid);
-  sd.vals = (const int8_t *)(base + off_vals(n));
   sd.codes = (const uint32_t *)(base + kOffCodes);
   sd.n16 = code_words(n);
   sd.ctot = (const uint16_t *)(base + kOffCtot);
@@ -195,6 +201,9 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
     bs.nb = 1;
     bs.unit_bytes = (long long)unit_scratch_bytes(c, S);
     memcpy(g_upload + kOffSets, &bs, sizeof bs);
+    const PrepSet ps{(uint64_t *)(base + kOffPlanes), (uint32_t *)(base + kOffCodes),
+                     (uint16_t *)(base + kOffCtot), g, c, 0, 0};
+    memcpy(g_upload + kOffPrep, &ps, sizeof ps);
     // the inputs, the first time; then decisions (the unit kernel zeroes the
     // masks it reads, so every attempt decides again), from masks and a chunk
     // bitmap that start at zero
@@ -202,13 +211,13 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
     if (cudaMemcpyAsync(base, g_upload, up, cudaMemcpyHostToDevice, st) != cudaSuccess)
       return bail(EDDY_ERR_CUDA);
     if (attempt == 0 &&
-        launch_prep((const int8_t *)(base + off_vals(n)), g, n, W, c, (uint64_t *)(base + kOffPlanes),
-                    (uint64_t *)(base + kOffValid), (uint16_t *)(base + kOffCtot),
-                    (uint32_t *)(base + kOffCodes), st) != cudaSuccess)
+        launch_prep((const PrepSet *)(base + kOffPrep), 1, g, prep_pair_blocks(c),
+                    (const int8_t *)(base + off_vals(n)), nullptr, n, W,
+                    (uint64_t *)(base + kOffValid), st) != cudaSuccess)
       return bail(EDDY_ERR_CUDA);
     if (cudaMemsetAsync(base + kOffDmask, 0, dmask_bytes(1, c), st) != cudaSuccess ||
         launch_pairs(d_sets, d_slot, (const uint64_t *)(base + kOffMask),
-                     (uint32_t *)(base + kOffDmask), 1, W, c, nullptr, st) != cudaSuccess)
+                     (uint32_t *)(base + kOffDmask), 1, W, g, nullptr, st) != cudaSuccess)
       return bail(EDDY_ERR_CUDA);
     BatchDev bd{};
     bd.B = 1;
