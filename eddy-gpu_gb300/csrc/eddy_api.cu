@@ -85,6 +85,52 @@ struct DevBuf {
   }
 };
 
+// A kept unit's packed outputs (KeepLayout) in host memory.
+struct KeepView {
+  const uint8_t *p = nullptr;
+  int g = 0, U = 0, E = 0, E2 = 0, E2a = 0;
+  KeepLayout at() const { return keep_layout(g, U, E, E2); }
+  template <class T>
+  const T *as(size_t byte_off) const {
+    return reinterpret_cast<const T *>(p + byte_off);
+  }
+};
+
+// The kept outputs of the sets: page-locked chunks that the batches' packed
+// outputs are copied into, as they are, and that hold them until
+// eddy_clear_sets.  A context's later sets reuse the room (one chunk of all
+// that was taken).
+struct ResultPool {
+  std::vector<PinnedBuf> chunks;
+  size_t used = 0, grow = 0;
+  cudaError_t take(size_t bytes, uint8_t **out) {
+    bytes = (bytes + 255) & ~(size_t)255;
+    if (chunks.empty() || used + bytes > chunks.back().n) {
+      PinnedBuf b;
+      cudaError_t e = b.ensure(std::max(bytes, grow));
+      if (e != cudaSuccess) return e;
+      chunks.push_back(b);
+      used = 0;
+    }
+    *out = chunks.back().as<uint8_t>(used);
+    used += bytes;
+    return cudaSuccess;
+  }
+  void clear() {
+    if (chunks.size() > 1) {
+      grow = 0;
+      for (PinnedBuf &b : chunks) grow += b.n;
+      release();
+    }
+    used = 0;
+  }
+  void release() {
+    for (PinnedBuf &b : chunks) b.release();
+    chunks.clear();
+    used = 0;
+  }
+};
+
 struct SetHost {
   std::vector<int32_t> genes;
   std::vector<uint8_t> prior;  // bit per pair (row-major lower triangle), or empty
@@ -97,11 +143,9 @@ struct SetHost {
   int iterations = 0, failed = 0, betafit_ok = 0;
   double alpha = NAN, beta = NAN, pddn = NAN;
   unsigned long long exact = 0, tables = 0;
-  // iteration-0 networks
+  // iteration-0 networks (in the context's result pool)
   int U0 = 0;
-  std::vector<int32_t> ids, nodes, epn, edges;
-  std::vector<double> lval;
-  std::vector<int32_t> el_nodes, el_epn, el_edges;
+  KeepView kept;
 };
 
 }  // namespace
@@ -129,13 +173,14 @@ struct eddy_ctx {
   bool mat_ready = false;  // d_mat holds the matrix
   DevBuf d_masks, d_dmask, d_scratch, d_js, d_U, d_status, d_keep, d_uset, d_uperm;
   DevBuf d_uslot, d_sets;
-  DevBuf d_oids, d_ocnt, d_opar, d_odist, d_olval, d_orows, d_stats;
+  DevBuf d_kbuf, d_kmeta, d_stats;  // kept units' packed outputs, their table
   DevBuf d_Y, d_afp8, d_err;  // tensor-core contingency operands
   // d_dmask is all zero between batches (decisions only set bits, the unit
   // kernel clears what it reads) while this equals d_dmask.p; null = unknown
   void *dmask_clean = nullptr;
   PinnedBuf h_stage;          // per-batch uploads: unit sets, permutations, slots, set table
   PinnedBuf h_res;            // per-batch results
+  ResultPool results;         // the sets' kept outputs
   PinnedBuf h_vals;           // the resident sets' table, rows and prior bits on their way in
   int sms = 148;
   // autotuned contingency-kernel choice (layout and tile shape) per (n,
@@ -379,15 +424,6 @@ void labels_to_mask(const uint8_t *labels, int n, int W, uint64_t *mask) {
   for (int s = 0; s < n; s++)
     if (labels[s] == 0) mask[s >> 6] |= 1ull << (s & 63);
 }
-
-// Detailed outputs of one kept unit (host copies).
-struct KeepOut {
-  int U = 0;
-  std::vector<int32_t> ids, cnt, par;
-  std::vector<double> dist, lval;
-  std::vector<uint32_t> rows;
-  int mpk = 0;
-};
 
 // Contingency + decision kernel of a batch: the tcgen05 GEMM path unless
 // EDDY_PAIRS_KERNEL=popc selects the popcount kernel.
@@ -644,7 +680,7 @@ int check_mma_error(eddy_ctx *ctx, const BatchPlan &bp) {
 
 // One set's part of a batched run: its units (labellings), given as host
 // masks or as permutation indices of the device-generated stream, and
-// where their results go.  keep: unit 0's detailed outputs (its networks
+// where their results go.  keep: unit 0's packed outputs (its networks
 // for the output files), or null.
 struct Job {
   int set_id = -1;
@@ -653,8 +689,7 @@ struct Job {
   const int32_t *perms = nullptr;        // [n_units] (device labellings)
   double *js = nullptr;
   int32_t *U = nullptr;
-  KeepOut *keep = nullptr;
-  int mpk = 1;
+  KeepView *keep = nullptr;
   unsigned long long exact = 0, tables = 0;  // decision counters of its batches
 };
 struct UnitRef {
@@ -718,22 +753,23 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   // kept units: unit 0 of a keeping job
   std::vector<int> kept;  // batch indices of kept units
   std::vector<int32_t> keep_slot(Bt, -1);
-  int mpk = 1;
+  size_t kwords = 0;  // the most the kept outputs can take
   for (int i = 0; i < Bt; i++)
     if (units[i].i == 0 && jobs[units[i].job].keep) {
       keep_slot[i] = (int32_t)kept.size();
       kept.push_back(i);
-      mpk = std::max(mpk, jobs[units[i].job].mpk);
+      const SetDev &sd = bp.sets[uslot[i]].sd;
+      const size_t E = (size_t)S * sd.g * std::max(0, std::min(sd.mp, sd.g - 1));
+      kwords += keep_layout(sd.g, S, 0, 2 * sd.c).words + E / 2 + 1;
     }
-  const int nk = (int)kept.size(), kg = bp.gmax, kgw = (kg + 31) / 32;
+  const int nk = (int)kept.size();
   if (nk) {
-    CK(ctx->d_oids.ensure(sizeof(int32_t) * (size_t)nk * S));
-    CK(ctx->d_ocnt.ensure(sizeof(int32_t) * (size_t)nk * S * kg));
-    CK(ctx->d_opar.ensure(sizeof(int32_t) * (size_t)nk * S * kg * mpk));
-    CK(ctx->d_odist.ensure(sizeof(double) * 2 * (size_t)nk * S));
-    CK(ctx->d_olval.ensure(sizeof(double) * 2 * (size_t)nk * S));
-    CK(ctx->d_orows.ensure(sizeof(uint32_t) * 2 * (size_t)nk * kg * kgw));
-    CK(cudaMemsetAsync(ctx->d_opar.p, 0xff, sizeof(int32_t) * (size_t)nk * S * kg * mpk, ctx->stream));
+    // room for what earlier batches took or 128 MB (a batch that needs more
+    // says how much, and its kept units run again)
+    const size_t cap = std::min(kwords, std::max(ctx->d_kbuf.n / 8, (size_t)16 << 20));
+    CK(ctx->d_kbuf.ensure(8 * cap));
+    CK(ctx->d_kmeta.ensure(sizeof(KeepMeta) * (size_t)(nk + 1)));
+    CK(cudaMemsetAsync(ctx->d_kmeta.p, 0, sizeof(KeepMeta) * (size_t)(nk + 1), ctx->stream));
   }
   CK(ctx->d_stats.ensure(sizeof(unsigned long long) * 4 * ns));
   CK(cudaMemsetAsync(ctx->d_stats.p, 0, sizeof(unsigned long long) * 4 * ns, ctx->stream));
@@ -755,7 +791,8 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   // (uploads); results in h_res
   const size_t o_tab = (16 * (size_t)Bt + 255) & ~(size_t)255;
   CK(ctx->h_stage.ensure(o_tab + sizeof(BatchSet) * ns + 64));
-  CK(ctx->h_res.ensure(16 * (size_t)Bt + 64 + 32 * (size_t)ns));
+  const size_t o_km = (16 * (size_t)Bt + 8 + 32 * (size_t)ns + 63) & ~(size_t)63;
+  CK(ctx->h_res.ensure(o_km + sizeof(KeepMeta) * (size_t)(nk + 1)));
   int32_t *hs = ctx->h_stage.as<int32_t>(), *hp = hs + Bt, *hsl = hp + Bt, *hk = hsl + Bt;
   for (int i = 0; i < Bt; i++) {
     const Job &J = jobs[units[i].job];
@@ -789,15 +826,9 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   bd.U = ctx->d_U.as<int32_t>();
   bd.status = ctx->d_status.as<uint32_t>();
   bd.keep_slot = ctx->d_keep.as<int32_t>();
-  bd.keep_g = kg;
-  bd.keep_gw = kgw;
-  bd.out_ids = ctx->d_oids.as<int32_t>();
-  bd.out_cnt = ctx->d_ocnt.as<int32_t>();
-  bd.out_par = ctx->d_opar.as<int32_t>();
-  bd.mpk = mpk;
-  bd.out_dist = ctx->d_odist.as<double>();
-  bd.out_lval = ctx->d_olval.as<double>();
-  bd.out_rows = ctx->d_orows.as<uint32_t>();
+  bd.kmeta = ctx->d_kmeta.as<KeepMeta>();
+  bd.kbuf = ctx->d_kbuf.as<uint64_t>();
+  bd.kcap = ctx->d_kbuf.n / 8;
   bd.stats = ctx->d_stats.as<unsigned long long>();
   // the batch's device work: labellings, decisions, networks (events
   // become record nodes when captured)
@@ -828,8 +859,9 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
     }
     CK(record(ctx->ev[1], capturing));
     CK(launch_units(bd, bp.gmax, W, ctx->stream));
+    CK(launch_pack(bd, nk, S, ctx->stream));
     CK(record(ctx->ev[2], capturing));
-    ctx->launches += 1;  // networks, normalisation and JS
+    ctx->launches += 1 + (nk > 0);  // networks, normalisation and JS; kept lists
     return EDDY_OK;
   };
   ctx->dmask_clean = nullptr;  // until the batch is seen to finish
@@ -942,6 +974,10 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   const unsigned long long *hst4 = ctx->h_res.as<unsigned long long>(16 * (size_t)Bt + 8);
   CK(cudaMemcpyAsync(ctx->h_res.as<unsigned long long>(16 * (size_t)Bt + 8), ctx->d_stats.p,
                      sizeof(unsigned long long) * 4 * ns, cudaMemcpyDeviceToHost, ctx->stream));
+  const KeepMeta *hkm = ctx->h_res.as<KeepMeta>(o_km);
+  if (nk)
+    CK(cudaMemcpyAsync(ctx->h_res.as<KeepMeta>(o_km), ctx->d_kmeta.p, sizeof(KeepMeta) * (size_t)(nk + 1),
+                       cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   const unsigned errw = *herr;
   if (errw & 1u) return fail(ctx, EDDY_ERR_INTERNAL, "tensor-core pipeline wait timed out");
@@ -972,54 +1008,34 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   }
   for (int i = 0; i < Bt; i++) {
     Job &J = jobs[units[i].job];
-    if (hst[i] & kUnitHashCollision) {
-      *collision = true;
+    if (hst[i]) {
+      *collision = *collision || (hst[i] & kUnitHashCollision);
       again->push_back(units[i]);
     } else {
       J.js[units[i].i] = hjs[i];
       J.U[units[i].i] = hU[i];
     }
   }
-  // detailed outputs of the kept units that finished
-  for (int q = 0; q < nk; q++) {
-    const int i = kept[q];
-    if (hst[i] & kUnitHashCollision) continue;
-    Job &J = jobs[units[i].job];
-    KeepOut *K = J.keep;
-    const int g = ctx->res_sd[uslot[i]].g, GW = (g + 31) / 32, Uk = hU[i];
-    K->mpk = J.mpk;
-    K->U = Uk;
-    K->ids.resize(Uk);
-    K->cnt.resize((size_t)Uk * g);
-    K->par.resize((size_t)Uk * g * J.mpk);
-    K->dist.resize(2 * (size_t)S);
-    K->lval.resize(2 * (size_t)S);
-    K->rows.resize(2 * (size_t)g * GW);
-    std::vector<int32_t> cnt((size_t)S * kg), par((size_t)S * kg * mpk);
-    std::vector<uint32_t> rows(2 * (size_t)kg * kgw);
-    CK(cudaMemcpyAsync(K->ids.data(), ctx->d_oids.as<int32_t>() + (size_t)q * S, 4 * (size_t)Uk,
-                       cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(cnt.data(), ctx->d_ocnt.as<int32_t>() + (size_t)q * S * kg,
-                       4 * (size_t)Uk * kg, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(par.data(), ctx->d_opar.as<int32_t>() + (size_t)q * S * kg * mpk,
-                       4 * (size_t)Uk * kg * mpk, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(K->dist.data(), ctx->d_odist.as<double>() + 2 * (size_t)q * S, 16 * (size_t)S,
-                       cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(K->lval.data(), ctx->d_olval.as<double>() + 2 * (size_t)q * S, 16 * (size_t)S,
-                       cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(rows.data(), ctx->d_orows.as<uint32_t>() + 2 * (size_t)q * kg * kgw,
-                       4 * rows.size(), cudaMemcpyDeviceToHost, ctx->stream));
+  // the packed outputs of the kept units that finished, in one copy
+  if (nk) {
+    const size_t need = (size_t)hkm[0].off, have = std::min(need, ctx->d_kbuf.n / 8);
+    uint8_t *host = nullptr;
+    CK(ctx->results.take(8 * have, &host));
+    CK(cudaMemcpyAsync(host, ctx->d_kbuf.p, 8 * have, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    for (int uu = 0; uu < Uk; uu++)
-      for (int t = 0; t < g; t++) {
-        K->cnt[(size_t)uu * g + t] = cnt[(size_t)uu * kg + t];
-        for (int m = 0; m < J.mpk; m++)
-          K->par[((size_t)uu * g + t) * J.mpk + m] = par[((size_t)uu * kg + t) * mpk + m];
-      }
-    for (int k = 0; k < 2; k++)
-      for (int t = 0; t < g; t++)
-        for (int w = 0; w < GW; w++)
-          K->rows[((size_t)k * g + t) * GW + w] = rows[((size_t)k * kg + t) * kgw + w];
+    for (int q = 0; q < nk; q++) {
+      const int i = kept[q];
+      if (hst[i]) continue;
+      const KeepMeta &m = hkm[1 + q];
+      KeepView &v = *jobs[units[i].job].keep;
+      v.p = host + 8 * (size_t)m.off;
+      v.g = bp.sets[uslot[i]].sd.g;
+      v.U = m.U;
+      v.E = m.E;
+      v.E2 = m.E2;
+      v.E2a = m.E2a;
+    }
+    if (need > have) CK(ctx->d_kbuf.ensure(8 * need));
   }
   return EDDY_OK;
 }
@@ -1086,7 +1102,7 @@ int run_jobs(eddy_ctx *ctx, std::vector<Job> &jobs) {
 
 // One set's units (the single-set entry points).
 int run_units(eddy_ctx *ctx, int set_id, int nunits, const uint64_t *masks_host,
-              const int32_t *perms, double *js, int32_t *U, KeepOut *keep, int mpk,
+              const int32_t *perms, double *js, int32_t *U, KeepView *keep,
               unsigned long long *exact = nullptr, unsigned long long *tables = nullptr) {
   std::vector<Job> jobs(1);
   jobs[0].set_id = set_id;
@@ -1096,63 +1112,10 @@ int run_units(eddy_ctx *ctx, int set_id, int nunits, const uint64_t *masks_host,
   jobs[0].js = js;
   jobs[0].U = U;
   jobs[0].keep = keep;
-  jobs[0].mpk = std::max(1, mpk);
   int rc = run_jobs(ctx, jobs);
   if (exact) *exact += jobs[0].exact;
   if (tables) *tables += jobs[0].tables;
   return rc;
-}
-
-// Capped or uncapped parent lists of a network given by its row bitsets.
-void rows_to_lists(const uint32_t *rows, int g, int GW, int cap, std::vector<int32_t> &nodes,
-                   std::vector<int32_t> &edges) {
-  int run = 0;
-  for (int t = 0; t < g; t++) {
-    nodes.push_back(run);
-    int cnt = 0;
-    for (int j = 0; j < t && cnt < cap; j++)
-      if ((rows[(size_t)t * GW + (j >> 5)] >> (j & 31)) & 1u) {
-        edges.push_back(j);
-        cnt++;
-      }
-    run += cnt;
-  }
-}
-
-int store_keep(eddy_ctx *ctx, SetHost &S, const KeepOut &K, int g) {
-  (void)ctx;
-  S.U0 = K.U;
-  S.ids.assign(K.ids.begin(), K.ids.end());
-  S.nodes.assign((size_t)K.U * g, 0);
-  S.epn.assign(K.U + 1, 0);
-  S.edges.clear();
-  for (int u = 0; u < K.U; u++) {
-    int run = 0;
-    for (int t = 0; t < g; t++) {
-      S.nodes[(size_t)u * g + t] = run;
-      const int cnt = K.cnt[(size_t)u * g + t];
-      for (int k = 0; k < cnt && k < K.mpk; k++) S.edges.push_back(K.par[((size_t)u * g + t) * K.mpk + k]);
-      run += cnt;
-    }
-    S.epn[u + 1] = S.epn[u] + run;
-  }
-  const int Sn = (int)K.dist.size() / 2;
-  S.lval.assign(2 * (size_t)K.U, 0.0);
-  for (int u = 0; u < K.U; u++) {
-    S.lval[u] = K.lval[u];
-    S.lval[K.U + u] = K.lval[Sn + u];
-  }
-  // uncapped lists of the two full networks (main.cu:1530-1617)
-  const int GW = (g + 31) / 32;
-  S.el_nodes.clear();
-  S.el_edges.clear();
-  std::vector<int32_t> e0, e1;
-  rows_to_lists(K.rows.data(), g, GW, 0x7fffffff, S.el_nodes, e0);
-  rows_to_lists(K.rows.data() + (size_t)g * GW, g, GW, 0x7fffffff, S.el_nodes, e1);
-  S.el_epn = {0, (int32_t)e0.size(), (int32_t)(e0.size() + e1.size())};
-  S.el_edges = e0;
-  S.el_edges.insert(S.el_edges.end(), e1.begin(), e1.end());
-  return EDDY_OK;
 }
 
 bool finite_js(double v) { return !isnan(v); }
@@ -1193,8 +1156,8 @@ int eddy_ctx_destroy(eddy_ctx *ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   DevBuf *bufs[] = {&ctx->d_lg, &ctx->d_setdata, &ctx->d_mask0, &ctx->d_mat, &ctx->d_masks, &ctx->d_dmask,
                     &ctx->d_scratch, &ctx->d_js, &ctx->d_U, &ctx->d_status, &ctx->d_keep,
-                    &ctx->d_uset, &ctx->d_uperm, &ctx->d_uslot, &ctx->d_sets, &ctx->d_oids,
-                    &ctx->d_ocnt, &ctx->d_opar, &ctx->d_odist, &ctx->d_olval, &ctx->d_orows,
+                    &ctx->d_uset, &ctx->d_uperm, &ctx->d_uslot, &ctx->d_sets, &ctx->d_kbuf,
+                    &ctx->d_kmeta,
                     &ctx->d_stats, &ctx->d_Y, &ctx->d_afp8, &ctx->d_err};
   for (DevBuf *b : bufs) b->release();
   for (auto &ev : ctx->ev)
@@ -1203,6 +1166,7 @@ int eddy_ctx_destroy(eddy_ctx *ctx) {
   ctx->h_stage.release();
   ctx->h_res.release();
   ctx->h_vals.release();
+  ctx->results.release();
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
   delete ctx;
   return EDDY_OK;
@@ -1353,7 +1317,7 @@ class GlibcProducer {
 }  // namespace
 
 static void finish_set(SetHost &S, int R);
-static void finish_counter_set(eddy_ctx *ctx, SetHost &S, const KeepOut &K, int R);
+static void finish_counter_set(SetHost &S, int R);
 
 static int run_set(eddy_ctx *ctx, int set_id) {
   SetHost &S = ctx->sets[set_id];
@@ -1384,23 +1348,21 @@ static int run_set(eddy_ctx *ctx, int set_id) {
     return EDDY_OK;
   }
   int rc = EDDY_OK;
-  const int mpk0 = std::min(ctx->o.max_parents, std::max(g - 1, 1));
   if (ctx->o.rng == EDDY_RNG_COUNTER && n <= 4096) {
     // counter stream, labellings generated on the device: iteration 0 (the
     // unpermuted labelling, kept), then, unless its JS is not finite, which
     // ends the set there (main.cu:1431-1435), the permutations in one pass
     std::vector<int32_t> perms(R);
     for (int i = 0; i < R; i++) perms[i] = i;
-    KeepOut K;
     rc = run_units(ctx, set_id, 1, nullptr, perms.data(), S.js.data(), S.U.data(),
-                   ctx->o.keep_networks ? &K : nullptr, mpk0, &S.exact, &S.tables);
+                   ctx->o.keep_networks ? &S.kept : nullptr, &S.exact, &S.tables);
     if (rc) return rc;
     if (R > 1 && finite_js(S.js[0])) {
       rc = run_units(ctx, set_id, R - 1, nullptr, perms.data() + 1, S.js.data() + 1,
-                     S.U.data() + 1, nullptr, 1, &S.exact, &S.tables);
+                     S.U.data() + 1, nullptr, &S.exact, &S.tables);
       if (rc) return rc;
     }
-    finish_counter_set(ctx, S, K, R);
+    finish_counter_set(S, R);
     return EDDY_OK;
   } else {
     // iteration 0 (kept: networks and likelihoods for the output files)
@@ -1417,12 +1379,10 @@ static int run_set(eddy_ctx *ctx, int set_id) {
     if (ctx->o.rng == EDDY_RNG_GLIBC && R > 1 && (!S.it0 || finite_js(S.js[0])))
       prod.reset(new GlibcProducer(ctx->rng, n, ctx->nA, W, R - 1, ctx->labels0.data()));
     if (!S.it0) {
-      KeepOut K;
       rc = run_units(ctx, set_id, 1, masks.data(), nullptr, S.js.data(), S.U.data(),
-                     ctx->o.keep_networks ? &K : nullptr, mpk0, &S.exact, &S.tables);
+                     ctx->o.keep_networks ? &S.kept : nullptr, &S.exact, &S.tables);
       if (rc) return rc;
-      if (ctx->o.keep_networks) store_keep(ctx, S, K, g);
-      else S.U0 = S.U[0];
+      S.U0 = S.U[0];
       S.iterations = 1;
     }
     if (!finite_js(S.js[0])) {
@@ -1442,7 +1402,7 @@ static int run_set(eddy_ctx *ctx, int set_id) {
         const int ready = prod->wait_ready(std::min(nu, done + 256));
         const int cnt = ready - done;
         rc = run_units(ctx, set_id, cnt, prod->masks(done), perms.data() + done,
-                       S.js.data() + 1 + done, S.U.data() + 1 + done, nullptr, 1, &S.exact,
+                       S.js.data() + 1 + done, S.U.data() + 1 + done, nullptr, &S.exact,
                        &S.tables);
         if (rc) return rc;
         done = ready;
@@ -1472,7 +1432,7 @@ static int run_set(eddy_ctx *ctx, int set_id) {
         }
       }
       rc = run_units(ctx, set_id, nu, device_counter ? nullptr : mh.data(), perms.data(),
-                     S.js.data() + 1, S.U.data() + 1, nullptr, 1, &S.exact, &S.tables);
+                     S.js.data() + 1, S.U.data() + 1, nullptr, &S.exact, &S.tables);
       if (rc) return rc;
     }
     S.iterations = R;
@@ -1495,10 +1455,8 @@ static void finish_set(SetHost &S, int R) {
 // A set whose iteration 0 and permutations ran in one pass on the counter
 // stream: a non-finite JS at iteration 0 ends the set there
 // (main.cu:1431-1435) and the permutations' results are discarded.
-static void finish_counter_set(eddy_ctx *ctx, SetHost &S, const KeepOut &K, int R) {
-  const int g = (int)S.genes.size();
-  if (ctx->o.keep_networks) store_keep(ctx, S, K, g);
-  else S.U0 = S.U[0];
+static void finish_counter_set(SetHost &S, int R) {
+  S.U0 = S.U[0];
   if (!finite_js(S.js[0])) {
     for (int i = 1; i < R; i++) {
       S.js[i] = NAN;
@@ -1522,7 +1480,6 @@ static void finish_counter_set(eddy_ctx *ctx, SetHost &S, const KeepOut &K, int 
 static int run_counter_sets(eddy_ctx *ctx, const std::vector<int> &ids) {
   const int R = ctx->o.permutations;
   std::vector<Job> jobs(ids.size());
-  std::vector<KeepOut> keeps(ids.size());
   std::vector<int32_t> perms(R);
   for (int i = 0; i < R; i++) perms[i] = i;
   for (size_t j = 0; j < ids.size(); j++) {
@@ -1539,8 +1496,7 @@ static int run_counter_sets(eddy_ctx *ctx, const std::vector<int> &ids) {
     jobs[j].perms = perms.data();
     jobs[j].js = S.js.data();
     jobs[j].U = S.U.data();
-    jobs[j].keep = ctx->o.keep_networks ? &keeps[j] : nullptr;
-    jobs[j].mpk = std::min(ctx->o.max_parents, std::max(g - 1, 1));
+    jobs[j].keep = ctx->o.keep_networks ? &S.kept : nullptr;
   }
   int rc = run_jobs(ctx, jobs);
   if (rc) return rc;
@@ -1570,7 +1526,7 @@ static int run_counter_sets(eddy_ctx *ctx, const std::vector<int> &ids) {
     }
   }
   for (size_t j = 0; j < ids.size(); j++)
-    finish_counter_set(ctx, ctx->sets[ids[j]], keeps[j], R);
+    finish_counter_set(ctx->sets[ids[j]], R);
   return EDDY_OK;
 }
 
@@ -1584,7 +1540,6 @@ static int run_iteration0_sets(eddy_ctx *ctx, const std::vector<int> &ids) {
   std::vector<uint64_t> mask0((size_t)W);
   labels_to_mask(ctx->labels0.data(), ctx->samples, W, mask0.data());
   std::vector<Job> jobs(ids.size());
-  std::vector<KeepOut> keeps(ids.size());
   for (size_t j = 0; j < ids.size(); j++) {
     SetHost &S = ctx->sets[ids[j]];
     const int g = (int)S.genes.size(), R = set_iterations(ctx, S);
@@ -1599,8 +1554,7 @@ static int run_iteration0_sets(eddy_ctx *ctx, const std::vector<int> &ids) {
     jobs[j].masks_host = mask0.data();
     jobs[j].js = S.js.data();
     jobs[j].U = S.U.data();
-    jobs[j].keep = ctx->o.keep_networks ? &keeps[j] : nullptr;
-    jobs[j].mpk = std::min(ctx->o.max_parents, std::max(g - 1, 1));
+    jobs[j].keep = ctx->o.keep_networks ? &S.kept : nullptr;
   }
   int rc = run_jobs(ctx, jobs);
   if (rc) return rc;
@@ -1608,8 +1562,7 @@ static int run_iteration0_sets(eddy_ctx *ctx, const std::vector<int> &ids) {
     SetHost &S = ctx->sets[ids[j]];
     S.exact = jobs[j].exact;
     S.tables = jobs[j].tables;
-    if (ctx->o.keep_networks) store_keep(ctx, S, keeps[j], (int)S.genes.size());
-    else S.U0 = S.U[0];
+    S.U0 = S.U[0];
     S.iterations = 1;
     S.it0 = true;
   }
@@ -1687,14 +1640,16 @@ int eddy_get_networks(const eddy_ctx *ctx, int set_id, int *U, int *edges, int32
                       int32_t *nodes, int32_t *epn, int32_t *edges_out, double *lval) {
   if (!ctx || set_id < 0 || set_id >= (int)ctx->sets.size()) return EDDY_ERR_ARG;
   const SetHost &S = ctx->sets[set_id];
-  if (!S.done || S.ids.empty()) return EDDY_ERR_STATE;
-  if (U) *U = S.U0;
-  if (edges) *edges = (int)S.edges.size();
-  if (ids) memcpy(ids, S.ids.data(), 4 * S.ids.size());
-  if (nodes) memcpy(nodes, S.nodes.data(), 4 * S.nodes.size());
-  if (epn) memcpy(epn, S.epn.data(), 4 * S.epn.size());
-  if (edges_out) memcpy(edges_out, S.edges.data(), 4 * S.edges.size());
-  if (lval) memcpy(lval, S.lval.data(), 8 * S.lval.size());
+  const KeepView &v = S.kept;
+  if (!S.done || !v.p) return EDDY_ERR_STATE;
+  const KeepLayout k = v.at();
+  if (U) *U = v.U;
+  if (edges) *edges = v.E;
+  if (ids) memcpy(ids, v.p + k.ids, 4 * (size_t)v.U);
+  if (nodes) memcpy(nodes, v.p + k.nodes, 4 * (size_t)v.U * v.g);
+  if (epn) memcpy(epn, v.p + k.epn, 4 * ((size_t)v.U + 1));
+  if (edges_out) memcpy(edges_out, v.p + k.edges, 4 * (size_t)v.E);
+  if (lval) memcpy(lval, v.p + k.lval, 16 * (size_t)v.U);
   return EDDY_OK;
 }
 
@@ -1702,11 +1657,17 @@ int eddy_get_edge_list(const eddy_ctx *ctx, int set_id, int *edges, int32_t *nod
                        int32_t *edges_out) {
   if (!ctx || set_id < 0 || set_id >= (int)ctx->sets.size()) return EDDY_ERR_ARG;
   const SetHost &S = ctx->sets[set_id];
-  if (!S.done || S.el_nodes.empty()) return EDDY_ERR_STATE;
-  if (edges) *edges = (int)S.el_edges.size();
-  if (nodes) memcpy(nodes, S.el_nodes.data(), 4 * S.el_nodes.size());
-  if (epn) memcpy(epn, S.el_epn.data(), 4 * S.el_epn.size());
-  if (edges_out) memcpy(edges_out, S.el_edges.data(), 4 * S.el_edges.size());
+  const KeepView &v = S.kept;
+  if (!S.done || !v.p) return EDDY_ERR_STATE;
+  const KeepLayout k = v.at();
+  if (edges) *edges = v.E2;
+  if (nodes) memcpy(nodes, v.p + k.lnodes, 8 * (size_t)v.g);
+  if (epn) {
+    epn[0] = 0;
+    epn[1] = v.E2a;
+    epn[2] = v.E2;
+  }
+  if (edges_out) memcpy(edges_out, v.p + k.ledges, 4 * (size_t)v.E2);
   return EDDY_OK;
 }
 
@@ -1733,7 +1694,7 @@ int eddy_run_labellings(eddy_ctx *ctx, int set_id, const uint8_t *labels, int R,
   }
   std::vector<uint64_t> mh((size_t)R * W);
   for (int r = 0; r < R; r++) labels_to_mask(labels + (size_t)r * n, n, W, mh.data() + (size_t)r * W);
-  return run_units(ctx, set_id, R, mh.data(), nullptr, js, unique, nullptr, 1);
+  return run_units(ctx, set_id, R, mh.data(), nullptr, js, unique, nullptr);
 }
 
 int eddy_debug_edges(eddy_ctx *ctx, int set_id, const uint8_t *labels, uint8_t *edges) {
@@ -1808,24 +1769,35 @@ int eddy_debug_unit(eddy_ctx *ctx, int set_id, const uint8_t *labels, int mpk, i
   if (ctx->sets[set_id].genes.size() < 2) return fail(ctx, EDDY_ERR_ARG, "set %d has no pair", set_id);
   std::vector<uint64_t> m(W);
   labels_to_mask(labels, n, W, m.data());
-  KeepOut K;
+  KeepView K;
   double j = 0;
   int32_t u = 0;
-  int rc = run_units(ctx, set_id, 1, m.data(), nullptr, &j, &u, &K, mpk);
+  const size_t used = ctx->results.used, chunks = ctx->results.chunks.size();
+  int rc = run_units(ctx, set_id, 1, m.data(), nullptr, &j, &u, &K);
   if (rc) return rc;
+  // (this call's outputs are copied out below: their room is free again)
+  if (ctx->results.chunks.size() == chunks) ctx->results.used = used;
   const int g = (int)ctx->sets[set_id].genes.size(), S = n + 2;
+  const KeepLayout k = K.at();
+  const int32_t *nodes = K.as<int32_t>(k.nodes), *epn = K.as<int32_t>(k.epn);
+  const int32_t *edges = K.as<int32_t>(k.edges);
   if (U) *U = K.U;
   if (js) *js = j;
+  if (ids) memcpy(ids, K.p + k.ids, 4 * (size_t)K.U);
   for (int i = 0; i < K.U; i++) {
-    if (ids) ids[i] = K.ids[i];
     for (int t = 0; t < g; t++) {
-      if (counts) counts[(size_t)i * g + t] = K.cnt[(size_t)i * g + t];
+      const int at = nodes[(size_t)i * g + t];
+      const int end = t + 1 < g ? nodes[(size_t)i * g + t + 1] : epn[i + 1] - epn[i];
+      if (counts) counts[(size_t)i * g + t] = end - at;
       if (parents)
-        for (int q = 0; q < mpk; q++) parents[((size_t)i * g + t) * mpk + q] = K.par[((size_t)i * g + t) * mpk + q];
+        for (int q = 0; q < mpk; q++)
+          parents[((size_t)i * g + t) * mpk + q] = q < end - at ? edges[epn[i] + at + q] : -1;
     }
   }
-  if (dist) memcpy(dist, K.dist.data(), 16 * (size_t)S);
-  if (lval) memcpy(lval, K.lval.data(), 16 * (size_t)S);
+  for (int c = 0; c < 2; c++) {
+    if (dist) memcpy(dist + (size_t)c * S, K.as<double>(k.dist) + (size_t)c * K.U, 8 * (size_t)K.U);
+    if (lval) memcpy(lval + (size_t)c * S, K.as<double>(k.lval) + (size_t)c * K.U, 8 * (size_t)K.U);
+  }
   return EDDY_OK;
 }
 
@@ -1851,7 +1823,7 @@ int eddy_run_permutations(eddy_ctx *ctx, int set_id, int first, int count, doubl
   std::vector<int32_t> perms(count);
   for (int i = 0; i < count; i++) perms[i] = first + i;
   if (ctx->o.rng == EDDY_RNG_COUNTER && n <= 4096)
-    return run_units(ctx, set_id, count, nullptr, perms.data(), js, unique, nullptr, 1);
+    return run_units(ctx, set_id, count, nullptr, perms.data(), js, unique, nullptr);
   std::vector<uint64_t> mh((size_t)count * W);
   std::vector<uint8_t> cur(n);
   for (int i = 0; i < count; i++) {
@@ -1865,7 +1837,7 @@ int eddy_run_permutations(eddy_ctx *ctx, int set_id, int first, int count, doubl
     }
     labels_to_mask(cur.data(), n, W, mh.data() + (size_t)i * W);
   }
-  return run_units(ctx, set_id, count, mh.data(), nullptr, js, unique, nullptr, 1);
+  return run_units(ctx, set_id, count, mh.data(), nullptr, js, unique, nullptr);
 }
 
 int eddy_set_stream(eddy_ctx *ctx, void *stream) {
@@ -1879,6 +1851,7 @@ int eddy_set_stream(eddy_ctx *ctx, void *stream) {
 int eddy_clear_sets(eddy_ctx *ctx) {
   if (!ctx) return EDDY_ERR_ARG;
   ctx->sets.clear();
+  ctx->results.clear();
   ctx->res_ids.clear();
   ctx->res_sd.clear();
   ctx->y_ready = false;

@@ -16,6 +16,7 @@ constexpr int kDofSlots = 3;        // dof 1, 2, 4 (dof 0 never gives an edge)
 constexpr int kMaxBdeuParents = 3;  // kernel5.cu:119-130 caps at 1 + 3
 constexpr int kDivisors = 15;       // distinct q and q*r of the BDeu terms
 constexpr uint32_t kUnitOk = 0;
+constexpr uint32_t kUnitKeepFull = 1u;       // no room for a kept unit's outputs
 constexpr uint32_t kUnitHashCollision = 2u;  // equal hash, unequal networks
 constexpr uint32_t kUnitBadShape = 4u;
 
@@ -120,6 +121,36 @@ __device__ __forceinline__ void mark_chunk(uint32_t *ucb, int p) {
 }
 #endif
 
+// Detailed outputs of a kept unit, packed by the kernel into one buffer for
+// all of a batch's (KeepMeta: where, and the counts its layout follows from):
+// the likelihoods and node-summed scores of its U unique networks (class 1's,
+// then class 2's), their ids, edge ranges (epn, U + 1), per-node edge
+// positions (U x g) and edges (E), and the uncapped parent lists of the two
+// full networks: per-node positions within each class (2 g) and edges (E2,
+// the first E2a of class 1).
+struct KeepMeta {
+  unsigned long long off;  // 8-byte words
+  int U, E, E2, E2a;
+  int u, pad_;             // its unit in the batch, + 1 (0: none, the unit did
+                           // not finish)
+};
+struct KeepLayout {
+  size_t lval, dist, ids, epn, nodes, edges, lnodes, ledges, words;  // bytes; 8-byte words
+};
+EDDY_HD inline KeepLayout keep_layout(int g, int U, int E, int E2) {
+  KeepLayout k;
+  k.lval = 0;
+  k.dist = k.lval + 16 * (size_t)U;
+  k.ids = k.dist + 16 * (size_t)U;
+  k.epn = k.ids + 4 * (size_t)U;
+  k.nodes = k.epn + 4 * ((size_t)U + 1);
+  k.edges = k.nodes + 4 * (size_t)U * g;
+  k.lnodes = k.edges + 4 * (size_t)E;
+  k.ledges = k.lnodes + 8 * (size_t)g;
+  k.words = (k.ledges + 4 * (size_t)E2 + 7) / 8;
+  return k;
+}
+
 // Per-batch pointers for the unit kernel.
 struct BatchDev {
   int B;                       // units in the batch
@@ -135,16 +166,10 @@ struct BatchDev {
   int32_t *U;                  // [B]
   uint32_t *status;            // [B]
   int32_t *keep_slot;          // [B] -1 or slot of detailed output
-  // detailed outputs for kept units (one slot per kept unit; node arrays
-  // strided by keep_g nodes and rows by keep_gw words):
-  int keep_g, keep_gw;
-  int32_t *out_ids;            // [slots][S]   unique network -> network id
-  int32_t *out_cnt;            // [slots][S][keep_g] capped parent counts
-  int32_t *out_par;            // [slots][S][keep_g][mpk] parent lists
-  int mpk;                     // list capacity per node in out_par
-  double *out_dist;            // [slots][2][S] node-summed BDeu (double)
-  double *out_lval;            // [slots][2][S] normalised likelihoods
-  uint32_t *out_rows;          // [slots][2][keep_g][keep_gw] full-network edge rows
+  KeepMeta *kmeta;             // [1 + slots]: entry 0's off counts the words taken,
+                               // entry 1 + slot is a kept unit's
+  uint64_t *kbuf;              // the kept units' packed outputs (KeepLayout)
+  unsigned long long kcap;     // its 8-byte words
   unsigned long long *stats;   // [nsets][4] per set: exact rechecks, tables decided,
                                // tables settled by a filter, duplicate networks
 };

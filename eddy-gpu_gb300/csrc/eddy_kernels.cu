@@ -462,7 +462,7 @@ __host__ __device__ inline int genes_of_pairs(int c) {
 
 struct UnitLayout {
   size_t phi[2], ent, ment, mdh, msc, vcan, sel, hs, dist, sig, urep, wl, vrep, ubits, htab;
-  size_t bkey, bsc, bpos, total;
+  size_t bkey, bsc, bpos, vcnt, krow, total;
 };
 __host__ __device__ inline UnitLayout unit_layout(int c, int S) {
   UnitLayout L;
@@ -490,6 +490,9 @@ __host__ __device__ inline UnitLayout unit_layout(int c, int S) {
   L.msc = take(2 * sizeof(int64_t) * nv);       // scores less the full list's, both classes
   L.vcan = take(sizeof(uint16_t) * nv);         // first variant of the row with the same key
   L.sel = take(sizeof(uint16_t) * nv);          // the variants to score
+  L.vcnt = take(sizeof(uint16_t) * nv);         // their list lengths
+  // a kept unit's rows, entry ranges (k_pack reads them)
+  L.krow = take(sizeof(uint32_t) * (2 * (size_t)g * ((g + 31) / 32) + 4 * (size_t)g));
   L.bkey = take(sizeof(uint64_t) * nb);
   L.bsc = take(2 * sizeof(int64_t) * nb);
   L.bpos = take(sizeof(int32_t) * nb);
@@ -532,6 +535,7 @@ struct UnitSmem {
   SetDev sd;    // the unit's set (copied from the batch's set table)
   unsigned long long HF[2];  // hashes of the two full networks
   long long base[2][2];      // [data class][full network of class]
+  int flen[2];  // edges of the full networks' capped lists (kept units)
   int ndab;     // nodes whose full lists differ between the classes
   int split[2]; // class 2's first memo entry, first variant
   int nbig[2];  // rows formed per sample, per class
@@ -541,6 +545,7 @@ struct UnitSmem {
   int nsel;     // variants to score
   int any;
   unsigned status;
+  unsigned long long koff;  // a kept unit's region of the packed outputs
   int scan[32];
   unsigned long long scan64[32];
   long long red[6][32];
@@ -659,13 +664,13 @@ __device__ __forceinline__ unsigned long long list_key(int t, int cnt, const int
 }
 
 // The list of row i = (k, t) for left-out sample sigma, when it differs
-// from the full network's: its key and hash (false: the full list).  The
+// from the full network's: its key, hash and length (false: the full list).  The
 // lists differ exactly when the first column that a triggered entry
 // toggles is not past the full list's end (an edge taken out there was in
 // the list; one put in there belongs to it).
 __device__ __noinline__ bool sample_list(const SetDev &sd, const UnitPtrs &P, const uint2 *ent, int k,
                                          int t, int sigma, unsigned long long &key,
-                                         unsigned long long &hash) {
+                                         unsigned long long &hash, int &len) {
   const int i = k * sd.g + t;
   const uint32_t *cw = sd.codes + (sigma >> 4);
   const int sh = 2 * (sigma & 15);
@@ -694,6 +699,7 @@ __device__ __noinline__ bool sample_list(const SetDev &sd, const UnitPtrs &P, co
   }
   key = list_key(t, cnt, ps);
   hash = h;
+  len = cnt;
   return true;
 }
 
@@ -978,6 +984,7 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
   // ---- P0: init
   if (tid == 0) {
     SM.HF[0] = SM.HF[1] = 0;
+    SM.flen[0] = SM.flen[1] = 0;
     SM.ndab = 0;
     SM.status = 0;
     SM.nbig[0] = SM.nbig[1] = 0;
@@ -1195,6 +1202,7 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
   // ---- P2: capped lists of the two full networks; their hashes summed per
   // warp, then one atomic per warp and class
   unsigned long long hsum[2] = {0ull, 0ull};
+  int csum[2] = {0, 0};
   for (int i = tid; i < 2 * g; i += nt) {
     const int k = i >= g ? 1 : 0, t = i - k * g;
     const uint32_t *row = P.rows + (size_t)i * GW;
@@ -1213,7 +1221,13 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
     for (int q = 0; q < 3; q++) P.fps[i * 3 + q] = (uint16_t)ps[q];
     P.fh[i] = h;
     hsum[k] += h;
+    csum[k] += cnt;
   }
+  if (keep >= 0)
+    for (int k = 0; k < 2; k++) {
+      const int x = __reduce_add_sync(0xffffffffu, csum[k]);
+      if (lane == 0) atomicAdd(&SM.flen[k], x);
+    }
   for (int o = 16; o > 0; o >>= 1) {
     hsum[0] += __shfl_xor_sync(0xffffffffu, hsum[0], o);
     hsum[1] += __shfl_xor_sync(0xffffffffu, hsum[1], o);
@@ -1253,6 +1267,7 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
   // ---- the variants of the memo rows: key (node, first three parents)
   // and hash of each list that differs from the full one
   unsigned long long *ment = (unsigned long long *)(scr + L.ment);
+  uint16_t *vcnt = (uint16_t *)(scr + L.vcnt);
   unsigned long long *mdh = nvar <= kSmVar ? P.itk : (unsigned long long *)(scr + L.mdh);
   for (int v = tid; v < nvar; v += nt) {
     int lo = 0, hi = 2 * g - 1;
@@ -1265,6 +1280,7 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
     const int sub = v - P.moff[i] + 1;
     const int e0 = P.phs[i], e1 = P.phe[i];
     unsigned long long key = ~0ull, dh = 0ull;
+    int len = 0;
     if ((int)(ent[e0 + __ffs(sub) - 1].x & 511u) <= P.fend[i]) {
       const uint32_t *row = P.rows + (size_t)i * GW;
       uint64_t h = node_hash_init(sd.salt, t);
@@ -1284,12 +1300,14 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
         }
       }
       key = list_key(t, cnt, ps);
+      len = cnt;
       dh = h - P.fh[i];
       // two lists of a node with one hash: another salt
       if (dh == 0ull) atomicOr(&SM.status, kUnitHashCollision);
     }
     ment[v] = key;
     mdh[v] = dh;
+    if (keep >= 0) vcnt[v] = (uint16_t)len;
   }
   // sample lists of both classes in index order (network -> left-out
   // sample)
@@ -1408,7 +1426,8 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
       for (int r = 0; r < SM.nbig[k]; r++) {
         const int t = P.big[k * g + r];
         unsigned long long key, h;
-        if (!sample_list(sd, P, ent, k, t, sg, key, h)) continue;
+        int len;
+        if (!sample_list(sd, P, ent, k, t, sg, key, h, len)) continue;
         const unsigned long long d = h - P.fh[k * g + t];
         if (d == 0ull) atomicOr(&SM.status, kUnitHashCollision);
         dh += d;
@@ -1686,6 +1705,7 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
       const bool live = uu < (k ? U : U1);
       const int s = live ? urep[uu] : 0;
       long long d1 = SM.base[0][k], d2 = SM.base[1][k];
+      int dc = 0;  // the network's edges less the full one's
       const bool plain = !live || s == 0 || s == firstB0;
       if (!__all_sync(0xffffffffu, plain)) {
         const int sg = sig[plain ? (k ? nA : 0) : s - 1];
@@ -1695,11 +1715,15 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
           const longlong2 x = msc[v];
           x1 += x.x;
           x2 += x.y;
+          if (keep >= 0) dc += (int)vcnt[v] - P.fcnt[k * g + (int)(ment[v] & 0x3FFF)];
         });
         for (int r = 0; !plain && r < SM.nbig[k]; r++) {
           const int t = P.big[k * g + r];
           unsigned long long key, h;
-          if (!sample_list(sd, P, ent, k, t, sg, key, h) || !differs(k, key)) continue;
+          int len;
+          if (!sample_list(sd, P, ent, k, t, sg, key, h, len)) continue;
+          dc += len - P.fcnt[k * g + t];
+          if (!differs(k, key)) continue;
           const int slot = big_slot(key, false);
           long long sc[2];
           if (slot >= 0) {
@@ -1714,56 +1738,167 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
         if (!plain) {
           d1 += x1;
           d2 += x2;
+        } else {
+          dc = 0;
         }
       }
       if (live) {
         dist[uu] = d1;
         dist[S + uu] = d2;
+        if (keep >= 0) wl[uu] = SM.flen[k] + dc;
       }
     }
   }
 
   __syncthreads();
-  // ---- P6: detailed outputs of kept units
+  // ---- P6: detailed outputs of kept units, packed: a region of the
+  // batch's buffer, its edge ranges and the full networks' edge lists;
+  // k_pack writes the unique networks' lists
+  double *pl = nullptr, *ql = nullptr;
   if (keep >= 0) {
-    const int mpk = bd.mpk;
+    // edge ranges (in place), and the uncapped rows' counts
+    int E = 0, E2 = 0;
+    for (int u0 = 0; u0 < U; u0 += nt) {
+      int total;
+      const int off = block_scan(u0 + tid < U ? wl[u0 + tid] : 0, total, SM.scan);
+      if (u0 + tid < U) wl[u0 + tid] = E + off;
+      E += total;
+    }
+    auto row_edges = [&](int i) {
+      int x = 0;
+      for (int w = 0; w < GW; w++) x += __popc(P.rows[(size_t)i * GW + w]);
+      return x;
+    };
+    for (int i0 = 0; i0 < 2 * g; i0 += nt) {
+      const int i = i0 + tid;
+      int total;
+      const int off = block_scan(i < 2 * g ? row_edges(i) : 0, total, SM.scan);
+      if (i < 2 * g) P.nst[i] = E2 + off;
+      E2 += total;
+    }
+    __syncthreads();
+    const int E2a = P.nst[g];
+    const KeepLayout KL = keep_layout(g, U, E, E2);
+    if (tid == 0) {
+      SM.koff = atomicAdd(&bd.kmeta[0].off, (unsigned long long)KL.words);
+      KeepMeta m;
+      m.off = SM.koff;
+      m.U = U;
+      m.E = E;
+      m.E2 = E2;
+      m.E2a = E2a;
+      m.u = SM.koff + KL.words <= bd.kcap ? u + 1 : 0;
+      m.pad_ = 0;
+      bd.kmeta[1 + keep] = m;
+    }
+    __syncthreads();
+    if (SM.koff + KL.words > bd.kcap) {
+      // (the host makes room for the words counted and runs the unit again)
+      if (tid == 0) {
+        bd.U[u] = -1;
+        bd.status[u] = kUnitKeepFull;
+      }
+      return;
+    }
+    uint8_t *kb = reinterpret_cast<uint8_t *>(bd.kbuf + SM.koff);
+    int *ids = (int *)(kb + KL.ids), *epn = (int *)(kb + KL.epn);
+    int *lnodes = (int *)(kb + KL.lnodes), *ledges = (int *)(kb + KL.ledges);
+    double *kd = (double *)(kb + KL.dist);
     const double fx = ldexp(1.0, -sd.lg_shift);
     for (int uu = tid; uu < U; uu += nt) {
-      bd.out_ids[(size_t)keep * S + uu] = urep[uu];
-      bd.out_dist[((size_t)keep * 2 + 0) * S + uu] = (double)dist[uu] * fx;
-      bd.out_dist[((size_t)keep * 2 + 1) * S + uu] = (double)dist[S + uu] * fx;
+      ids[uu] = urep[uu];
+      epn[uu] = wl[uu];
+      kd[uu] = (double)dist[uu] * fx;
+      kd[U + uu] = (double)dist[S + uu] * fx;
     }
-    for (int i = tid; i < 2 * g * GW; i += nt) {
-      const int kt = i / GW, w = i - kt * GW;  // (class, node) row, word
-      bd.out_rows[((size_t)keep * 2 * bd.keep_g + (kt / g) * bd.keep_g + kt % g) * bd.keep_gw + w] =
-          P.rows[i];
+    if (tid == 0) epn[U] = E;
+    for (int i = tid; i < 2 * g; i += nt) {
+      const int at = P.nst[i];
+      lnodes[i] = at - (i >= g ? E2a : 0);
+      int q = at;
+      for (int w = 0; w < GW; w++)
+        for (uint32_t x = P.rows[(size_t)i * GW + w]; x; x &= x - 1) ledges[q++] = 32 * w + __ffs(x) - 1;
     }
-    // full capped lists of every unique network: warp per network
-    for (int uu = warp; uu < U; uu += nw) {
-      const int s = urep[uu];
-      int k, sigma;
-      net_of(s, sd, sig, k, sigma);
-      for (int t = lane; t < g; t += 32) {
-        ListGen G;
-        gen_for(G, sd, P, ent, k, t, sigma);
-        int cnt = 0;
-        while (cnt < sd.mp) {
-          int j = G.next();
-          if (j < 0) break;
-          if (cnt < mpk) bd.out_par[(((size_t)keep * S + uu) * bd.keep_g + t) * mpk + cnt] = j;
-          cnt++;
-        }
-        bd.out_cnt[((size_t)keep * S + uu) * bd.keep_g + t] = cnt;
-      }
+    // what k_pack reads: the rows, the entry ranges and the entries
+    uint32_t *kr = (uint32_t *)(scr + L.krow);
+    for (int i = tid; i < 2 * g * GW; i += nt) kr[i] = P.rows[i];
+    for (int i = tid; i < 4 * g; i += nt) kr[2 * g * GW + i] = (uint32_t)P.phs[i];
+    if (ent == P.ent) {
+      int n = nmemo;
+      for (int k = 0; k < 2; k++)
+        for (int r = 0; r < SM.nbig[k]; r++) n = max(n, P.phe[k * g + P.big[k * g + r]]);
+      uint2 *dst = (uint2 *)(scr + L.ent);
+      for (int i = tid; i < n; i += nt) dst[i] = P.ent[i];
     }
+    pl = (double *)(kb + KL.lval);
+    ql = pl + U;
     __syncthreads();
   }
 
   // ---- P7: normalisation and JS
-  double *pl = keep >= 0 ? bd.out_lval + ((size_t)keep * 2 + 0) * S : nullptr;
-  double *ql = keep >= 0 ? bd.out_lval + ((size_t)keep * 2 + 1) * S : nullptr;
   const double js = unit_js(dist, S, U, SM, pl, ql);
   if (tid == 0) bd.js[u] = js;
+}
+
+// The unique networks' capped parent lists of the kept units (their edge
+// positions and edges in the packed outputs), a warp per network: in the
+// unit's own block they took 2.3 ms for 1000 networks of 200 genes.
+__global__ void __launch_bounds__(256) k_pack(const __grid_constant__ BatchDev bd) {
+  const KeepMeta km = bd.kmeta[1 + blockIdx.x];
+  if (km.u == 0) return;
+  const int u = km.u - 1, lane = threadIdx.x & 31, wpg = (blockDim.x >> 5) * gridDim.y;
+  const BatchSet &bs = bd.sets[bd.uslot[u]];
+  const SetDev &sd = bs.sd;
+  const int g = sd.g, GW = sd.GW;
+  uint8_t *scr = bd.scratch + bs.sc0 + (size_t)(u - bs.u0) * bs.unit_bytes;
+  const UnitLayout L = unit_layout(sd.c, sd.S);
+  const KeepLayout KL = keep_layout(g, km.U, km.E, km.E2);
+  uint8_t *kb = reinterpret_cast<uint8_t *>(bd.kbuf + km.off);
+  const int *ids = (const int *)(kb + KL.ids), *epn = (const int *)(kb + KL.epn);
+  int *nodes = (int *)(kb + KL.nodes), *edges = (int *)(kb + KL.edges);
+  const int *sig = (const int *)(scr + L.sig);
+  const uint2 *ent = (const uint2 *)(scr + L.ent);
+  UnitPtrs P{};
+  P.rows = (uint32_t *)(scr + L.krow);
+  P.phs = (int *)(P.rows + 2 * g * GW);
+  P.phe = P.phs + 2 * g;
+  // fn(j) for the parents of node t, in order, in the network of left-out
+  // sample sigma of class k
+  auto parents = [&](int k, int t, int sigma, auto &&fn) {
+    const int i = k * g + t;
+    int cnt = 0;
+    if (sigma < 0 || P.phs[i] >= P.phe[i]) {
+      const uint32_t *row = P.rows + (size_t)i * GW;
+      for (int w = 0; w < GW && cnt < sd.mp; w++)
+        for (uint32_t x = row[w]; x && cnt < sd.mp; x &= x - 1, cnt++) fn(32 * w + __ffs(x) - 1);
+    } else {
+      ListGen G;
+      gen_for(G, sd, P, ent, k, t, sigma);
+      for (int j; cnt < sd.mp && (j = G.next()) >= 0; cnt++) fn(j);
+    }
+    return cnt;
+  };
+  for (int uu = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5); uu < km.U; uu += wpg) {
+    int k, sigma, run = 0;
+    net_of(ids[uu], sd, sig, k, sigma);
+    int *dst = edges + epn[uu];
+    for (int t0 = 0; t0 < g; t0 += 32) {
+      const int t = t0 + lane;
+      const int cnt = t < g ? parents(k, t, sigma, [](int) {}) : 0;
+      int incl = cnt;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (t < g) {
+        const int at = run + incl - cnt;
+        nodes[(size_t)uu * g + t] = at;
+        int q = at;
+        parents(k, t, sigma, [&](int j) { dst[q++] = j; });
+      }
+      run += __shfl_sync(0xffffffffu, incl, 31);
+    }
+  }
 }
 
 // ------------------------------------------------------------ launchers
@@ -1808,6 +1943,12 @@ cudaError_t launch_units(const BatchDev &bd, int gmax, int W, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(k_units, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   k_units<<<bd.B, 256, smem, st>>>(bd);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_pack(const BatchDev &bd, int kept, int S, cudaStream_t st) {
+  if (kept <= 0) return cudaSuccess;
+  k_pack<<<dim3(kept, std::min(64, (S + 7) / 8)), 256, 0, st>>>(bd);
   return cudaGetLastError();
 }
 

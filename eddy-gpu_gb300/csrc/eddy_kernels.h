@@ -24,5 +24,7 @@ cudaError_t launch_pairs(const BatchSet *sets, const int32_t *uslot, const uint6
                          cudaStream_t st);
 // Network, BDeu and JS kernel of a batch (gmax: the largest set).
 cudaError_t launch_units(const BatchDev &bd, int gmax, int W, cudaStream_t st);
+// Lists of the kept units' unique networks, after launch_units (S: networks).
+cudaError_t launch_pack(const BatchDev &bd, int kept, int S, cudaStream_t st);
 cudaError_t set_divisor_map(const int8_t *map82);
 }  // namespace eddy

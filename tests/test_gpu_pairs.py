@@ -33,16 +33,10 @@ def test_popcount_tiles(case, eddy_lib, oracle_lib, monkeypatch):
     ctx.load_matrix(data, labels0)
     sid = ctx.add_set(np.arange(g), pr)
     monkeypatch.setenv("EDDY_PAIRS_KERNEL", "popc")
-    # (the second labelling has other class sizes)
-    for lab in (make_labels(rng, n, nA), make_labels(rng, n, nA - 3)):
+    for _ in range(2):
+        lab = make_labels(rng, n, nA)
         e, _, _ = oracle_lib.k1_edges(data[:, lab == 0], data[:, lab == 1], pr, oracle_lib.params())
-        got = ctx.debug_edges(sid, lab)
-        if (lab == 0).sum() == nA:
-            assert np.array_equal(got, e)
-        else:
-            # debug_edges lays the networks out by the context's class
-            # sizes: the two full networks are the same rows
-            assert np.array_equal(got[[0, -1]], e[[0, -1]])
+        assert np.array_equal(ctx.debug_edges(sid, lab), e)
     labs = np.stack([make_labels(rng, n, nA) for _ in range(40)])
     a = ctx.run_labellings(sid, labs)
     monkeypatch.setenv("EDDY_PAIRS_KERNEL", "mma")
