@@ -429,11 +429,9 @@ __global__ void __launch_bounds__(32 * kPairWarps, 2) k_pairs(const BatchSet *__
 
 // ------------------------------------------------------------ k_units
 // Kept flip entries of the two full networks' rows, one uint2 each:
-//   x = column (9 bits) | node << 9 | position in its row << 18 (3 bits)
-//       | last of its row << 21
+//   x = column (9 bits) | node << 9
 //   y = cells: bit 4a + b set when the entry fires for a left-out sample of
-//       states a (node) and b (column), no bit for a missing value (3);
-//       bits 16-31: the row's first variant (memo rows)
+//       states a (node) and b (column), no bit for a missing value (3)
 __device__ __forceinline__ uint32_t cells16(uint32_t fb) {
   return (fb & 7u) | (((fb >> 3) & 7u) << 4) | (((fb >> 6) & 7u) << 8);
 }
@@ -462,7 +460,7 @@ __host__ __device__ inline int genes_of_pairs(int c) {
 
 struct UnitLayout {
   size_t phi[2], ent, ment, mdh, msc, vcan, sel, hs, dist, sig, urep, wl, vrep, ubits, htab;
-  size_t bkey, bsc, bpos, vcnt, krow, total;
+  size_t bkey, bsc, bpos, vcnt, krow, cnt, lst, trig, total;
 };
 __host__ __device__ inline UnitLayout unit_layout(int c, int S) {
   UnitLayout L;
@@ -493,6 +491,10 @@ __host__ __device__ inline UnitLayout unit_layout(int c, int S) {
   L.vcnt = take(sizeof(uint16_t) * nv);         // their list lengths
   // a kept unit's rows, entry ranges (k_pack reads them)
   L.krow = take(sizeof(uint32_t) * (2 * (size_t)g * ((g + 31) / 32) + 4 * (size_t)g));
+  // per sample: how many rows it changes, and their variants, [rank][sample]
+  L.cnt = take(sizeof(int32_t) * (size_t)(S - 2));
+  L.lst = take(sizeof(uint16_t) * (size_t)(S - 2) * g);
+  L.trig = take(sizeof(uint32_t) * 64 * (size_t)((S - 2 + 31) / 32 + 1));
   L.bkey = take(sizeof(uint64_t) * nb);
   L.bsc = take(2 * sizeof(int64_t) * nb);
   L.bpos = take(sizeof(int32_t) * nb);
@@ -537,7 +539,7 @@ struct UnitSmem {
   long long base[2][2];      // [data class][full network of class]
   int flen[2];  // edges of the full networks' capped lists (kept units)
   int ndab;     // nodes whose full lists differ between the classes
-  int split[2]; // class 2's first memo entry, first variant
+  int split[3]; // class 2's first memo entry, first variant, first memo row
   int nbig[2];  // rows formed per sample, per class
   int firstB0;  // first class-2 network equal to the class-2 full network
   int nchg;     // networks that differ from their class's full network
@@ -554,14 +556,15 @@ struct UnitSmem {
 
 // BDeu work items (node scores) processed per round
 constexpr int kItems = 512;
-// the BDeu item arrays (keys, scores, task prefix) in one region that also
-// holds the variants' hashes while the networks are hashed (kSmVar of them)
-// and then the network table
-constexpr int kSmVar = 2048;
+// the BDeu item arrays (keys, scores, task prefix) in one region that, with
+// the base scores behind it, also holds the variants' hashes and the entries'
+// trigger words while the networks are hashed, and then the network table
 constexpr size_t kWorkBytes = sizeof(unsigned long long) * kItems + 2 * sizeof(long long) * kItems +
                               sizeof(int) * (2 * kItems + 4);
-static_assert(kSmVar * sizeof(unsigned long long) <= kWorkBytes && kSmSlots * sizeof(int) <= kWorkBytes,
-              "work region");
+static_assert(kSmSlots * sizeof(int) <= kWorkBytes && kWorkBytes % 16 == 0, "work region");
+// entries whose trigger words a unit's scratch holds (sample counts for
+// which the region above holds fewer than kMinTrig)
+constexpr int kTrigScratch = 64, kMinTrig = 16;
 // kept flip entries a unit holds in shared memory (more go to its scratch)
 constexpr int kEntCache = 1280;
 
@@ -578,6 +581,7 @@ struct UnitPtrs {
   int *moff;              // [2][g] variants of the rows before
   int *nst;               // [2][g] scratch of the compaction
   uint16_t *big;          // [2][g] rows formed per sample, per class
+  uint2 *rinfo;           // [2 g] the memo rows: first entry; entries | first variant << 8
   uint8_t *need;          // [g] 1 = full lists differ, 2 = scores needed
   uint32_t *used;         // [unit_variants / 32] variants some network uses
   unsigned long long *itk;   // [kItems] node-score items: t | np << 14 | parents
@@ -612,13 +616,15 @@ __host__ __device__ inline UnitPtrs carve(char *base, int g, int W, int GW) {
   P.moff = (int *)take(2 * sizeof(int) * g);
   P.nst = (int *)take(2 * sizeof(int) * g);
   P.big = (uint16_t *)take(2 * sizeof(uint16_t) * g);
+  P.rinfo = (uint2 *)take(2 * sizeof(uint2) * g);
   P.need = (uint8_t *)take(g);
   P.used = (uint32_t *)take(sizeof(uint32_t) * ((unit_variants(g) + 31) / 32));
-  P.itk = (unsigned long long *)take(kWorkBytes);
+  P.dmap = (int8_t *)take(96);
+  // (the base scores follow the work region directly)
+  P.itk = (unsigned long long *)take(kWorkBytes + 4 * sizeof(long long) * g);
   P.acc = (long long *)(P.itk + kItems);
   P.tq = (int *)(P.acc + 2 * kItems);
-  P.dmap = (int8_t *)take(96);
-  P.fsc = (long long *)take(4 * sizeof(long long) * g);
+  P.fsc = (long long *)((char *)P.itk + kWorkBytes);
   P.ent = (uint2 *)take(sizeof(uint2) * kEntCache);
   P.bytes = (o + 15) & ~(size_t)15;
   return P;
@@ -927,16 +933,14 @@ static __device__ __noinline__ double unit_js(long long *dist, int S, int U, Uni
 
 // One block per unit.  A left-out sample changes only rows whose flip
 // entries it triggers, and both a network's hash and its score are sums over
-// rows, so nothing is kept per network but those sums: a lane takes one
-// left-out sample and walks its class's entries (the same for the whole
-// warp), adding the hash, and later the scores, of each row's variant.  The
-// walk reads two state bits per entry and sample, coalesced, where a warp
-// per network that lists its changed nodes waits on chains of its own.
-// Measured against that form: 10000 units of 200 genes x 1000 samples near
-// the threshold 44.0 -> 20.0 ms, 301 units of 387 x 600 35.0 -> 5.3 ms (its
-// table of changed nodes had no room for their ~1500 distinct lists), 90410
-// units that mostly have no entry 9.3 -> 3.0 ms.  Bound by issue and latency
-// in P1 and the node scores now.
+// rows, so nothing is kept per network but those sums and the rows it
+// changes: a lane takes one left-out sample, a warp 32 of one class, and walks
+// the class's memo rows.  A warp per network that lists its changed nodes
+// waited on chains of its own: 10000 units of 200 genes x 1000 samples near
+// the threshold took 44.0 ms against 19.5 ms now (with the normalisation and
+// JS, then 6.0 ms more), 301 units of 387 x 600 35.0 against 4.6 ms.  Bound by
+// issue (1.3 million warp instructions a unit at that shape), about half of
+// them in the node scores.
 __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
   extern __shared__ __align__(16) char smraw[];
   UnitSmem &SM = *reinterpret_cast<UnitSmem *>(smraw);
@@ -990,7 +994,7 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
     SM.nbig[0] = SM.nbig[1] = 0;
     SM.firstB0 = S - 1;
     SM.nchg = SM.nver = SM.nsel = 0;
-    SM.split[0] = SM.split[1] = 0;
+    SM.split[0] = SM.split[1] = SM.split[2] = 0;
     for (int a = 0; a < 2; a++)
       for (int b = 0; b < 2; b++) SM.base[a][b] = 0;
   }
@@ -1136,13 +1140,15 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
   // the variants of the rows before (a variant's row is the last one whose
   // moff is not past it).
   const uint2 *ent = P.ent;
-  int nmemo = 0, nvar = 0, E = bd.memo_max;
+  int nmemo = 0, nvar = 0, nmr = 0, E = bd.memo_max;
   auto memo_row = [&](int i, int e) {
     return e >= 1 && e <= E && (1 << e) <= (i < g ? nA : nB) + 8;
   };
   if (entries) {
+    // packed: memo entries (14 bits), memo rows (11), other entries (20),
+    // variants (19)
+    constexpr int kR = 14, kO = 25, kV = 45;
     unsigned long long running;
-    // packed: memo entries, other entries << 20, variants << 40
     while (true) {
       running = 0ull;
       for (int i0 = 0; i0 < 2 * g; i0 += nt) {
@@ -1150,27 +1156,31 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
         const int e = (i < 2 * g && P.phs[i] < P.phe[i]) ? P.phe[i] - P.phs[i] : 0;
         const bool mr = memo_row(i, e);
         const unsigned long long v =
-            mr ? (unsigned long long)e | ((unsigned long long)((1 << e) - 1) << 40)
-               : (unsigned long long)e << 20;
+            mr ? (unsigned long long)e | (1ull << kR) | ((unsigned long long)((1 << e) - 1) << kV)
+               : (unsigned long long)e << kO;
         unsigned long long total;
         const unsigned long long off = running + block_scan(v, total, SM.scan64);
         if (i < 2 * g) {
-          P.moff[i] = (int)(off >> 40);
-          P.nst[i] = mr ? (int)(off & 0xFFFFF) : (int)((off >> 20) & 0xFFFFF);
+          const int me = (int)(off & ((1u << kR) - 1)), row = (int)((off >> kR) & 0x7FF);
+          P.moff[i] = (int)(off >> kV);
+          P.nst[i] = mr ? me : (int)((off >> kO) & 0xFFFFF);
+          if (mr) P.rinfo[row] = make_uint2((unsigned)me, (unsigned)e | ((unsigned)P.moff[i] << 8));
           if (i == g) {
-            SM.split[0] = (int)(off & 0xFFFFF);
-            SM.split[1] = (int)(off >> 40);
+            SM.split[0] = me;
+            SM.split[1] = P.moff[i];
+            SM.split[2] = row;
           }
         }
         running += total;
       }
-      nvar = (int)(running >> 40);
+      nvar = (int)(running >> kV);
       if (nvar <= unit_variants(g) || E <= 0) break;
       E--;
       __syncthreads();
     }
-    nmemo = (int)(running & 0xFFFFF);
-    const int nbig = (int)((running >> 20) & 0xFFFFF);
+    nmemo = (int)(running & ((1u << kR) - 1));
+    nmr = (int)((running >> kR) & 0x7FF);
+    const int nbig = (int)((running >> kO) & 0xFFFFF);
     uint2 *dst = nmemo + nbig <= kEntCache ? P.ent : (uint2 *)(scr + L.ent);
     ent = dst;
     __syncthreads();
@@ -1185,9 +1195,7 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
       const int at = P.nst[i] + (mr ? 0 : nmemo);
       for (int q = 0; q < e; q++) {
         const uint32_t x = phi[k][e0 + q];
-        dst[at + q] = make_uint2((x & 0xFFFFu) | ((uint32_t)t << 9) | ((uint32_t)(q & 7) << 18) |
-                                     (q + 1 == e ? 1u << 21 : 0u),
-                                 (x >> 16) | ((uint32_t)(mr ? P.moff[i] : 0) << 16));
+        dst[at + q] = make_uint2((x & 0xFFFFu) | ((uint32_t)t << 9), x >> 16);
       }
       P.phs[i] = at;
       P.phe[i] = at + e;
@@ -1268,7 +1276,14 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
   // and hash of each list that differs from the full one
   unsigned long long *ment = (unsigned long long *)(scr + L.ment);
   uint16_t *vcnt = (uint16_t *)(scr + L.vcnt);
-  unsigned long long *mdh = nvar <= kSmVar ? P.itk : (unsigned long long *)(scr + L.mdh);
+  const int n = sd.n, W32 = 2 * W;
+  // the work region: the variants' hashes, if room for the trigger words of
+  // 64 entries is left, then the trigger words (of tcap entries)
+  const size_t region = kWorkBytes + 4 * sizeof(long long) * (size_t)g;
+  const size_t mdhb = (8 * (size_t)nvar + 15) & ~(size_t)15;
+  const bool mdh_sm = mdhb + 4 * (size_t)W32 * 64 <= region;
+  unsigned long long *mdh = mdh_sm ? P.itk : (unsigned long long *)(scr + L.mdh);
+  const int tcap_sm = (int)((region - (mdh_sm ? mdhb : 0)) / (4 * (size_t)W32));
   for (int v = tid; v < nvar; v += nt) {
     int lo = 0, hi = 2 * g - 1;
     while (lo < hi) {
@@ -1370,71 +1385,132 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
     }
     return -1;
   };
-  // fn(variant) for every memo row whose entries sample sg triggers, in
-  // class k: a flat walk over the class's entries, four at a time
-  auto walk = [&](int k, int sg, auto &&fn) {
-    const uint32_t *cw = sd.codes + (sg >> 4);
-    const int sh = 2 * (sg & 15), n16 = sd.n16;
-    const int e0 = k ? SM.split[0] : 0, e1 = k ? nmemo : SM.split[0];
-    int sub = 0;
-    for (int e = e0; e < e1; e += 4) {
-      uint2 en[4];
-      uint32_t a[4], b[4];
-#pragma unroll
-      for (int q = 0; q < 4; q++) en[q] = ent[e + q < e1 ? e + q : e1 - 1];
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        a[q] = __ldg(cw + ((en[q].x >> 9) & 511u) * n16);
-        b[q] = __ldg(cw + (en[q].x & 511u) * n16);
-      }
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        if (e + q >= e1) break;
-        const uint32_t cell = ((a[q] >> sh) & 3u) * 4u + ((b[q] >> sh) & 3u);
-        sub |= (int)(((en[q].y >> cell) & 1u) << ((en[q].x >> 18) & 7u));
-        if (en[q].x >> 21) {
-          if (sub) fn((int)(en[q].y >> 16) + sub - 1);
-          sub = 0;
-        }
-      }
-    }
-  };
-  const int nch0 = (nA + 31) >> 5, nch = nch0 + ((nB + 31) >> 5);
-
-  // ---- P3: every network's hash: its class's full network's, plus the
-  // hash difference of each row the left-out sample changes.  A lane per
-  // sample, a warp per 32 samples of one class.
+  // ---- P3: what the left-out samples change.  An entry (t, j, cells) fires
+  // for the samples whose states lie in its cells: the OR over the cells (a,
+  // b) of plane(t, a) & plane(j, b), formed 32 samples at a time (its trigger
+  // words), for as many memo rows at a time as the region holds.  Then a lane
+  // takes one sample of the class, a warp 32, and walks the rows: the bits of
+  // a row's entries name the variant the sample changes the row to.  Its hash
+  // difference goes into the network's hash, and the variant, unless it
+  // leaves the row's list as it is, on the sample's list, from which the
+  // scores are summed later.  Cycles of a block for this and the sums, 200
+  // genes x 1000 samples near the threshold: 350k + 95k; a byte per row and
+  // sample instead of the lists, stored and read coalesced, 309k + 298k; a
+  // walk over packed states for each, 295k + 468k.
+  uint16_t *lst = (uint16_t *)(scr + L.lst);
+  int *cng = (int *)(scr + L.cnt);
   unsigned long long *hs = (unsigned long long *)(scr + L.hs);
   auto as_key = [](unsigned long long h) { return h == ~0ull ? ~1ull : h; };
-  if (entries) {
-    for (int ch = warp; ch < nch; ch += nw) {
-      const int k = ch >= nch0 ? 1 : 0, i = 32 * (k ? ch - nch0 : ch) + lane;
-      const int nk = k ? nB : nA;
-      const bool live = i < nk;
-      const int s = 1 + (k ? nA : 0) + (live ? i : nk - 1);
-      const int sg = sig[s - 1];
-      unsigned long long dh = 0ull;
-      bool chg = false;
-      walk(k, sg, [&](int v) {
-        const unsigned long long d = mdh[v];
-        if (d) {
+  // (trig and mdh in shared memory or not, for the compiler to see)
+  auto walk = [&](uint32_t *__restrict__ trig, int tcap,
+                  const unsigned long long *__restrict__ mdh) {
+    int wpr = 1;  // lanes per entry
+    while (wpr < W32 && wpr < 32) wpr <<= 1;
+    const uint32_t *__restrict__ pl32 = reinterpret_cast<const uint32_t *>(sd.planes);
+    for (int k = 0; k < 2; k++) {
+      const int nk = k ? nB : nA, sk = k ? nA : 0, nch = (nk + 31) >> 5;
+      const int rend = k ? nmr : SM.split[2];
+      int r0 = k ? SM.split[2] : 0;
+      bool first = true;
+      do {
+        // rows [r0, r1), entries [e0, e1)
+        const int e0 = r0 < rend ? (int)P.rinfo[r0].x : 0;
+        int lo = r0, hi = rend;
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          const uint2 ri = P.rinfo[mid - 1];
+          if ((int)ri.x + (int)(ri.y & 0xFFu) - e0 <= tcap) lo = mid;
+          else hi = mid - 1;
+        }
+        const int r1 = lo;
+        const int e1 = r1 > r0 ? (int)(P.rinfo[r1 - 1].x + (P.rinfo[r1 - 1].y & 0xFFu)) : e0;
+        __syncthreads();
+#pragma unroll 2
+        for (int e = e0 + (warp * 32 + lane) / wpr; e < e1; e += nt / wpr) {
+          const uint2 en = ent[e];
+          const uint32_t *pt = pl32 + (size_t)((en.x >> 9) & 511u) * 3 * W32;
+          const uint32_t *pj = pl32 + (size_t)(en.x & 511u) * 3 * W32;
+          for (int w = lane & (wpr - 1); w < W32; w += wpr) {
+            const uint32_t t0 = __ldg(pt + w), t1 = __ldg(pt + W32 + w), t2 = __ldg(pt + 2 * W32 + w);
+            const uint32_t j0 = __ldg(pj + w), j1 = __ldg(pj + W32 + w), j2 = __ldg(pj + 2 * W32 + w);
+            auto cells = [&](uint32_t f) {
+              return ((f & 1u) ? j0 : 0u) | ((f & 2u) ? j1 : 0u) | ((f & 4u) ? j2 : 0u);
+            };
+            trig[(e - e0) * W32 + w] =
+                (t0 & cells(en.y)) | (t1 & cells(en.y >> 4)) | (t2 & cells(en.y >> 8));
+          }
+        }
+        __syncthreads();
+        for (int ch = warp; ch < nch; ch += nw) {
+          const int i = 32 * ch + lane;
+          const bool live = i < nk;
+          const int s = 1 + sk + (live ? i : nk - 1), sg = sig[s - 1];
+          const uint32_t *tw = trig + (sg >> 5);
+          const int sh = sg & 31;
+          unsigned long long dh = 0ull;
+          int c = first ? 0 : cng[sg];
+          unsigned at = (unsigned)c * (unsigned)n + (unsigned)sg;
+          constexpr int kRows = 4;
+          for (int r = r0; r < r1; r += kRows) {
+            uint2 ri[kRows];
+            unsigned x[kRows];
+#pragma unroll
+            for (int q = 0; q < kRows; q++) ri[q] = P.rinfo[r + q < r1 ? r + q : r1 - 1];
+#pragma unroll
+            for (int q = 0; q < kRows; q++) x[q] = tw[(ri[q].x - (unsigned)e0) * W32];
+#pragma unroll
+            for (int q = 0; q < kRows; q++) {
+              if (r + q >= r1) break;
+              const int cnt = (int)(ri[q].y & 0xFFu);
+              const uint32_t *tr = tw + (ri[q].x - (unsigned)e0) * W32;
+              unsigned sub = (x[q] >> sh) & 1u;
+              for (int j = 1; j < cnt; j++) sub |= ((tr[j * W32] >> sh) & 1u) << j;
+              if (sub) {
+                const int v = (int)(ri[q].y >> 8) + (int)sub - 1;
+                const unsigned long long d = mdh[v];
+                if (d) {  // (0: the full list)
+                  dh += d;
+                  if (!((P.used[v >> 5] >> (v & 31)) & 1u)) atomicOr(&P.used[v >> 5], 1u << (v & 31));
+                  lst[at] = (uint16_t)v;
+                  at += (unsigned)n;
+                  c++;
+                }
+              }
+            }
+          }
+          if (live) {
+            hs[s] = (first ? SM.HF[k] : hs[s]) + dh;
+            cng[sg] = c;
+          }
+        }
+        r0 = r1;
+        first = false;
+      } while (r0 < rend);
+    }
+    __syncthreads();
+  };
+  // the rows formed per sample, and the changed networks counted
+  auto finish = [&]() {
+    for (int s0 = 32 * warp; s0 < n; s0 += nt) {
+      const int s = 1 + s0 + lane;
+      const bool live = s0 + lane < n;
+      const int k = s <= nA ? 0 : 1, sg = live ? sig[s - 1] : 0;
+      unsigned long long dh = live ? hs[s] : 0ull;
+      bool chg = live && cng[sg] > 0;
+      for (int kk = 0; kk < 2; kk++)
+        for (int r = 0; r < SM.nbig[kk]; r++) {
+          if (!live || k != kk) continue;
+          const int t = P.big[k * g + r];
+          unsigned long long key, h;
+          int len;
+          if (!sample_list(sd, P, ent, k, t, sg, key, h, len)) continue;
+          const unsigned long long d = h - P.fh[k * g + t];
+          if (d == 0ull) atomicOr(&SM.status, kUnitHashCollision);
           dh += d;
           chg = true;
-          if (!((P.used[v >> 5] >> (v & 31)) & 1u)) atomicOr(&P.used[v >> 5], 1u << (v & 31));
+          if (differs(k, key)) big_slot(key, true);
         }
-      });
-      for (int r = 0; r < SM.nbig[k]; r++) {
-        const int t = P.big[k * g + r];
-        unsigned long long key, h;
-        int len;
-        if (!sample_list(sd, P, ent, k, t, sg, key, h, len)) continue;
-        const unsigned long long d = h - P.fh[k * g + t];
-        if (d == 0ull) atomicOr(&SM.status, kUnitHashCollision);
-        dh += d;
-        chg = true;
-        if (differs(k, key)) big_slot(key, true);
-      }
-      if (live) hs[s] = chg ? as_key(SM.HF[k] + dh) : ~0ull;
+      if (live) hs[s] = chg ? as_key(dh) : ~0ull;
       const unsigned nc = __ballot_sync(0xffffffffu, live && chg);
       const int first0 = __reduce_min_sync(0xffffffffu, (k && live && !chg) ? s : S - 1);
       if (lane == 0) {
@@ -1442,6 +1518,14 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
         if (first0 < S - 1) atomicMin(&SM.firstB0, first0);
       }
     }
+  };
+  if (entries) {
+    uint32_t *tr_sm = (uint32_t *)P.itk;
+    const unsigned long long *gdh = (const unsigned long long *)(scr + L.mdh);
+    if (tcap_sm < kMinTrig) walk((uint32_t *)(scr + L.trig), kTrigScratch, gdh);
+    else if (mdh_sm) walk((uint32_t *)((char *)P.itk + mdhb), tcap_sm, P.itk);
+    else walk(tr_sm, tcap_sm, gdh);
+    finish();
   } else if (tid == 0) {
     SM.firstB0 = nA + 1;  // the first class-2 network
   }
@@ -1708,15 +1792,18 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
       int dc = 0;  // the network's edges less the full one's
       const bool plain = !live || s == 0 || s == firstB0;
       if (!__all_sync(0xffffffffu, plain)) {
-        const int sg = sig[plain ? (k ? nA : 0) : s - 1];
+        const int sg = plain ? 0 : sig[s - 1];
+        const int c = plain ? 0 : cng[sg];
+        unsigned at = (unsigned)sg;
         long long x1 = 0, x2 = 0;
-        walk(k, sg, [&](int v) {
-          if (!is_used(v)) return;
+#pragma unroll 4
+        for (int q = 0; q < c; q++, at += (unsigned)n) {
+          const int v = lst[at];
           const longlong2 x = msc[v];
           x1 += x.x;
           x2 += x.y;
           if (keep >= 0) dc += (int)vcnt[v] - P.fcnt[k * g + (int)(ment[v] & 0x3FFF)];
-        });
+        }
         for (int r = 0; !plain && r < SM.nbig[k]; r++) {
           const int t = P.big[k * g + r];
           unsigned long long key, h;
@@ -1735,12 +1822,8 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
           x1 += sc[0] - P.fsc[(k * 2 + 0) * g + t];
           x2 += sc[1] - P.fsc[(k * 2 + 1) * g + t];
         }
-        if (!plain) {
-          d1 += x1;
-          d2 += x2;
-        } else {
-          dc = 0;
-        }
+        d1 += x1;
+        d2 += x2;
       }
       if (live) {
         dist[uu] = d1;
