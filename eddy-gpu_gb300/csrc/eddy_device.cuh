@@ -629,103 +629,98 @@ static __device__ int64_t bdeu_score0(const SetDev &sd, int t,
   return sc - sd.lg[(size_t)c_dmap[1] * sd.lg_stride + nij];
 }
 
-// Parent configurations of node t's score (np >= 1 parents) in one class:
-// q = product of the parents' observed-state counts (0: the score is 0).
-__device__ __forceinline__ int bdeu_q(const uint16_t *cnt3, int np, int p0, int p1, int p2) {
-  const int idx[3] = {p0, p1, p2};
-  int q = 1;
-  for (int k = 0; k < np; k++) {
-    const uint16_t *c = cnt3 + idx[k] * 3;
-    q *= (c[0] > 0) + (c[1] > 0) + (c[2] > 0);
-  }
-  return q;
-}
-// Tasks of node t's score in one class: one per configuration of the
-// parents after the first (the first parent's states are summed within a
-// task), q / (the first parent's observed-state count), 0 when q is 0.
-__device__ __forceinline__ int bdeu_tasks(const uint16_t *cnt3, int np, int p0, int p1, int p2) {
-  const int q = bdeu_q(cnt3, np, p0, p1, p2);
-  if (q == 0) return 0;
-  const uint16_t *c = cnt3 + p0 * 3;
-  return q / ((c[0] > 0) + (c[1] > 0) + (c[2] > 0));
-}
+// A unit's samples by class: word w of gene i, planes[w g + i], holds bit 0 (x)
+// and bit 1 (y) of the states (0-2, 3: missing or past the end) of 32 samples
+// of a class, packed without the other class's (an even number of words).  A
+// parent configuration is then counted over the class's own words, and one
+// 8-byte load gives a gene at 32 samples, next to the other genes at the same
+// samples.
+struct ClassPlanes {
+  const uint2 *p;
+  int g, words;
+};
+__host__ __device__ constexpr int class_words(int nk) { return (nk + 63) / 64 * 2; }
 
-// The terms of kernel5.cu:30-218 for the parent configurations of task j
-// of node t's score over class mask m: configuration j of the parents after
-// the first, with every observed state of the first parent, i.e.
-//   sum over those configurations of  sum_k LG(q r)[N_jk] - LG(q)[N_j].
-// Summing the terms of all tasks gives the node's score (fixed point,
-// exact, in any order).  dmap: the divisor map in shared memory.
-static __device__ __noinline__ int64_t bdeu_config_term(const SetDev &sd, int t, int np, int p0,
-                                                        int p1, int p2, const uint64_t *m,
-                                                        const uint16_t *cnt3, int j,
-                                                        const int8_t *dmap) {
-  int nstate[4], st[4][3];
-  const int idx[4] = {t, p0, p1, p2};
-  for (int k = 0; k <= np; k++) {
-    int c = 0;
-    for (int a = 0; a < 3; a++)
-      if (cnt3[idx[k] * 3 + a] > 0) st[k][c++] = a;
-    nstate[k] = c;
+// Tasks of a score with np >= 1 parents in one class: one per state of the
+// third parent.
+__device__ __forceinline__ int bdeu_tasks(int np) { return np <= 2 ? 1 : 3; }
+
+// The terms of kernel5.cu:30-218 for task j of node t's score: state j of the
+// third parent with every state of the first two, i.e. the sum over those
+// configurations of sum_k LG(q r)[N_jk] - LG(q)[N_j] (an unobserved state
+// counts nothing and adds 0).  Summing the terms of all tasks gives the
+// node's score (fixed point, exact, in any order).  One thread takes nine
+// configurations: the loads and the states' masks serve 27 counters.  Two words
+// a step: one IADD3 adds both their popcounts.  (k_units, 10000 units of 200
+// genes x 1000 samples near the threshold: 19.5 ms with a thread per three
+// configurations over all samples' words, masked by class; 18.1 over packed
+// words; 15.3 with nine a thread.)
+template <bool kTwo>
+__device__ __forceinline__ int64_t bdeu_terms(const ClassPlanes &cp, int t, bool has2, int p0, int p1,
+                                              int p2, int j, const int64_t *__restrict__ LGq,
+                                              const int64_t *__restrict__ LGqr) {
+  constexpr int kS1 = kTwo ? 3 : 1;
+  int c[kS1][9];
+#pragma unroll
+  for (int s = 0; s < kS1; s++)
+#pragma unroll
+    for (int k = 0; k < 9; k++) c[s][k] = 0;
+  // state j of a gene: (y ^ hi) & (x ^ lo)
+  const uint32_t hi = j == 2 ? 0u : ~0u, lo = j == 1 ? 0u : ~0u;
+  const uint2 *Pt = cp.p + t, *Pa = cp.p + p0, *Pb = cp.p + p1, *Pc = cp.p + p2;
+  const int g = cp.g;
+#pragma unroll 1
+  for (int w = 0; w < cp.words; w += 2) {
+    uint32_t x[2][3], y[2][3], b[2][3];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const uint2 T = Pt[h * g], A = Pa[h * g];
+      uint32_t pm = ~0u;
+      if (has2) {
+        const uint2 C = Pc[h * g];
+        pm = (C.y ^ hi) & (C.x ^ lo);
+      }
+      x[h][0] = ~T.y & ~T.x;
+      x[h][1] = ~T.y & T.x;
+      x[h][2] = T.y & ~T.x;
+      y[h][0] = pm & ~A.y & ~A.x;
+      y[h][1] = pm & ~A.y & A.x;
+      y[h][2] = pm & A.y & ~A.x;
+      if (kTwo) {
+        const uint2 B = Pb[h * g];
+        b[h][0] = ~B.y & ~B.x;
+        b[h][1] = ~B.y & B.x;
+        b[h][2] = B.y & ~B.x;
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < kS1; s++)
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+          c[s][3 * i + k] += kTwo ? __popc(y[0][i] & x[0][k] & b[0][s]) + __popc(y[1][i] & x[1][k] & b[1][s])
+                                  : __popc(y[0][i] & x[0][k]) + __popc(y[1][i] & x[1][k]);
+    Pt += 2 * g;
+    Pa += 2 * g;
+    Pb += 2 * g;
+    Pc += 2 * g;
   }
-  const int r = nstate[0];
-  int q = 1;
-  for (int k = 1; k <= np; k++) q *= nstate[k];
-  const int W = sd.W;
-  const uint64_t *P = sd.planes;
-  const int64_t *LGq = sd.lg + (size_t)dmap[q] * sd.lg_stride;
-  const int64_t *LGqr = (r > 0) ? sd.lg + (size_t)dmap[q * r] * sd.lg_stride : LGq;
-  // plane rows as word offsets into the planes: the other parents' (the
-  // first parent's own row again when absent: ANDing it twice changes
-  // nothing), the first parent's observed states (repeated past its count;
-  // unused), the child's states
-  auto row_of = [&](int gene, int s) { return (gene * 3 + s) * W; };
-  int rem = j;
-  const int n1 = nstate[1];
-  const int oa0 = row_of(p0, st[1][0]);
-  const int oa1 = row_of(p0, st[1][n1 > 1 ? 1 : 0]);
-  const int oa2 = row_of(p0, st[1][n1 > 2 ? 2 : 0]);
-  int ob[2] = {-1, -1};
-  for (int k = 2; k <= np; k++) {
-    const int s = st[k][rem % nstate[k]];
-    rem /= nstate[k];
-    ob[k - 2] = row_of(idx[k], s);
-  }
-  const int ot0 = row_of(t, r > 0 ? st[0][0] : 0);
-  const int ot1 = row_of(t, r > 1 ? st[0][1] : 0);
-  const int ot2 = row_of(t, r > 2 ? st[0][2] : 0);
-  int c00 = 0, c01 = 0, c02 = 0, c10 = 0, c11 = 0, c12 = 0, c20 = 0, c21 = 0, c22 = 0;
-  const bool has2 = ob[0] >= 0, has3 = ob[1] >= 0;
-  const int ob0 = has2 ? ob[0] : 0, ob1 = has3 ? ob[1] : 0;
-  for (int w = 0; w < W; w++) {
-    uint64_t pm = m[w];
-    if (has2) pm &= P[ob0 + w];
-    if (has3) pm &= P[ob1 + w];
-    const uint64_t x0 = P[ot0 + w], x1 = P[ot1 + w], x2 = P[ot2 + w];
-    const uint64_t y0 = pm & P[oa0 + w], y1 = pm & P[oa1 + w], y2 = pm & P[oa2 + w];
-    c00 += __popcll(y0 & x0);
-    c01 += __popcll(y0 & x1);
-    c02 += __popcll(y0 & x2);
-    c10 += __popcll(y1 & x0);
-    c11 += __popcll(y1 & x1);
-    c12 += __popcll(y1 & x2);
-    c20 += __popcll(y2 & x0);
-    c21 += __popcll(y2 & x1);
-    c22 += __popcll(y2 & x2);
-  }
-  // one configuration's terms: counts x0, x1, x2 of the child's states
-  auto conf = [&](int x0, int x1, int x2) -> int64_t {
-    int64_t v = 0;
-    int nij = 0;
-    if (r > 0) { nij += x0; v += LGqr[x0]; }
-    if (r > 1) { nij += x1; v += LGqr[x1]; }
-    if (r > 2) { nij += x2; v += LGqr[x2]; }
-    return v - LGq[nij];
-  };
-  int64_t term = conf(c00, c01, c02);
-  if (n1 > 1) term += conf(c10, c11, c12);
-  if (n1 > 2) term += conf(c20, c21, c22);
+  int64_t term = 0;
+#pragma unroll
+  for (int s = 0; s < kS1; s++)
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const int c0 = c[s][3 * i], c1 = c[s][3 * i + 1], c2 = c[s][3 * i + 2];
+      term += LGqr[c0] + LGqr[c1] + LGqr[c2] - LGq[c0 + c1 + c2];
+    }
   return term;
+}
+static __device__ __noinline__ int64_t bdeu_config_term(const ClassPlanes cp, int t, int np, int p0,
+                                                        int p1, int p2, int j, const int64_t *LGq,
+                                                        const int64_t *LGqr) {
+  return np > 1 ? bdeu_terms<true>(cp, t, np > 2, p0, p1, np > 2 ? p2 : p1, j, LGq, LGqr)
+                : bdeu_terms<false>(cp, t, false, p0, p0, p0, 0, LGq, LGqr);
 }
 
 }  // namespace eddy

@@ -460,7 +460,7 @@ __host__ __device__ inline int genes_of_pairs(int c) {
 
 struct UnitLayout {
   size_t phi[2], ent, ment, mdh, msc, vcan, sel, hs, dist, sig, urep, wl, vrep, ubits, htab;
-  size_t bkey, bsc, bpos, vcnt, krow, cnt, lst, trig, total;
+  size_t bkey, bsc, bpos, vcnt, krow, cnt, lst, trig, cp, total;
 };
 __host__ __device__ inline UnitLayout unit_layout(int c, int S) {
   UnitLayout L;
@@ -486,7 +486,7 @@ __host__ __device__ inline UnitLayout unit_layout(int c, int S) {
   L.ment = take(sizeof(uint64_t) * nv);         // variants: key (or ~0: the full list)
   L.mdh = take(sizeof(uint64_t) * nv);          // hash less the full list's
   L.msc = take(2 * sizeof(int64_t) * nv);       // scores less the full list's, both classes
-  L.vcan = take(sizeof(uint16_t) * nv);         // first variant of the row with the same key
+  L.vcan = take(sizeof(uint16_t) * nv);         // a variant with the same key, scored for it
   L.sel = take(sizeof(uint16_t) * nv);          // the variants to score
   L.vcnt = take(sizeof(uint16_t) * nv);         // their list lengths
   // a kept unit's rows, entry ranges (k_pack reads them)
@@ -495,6 +495,7 @@ __host__ __device__ inline UnitLayout unit_layout(int c, int S) {
   L.cnt = take(sizeof(int32_t) * (size_t)(S - 2));
   L.lst = take(sizeof(uint16_t) * (size_t)(S - 2) * g);
   L.trig = take(sizeof(uint32_t) * 64 * (size_t)((S - 2 + 31) / 32 + 1));
+  L.cp = take(sizeof(uint2) * (size_t)g * ((S - 2) / 32 + 4));  // both classes' ClassPlanes
   L.bkey = take(sizeof(uint64_t) * nb);
   L.bsc = take(2 * sizeof(int64_t) * nb);
   L.bpos = take(sizeof(int32_t) * nb);
@@ -583,6 +584,7 @@ struct UnitPtrs {
   uint16_t *big;          // [2][g] rows formed per sample, per class
   uint2 *rinfo;           // [2 g] the memo rows: first entry; entries | first variant << 8
   uint8_t *need;          // [g] 1 = full lists differ, 2 = scores needed
+  uint8_t *nobs;          // [2][g] observed states per class
   uint32_t *used;         // [unit_variants / 32] variants some network uses
   unsigned long long *itk;   // [kItems] node-score items: t | np << 14 | parents
   long long *acc;            // [kItems][2] their scores per class
@@ -618,6 +620,7 @@ __host__ __device__ inline UnitPtrs carve(char *base, int g, int W, int GW) {
   P.big = (uint16_t *)take(2 * sizeof(uint16_t) * g);
   P.rinfo = (uint2 *)take(2 * sizeof(uint2) * g);
   P.need = (uint8_t *)take(g);
+  P.nobs = (uint8_t *)take(2 * g);
   P.used = (uint32_t *)take(sizeof(uint32_t) * ((unit_variants(g) + 31) / 32));
   P.dmap = (int8_t *)take(96);
   // (the base scores follow the work region directly)
@@ -715,9 +718,22 @@ __device__ __noinline__ bool sample_list(const SetDev &sd, const UnitPtrs &P, co
 // score); emit(i, key, class-1 score, class-2 score).  Fixed-point terms are
 // summed with atomics: exact, in any order.  Nodes without parents are
 // scored from the state counts.
+// divisor rows of a score's terms in one class (false: no observed
+// configuration or child state, the score is 0)
+__device__ __forceinline__ bool bdeu_rows(const SetDev &sd, const UnitPtrs &P, int cls, int t, int np,
+                                          int p0, int p1, int p2, const int64_t *&LGq,
+                                          const int64_t *&LGqr) {
+  const uint8_t *no = P.nobs + cls * sd.g;
+  const int q = no[p0] * (np > 1 ? no[p1] : 1) * (np > 2 ? no[p2] : 1), r = no[t];
+  if (q == 0 || r == 0) return false;
+  LGq = sd.lg + (size_t)P.dmap[q] * sd.lg_stride;
+  LGqr = sd.lg + (size_t)P.dmap[q * r] * sd.lg_stride;
+  return true;
+}
+
 template <class Get, class Emit>
-__device__ void bdeu_items(const SetDev &sd, const UnitPtrs &P, int *scan, int n, Get get,
-                           Emit emit) {
+__device__ void bdeu_items(const SetDev &sd, const UnitPtrs &P, const ClassPlanes *cp, int *scan, int n,
+                           Get get, Emit emit) {
   const int tid = threadIdx.x, nt = blockDim.x, g = sd.g;
   for (int b0 = 0; b0 < n; b0 += kItems) {
     const int m = n - b0 < kItems ? n - b0 : kItems;
@@ -725,10 +741,8 @@ __device__ void bdeu_items(const SetDev &sd, const UnitPtrs &P, int *scan, int n
       const unsigned long long key = get(b0 + i);
       P.itk[i] = key;
       const int np = (key == ~0ull) ? 0 : (int)((key >> 14) & 3);
-      const int p0 = (int)((key >> 16) & 0xFFFF), p1 = (int)((key >> 32) & 0xFFFF),
-                p2 = (int)((key >> 48) & 0xFFFF);
       for (int cls = 0; cls < 2; cls++) {
-        P.tq[2 * i + cls] = np ? bdeu_tasks(P.cnt3 + 3 * g * cls, np, p0, p1, p2) : 0;
+        P.tq[2 * i + cls] = np ? bdeu_tasks(np) : 0;
         P.acc[2 * i + cls] = (key != ~0ull && np == 0)
                                  ? bdeu_score0(sd, (int)(key & 0x3FFF), P.cnt3 + 3 * g * cls)
                                  : 0;
@@ -763,9 +777,11 @@ __device__ void bdeu_items(const SetDev &sd, const UnitPtrs &P, int *scan, int n
         const int i = lo >> 1, cls = lo & 1, j = task - P.tq[lo];
         const unsigned long long key = P.itk[i];
         const int t = (int)(key & 0x3FFF), np = (int)((key >> 14) & 3);
-        term = bdeu_config_term(sd, t, np, (int)((key >> 16) & 0xFFFF),
-                                (int)((key >> 32) & 0xFFFF), (int)((key >> 48) & 0xFFFF),
-                                cls ? P.mB : P.mA, P.cnt3 + 3 * g * cls, j, P.dmap);
+        const int p0 = (int)((key >> 16) & 0xFFFF), p1 = (int)((key >> 32) & 0xFFFF),
+                  p2 = (int)((key >> 48) & 0xFFFF);
+        const int64_t *LGq, *LGqr;
+        if (bdeu_rows(sd, P, cls, t, np, p0, p1, p2, LGq, LGqr))
+          term = bdeu_config_term(cp[cls], t, np, p0, p1, p2, j, LGq, LGqr);
         seg = lo;
       }
 #pragma unroll
@@ -785,22 +801,98 @@ __device__ void bdeu_items(const SetDev &sd, const UnitPtrs &P, int *scan, int n
 }
 
 // Both classes' scores of one key by one thread.
-__device__ __noinline__ void key_scores(const SetDev &sd, const UnitPtrs &P, unsigned long long key,
-                                        long long *s) {
+__device__ __noinline__ void key_scores(const SetDev &sd, const UnitPtrs &P, const ClassPlanes *cp,
+                                        unsigned long long key, long long *s) {
   const int t = (int)(key & 0x3FFF), np = (int)((key >> 14) & 3);
   const int p0 = (int)((key >> 16) & 0xFFFF), p1 = (int)((key >> 32) & 0xFFFF),
             p2 = (int)((key >> 48) & 0xFFFF);
   for (int cls = 0; cls < 2; cls++) {
-    const uint16_t *cnt3 = P.cnt3 + 3 * sd.g * cls;
     if (np == 0) {
-      s[cls] = bdeu_score0(sd, t, cnt3);
+      s[cls] = bdeu_score0(sd, t, P.cnt3 + 3 * sd.g * cls);
       continue;
     }
-    const int q = bdeu_tasks(cnt3, np, p0, p1, p2);
+    const int64_t *LGq, *LGqr;
     s[cls] = 0;
-    for (int j = 0; j < q; j++)
-      s[cls] += bdeu_config_term(sd, t, np, p0, p1, p2, cls ? P.mB : P.mA, cnt3, j, P.dmap);
+    if (bdeu_rows(sd, P, cls, t, np, p0, p1, p2, LGq, LGqr))
+      for (int j = 0; j < bdeu_tasks(np); j++)
+        s[cls] += bdeu_config_term(cp[cls], t, np, p0, p1, p2, j, LGq, LGqr);
   }
+}
+
+// The states of a unit's samples packed by class (ClassPlanes), a lane per
+// gene, a warp per 32 genes and class: the class's bits of each sample word
+// are moved together (Hacker's Delight's compress, its five move masks
+// formed once per word and class) and appended to the gene's current output
+// word; the lanes share the masks, so they fill and store words together.
+__device__ __noinline__ void pack_classes(const SetDev &sd, const UnitPtrs &P, uint32_t *moves,
+                                          uint2 *out) {
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+  const int g = sd.g, W32 = 2 * sd.W;
+  for (int i = tid; i < 2 * W32; i += nt) {
+    const int cls = i >= W32 ? 1 : 0;
+    uint32_t m = reinterpret_cast<const uint32_t *>(cls ? P.mB : P.mA)[i - cls * W32];
+    uint32_t *mv = moves + 8 * i;
+    mv[5] = m;
+    uint32_t mk = ~m << 1;
+#pragma unroll
+    for (int b = 0; b < 5; b++) {
+      uint32_t mp = mk ^ (mk << 1);
+      mp ^= mp << 2;
+      mp ^= mp << 4;
+      mp ^= mp << 8;
+      mp ^= mp << 16;
+      const uint32_t v = mp & m;
+      mv[b] = v;
+      m = (m ^ v) | (v >> (1 << b));
+      mk &= ~mp;
+    }
+  }
+  __syncthreads();
+  const int gb = (g + 31) >> 5;
+  for (int task = warp; task < 2 * gb; task += nw) {
+    const int cls = task >= gb ? 1 : 0, i = 32 * (task - cls * gb) + lane;
+    const bool live = i < g;
+    const uint64_t *pl = sd.planesT + 3 * (size_t)(live ? i : g - 1);
+    uint2 *dst = out + (cls ? (size_t)class_words(sd.nA) * g : 0) + i;
+    const uint2 *end = dst + (size_t)class_words(cls ? sd.nB : sd.nA) * g;
+    const uint4 *mv4 = reinterpret_cast<const uint4 *>(moves + 8 * (size_t)cls * W32);
+    uint32_t a0 = 0u, a1 = 0u;
+    int fill = 0;
+    for (int w = 0; w < sd.W; w++, pl += 3 * (size_t)g) {
+      const uint64_t q0 = pl[0], q1 = pl[1], q2 = pl[2];
+      const uint64_t mis = ~(q0 | q1 | q2), b0 = q1 | mis, b1 = q2 | mis;
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const uint4 u = mv4[2 * (2 * w + h)], v = mv4[2 * (2 * w + h) + 1];
+        const uint32_t mv[5] = {u.x, u.y, u.z, u.w, v.x};
+        uint32_t x0 = (uint32_t)(b0 >> (32 * h)) & v.y, x1 = (uint32_t)(b1 >> (32 * h)) & v.y;
+#pragma unroll
+        for (int b = 0; b < 5; b++) {
+          const uint32_t t0 = x0 & mv[b], t1 = x1 & mv[b];
+          x0 = (x0 ^ t0) | (t0 >> (1 << b));
+          x1 = (x1 ^ t1) | (t1 >> (1 << b));
+        }
+        a0 |= x0 << fill;
+        a1 |= x1 << fill;
+        const int c = __popc(v.y);
+        if (fill + c >= 32) {
+          if (live) *dst = make_uint2(a0, a1);
+          dst += g;
+          a0 = fill ? x0 >> (32 - fill) : 0u;
+          a1 = fill ? x1 >> (32 - fill) : 0u;
+          fill -= 32;
+        }
+        fill += c;
+      }
+    }
+    // the rest of the class's words: no value
+    if (fill) {
+      if (live) *dst = make_uint2(a0 | (~0u << fill), a1 | (~0u << fill));
+      dst += g;
+    }
+    if (dst != end && live) *dst = make_uint2(~0u, ~0u);
+  }
+  __syncthreads();
 }
 
 // Normalisation (main.cu:1302-1404) and JS (main.cu:1406-1428) of a unit
@@ -1678,6 +1770,14 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
     P.cnt3[i] = (uint16_t)a;
     P.cnt3[3 * g + i] = (uint16_t)b;
   }
+  uint2 *cpw = (uint2 *)(scr + L.cp);
+  pack_classes(sd, P, (uint32_t *)(scr + L.trig), cpw);
+  const ClassPlanes cp[2] = {{cpw, g, class_words(nA)},
+                             {cpw + (size_t)class_words(nA) * g, g, class_words(nB)}};
+  for (int i = tid; i < 2 * g; i += nt) {
+    const uint16_t *c3 = P.cnt3 + 3 * i;
+    P.nobs[i] = (uint8_t)((c3[0] > 0) + (c3[1] > 0) + (c3[2] > 0));
+  }
   for (int t = tid; t < g; t += nt)
     if (keep >= 0 || P.need[t] || P.phs[t] < P.phe[t] || P.phs[g + t] < P.phe[g + t]) P.need[t] |= 2;
   for (int i = tid; i < 4 * g; i += nt) P.fsc[i] = 0;
@@ -1692,7 +1792,7 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
     return true;
   };
   bdeu_items(
-      sd, P, SM.scan, 2 * g,
+      sd, P, cp, SM.scan, 2 * g,
       [&](int i) -> unsigned long long {
         const int k = i >= g ? 1 : 0, t = i - k * g;
         if (!(P.need[t] & 2) || (k == 1 && same_as_class1(t))) return ~0ull;
@@ -1718,14 +1818,24 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) SM.base[warp & 1][warp >> 1] = s;
   }
-  // the used variants' distinct keys within each row, and the keys of the
-  // lists formed per sample, scored once each
+  // the used variants' distinct keys, and the keys of the lists formed per
+  // sample, scored once each.  A table in the work region (free between the
+  // two rounds of scores) gives each key its first variant: 38 bits of key
+  // (genes below 512) and 16 of the variant a slot.  A variant that finds no
+  // room is scored on its own.
   longlong2 *msc = (longlong2 *)(scr + L.msc);
   longlong2 *bsc = (longlong2 *)(scr + L.bsc);
   uint16_t *vcan = (uint16_t *)(scr + L.vcan), *sel = (uint16_t *)(scr + L.sel);
   const int vsplit = SM.split[1];
   auto is_used = [&](int v) { return ((P.used[v >> 5] >> (v & 31)) & 1u) != 0u; };
   if (SM.nchg) {
+    constexpr int kKeySlots = 2048;
+    static_assert(kKeySlots * sizeof(unsigned long long) <= kWorkBytes, "key table");
+    unsigned long long *kt = P.itk;
+    int slots = 64;
+    while (slots < 2 * nvar && slots < kKeySlots) slots <<= 1;
+    for (int i = tid; i < slots; i += nt) kt[i] = ~0ull;
+    __syncthreads();
     for (int v = tid; v < nvar; v += nt) {
       if (!is_used(v)) continue;
       const unsigned long long key = ment[v];
@@ -1734,13 +1844,19 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
         vcan[v] = (uint16_t)v;
         continue;
       }
-      // the row's first used variant with this key (a key names its node)
+      const unsigned long long k38 = (key & 511u) | (((key >> 14) & 3u) << 9) |
+                                     (((key >> 16) & 511u) << 11) | (((key >> 32) & 511u) << 20) |
+                                     (((key >> 48) & 511u) << 29);
       int can = v;
-      for (int w = v - 1; w >= 0 && can - w < 256; w--) {
-        const unsigned long long kw = ment[w];
-        if (kw != ~0ull && (kw & 0x3FFF) != (key & 0x3FFF)) break;
-        if (w < vsplit && v >= vsplit) break;
-        if (kw == key && is_used(w)) can = w;
+      unsigned slot = (unsigned)(mix64(k38) & (slots - 1));
+      for (int pr = 0; pr < 32; pr++, slot = (slot + 1u) & (slots - 1)) {
+        unsigned long long cur = *(volatile unsigned long long *)&kt[slot];
+        if (cur == ~0ull) cur = atomicCAS(&kt[slot], ~0ull, (k38 << 16) | (unsigned)v);
+        if (cur == ~0ull) break;
+        if (cur >> 16 == k38) {
+          can = (int)(cur & 0xFFFFu);
+          break;
+        }
       }
       vcan[v] = (uint16_t)can;
       if (can == v) sel[atomicAdd(&SM.nsel, 1)] = (uint16_t)v;
@@ -1759,7 +1875,7 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
     __syncthreads();
     const int nsel = SM.nsel;
     bdeu_items(
-        sd, P, SM.scan, nsel + nbk,
+        sd, P, cp, SM.scan, nsel + nbk,
         [&](int i) -> unsigned long long { return i < nsel ? ment[sel[i]] : bkey[bpos[i - nsel]]; },
         [&](int i, unsigned long long key, long long s1, long long s2) {
           if (i < nsel) {
@@ -1769,8 +1885,16 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
             bsc[bpos[i - nsel]] = make_longlong2(s1, s2);
           }
         });
-    for (int v = tid; v < nvar; v += nt)
-      if (is_used(v) && vcan[v] != v) msc[v] = msc[vcan[v]];
+    for (int v = tid; v < nvar; v += nt) {
+      const int c = is_used(v) ? vcan[v] : v;
+      if (c == v) continue;
+      // the same list of the same node, in either class
+      const int t = (int)(ment[v] & 0x3FFF), k = v >= vsplit ? 1 : 0, kc = c >= vsplit ? 1 : 0;
+      longlong2 x = msc[c];
+      x.x += P.fsc[(kc * 2 + 0) * g + t] - P.fsc[(k * 2 + 0) * g + t];
+      x.y += P.fsc[(kc * 2 + 1) * g + t] - P.fsc[(k * 2 + 1) * g + t];
+      msc[v] = x;
+    }
   }
   __syncthreads();
   // unique networks: base of their class plus the variants' differences, a
@@ -1817,7 +1941,7 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
             sc[0] = bsc[slot].x;
             sc[1] = bsc[slot].y;
           } else {
-            key_scores(sd, P, key, sc);  // the table had no room
+            key_scores(sd, P, cp, key, sc);  // the table had no room
           }
           x1 += sc[0] - P.fsc[(k * 2 + 0) * g + t];
           x2 += sc[1] - P.fsc[(k * 2 + 1) * g + t];
