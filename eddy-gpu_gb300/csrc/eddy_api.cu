@@ -171,15 +171,15 @@ struct eddy_ctx {
   // decisions, per-unit scratch, results, the set table and unit slots
   DevBuf d_lg, d_setdata, d_mask0, d_mat;
   bool mat_ready = false;  // d_mat holds the matrix
-  DevBuf d_masks, d_dmask, d_scratch, d_js, d_U, d_status, d_keep, d_uset, d_uperm;
-  DevBuf d_uslot, d_sets;
-  DevBuf d_kbuf, d_kmeta, d_stats;  // kept units' packed outputs, their table
-  DevBuf d_Y, d_afp8, d_err;  // tensor-core contingency operands
+  DevBuf d_masks, d_dmask, d_scratch;
+  DevBuf d_in, d_out;  // a batch's uploads and results, one copy each
+  DevBuf d_kbuf;       // kept units' packed outputs
+  DevBuf d_Y, d_afp8;  // tensor-core contingency operands
   // d_dmask is all zero between batches (decisions only set bits, the unit
   // kernel clears what it reads) while this equals d_dmask.p; null = unknown
   void *dmask_clean = nullptr;
-  PinnedBuf h_stage;          // per-batch uploads: unit sets, permutations, slots, set table
-  PinnedBuf h_res;            // per-batch results
+  PinnedBuf h_stage;          // d_in's contents on their way in
+  PinnedBuf h_res;            // d_out's on their way out
   ResultPool results;         // the sets' kept outputs
   PinnedBuf h_vals;           // the resident sets' table, rows and prior bits on their way in
   int sms = 148;
@@ -540,12 +540,17 @@ int dmask_ready(eddy_ctx *ctx, size_t bytes) {
 }
 
 // A batch as the decision kernels see it: the host copy of its set table
-// (device descriptors, unit ranges and slices filled in), each unit's slot,
-// and the table's device copy.
+// (device descriptors, unit ranges and slices filled in), where the table,
+// each unit's slot and the error word are on the device, and the table's
+// staging.
 struct BatchPlan {
   std::vector<BatchSet> sets;
   int B = 0, gmax = 0, cmax = 0;
   bool fp64 = false;  // every set decides in FP64 (the popcount path)
+  BatchSet *d_sets = nullptr, *h_tab = nullptr;
+  const int32_t *d_uslot = nullptr;
+  unsigned *d_err = nullptr;
+  int uploaded = -1;  // the tile shape the device's table is planned for (-1: none)
 };
 
 // The set table in layout `core` for tile shape `variant`: each slot's
@@ -560,21 +565,22 @@ MmaPlan plan_mma(eddy_ctx *ctx, BatchPlan &bp, int variant) {
   return mma_plan(bp.sets.data(), (int)bp.sets.size(), variant, core);
 }
 
-// Uploads the set table through the pinned staging at byte offset `off`.
-int upload_table(eddy_ctx *ctx, const BatchPlan &bp, size_t off) {
+// Uploads the set table as planned for tile shape v, once the copy before
+// has left the staging (tuning and checks: a batch whose shape is known has
+// the planned table in its one upload).
+int upload_table(eddy_ctx *ctx, BatchPlan &bp, int v) {
+  CK(cudaStreamSynchronize(ctx->stream));
   const size_t tb = sizeof(BatchSet) * bp.sets.size();
-  CK(ctx->d_sets.ensure(tb));
-  memcpy(ctx->h_stage.as<char>(off), bp.sets.data(), tb);
-  CK(cudaMemcpyAsync(ctx->d_sets.p, ctx->h_stage.as<char>(off), tb, cudaMemcpyHostToDevice,
-                     ctx->stream));
+  memcpy(bp.h_tab, bp.sets.data(), tb);
+  CK(cudaMemcpyAsync(bp.d_sets, bp.h_tab, tb, cudaMemcpyHostToDevice, ctx->stream));
+  bp.uploaded = v;
   return EDDY_OK;
 }
 
 // The Y arena of the resident sets, from the uploaded set table (planned).
 int build_y(eddy_ctx *ctx, const BatchPlan &bp, bool core) {
   if (ctx->y_ready) return EDDY_OK;
-  CK(launch_build_y(ctx->d_sets.as<BatchSet>(), (int)bp.sets.size(), core, ctx->y, ctx->W,
-                    ctx->stream));
+  CK(launch_build_y(bp.d_sets, (int)bp.sets.size(), core, ctx->y, ctx->W, ctx->stream));
   ctx->launches += 1;
   ctx->y_ready = true;
   return EDDY_OK;
@@ -583,34 +589,25 @@ int build_y(eddy_ctx *ctx, const BatchPlan &bp, bool core) {
 // Decisions of a batch: the popcount kernel, or the tensor-core path in the
 // variant picked (tuning it on this batch when it is the first of its shape
 // with >= 512 units: every choice is timed once, same results, the fastest
-// kept).  The table is uploaded from the staging at byte offset toff.
+// kept; the table goes up again for each).  The error word is 0 before.
 // ev_mid, when given, is recorded where the contraction ends and the
 // general-path decisions begin (right after the pair kernel on the popcount
 // path, which has no separate decision kernels).
 int launch_pairs_any(eddy_ctx *ctx, BatchPlan &bp, const uint64_t *masks, uint32_t *dmask,
-                     unsigned long long *stats, size_t toff, bool force_popc = false,
+                     unsigned long long *stats, bool force_popc = false,
                      cudaEvent_t ev_mid = nullptr) {
   auto mark = [&]() -> cudaError_t { return ev_mid ? cudaEventRecord(ev_mid, ctx->stream) : cudaSuccess; };
   if (bp.cmax == 0) {
-    int rc = upload_table(ctx, bp, toff);
-    if (rc) return rc;
     CK(mark());
     return EDDY_OK;
   }
   const int ns = (int)bp.sets.size();
   if (use_popc() || bp.fp64 || force_popc) {
-    {
-      int rc = upload_table(ctx, bp, toff);
-      if (rc) return rc;
-    }
-    CK(launch_pairs(ctx->d_sets.as<BatchSet>(), ctx->d_uslot.as<int32_t>(), masks, dmask, bp.B,
-                    ctx->W, bp.gmax, stats, ctx->stream));
+    CK(launch_pairs(bp.d_sets, bp.d_uslot, masks, dmask, bp.B, ctx->W, bp.gmax, stats, ctx->stream));
     CK(mark());
     ctx->launches += 1;
     return EDDY_OK;
   }
-  CK(ctx->d_err.ensure(sizeof(unsigned)));
-  CK(cudaMemsetAsync(ctx->d_err.p, 0, sizeof(unsigned), ctx->stream));
   Shape sh{bp.sets[0].sd.g, bp.sets[0].sd.c, shape_of(ctx, ctx->res_ids[0]).core};
   int variant = pick_variant(ctx, sh, bp.B);
   const int g_single = ns == 1 ? bp.sets[0].sd.g : 0;
@@ -622,15 +619,14 @@ int launch_pairs_any(eddy_ctx *ctx, BatchPlan &bp, const uint64_t *masks, uint32
     const MmaPlan mp = plan_mma(ctx, bp, v);
     CK(ctx->d_afp8.ensure(mma_a_bytes(mp, ctx->samples, layout_core(v))));
     {
-      int rc = upload_table(ctx, bp, toff);
+      int rc = bp.uploaded == v ? EDDY_OK : upload_table(ctx, bp, v);
       if (rc) return rc;
       rc = build_y(ctx, bp, layout_core(v));
       if (rc) return rc;
     }
-    CK(launch_pairs_mma(ctx->d_sets.as<BatchSet>(), ns, mp, masks, ctx->d_uslot.as<int32_t>(),
-                        ctx->samples, ctx->W, ctx->d_afp8.as<uint8_t>(), ctx->y, dmask, st,
-                        ctx->d_err.as<unsigned>(), ctx->sms, ctx->stream, v, layout_core(v),
-                        g_single, evm));
+    CK(launch_pairs_mma(bp.d_sets, ns, mp, masks, bp.d_uslot, ctx->samples, ctx->W,
+                        ctx->d_afp8.as<uint8_t>(), ctx->y, dmask, st, bp.d_err, ctx->sms, ctx->stream,
+                        v, layout_core(v), g_single, evm));
     ctx->launches += mma_launches();
     return EDDY_OK;
   };
@@ -643,9 +639,6 @@ int launch_pairs_any(eddy_ctx *ctx, BatchPlan &bp, const uint64_t *masks, uint32
     const int ncand = choices(sh, cand);
     for (int ci = 0; ci < ncand; ci++) {
       const int v = cand[ci];
-      // (the staging slot of the table is rewritten for the next choice
-      // only after this one's upload has run)
-      if (ci > 0) CK(cudaStreamSynchronize(ctx->stream));
       CK(cudaEventRecord(ctx->ev[2], ctx->stream));
       {
         int rc = run(v, nullptr, nullptr);
@@ -663,16 +656,14 @@ int launch_pairs_any(eddy_ctx *ctx, BatchPlan &bp, const uint64_t *masks, uint32
     }
     ctx->tuned[tune_key(ctx->samples, sh)] = bi;
     variant = bi;
-    CK(cudaStreamSynchronize(ctx->stream));
   }
   ctx->tuned_variant = variant;
   return run(variant, stats, ev_mid);
 }
 
 int check_mma_error(eddy_ctx *ctx, const BatchPlan &bp) {
-  if (use_popc() || bp.fp64 || ctx->d_err.p == nullptr) return EDDY_OK;
   unsigned e = 0;
-  CK(cudaMemcpyAsync(&e, ctx->d_err.p, sizeof e, cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaMemcpyAsync(&e, bp.d_err, sizeof e, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   if (e) return fail(ctx, EDDY_ERR_INTERNAL, "tensor-core pipeline wait timed out");
   return EDDY_OK;
@@ -768,68 +759,87 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
     // says how much, and its kept units run again)
     const size_t cap = std::min(kwords, std::max(ctx->d_kbuf.n / 8, (size_t)16 << 20));
     CK(ctx->d_kbuf.ensure(8 * cap));
-    CK(ctx->d_kmeta.ensure(sizeof(KeepMeta) * (size_t)(nk + 1)));
-    CK(cudaMemsetAsync(ctx->d_kmeta.p, 0, sizeof(KeepMeta) * (size_t)(nk + 1), ctx->stream));
   }
-  CK(ctx->d_stats.ensure(sizeof(unsigned long long) * 4 * ns));
-  CK(cudaMemsetAsync(ctx->d_stats.p, 0, sizeof(unsigned long long) * 4 * ns, ctx->stream));
-  CK(ctx->d_masks.ensure(sizeof(uint64_t) * (size_t)Bt * W));
   {
     int rc = dmask_ready(ctx, sizeof(uint32_t) * std::max<size_t>(dmw, 1));
     if (rc) return rc;
   }
   CK(ctx->d_scratch.ensure(std::max<size_t>(scb, 1)));
-  CK(ctx->d_js.ensure(sizeof(double) * Bt));
-  CK(ctx->d_U.ensure(sizeof(int32_t) * Bt));
-  CK(ctx->d_status.ensure(sizeof(uint32_t) * Bt));
-  CK(ctx->d_keep.ensure(sizeof(int32_t) * Bt));
-  CK(ctx->d_uslot.ensure(sizeof(int32_t) * Bt));
-  CK(ctx->d_uset.ensure(sizeof(int32_t) * Bt));
-  CK(ctx->d_uperm.ensure(sizeof(int32_t) * Bt));
-  CK(ctx->d_sets.ensure(sizeof(BatchSet) * ns));
-  // pinned staging: [set ids][permutations][slots][kept slots][set table]
-  // (uploads); results in h_res
-  const size_t o_tab = (16 * (size_t)Bt + 255) & ~(size_t)255;
-  CK(ctx->h_stage.ensure(o_tab + sizeof(BatchSet) * ns + 64));
-  const size_t o_km = (16 * (size_t)Bt + 8 + 32 * (size_t)ns + 63) & ~(size_t)63;
-  CK(ctx->h_res.ensure(o_km + sizeof(KeepMeta) * (size_t)(nk + 1)));
-  int32_t *hs = ctx->h_stage.as<int32_t>(), *hp = hs + Bt, *hsl = hp + Bt, *hk = hsl + Bt;
-  for (int i = 0; i < Bt; i++) {
-    const Job &J = jobs[units[i].job];
-    hs[i] = J.set_id;
-    hp[i] = J.perms ? J.perms[units[i].i] : 0;
-    hsl[i] = uslot[i];
-    hk[i] = keep_slot[i];
+  // uploads, in one copy: [set table][slots][kept slots], then the labellings'
+  // masks, or the sets and permutations they are drawn from.  (A batch of
+  // one unit is bound by its copies, launches and their gaps: with one copy
+  // each way and one memset, for up to five, six and three, one labelling of
+  // 20 genes x 200 samples takes 0.103 ms for 0.125.)
+  const bool mma = !popc_batch && !use_popc() && !bp.fp64 && bp.cmax > 0;
+  const size_t Bz = (size_t)Bt;
+  const size_t i_slot = (sizeof(BatchSet) * ns + 255) & ~(size_t)255, i_keep = i_slot + 4 * Bz;
+  const size_t i_lab = (i_keep + 4 * Bz + 255) & ~(size_t)255;
+  const size_t in_bytes = i_lab + (masks_host ? 8 * Bz * W : 8 * Bz);
+  // results, in one copy: [JS][U][status], then, 0 before the batch, the error
+  // word, the sets' decision counters and the kept units' table
+  const size_t o_U = 8 * Bz, o_st = o_U + 4 * Bz, o_err = o_st + 4 * Bz, o_cnt = o_err + 8;
+  const size_t o_km = o_cnt + 32 * (size_t)ns;
+  const size_t out_bytes = o_km + sizeof(KeepMeta) * (size_t)(nk + 1);
+  CK(ctx->d_in.ensure(in_bytes));
+  CK(ctx->h_stage.ensure(in_bytes));
+  CK(ctx->d_out.ensure(out_bytes));
+  CK(ctx->h_res.ensure(out_bytes));
+  if (!masks_host) CK(ctx->d_masks.ensure(8 * Bz * W));
+  uint8_t *din = ctx->d_in.as<uint8_t>(), *dout = ctx->d_out.as<uint8_t>();
+  bp.d_sets = (BatchSet *)din;
+  bp.h_tab = ctx->h_stage.as<BatchSet>();
+  bp.d_uslot = (const int32_t *)(din + i_slot);
+  bp.d_err = (unsigned *)(dout + o_err);
+  const int32_t *d_uset = (const int32_t *)(din + i_lab), *d_uperm = d_uset + Bt;
+  {
+    int32_t *hsl = ctx->h_stage.as<int32_t>(i_slot), *hk = ctx->h_stage.as<int32_t>(i_keep);
+    memcpy(hsl, uslot.data(), 4 * Bz);
+    memcpy(hk, keep_slot.data(), 4 * Bz);
+    if (masks_host) {
+      uint64_t *hm = ctx->h_stage.as<uint64_t>(i_lab);
+      for (int i = 0; i < Bt; i++)
+        memcpy(hm + (size_t)i * W, jobs[units[i].job].masks_host + (size_t)units[i].i * W, 8 * W);
+    } else {
+      int32_t *hs = ctx->h_stage.as<int32_t>(i_lab), *hp = hs + Bt;
+      for (int i = 0; i < Bt; i++) {
+        const Job &J = jobs[units[i].job];
+        hs[i] = J.set_id;
+        hp[i] = J.perms ? J.perms[units[i].i] : 0;
+      }
+    }
   }
-  CK(cudaMemcpyAsync(ctx->d_uslot.p, hsl, 4 * (size_t)Bt, cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemcpyAsync(ctx->d_keep.p, hk, 4 * (size_t)Bt, cudaMemcpyHostToDevice, ctx->stream));
-  if (masks_host) {
-    std::vector<uint64_t> mh((size_t)Bt * W);
-    for (int i = 0; i < Bt; i++)
-      memcpy(mh.data() + (size_t)i * W, jobs[units[i].job].masks_host + (size_t)units[i].i * W, 8 * W);
-    CK(cudaMemcpyAsync(ctx->d_masks.p, mh.data(), 8 * mh.size(), cudaMemcpyHostToDevice, ctx->stream));
-  } else {
-    CK(cudaMemcpyAsync(ctx->d_uset.p, hs, 4 * (size_t)Bt, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->d_uperm.p, hp, 4 * (size_t)Bt, cudaMemcpyHostToDevice, ctx->stream));
+  // the table, planned when the tile shape is known
+  Shape sh0 = shape_of(ctx, ids[0]);
+  const int vknown = mma ? pick_variant(ctx, sh0, Bt) : -1;
+  MmaPlan mp{};
+  if (vknown >= 0) {
+    int rc = layout_y(ctx, layout_core(vknown));
+    if (rc) return rc;
+    mp = plan_mma(ctx, bp, vknown);
+    CK(ctx->d_afp8.ensure(mma_a_bytes(mp, n, layout_core(vknown))));
   }
+  memcpy(bp.h_tab, bp.sets.data(), sizeof(BatchSet) * ns);
+  bp.uploaded = vknown;
+  CK(cudaMemcpyAsync(din, ctx->h_stage.p, in_bytes, cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemsetAsync(dout + o_err, 0, out_bytes - o_err, ctx->stream));
   BatchDev bd{};
   bd.B = Bt;
   bd.nsets = ns;
   bd.memo_max = kMemoMax;
   if (const char *em = getenv("EDDY_MEMO_MAX")) bd.memo_max = std::max(0, std::min(kMemoMax, atoi(em)));
-  bd.sets = ctx->d_sets.as<BatchSet>();
-  bd.uslot = ctx->d_uslot.as<int32_t>();
-  bd.masks = ctx->d_masks.as<uint64_t>();
+  bd.sets = bp.d_sets;
+  bd.uslot = bp.d_uslot;
+  bd.masks = masks_host ? (const uint64_t *)(din + i_lab) : ctx->d_masks.as<uint64_t>();
   bd.dmask = ctx->d_dmask.as<uint32_t>();
   bd.scratch = ctx->d_scratch.as<uint8_t>();
-  bd.js = ctx->d_js.as<double>();
-  bd.U = ctx->d_U.as<int32_t>();
-  bd.status = ctx->d_status.as<uint32_t>();
-  bd.keep_slot = ctx->d_keep.as<int32_t>();
-  bd.kmeta = ctx->d_kmeta.as<KeepMeta>();
+  bd.js = (double *)dout;
+  bd.U = (int32_t *)(dout + o_U);
+  bd.status = (uint32_t *)(dout + o_st);
+  bd.keep_slot = (int32_t *)(din + i_keep);
+  bd.kmeta = (KeepMeta *)(dout + o_km);
   bd.kbuf = ctx->d_kbuf.as<uint64_t>();
   bd.kcap = ctx->d_kbuf.n / 8;
-  bd.stats = ctx->d_stats.as<unsigned long long>();
+  bd.stats = (unsigned long long *)(dout + o_cnt);
   // the batch's device work: labellings, decisions, networks (events
   // become record nodes when captured)
   auto record = [&](cudaEvent_t e, bool capturing) -> cudaError_t {
@@ -840,20 +850,16 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   // the sets resident) that repeats the previous one's sets, shape and
   // buffers is captured as one CUDA graph and later replayed; the uploads
   // above stay outside the graph
-  Shape sh0 = shape_of(ctx, ids[0]);
-  const bool mma = !popc_batch && !use_popc() && !bp.fp64 && bp.cmax > 0;
-  const bool graphable = !masks_host && nk == 0 && mma && ctx->stream != nullptr &&
-                         pick_variant(ctx, sh0, Bt) >= 0;
+  const bool graphable = !masks_host && nk == 0 && vknown >= 0 && ctx->stream != nullptr;
   auto enqueue = [&](bool capturing) -> int {
     if (!masks_host) {
-      CK(launch_counter_masks(n, ctx->nA, W, ctx->o.seed, ctx->d_uset.as<int32_t>(),
-                              ctx->d_uperm.as<int32_t>(), ctx->d_mask0.as<uint64_t>(),
+      CK(launch_counter_masks(n, ctx->nA, W, ctx->o.seed, d_uset, d_uperm, ctx->d_mask0.as<uint64_t>(),
                               ctx->d_masks.as<uint64_t>(), Bt, ctx->stream));
       ctx->launches++;
     }
     CK(record(ctx->ev[0], capturing));
     {
-      int rc = launch_pairs_any(ctx, bp, bd.masks, bd.dmask, bd.stats, o_tab, popc_batch,
+      int rc = launch_pairs_any(ctx, bp, bd.masks, bd.dmask, bd.stats, popc_batch,
                                 ctx->ev[4]);
       if (rc) return rc;
     }
@@ -866,27 +872,15 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   };
   ctx->dmask_clean = nullptr;  // until the batch is seen to finish
   if (graphable) {
-    // the table of the tuned shape, uploaded outside the graph
-    const int v = pick_variant(ctx, sh0, Bt);
-    {
-      int rc = layout_y(ctx, layout_core(v));
-      if (rc) return rc;
-    }
-    const MmaPlan mp = plan_mma(ctx, bp, v);
-    CK(ctx->d_afp8.ensure(mma_a_bytes(mp, n, layout_core(v))));
-    CK(ctx->d_err.ensure(sizeof(unsigned)));
+    const int v = vknown;
     // everything a replay bakes in: the sets, their state, the batch shape
     // and every buffer address
     std::vector<uintptr_t> key = {(uintptr_t)ctx->prep_gen, (uintptr_t)ctx->salt,
                                   (uintptr_t)Bt, (uintptr_t)v,
                                   (uintptr_t)ctx->o.seed, (uintptr_t)ctx->d_masks.p,
                                   (uintptr_t)ctx->d_dmask.p, (uintptr_t)ctx->d_scratch.p,
-                                  (uintptr_t)ctx->d_js.p, (uintptr_t)ctx->d_U.p,
-                                  (uintptr_t)ctx->d_status.p, (uintptr_t)ctx->d_keep.p,
-                                  (uintptr_t)ctx->d_uset.p, (uintptr_t)ctx->d_uperm.p,
-                                  (uintptr_t)ctx->d_uslot.p, (uintptr_t)ctx->d_sets.p,
-                                  (uintptr_t)ctx->d_stats.p, (uintptr_t)ctx->d_afp8.p,
-                                  (uintptr_t)ctx->d_Y.p, (uintptr_t)ctx->d_err.p,
+                                  (uintptr_t)ctx->d_in.p, (uintptr_t)ctx->d_out.p,
+                                  (uintptr_t)ctx->d_afp8.p, (uintptr_t)ctx->d_Y.p,
                                   (uintptr_t)ctx->d_mask0.p, (uintptr_t)ctx->stream,
                                   (uintptr_t)bp.sets[0].sd.exact_all, (uintptr_t)bd.memo_max};
     for (int k = 0; k < ns; k++) {
@@ -900,15 +894,11 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
       int rc = enqueue(false);
       if (rc) return rc;
     } else {
-      // the uploads of the table and the error word happen outside the
-      // graph, before its launch
+      // (the upload and the zeroing happen outside the graph, above)
       {
-        int rc = upload_table(ctx, bp, o_tab);
-        if (rc) return rc;
-        rc = build_y(ctx, bp, layout_core(v));
+        int rc = build_y(ctx, bp, layout_core(v));
         if (rc) return rc;
       }
-      CK(cudaMemsetAsync(ctx->d_err.p, 0, sizeof(unsigned), ctx->stream));
       if (!replay) {
         if (ctx->graph_exec) {
           cudaGraphExecDestroy(ctx->graph_exec);
@@ -923,13 +913,13 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
             if (e != cudaSuccess && rc == EDDY_OK)
               rc = fail(ctx, EDDY_ERR_CUDA, "capture: %s", cudaGetErrorString(e));
           };
-          cap_ck(launch_counter_masks(n, ctx->nA, W, ctx->o.seed, ctx->d_uset.as<int32_t>(),
-                                      ctx->d_uperm.as<int32_t>(), ctx->d_mask0.as<uint64_t>(),
-                                      ctx->d_masks.as<uint64_t>(), Bt, ctx->stream));
+          cap_ck(launch_counter_masks(n, ctx->nA, W, ctx->o.seed, d_uset, d_uperm,
+                                      ctx->d_mask0.as<uint64_t>(), ctx->d_masks.as<uint64_t>(), Bt,
+                                      ctx->stream));
           cap_ck(record(ctx->ev[0], true));
-          cap_ck(launch_pairs_mma(ctx->d_sets.as<BatchSet>(), ns, mp, bd.masks, bd.uslot, n, W,
-                                  ctx->d_afp8.as<uint8_t>(), ctx->y, bd.dmask, bd.stats,
-                                  ctx->d_err.as<unsigned>(), ctx->sms, ctx->stream, v,
+          cap_ck(launch_pairs_mma(bp.d_sets, ns, mp, bd.masks, bd.uslot, n, W,
+                                  ctx->d_afp8.as<uint8_t>(), ctx->y, bd.dmask, bd.stats, bp.d_err,
+                                  ctx->sms, ctx->stream, v,
                                   layout_core(v), ns == 1 ? bp.sets[0].sd.g : 0, ctx->ev[4],
                                   true));
           cap_ck(record(ctx->ev[1], true));
@@ -959,25 +949,13 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
     int rc = enqueue(false);
     if (rc) return rc;
   }
-  // results (and the tensor-core kernel's timeout word) through the pinned
-  // staging: JS, U, status, error word
-  double *hjs = ctx->h_res.as<double>();
-  int32_t *hU = ctx->h_res.as<int32_t>(8 * (size_t)Bt);
-  uint32_t *hst = ctx->h_res.as<uint32_t>(12 * (size_t)Bt);
-  unsigned *herr = ctx->h_res.as<unsigned>(16 * (size_t)Bt);
-  *herr = 0;
-  CK(cudaMemcpyAsync(hjs, ctx->d_js.p, 8 * (size_t)Bt, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaMemcpyAsync(hU, ctx->d_U.p, 4 * (size_t)Bt, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaMemcpyAsync(hst, ctx->d_status.p, 4 * (size_t)Bt, cudaMemcpyDeviceToHost, ctx->stream));
-  if (mma) CK(cudaMemcpyAsync(herr, ctx->d_err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
-  // the decision counters of each set
-  const unsigned long long *hst4 = ctx->h_res.as<unsigned long long>(16 * (size_t)Bt + 8);
-  CK(cudaMemcpyAsync(ctx->h_res.as<unsigned long long>(16 * (size_t)Bt + 8), ctx->d_stats.p,
-                     sizeof(unsigned long long) * 4 * ns, cudaMemcpyDeviceToHost, ctx->stream));
+  const double *hjs = ctx->h_res.as<double>();
+  const int32_t *hU = ctx->h_res.as<int32_t>(o_U);
+  const uint32_t *hst = ctx->h_res.as<uint32_t>(o_st);
+  const unsigned *herr = ctx->h_res.as<unsigned>(o_err);
+  const unsigned long long *hst4 = ctx->h_res.as<unsigned long long>(o_cnt);
   const KeepMeta *hkm = ctx->h_res.as<KeepMeta>(o_km);
-  if (nk)
-    CK(cudaMemcpyAsync(ctx->h_res.as<KeepMeta>(o_km), ctx->d_kmeta.p, sizeof(KeepMeta) * (size_t)(nk + 1),
-                       cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaMemcpyAsync(ctx->h_res.p, dout, out_bytes, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   const unsigned errw = *herr;
   if (errw & 1u) return fail(ctx, EDDY_ERR_INTERNAL, "tensor-core pipeline wait timed out");
@@ -1155,10 +1133,7 @@ int eddy_ctx_destroy(eddy_ctx *ctx) {
   cudaSetDevice(ctx->o.device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   DevBuf *bufs[] = {&ctx->d_lg, &ctx->d_setdata, &ctx->d_mask0, &ctx->d_mat, &ctx->d_masks, &ctx->d_dmask,
-                    &ctx->d_scratch, &ctx->d_js, &ctx->d_U, &ctx->d_status, &ctx->d_keep,
-                    &ctx->d_uset, &ctx->d_uperm, &ctx->d_uslot, &ctx->d_sets, &ctx->d_kbuf,
-                    &ctx->d_kmeta,
-                    &ctx->d_stats, &ctx->d_Y, &ctx->d_afp8, &ctx->d_err};
+                    &ctx->d_scratch, &ctx->d_in, &ctx->d_out, &ctx->d_kbuf, &ctx->d_Y, &ctx->d_afp8};
   for (DevBuf *b : bufs) b->release();
   for (auto &ev : ctx->ev)
     if (ev) cudaEventDestroy(ev);
@@ -1717,16 +1692,25 @@ int eddy_debug_edges(eddy_ctx *ctx, int set_id, const uint8_t *labels, uint8_t *
   const int c = sd.c, S = sd.S;
   std::vector<uint64_t> m(W);
   labels_to_mask(labels, n, W, m.data());
-  CK(ctx->d_masks.ensure(8 * W));
   rc = dmask_ready(ctx, dmask_bytes(1, c));
   if (rc) return rc;
   ctx->dmask_clean = nullptr;  // no unit kernel reads (and clears) these masks
-  CK(ctx->h_stage.ensure(512 + sizeof(BatchSet)));
-  CK(ctx->d_uslot.ensure(sizeof(int32_t)));
-  CK(cudaMemsetAsync(ctx->d_uslot.p, 0, sizeof(int32_t), ctx->stream));
-  CK(cudaMemcpyAsync(ctx->d_masks.p, m.data(), 8 * W, cudaMemcpyHostToDevice, ctx->stream));
-  rc = launch_pairs_any(ctx, bp, ctx->d_masks.as<uint64_t>(), ctx->d_dmask.as<uint32_t>(), nullptr,
-                        256);
+  // [set table][the unit's slot, 0][its mask] in one upload; the error word
+  const size_t i_slot = (sizeof(BatchSet) + 255) & ~(size_t)255, i_mask = i_slot + 256;
+  CK(ctx->d_in.ensure(i_mask + 8 * W));
+  CK(ctx->h_stage.ensure(i_mask + 8 * W));
+  CK(ctx->d_out.ensure(8));
+  bp.d_sets = ctx->d_in.as<BatchSet>();
+  bp.h_tab = ctx->h_stage.as<BatchSet>();
+  bp.d_uslot = (const int32_t *)(ctx->d_in.as<uint8_t>() + i_slot);
+  bp.d_err = ctx->d_out.as<unsigned>();
+  memcpy(bp.h_tab, bp.sets.data(), sizeof(BatchSet));
+  *ctx->h_stage.as<int64_t>(i_slot) = 0;
+  memcpy(ctx->h_stage.as<uint8_t>(i_mask), m.data(), 8 * W);
+  CK(cudaMemcpyAsync(ctx->d_in.p, ctx->h_stage.p, i_mask + 8 * W, cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemsetAsync(ctx->d_out.p, 0, 8, ctx->stream));
+  rc = launch_pairs_any(ctx, bp, (const uint64_t *)(ctx->d_in.as<uint8_t>() + i_mask),
+                        ctx->d_dmask.as<uint32_t>(), nullptr);
   if (rc) return rc;
   rc = check_mma_error(ctx, bp);
   if (rc) return rc;
