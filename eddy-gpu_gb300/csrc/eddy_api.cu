@@ -715,7 +715,7 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   bp.B = Bt;
   bp.sets.assign(ns, BatchSet{});
   bp.fp64 = true;
-  size_t dmw = 0, scb = 0;
+  size_t dmw = 0;
   for (int k = 0, u = 0; k < ns; k++) {
     BatchSet &b = bp.sets[k];
     b.sd = ctx->res_sd[k];
@@ -728,9 +728,6 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
     b.nb = nb;
     b.dm0 = (long long)dmw;
     dmw += dmask_words(nb, b.sd.c);
-    b.unit_bytes = (long long)unit_scratch_bytes(b.sd.c, S);
-    b.sc0 = (long long)scb;
-    scb += (size_t)nb * b.unit_bytes;
     bp.gmax = std::max(bp.gmax, b.sd.g);
     bp.cmax = std::max(bp.cmax, b.sd.c);
     bp.fp64 = bp.fp64 && use_popc(b.sd);
@@ -764,7 +761,10 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
     int rc = dmask_ready(ctx, sizeof(uint32_t) * std::max<size_t>(dmw, 1));
     if (rc) return rc;
   }
-  CK(ctx->d_scratch.ensure(std::max<size_t>(scb, 1)));
+  BatchDev bd{};
+  bd.B = Bt;
+  plan_units(bd, bp.gmax, n, ctx->sms);
+  CK(ctx->d_scratch.ensure(bd.lay.total * (size_t)(bd.blocks + nk)));
   // uploads, in one copy: [set table][slots][kept slots], then the labellings'
   // masks, or the sets and permutations they are drawn from.  (A batch of
   // one unit is bound by its copies, launches and their gaps: with one copy
@@ -776,7 +776,7 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   const size_t i_lab = (i_keep + 4 * Bz + 255) & ~(size_t)255;
   const size_t in_bytes = i_lab + (masks_host ? 8 * Bz * W : 8 * Bz);
   // results, in one copy: [JS][U][status], then, 0 before the batch, the error
-  // word, the sets' decision counters and the kept units' table
+  // word, the unit kernel's counter of units taken, the sets' decision counters and the kept units' table
   const size_t o_U = 8 * Bz, o_st = o_U + 4 * Bz, o_err = o_st + 4 * Bz, o_cnt = o_err + 8;
   const size_t o_km = o_cnt + 32 * (size_t)ns;
   const size_t out_bytes = o_km + sizeof(KeepMeta) * (size_t)(nk + 1);
@@ -822,8 +822,6 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   bp.uploaded = vknown;
   CK(cudaMemcpyAsync(din, ctx->h_stage.p, in_bytes, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemsetAsync(dout + o_err, 0, out_bytes - o_err, ctx->stream));
-  BatchDev bd{};
-  bd.B = Bt;
   bd.nsets = ns;
   bd.memo_max = kMemoMax;
   if (const char *em = getenv("EDDY_MEMO_MAX")) bd.memo_max = std::max(0, std::min(kMemoMax, atoi(em)));
@@ -832,6 +830,7 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   bd.masks = masks_host ? (const uint64_t *)(din + i_lab) : ctx->d_masks.as<uint64_t>();
   bd.dmask = ctx->d_dmask.as<uint32_t>();
   bd.scratch = ctx->d_scratch.as<uint8_t>();
+  bd.taken = (unsigned *)(dout + o_err + 4);
   bd.js = (double *)dout;
   bd.U = (int32_t *)(dout + o_U);
   bd.status = (uint32_t *)(dout + o_st);
@@ -864,7 +863,7 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
       if (rc) return rc;
     }
     CK(record(ctx->ev[1], capturing));
-    CK(launch_units(bd, bp.gmax, W, ctx->stream));
+    CK(launch_units(bd, ctx->stream));
     CK(launch_pack(bd, nk, S, ctx->stream));
     CK(record(ctx->ev[2], capturing));
     ctx->launches += 1 + (nk > 0);  // networks, normalisation and JS; kept lists
@@ -923,7 +922,7 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
                                   layout_core(v), ns == 1 ? bp.sets[0].sd.g : 0, ctx->ev[4],
                                   true));
           cap_ck(record(ctx->ev[1], true));
-          cap_ck(launch_units(bd, bp.gmax, W, ctx->stream));
+          cap_ck(launch_units(bd, ctx->stream));
           cap_ck(record(ctx->ev[2], true));
           ctx->launches += 1 + mma_launches() + 1;
         }
@@ -1030,9 +1029,9 @@ int run_jobs(eddy_ctx *ctx, std::vector<Job> &jobs) {
     const int g = (int)ctx->sets[J.set_id].genes.size(), c = g * (g - 1) / 2;
     cmax = std::max(cmax, c);
     total += J.n_units;
-    per_unit_max = std::max(per_unit_max, unit_scratch_bytes(c, S) + 4 * (size_t)c + 8 * W + 64);
+    per_unit_max = std::max(per_unit_max, (J.keep ? unit_scratch_bytes(c, S) : 0) + 4 * (size_t)c + 8 * W + 64);
   }
-  // batch size: bounded by memory (masks, decisions and scratch, up to 16 GB),
+  // batch size: bounded by memory (masks, decisions, kept units' scratch, up to 16 GB),
   // by 16384 units (the general-path queue holds unit indices below 2^15)
   // and by the queue's room for every table of the batch (2^28): the units
   // are then split into batches of equal size (later calls of the same
@@ -1684,7 +1683,6 @@ int eddy_debug_edges(eddy_ctx *ctx, int set_id, const uint8_t *labels, uint8_t *
   bp.sets.assign(1, BatchSet{});
   bp.sets[0].sd = ctx->res_sd[0];
   bp.sets[0].nb = 1;
-  bp.sets[0].unit_bytes = 0;
   bp.gmax = bp.sets[0].sd.g;
   bp.cmax = bp.sets[0].sd.c;
   bp.fp64 = use_popc(bp.sets[0].sd);

@@ -103,10 +103,8 @@ struct BatchSet {
   int marg_b0;         // first block of its class-count work (4-cell layout)
   int pad_;
   long long dm0;       // u32 words: its decision masks, then its chunk bitmap
-  long long sc0;       // bytes: its per-unit scratch, unit_bytes per unit
   long long mg0;       // u32 words (4-cell layout): class counts [g][128
                        // mblocks], then the class-1 sizes [128 mblocks]
-  long long unit_bytes;
 };
 #ifdef __CUDACC__
 __device__ __forceinline__ uint32_t *unit_dmask(uint32_t *dmask, const BatchSet &bs, int u) {
@@ -152,6 +150,19 @@ EDDY_HD inline KeepLayout keep_layout(int g, int U, int E, int E2) {
 }
 
 // Per-batch pointers for the unit kernel.
+// Byte offsets of a unit's arrays in its block's scratch and in its shared
+// memory (eddy_kernels.cu), for the largest set of a batch.
+struct UnitLayout {
+  uint32_t phi[2], ent, ment, mdh, msc, vcan, sel, hs, dist, sig, urep, wl, vrep, ubits, htab;
+  uint32_t bkey, bsc, bpos, vcnt, krow, vinf, uv, vw, xs, dc, moves, cp;
+  uint32_t total;
+};
+struct UnitSlices {
+  uint32_t mA, mB, pcA, pcB, rows, cnt3, fcnt, fend, fps, fh, phs, phe, moff, nst, big, need, nobs;
+  uint32_t used, chg, dmap, itk, acc, tq, fsc, ent;
+  uint32_t total;
+};
+
 struct BatchDev {
   int B;                       // units in the batch
   int nsets;                   // sets in the batch
@@ -161,7 +172,13 @@ struct BatchDev {
   const int32_t *uslot;        // [B] set of each unit (index into sets)
   const uint64_t *masks;       // [B][W] class-1 sample mask per unit
   uint32_t *dmask;             // decision masks and chunk bitmaps (per set: dm0)
-  uint8_t *scratch;            // per-unit scratch (per set: sc0)
+  uint8_t *scratch;            // unit scratch: a slot of lay.total bytes per block of the
+                               // unit kernel, then one per kept unit
+  UnitLayout lay;
+  UnitSlices sm;
+  int blocks;                  // blocks of the unit kernel
+  unsigned *taken;             // units taken past the first of every block, 0 before
+                               // (not read when every unit has a block)
   double *js;                  // [B]
   int32_t *U;                  // [B]
   uint32_t *status;            // [B]

@@ -442,6 +442,8 @@ __device__ __forceinline__ uint32_t cells16(uint32_t fb) {
 // unit's variants fit unit_variants(g), which rows of up to five entries
 // always do.
 __host__ __device__ constexpr int unit_variants(int g) { return 62 * g + 64; }
+// variants whose sample words (variant_word) the unit's scratch keeps
+__host__ __device__ constexpr int kept_words(int g) { return 8 * g + 64; }
 // slots of the table of the lists formed per sample (in the unit's scratch)
 __host__ __device__ constexpr int big_slots(int g) {
   int s = 256;
@@ -451,24 +453,20 @@ __host__ __device__ constexpr int big_slots(int g) {
 // network table: slots held in shared memory (larger ones in the scratch)
 constexpr int kSmSlots = 4096;
 // genes of a set of c pairs (c = g (g - 1) / 2, so 1 + 8 c = (2 g - 1)^2)
-__host__ __device__ inline int genes_of_pairs(int c) {
+static int genes_of_pairs(int c) {
   int r = (int)sqrt((double)(1 + 8 * (long long)c));
   while ((long long)r * r > 1 + 8 * (long long)c) r--;
   while ((long long)(r + 1) * (r + 1) <= 1 + 8 * (long long)c) r++;
   return (r + 1) / 2;
 }
 
-struct UnitLayout {
-  size_t phi[2], ent, ment, mdh, msc, vcan, sel, hs, dist, sig, urep, wl, vrep, ubits, htab;
-  size_t bkey, bsc, bpos, vcnt, krow, cnt, lst, trig, cp, total;
-};
-__host__ __device__ inline UnitLayout unit_layout(int c, int S) {
+static UnitLayout unit_layout(int c, int S) {
   UnitLayout L;
   size_t o = 0;
   auto take = [&](size_t bytes) {
     const size_t at = o;
     o = (o + bytes + 255) & ~(size_t)255;
-    return at;
+    return (uint32_t)at;
   };
   const size_t cc = c > 0 ? c : 1;
   const int g = genes_of_pairs(c);
@@ -491,17 +489,19 @@ __host__ __device__ inline UnitLayout unit_layout(int c, int S) {
   L.vcnt = take(sizeof(uint16_t) * nv);         // their list lengths
   // a kept unit's rows, entry ranges (k_pack reads them)
   L.krow = take(sizeof(uint32_t) * (2 * (size_t)g * ((g + 31) / 32) + 4 * (size_t)g));
-  // per sample: how many rows it changes, and their variants, [rank][sample]
-  L.cnt = take(sizeof(int32_t) * (size_t)(S - 2));
-  L.lst = take(sizeof(uint16_t) * (size_t)(S - 2) * g);
-  L.trig = take(sizeof(uint32_t) * 64 * (size_t)((S - 2 + 31) / 32 + 1));
+  L.vinf = take(sizeof(uint32_t) * nv);         // variants: entries and subset (variant_info)
+  L.uv = take(sizeof(uint2) * nv);              // the used ones: number, info
+  L.vw = take(sizeof(uint32_t) * kept_words(g) * class_words(S - 2));  // words of the first ones
+  L.xs = take(2 * sizeof(int64_t) * (size_t)S); // per network: scores less the full one's
+  L.dc = take(sizeof(int32_t) * (size_t)S);     // and its lists' edges (kept units)
+  L.moves = take(sizeof(uint32_t) * 32 * ((size_t)(S - 2 + 63) / 64));  // pack_classes' masks
   L.cp = take(sizeof(uint2) * (size_t)g * ((S - 2) / 32 + 4));  // both classes' ClassPlanes
   L.bkey = take(sizeof(uint64_t) * nb);
   L.bsc = take(2 * sizeof(int64_t) * nb);
   L.bpos = take(sizeof(int32_t) * nb);
   for (int k = 0; k < 2; k++) L.phi[k] = take(sizeof(uint32_t) * cc);
   L.ent = take(2 * sizeof(uint2) * cc);
-  L.total = o;
+  L.total = (uint32_t)o;
   return L;
 }
 
@@ -533,42 +533,6 @@ __device__ __forceinline__ T block_scan(T v, T &total, T *sbuf) {
   return excl;
 }
 
-struct UnitSmem {
-  // fixed part; variable arrays follow in dynamic shared memory
-  SetDev sd;    // the unit's set (copied from the batch's set table)
-  unsigned long long HF[2];  // hashes of the two full networks
-  long long base[2][2];      // [data class][full network of class]
-  int flen[2];  // edges of the full networks' capped lists (kept units)
-  int ndab;     // nodes whose full lists differ between the classes
-  int split[3]; // class 2's first memo entry, first variant, first memo row
-  int nbig[2];  // rows formed per sample, per class
-  int firstB0;  // first class-2 network equal to the class-2 full network
-  int nchg;     // networks that differ from their class's full network
-  int nver;     // networks merged by hash
-  int nsel;     // variants to score
-  int any;
-  unsigned status;
-  unsigned long long koff;  // a kept unit's region of the packed outputs
-  int scan[32];
-  unsigned long long scan64[32];
-  long long red[6][32];
-  double redd[3][32];
-};
-
-// BDeu work items (node scores) processed per round
-constexpr int kItems = 512;
-// the BDeu item arrays (keys, scores, task prefix) in one region that, with
-// the base scores behind it, also holds the variants' hashes and the entries'
-// trigger words while the networks are hashed, and then the network table
-constexpr size_t kWorkBytes = sizeof(unsigned long long) * kItems + 2 * sizeof(long long) * kItems +
-                              sizeof(int) * (2 * kItems + 4);
-static_assert(kSmSlots * sizeof(int) <= kWorkBytes && kWorkBytes % 16 == 0, "work region");
-// entries whose trigger words a unit's scratch holds (sample counts for
-// which the region above holds fewer than kMinTrig)
-constexpr int kTrigScratch = 64, kMinTrig = 16;
-// kept flip entries a unit holds in shared memory (more go to its scratch)
-constexpr int kEntCache = 1280;
-
 struct UnitPtrs {
   uint64_t *mA, *mB;      // [W]
   int *pcA, *pcB;         // [W]
@@ -582,57 +546,121 @@ struct UnitPtrs {
   int *moff;              // [2][g] variants of the rows before
   int *nst;               // [2][g] scratch of the compaction
   uint16_t *big;          // [2][g] rows formed per sample, per class
-  uint2 *rinfo;           // [2 g] the memo rows: first entry; entries | first variant << 8
   uint8_t *need;          // [g] 1 = full lists differ, 2 = scores needed
   uint8_t *nobs;          // [2][g] observed states per class
   uint32_t *used;         // [unit_variants / 32] variants some network uses
   unsigned long long *itk;   // [kItems] node-score items: t | np << 14 | parents
   long long *acc;            // [kItems][2] their scores per class
   int *tq;                   // [2 kItems + 1] task prefix per (item, class)
+  uint32_t *chg;             // [class_words of both classes] networks with a changed list
   int8_t *dmap;              // [96] divisor map (copy of the constant one)
   long long *fsc;            // [2 full][2 data][g] base node scores
   uint2 *ent;                // [kEntCache] the kept flip entries
-  size_t bytes;
 };
-__host__ __device__ inline UnitPtrs carve(char *base, int g, int W, int GW) {
-  UnitPtrs P;
+
+struct UnitSmem {
+  // fixed part; variable arrays follow in dynamic shared memory
+  SetDev sd;    // the unit's set (copied from the batch's set table)
+  UnitPtrs P;   // the variable arrays (for the functions not inlined)
+  unsigned long long HF[2];  // hashes of the two full networks
+  long long base[2][2];      // [data class][full network of class]
+  int flen[2];  // edges of the full networks' capped lists (kept units)
+  int ndab;     // nodes whose full lists differ between the classes
+  int split[2]; // class 2's first memo entry, first variant
+  int nbig[2];  // rows formed per sample, per class
+  int firstB0;  // first class-2 network equal to the class-2 full network
+  int nchg;     // networks that differ from their class's full network
+  int nver;     // networks merged by hash
+  int nsel;     // variants to score
+  int any;
+  int next[2];  // the block's next unit (by turns)
+  unsigned status;
+  unsigned long long koff;  // a kept unit's region of the packed outputs
+  int scan[32];
+  unsigned long long scan64[32];
+  long long red[6][32];
+  double redd[3][32];
+};
+
+// BDeu work items (node scores) processed per round
+constexpr int kItems = 512;
+// the BDeu item arrays (keys, scores, task prefix) in one region that also
+// holds the operands of the networks' sums (unit_walk) and then the network
+// table
+constexpr size_t kWorkBytes = sizeof(unsigned long long) * kItems + 2 * sizeof(long long) * kItems +
+                              sizeof(int) * (2 * kItems + 4);
+static_assert(kSmSlots * sizeof(int) <= kWorkBytes && kWorkBytes % 16 == 0, "work region");
+// kept flip entries a unit holds in shared memory (more go to its scratch)
+constexpr int kEntCache = 1280;
+
+static UnitSlices unit_slices(int g, int W) {
+  UnitSlices P;
+  const int GW = (g + 31) / 32;
   size_t o = sizeof(UnitSmem);
   auto take = [&](size_t bytes) {
     o = (o + 15) & ~(size_t)15;
-    char *p = base + o;
+    const size_t at = o;
     o += bytes;
-    return p;
+    return (uint32_t)at;
   };
-  P.mA = (uint64_t *)take(2 * sizeof(uint64_t) * W);
-  P.mB = P.mA + W;
-  P.pcA = (int *)take(2 * sizeof(int) * W);
-  P.pcB = P.pcA + W;
-  P.rows = (uint32_t *)take(2 * sizeof(uint32_t) * (size_t)g * GW);
-  P.cnt3 = (uint16_t *)take(2 * 3 * sizeof(uint16_t) * g);
-  P.fcnt = (uint16_t *)take(2 * sizeof(uint16_t) * g);
-  P.fend = (int16_t *)take(2 * sizeof(int16_t) * g);
-  P.fps = (uint16_t *)take(2 * 3 * sizeof(uint16_t) * g);
-  P.fh = (unsigned long long *)take(2 * sizeof(unsigned long long) * g);
-  P.phs = (int *)take(4 * sizeof(int) * g);
-  P.phe = P.phs + 2 * g;
-  P.moff = (int *)take(2 * sizeof(int) * g);
-  P.nst = (int *)take(2 * sizeof(int) * g);
-  P.big = (uint16_t *)take(2 * sizeof(uint16_t) * g);
-  P.rinfo = (uint2 *)take(2 * sizeof(uint2) * g);
-  P.need = (uint8_t *)take(g);
-  P.nobs = (uint8_t *)take(2 * g);
-  P.used = (uint32_t *)take(sizeof(uint32_t) * ((unit_variants(g) + 31) / 32));
-  P.dmap = (int8_t *)take(96);
+  P.mA = take(2 * sizeof(uint64_t) * W);
+  P.mB = P.mA + sizeof(uint64_t) * W;
+  P.pcA = take(2 * sizeof(int) * W);
+  P.pcB = P.pcA + sizeof(int) * W;
+  P.rows = take(2 * sizeof(uint32_t) * (size_t)g * GW);
+  P.cnt3 = take(2 * 3 * sizeof(uint16_t) * g);
+  P.fcnt = take(2 * sizeof(uint16_t) * g);
+  P.fend = take(2 * sizeof(uint16_t) * g);
+  P.fps = take(2 * 3 * sizeof(uint16_t) * g);
+  P.fh = take(2 * sizeof(unsigned long long) * g);
+  P.phs = take(4 * sizeof(int) * g);
+  P.moff = take(2 * sizeof(int) * g);
+  P.nst = take(2 * sizeof(int) * g);
+  P.big = take(2 * sizeof(uint16_t) * g);
+  P.need = take(g);
+  P.nobs = take(2 * g);
+  P.used = take(sizeof(uint32_t) * ((unit_variants(g) + 31) / 32));
+  P.chg = take(sizeof(uint32_t) * (2 * W + 2));
+  P.dmap = take(96);
   // (the base scores follow the work region directly)
-  P.itk = (unsigned long long *)take(kWorkBytes + 4 * sizeof(long long) * g);
-  P.acc = (long long *)(P.itk + kItems);
-  P.tq = (int *)(P.acc + 2 * kItems);
-  P.fsc = (long long *)((char *)P.itk + kWorkBytes);
-  P.ent = (uint2 *)take(sizeof(uint2) * kEntCache);
-  P.bytes = (o + 15) & ~(size_t)15;
+  P.itk = take(kWorkBytes + 4 * sizeof(long long) * g);
+  P.acc = P.itk + sizeof(unsigned long long) * kItems;
+  P.tq = P.acc + 2 * sizeof(long long) * kItems;
+  P.fsc = P.itk + kWorkBytes;
+  P.ent = take(sizeof(uint2) * kEntCache);
+  P.total = (uint32_t)((o + 15) & ~(size_t)15);
   return P;
 }
-static size_t unit_smem_bytes(int g, int W) { return carve(nullptr, g, W, (g + 31) / 32).bytes; }
+// (phe follows phs, both by the unit's own genes: they are copied as one)
+__device__ __forceinline__ UnitPtrs unit_ptrs(char *base, const UnitSlices &o, int g) {
+  UnitPtrs P;
+  P.mA = (uint64_t *)(base + o.mA);
+  P.mB = (uint64_t *)(base + o.mB);
+  P.pcA = (int *)(base + o.pcA);
+  P.pcB = (int *)(base + o.pcB);
+  P.rows = (uint32_t *)(base + o.rows);
+  P.cnt3 = (uint16_t *)(base + o.cnt3);
+  P.fcnt = (uint16_t *)(base + o.fcnt);
+  P.fend = (int16_t *)(base + o.fend);
+  P.fps = (uint16_t *)(base + o.fps);
+  P.fh = (unsigned long long *)(base + o.fh);
+  P.phs = (int *)(base + o.phs);
+  P.phe = P.phs + 2 * g;
+  P.moff = (int *)(base + o.moff);
+  P.nst = (int *)(base + o.nst);
+  P.big = (uint16_t *)(base + o.big);
+  P.need = (uint8_t *)(base + o.need);
+  P.nobs = (uint8_t *)(base + o.nobs);
+  P.used = (uint32_t *)(base + o.used);
+  P.chg = (uint32_t *)(base + o.chg);
+  P.dmap = (int8_t *)(base + o.dmap);
+  P.itk = (unsigned long long *)(base + o.itk);
+  P.acc = (long long *)(base + o.acc);
+  P.tq = (int *)(base + o.tq);
+  P.fsc = (long long *)(base + o.fsc);
+  P.ent = (uint2 *)(base + o.ent);
+  return P;
+}
 
 // Network s of a unit: class k (0 = class 1, 1 = class 2) and left-out
 // sample sigma (-1 for the two full networks), kernel1.cu:85-88, 412-416.
@@ -895,6 +923,236 @@ __device__ __noinline__ void pack_classes(const SetDev &sd, const UnitPtrs &P, u
   __syncthreads();
 }
 
+// Where a variant comes from: its row's first kept entry, their number and
+// the subset of them that fires.
+__device__ __forceinline__ uint32_t variant_info(int e0, int e, int sub) {
+  return (uint32_t)e0 | ((uint32_t)e << 14) | ((uint32_t)sub << 18);
+}
+__device__ __forceinline__ int info_first(uint32_t x) { return (int)(x & 0x3FFFu); }
+__device__ __forceinline__ int info_count(uint32_t x) { return (int)((x >> 14) & 15u); }
+__device__ __forceinline__ int info_end(uint32_t x) { return info_first(x) + info_count(x); }
+
+// The 32 samples of a class that fire an entry (t, j, cells): the OR over the
+// cells (a, b) of state a of node t and state b of column j.
+__device__ __forceinline__ uint32_t trigger_word(const uint2 *cw, uint2 en) {
+  const uint2 a = cw[(en.x >> 9) & 511u], b = cw[en.x & 511u];
+  const uint32_t j0 = ~(b.x | b.y), j1 = b.x & ~b.y, j2 = b.y & ~b.x;
+  auto cells = [&](uint32_t f) {
+    return ((f & 1u) ? j0 : 0u) | ((f & 2u) ? j1 : 0u) | ((f & 4u) ? j2 : 0u);
+  };
+  return (~(a.x | a.y) & cells(en.y)) | ((a.x & ~a.y) & cells(en.y >> 4)) |
+         ((a.y & ~a.x) & cells(en.y >> 8));
+}
+
+constexpr int kFewVariants = 16;
+constexpr int kUnitThreads = 256, kUnitWarps = kUnitThreads / 32, kUnitRegs = 80;
+
+// The samples of class word w that fire exactly the variant's subset of its
+// row's entries, from the class planes.
+__device__ __noinline__ uint32_t variant_word(const uint2 *cw, const uint2 *ent, uint32_t info) {
+  uint32_t x = ~0u, sub = info >> 18;
+  const uint2 *e = ent + info_first(info);
+  for (int j = info_count(info); j > 0; j--, e++, sub >>= 1)
+    x &= trigger_word(cw, *e) ^ ((sub & 1u) - 1u);
+  return x;
+}
+
+// Which of the variants [v0, v1) of a class of nk samples some left-out
+// sample changes its row to (P.used), which samples have a changed list
+// (chg), and the variants' words (vw[v][stride], the first `keep` variants').
+// 8, 16 or 32 words of the class at a time, a lane per variant and word; the
+// entries' trigger words are formed first, as many as `bytes` of the work
+// region hold, word by word (a warp's 32 entries share their nodes' planes;
+// an odd pitch keeps the lanes' words in different banks).
+__device__ __noinline__ void mark_variants(const UnitPtrs &P, const uint2 *cpw, int g, int nk,
+                                           uint32_t *chg, const uint2 *ent, const uint32_t *vinf,
+                                           const unsigned long long *mdh, int v0, int v1, uint32_t *vw,
+                                           int stride, int keep, int bytes) {
+  uint32_t *T = (uint32_t *)P.itk;
+  const int tid = threadIdx.x, lane = tid & 31, words = (nk + 31) >> 5;
+  const int lw = words <= 8 ? 3 : words <= 16 ? 4 : 5, nw = 1 << lw;
+  const int pitch = ((bytes >> (lw + 2)) - 1) | 1, w = tid & (nw - 1);
+  for (int w0 = 0; w0 < words; w0 += nw) {
+    const int live = min(nw, words - w0);
+    uint32_t c = 0u;
+    for (int q = v0, qe; q < v1; q = qe) {
+      const int e0 = info_first(vinf[q]);
+      qe = v1;
+      if (info_end(vinf[v1 - 1]) - e0 > pitch) {
+        // the longest run of variants whose rows' entries fit
+        int lo = q + 1;
+        while (lo < qe) {
+          const int mid = (lo + qe + 1) >> 1;
+          if (info_end(vinf[mid - 1]) - e0 <= pitch) lo = mid;
+          else qe = mid - 1;
+        }
+      }
+      const int ne = info_end(vinf[qe - 1]) - e0;
+      __syncthreads();
+      for (int i = tid, x = tid / ne, e = tid - x * ne; i < live * ne; i += kUnitThreads) {
+        T[x * pitch + e] = trigger_word(cpw + (size_t)(w0 + x) * g, ent[e0 + e]);
+        e += kUnitThreads;
+        while (e >= ne) e -= ne, x++;
+      }
+      __syncthreads();
+      const uint32_t *t0 = T + w * pitch - e0;
+#pragma unroll 2
+      for (int b = q; b < qe; b += kUnitThreads >> lw) {
+        const int v = b + (tid >> lw);
+        uint32_t x = 0u;
+        if (v < qe && w < live) {
+          const uint32_t info = vinf[v];
+          const uint32_t *t = t0 + info_first(info);
+          uint32_t sub = info >> 18;
+          x = ~0u;
+          for (int j = info_count(info); j > 0; j--, t++, sub >>= 1) x &= *t ^ ((sub & 1u) - 1u);
+          if (mdh[v] == 0ull) x = 0u;  // (0: the full list)
+          if (v < keep) vw[(size_t)v * stride + w0 + w] = x;
+        }
+        c |= x;
+        const uint32_t any = __ballot_sync(0xffffffffu, x != 0u) >> (lane & ~(nw - 1));
+        if (w == 0 && (any & (~0u >> (32 - nw)))) atomicOr(&P.used[v >> 5], 1u << (v & 31));
+      }
+    }
+    for (int o = nw; o < 32; o <<= 1) c |= __shfl_xor_sync(0xffffffffu, c, o);
+    if (lane < nw && c) atomicOr(&chg[w0 + w], c);
+  }
+}
+
+__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
+                                         uint32_t a3, uint2 b) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b.x), "r"(b.y));
+}
+
+// What the left-out samples of a class of nk change: for every sample the sum
+// over the used variants uv[0 .. nu) that it fires of the variant's hash
+// difference and of its two score differences (and, J = 4, of its list's
+// length difference), put(i, sums) for sample i of the class.
+//
+// The sums are a contraction of the samples' bits with the variants' values,
+// so they go through the matrix units: the values' eight bytes are the
+// columns of bf16 operand B (0 .. 255, exact), the bits, as 0 or 2, are
+// operand A (a sample fires at most one variant of a row, so a column sums to
+// at most 2 x 512 x 255: exact in FP32), and the bytes' sums are put together
+// modulo 2^64.  A warp takes 32 samples, eight words of the class at a time;
+// the variants go by in blocks of 160, the next one's words and values loaded
+// while this one's are multiplied.  mma.sync tiles, M = samples, N = 24, K =
+// variants: a block's operands are read once, so the descriptors, fences and
+// TMEM round trips of tcgen05.mma would cost more than the 60 instructions a
+// warp issues for it.  The bits pass into registers by shift and mask: a pair
+// of variants' words is held as its low and its high halves, so that bit r of
+// both variants lands in the exponents' top bits of one register.
+template <int J, class Word, class Value, class Put>
+__device__ __noinline__ void unit_walk(void *region, int nk, int nu, Word word, Value value,
+                                       Put put) {
+  constexpr int kK = 160;                                  // variants of a block
+  constexpr int kB = (kK / 2 * J + kUnitThreads - 1) / kUnitThreads;  // pairs of values
+  static_assert(kK * (4 * kUnitWarps + 16 * J) <= (int)kWorkBytes, "work region");
+  uint2 *A = (uint2 *)region;                              // [kK / 16][8 words][4][2]
+  uint32_t *B = (uint32_t *)(A + kK / 2 * kUnitWarps);     // [kK / 16][J][8][4][2]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, words = (nk + 31) >> 5;
+  const int r8 = lane >> 2, t4 = lane & 3, aw = tid & (kUnitWarps - 1), ap = tid / kUnitWarps;
+  const uint32_t sh0 = 14 - r8, sh1 = (6 - r8) & 31;
+  auto bits = [](uint32_t x, uint32_t sh) { return __funnelshift_l(x, x, sh) & 0x40004000u; };
+  constexpr int kPairs = kUnitThreads / kUnitWarps;          // pairs of operand A at a time
+  constexpr int kAp = (kK / 2 + kPairs - 1) / kPairs;
+  for (int w0 = 0; w0 < words; w0 += kUnitWarps) {
+    float acc[2][J][4];
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+      for (int j = 0; j < J; j++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) acc[m][j][q] = 0.f;
+    uint32_t xa[kAp][2];
+    unsigned long long xb[kB][2];
+    auto load = [&](int q) {
+#pragma unroll
+      for (int r = 0; r < kAp; r++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int p = ap + r * kPairs, i = q + 2 * p + h;
+          xa[r][h] = 2 * p < kK && i < nu && w0 + aw < words ? word(i, w0 + aw) : 0u;
+        }
+#pragma unroll
+      for (int r = 0; r < kB; r++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int x = tid + r * kUnitThreads, j = x / (kK / 2), i = q + 2 * (x - j * (kK / 2)) + h;
+          xb[r][h] = j < J && i < nu ? value(i, j) : 0ull;
+        }
+    };
+    load(0);
+    for (int q = 0; q < nu; q += kK) {
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < kAp; r++) {
+        const int p = ap + r * kPairs;
+        if (2 * p < kK)
+          A[(((p >> 3) * kUnitWarps + aw) * 4 + (p & 3)) * 2 + ((p >> 2) & 1)] = make_uint2(
+              __byte_perm(xa[r][0], xa[r][1], 0x5410), __byte_perm(xa[r][0], xa[r][1], 0x7632));
+      }
+#pragma unroll
+      for (int r = 0; r < kB; r++) {
+        const int x = tid + r * kUnitThreads, j = x / (kK / 2), p = x - j * (kK / 2);
+        if (j >= J) continue;
+        uint32_t *b = B + ((p >> 3) * J + j) * 64 + 2 * (p & 3) + ((p >> 2) & 1);
+#pragma unroll
+        for (int l = 0; l < 8; l++) {
+          // a byte as a float: 2^23 + x, less 2^23
+          float f[2];
+#pragma unroll
+          for (int h = 0; h < 2; h++)
+            f[h] = __uint_as_float(__byte_perm((uint32_t)(xb[r][h] >> (l < 4 ? 0 : 32)), 0x4B000000u,
+                                               0x7540u + (l & 3))) - 8388608.f;
+          b[8 * l] = __byte_perm(__float_as_uint(f[0]), __float_as_uint(f[1]), 0x7632);
+        }
+      }
+      __syncthreads();
+      if (q + kK < nu) load(q + kK);
+      if (w0 + warp < words) {
+        const int steps = (min(kK, nu - q) + 15) >> 4;
+        const uint4 *a4 = reinterpret_cast<const uint4 *>(A) + warp * 4 + t4;
+        const uint2 *b2 = reinterpret_cast<const uint2 *>(B) + lane;
+        for (int ks = 0; ks < steps; ks++, a4 += 4 * kUnitWarps, b2 += 32 * J) {
+          const uint4 a = *a4;
+          const uint32_t l0 = bits(a.x, sh0), l1 = bits(a.x, sh1), l2 = bits(a.z, sh0), l3 = bits(a.z, sh1);
+          const uint32_t h0 = bits(a.y, sh0), h1 = bits(a.y, sh1), h2 = bits(a.w, sh0), h3 = bits(a.w, sh1);
+#pragma unroll
+          for (int j = 0; j < J; j++) {
+            const uint2 b = b2[32 * j];
+            mma_bf16(acc[0][j], l0, l1, l2, l3, b);
+            mma_bf16(acc[1][j], h0, h1, h2, h3, b);
+          }
+        }
+      }
+    }
+    if (w0 + warp >= words) continue;
+    // a lane's two bytes' sums of samples r8 + 8 x, the four lanes' together
+    // the value's; lane t4 keeps sample r8 + 8 t4
+    unsigned long long sum[J];
+#pragma unroll
+    for (int j = 0; j < J; j++) {
+      sum[j] = 0ull;
+#pragma unroll
+      for (int x = 0; x < 4; x++) {
+        const unsigned lo = (unsigned)(acc[x >> 1][j][2 * (x & 1)] * 0.5f);
+        const unsigned hi = (unsigned)(acc[x >> 1][j][2 * (x & 1) + 1] * 0.5f);
+        unsigned long long y = ((unsigned long long)lo + ((unsigned long long)hi << 8)) << (16 * t4);
+        y += __shfl_xor_sync(0xffffffffu, y, 1);
+        y += __shfl_xor_sync(0xffffffffu, y, 2);
+        if (x == t4) sum[j] = y;
+      }
+    }
+    const int i = 32 * (w0 + warp) + r8 + 8 * t4;
+    if (i < nk) put(i, sum);
+  }
+}
+
 // Normalisation (main.cu:1302-1404) and JS (main.cu:1406-1428) of a unit
 // from its unique networks' node-summed fixed-point scores dist[U], dist[S
 // + U]: per class min, max and mean of the scores (exact integers),
@@ -1033,18 +1291,17 @@ static __device__ __noinline__ double unit_js(long long *dist, int S, int U, Uni
 // JS, then 6.0 ms more), 301 units of 387 x 600 35.0 against 4.6 ms.  Bound by
 // issue (1.3 million warp instructions a unit at that shape), about half of
 // them in the node scores.
-__global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
-  extern __shared__ __align__(16) char smraw[];
+__device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw) {
   UnitSmem &SM = *reinterpret_cast<UnitSmem *>(smraw);
   const int nw = blockDim.x >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tid = threadIdx.x, nt = blockDim.x;
-  const int u = blockIdx.x;
   // the unit's set: its descriptor into shared memory, its slices of the
-  // batch's masks and scratch
+  // batch's masks
   const BatchSet &bs = bd.sets[bd.uslot[u]];
   const int ul = u - bs.u0, bs_nb = bs.nb;
   const long long bs_dm0 = bs.dm0;
-  uint8_t *scr = bd.scratch + bs.sc0 + (size_t)ul * bs.unit_bytes;
+  const int keep = bd.keep_slot ? bd.keep_slot[u] : -1;
+  uint8_t *scr = bd.scratch + (size_t)(keep < 0 ? (int)blockIdx.x : bd.blocks + keep) * bd.lay.total;
   {
     const int *src = reinterpret_cast<const int *>(&bs.sd);
     int *dst = reinterpret_cast<int *>(&SM.sd);
@@ -1054,7 +1311,6 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
   __syncthreads();
   const SetDev &sd = SM.sd;
   const int g = sd.g, W = sd.W, GW = sd.GW, S = sd.S, c = sd.c, nA = sd.nA, nB = sd.nB;
-  const int keep = bd.keep_slot ? bd.keep_slot[u] : -1;
   uint32_t *ucb = bd.dmask + bs_dm0 + (size_t)bs_nb * c + (size_t)ul * chunk_words(c);
   uint32_t *dm = bd.dmask + bs_dm0 + (size_t)ul * c;
   // a unit without a nonzero mask has empty networks only: one unique
@@ -1071,8 +1327,9 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
     }
     return;
   }
-  const UnitPtrs P = carve(smraw, g, W, GW);
-  const UnitLayout L = unit_layout(c, S);
+  const UnitPtrs P = unit_ptrs(smraw, bd.sm, g);
+  const UnitLayout &L = bd.lay;
+  if (tid == 0) SM.P = P;
   uint32_t *phi[2] = {(uint32_t *)(scr + L.phi[0]), (uint32_t *)(scr + L.phi[1])};
   long long *dist = (long long *)(scr + L.dist);
   int *sig = (int *)(scr + L.sig);
@@ -1086,7 +1343,7 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
     SM.nbig[0] = SM.nbig[1] = 0;
     SM.firstB0 = S - 1;
     SM.nchg = SM.nver = SM.nsel = 0;
-    SM.split[0] = SM.split[1] = SM.split[2] = 0;
+    SM.split[0] = SM.split[1] = 0;
     for (int a = 0; a < 2; a++)
       for (int b = 0; b < 2; b++) SM.base[a][b] = 0;
   }
@@ -1098,6 +1355,7 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
   for (int i = tid; i < 2 * g * GW; i += nt) P.rows[i] = 0;
   // entry ranges of rows: start = INT_MAX, end = 0 until an entry lands
   for (int i = tid; i < 4 * g; i += nt) P.phs[i] = (i < 2 * g) ? 0x7fffffff : 0;
+  for (int i = tid; i < 2 * W + 2; i += nt) P.chg[i] = 0u;
   for (int i = tid; i < 82; i += nt) P.dmap[i] = c_dmap[i];
   __syncthreads();
 
@@ -1232,14 +1490,13 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
   // the variants of the rows before (a variant's row is the last one whose
   // moff is not past it).
   const uint2 *ent = P.ent;
-  int nmemo = 0, nvar = 0, nmr = 0, E = bd.memo_max;
+  int nmemo = 0, nvar = 0, E = bd.memo_max;
   auto memo_row = [&](int i, int e) {
     return e >= 1 && e <= E && (1 << e) <= (i < g ? nA : nB) + 8;
   };
   if (entries) {
-    // packed: memo entries (14 bits), memo rows (11), other entries (20),
-    // variants (19)
-    constexpr int kR = 14, kO = 25, kV = 45;
+    // packed: memo entries (14 bits), other entries (20), variants (30)
+    constexpr int kO = 14, kV = 34;
     unsigned long long running;
     while (true) {
       running = 0ull;
@@ -1248,19 +1505,17 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
         const int e = (i < 2 * g && P.phs[i] < P.phe[i]) ? P.phe[i] - P.phs[i] : 0;
         const bool mr = memo_row(i, e);
         const unsigned long long v =
-            mr ? (unsigned long long)e | (1ull << kR) | ((unsigned long long)((1 << e) - 1) << kV)
+            mr ? (unsigned long long)e | ((unsigned long long)((1 << e) - 1) << kV)
                : (unsigned long long)e << kO;
         unsigned long long total;
         const unsigned long long off = running + block_scan(v, total, SM.scan64);
         if (i < 2 * g) {
-          const int me = (int)(off & ((1u << kR) - 1)), row = (int)((off >> kR) & 0x7FF);
+          const int me = (int)(off & ((1u << kO) - 1));
           P.moff[i] = (int)(off >> kV);
           P.nst[i] = mr ? me : (int)((off >> kO) & 0xFFFFF);
-          if (mr) P.rinfo[row] = make_uint2((unsigned)me, (unsigned)e | ((unsigned)P.moff[i] << 8));
           if (i == g) {
             SM.split[0] = me;
             SM.split[1] = P.moff[i];
-            SM.split[2] = row;
           }
         }
         running += total;
@@ -1270,8 +1525,7 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
       E--;
       __syncthreads();
     }
-    nmemo = (int)(running & ((1u << kR) - 1));
-    nmr = (int)((running >> kR) & 0x7FF);
+    nmemo = (int)(running & ((1u << kO) - 1));
     const int nbig = (int)((running >> kO) & 0xFFFFF);
     uint2 *dst = nmemo + nbig <= kEntCache ? P.ent : (uint2 *)(scr + L.ent);
     ent = dst;
@@ -1368,14 +1622,8 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
   // and hash of each list that differs from the full one
   unsigned long long *ment = (unsigned long long *)(scr + L.ment);
   uint16_t *vcnt = (uint16_t *)(scr + L.vcnt);
-  const int n = sd.n, W32 = 2 * W;
-  // the work region: the variants' hashes, if room for the trigger words of
-  // 64 entries is left, then the trigger words (of tcap entries)
-  const size_t region = kWorkBytes + 4 * sizeof(long long) * (size_t)g;
-  const size_t mdhb = (8 * (size_t)nvar + 15) & ~(size_t)15;
-  const bool mdh_sm = mdhb + 4 * (size_t)W32 * 64 <= region;
-  unsigned long long *mdh = mdh_sm ? P.itk : (unsigned long long *)(scr + L.mdh);
-  const int tcap_sm = (int)((region - (mdh_sm ? mdhb : 0)) / (4 * (size_t)W32));
+  unsigned long long *mdh = (unsigned long long *)(scr + L.mdh);
+  uint32_t *vinf = (uint32_t *)(scr + L.vinf);
   for (int v = tid; v < nvar; v += nt) {
     int lo = 0, hi = 2 * g - 1;
     while (lo < hi) {
@@ -1414,6 +1662,7 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
     }
     ment[v] = key;
     mdh[v] = dh;
+    vinf[v] = variant_info(e0, e1 - e0, sub);
     if (keep >= 0) vcnt[v] = (uint16_t)len;
   }
   // sample lists of both classes in index order (network -> left-out
@@ -1477,154 +1726,287 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
     }
     return -1;
   };
-  // ---- P3: what the left-out samples change.  An entry (t, j, cells) fires
-  // for the samples whose states lie in its cells: the OR over the cells (a,
-  // b) of plane(t, a) & plane(j, b), formed 32 samples at a time (its trigger
-  // words), for as many memo rows at a time as the region holds.  Then a lane
-  // takes one sample of the class, a warp 32, and walks the rows: the bits of
-  // a row's entries name the variant the sample changes the row to.  Its hash
-  // difference goes into the network's hash, and the variant, unless it
-  // leaves the row's list as it is, on the sample's list, from which the
-  // scores are summed later.  Cycles of a block for this and the sums, 200
-  // genes x 1000 samples near the threshold: 350k + 95k; a byte per row and
-  // sample instead of the lists, stored and read coalesced, 309k + 298k; a
-  // walk over packed states for each, 295k + 468k.
-  uint16_t *lst = (uint16_t *)(scr + L.lst);
-  int *cng = (int *)(scr + L.cnt);
+  // ---- P3: which variants the left-out samples change their rows to, and
+  // which samples have a changed list (both from the trigger words of the
+  // entries, 32 samples of a class at a time)
+  const int n = sd.n, vsplit = SM.split[1];
   unsigned long long *hs = (unsigned long long *)(scr + L.hs);
   auto as_key = [](unsigned long long h) { return h == ~0ull ? ~1ull : h; };
-  // (trig and mdh in shared memory or not, for the compiler to see)
-  auto walk = [&](uint32_t *__restrict__ trig, int tcap,
-                  const unsigned long long *__restrict__ mdh) {
-    int wpr = 1;  // lanes per entry
-    while (wpr < W32 && wpr < 32) wpr <<= 1;
-    const uint32_t *__restrict__ pl32 = reinterpret_cast<const uint32_t *>(sd.planes);
-    for (int k = 0; k < 2; k++) {
-      const int nk = k ? nB : nA, sk = k ? nA : 0, nch = (nk + 31) >> 5;
-      const int rend = k ? nmr : SM.split[2];
-      int r0 = k ? SM.split[2] : 0;
-      bool first = true;
-      do {
-        // rows [r0, r1), entries [e0, e1)
-        const int e0 = r0 < rend ? (int)P.rinfo[r0].x : 0;
-        int lo = r0, hi = rend;
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          const uint2 ri = P.rinfo[mid - 1];
-          if ((int)ri.x + (int)(ri.y & 0xFFu) - e0 <= tcap) lo = mid;
-          else hi = mid - 1;
-        }
-        const int r1 = lo;
-        const int e1 = r1 > r0 ? (int)(P.rinfo[r1 - 1].x + (P.rinfo[r1 - 1].y & 0xFFu)) : e0;
-        __syncthreads();
-#pragma unroll 2
-        for (int e = e0 + (warp * 32 + lane) / wpr; e < e1; e += nt / wpr) {
-          const uint2 en = ent[e];
-          const uint32_t *pt = pl32 + (size_t)((en.x >> 9) & 511u) * 3 * W32;
-          const uint32_t *pj = pl32 + (size_t)(en.x & 511u) * 3 * W32;
-          for (int w = lane & (wpr - 1); w < W32; w += wpr) {
-            const uint32_t t0 = __ldg(pt + w), t1 = __ldg(pt + W32 + w), t2 = __ldg(pt + 2 * W32 + w);
-            const uint32_t j0 = __ldg(pj + w), j1 = __ldg(pj + W32 + w), j2 = __ldg(pj + 2 * W32 + w);
-            auto cells = [&](uint32_t f) {
-              return ((f & 1u) ? j0 : 0u) | ((f & 2u) ? j1 : 0u) | ((f & 4u) ? j2 : 0u);
-            };
-            trig[(e - e0) * W32 + w] =
-                (t0 & cells(en.y)) | (t1 & cells(en.y >> 4)) | (t2 & cells(en.y >> 8));
-          }
-        }
-        __syncthreads();
-        for (int ch = warp; ch < nch; ch += nw) {
-          const int i = 32 * ch + lane;
-          const bool live = i < nk;
-          const int s = 1 + sk + (live ? i : nk - 1), sg = sig[s - 1];
-          const uint32_t *tw = trig + (sg >> 5);
-          const int sh = sg & 31;
-          unsigned long long dh = 0ull;
-          int c = first ? 0 : cng[sg];
-          unsigned at = (unsigned)c * (unsigned)n + (unsigned)sg;
-          constexpr int kRows = 4;
-          for (int r = r0; r < r1; r += kRows) {
-            uint2 ri[kRows];
-            unsigned x[kRows];
-#pragma unroll
-            for (int q = 0; q < kRows; q++) ri[q] = P.rinfo[r + q < r1 ? r + q : r1 - 1];
-#pragma unroll
-            for (int q = 0; q < kRows; q++) x[q] = tw[(ri[q].x - (unsigned)e0) * W32];
-#pragma unroll
-            for (int q = 0; q < kRows; q++) {
-              if (r + q >= r1) break;
-              const int cnt = (int)(ri[q].y & 0xFFu);
-              const uint32_t *tr = tw + (ri[q].x - (unsigned)e0) * W32;
-              unsigned sub = (x[q] >> sh) & 1u;
-              for (int j = 1; j < cnt; j++) sub |= ((tr[j * W32] >> sh) & 1u) << j;
-              if (sub) {
-                const int v = (int)(ri[q].y >> 8) + (int)sub - 1;
-                const unsigned long long d = mdh[v];
-                if (d) {  // (0: the full list)
-                  dh += d;
-                  if (!((P.used[v >> 5] >> (v & 31)) & 1u)) atomicOr(&P.used[v >> 5], 1u << (v & 31));
-                  lst[at] = (uint16_t)v;
-                  at += (unsigned)n;
-                  c++;
-                }
-              }
-            }
-          }
-          if (live) {
-            hs[s] = (first ? SM.HF[k] : hs[s]) + dh;
-            cng[sg] = c;
-          }
-        }
-        r0 = r1;
-        first = false;
-      } while (r0 < rend);
+  uint2 *cpw = (uint2 *)(scr + L.cp);
+  const int cw1 = class_words(nA);
+  const ClassPlanes cp[2] = {{cpw, g, cw1}, {cpw + (size_t)cw1 * g, g, class_words(nB)}};
+  if (networks || SM.ndab) pack_classes(sd, SM.P, (uint32_t *)(scr + L.moves), cpw);
+  uint2 *uv = (uint2 *)(scr + L.uv);
+  uint32_t *vw = (uint32_t *)(scr + L.vw);
+  const int vws = max(cw1, class_words(nB));
+  int nul = 0, ulsplit = 0;
+  if (entries) {
+    // (the base scores' room behind the work region is free until then)
+    const int room = (int)(kWorkBytes + 4 * sizeof(long long) * (size_t)g);
+    if (vsplit > 0)
+      mark_variants(SM.P, cp[0].p, g, nA, P.chg, ent, vinf, mdh, 0, vsplit, vw, vws, kept_words(g), room);
+    if (nvar > vsplit)
+      mark_variants(SM.P, cp[1].p, g, nB, P.chg + cw1, ent, vinf, mdh, vsplit, nvar, vw, vws,
+                    kept_words(g), room);
+    // the rows formed per sample: their hash differences, and their keys
+    // into the table
+    for (int s0 = 32 * warp; nbigs && s0 < n; s0 += nt) {
+      const int s = 1 + s0 + lane;
+      if (s > n) continue;
+      const int k = s <= nA ? 0 : 1, sg = sig[s - 1], i = s - 1 - (k ? nA : 0);
+      unsigned long long dh = 0ull;
+      bool chg = false;
+      for (int r = 0; r < SM.nbig[k]; r++) {
+        const int t = P.big[k * g + r];
+        unsigned long long key, h;
+        int len;
+        if (!sample_list(sd, SM.P, ent, k, t, sg, key, h, len)) continue;
+        const unsigned long long d = h - P.fh[k * g + t];
+        if (d == 0ull) atomicOr(&SM.status, kUnitHashCollision);
+        dh += d;
+        chg = true;
+        if (differs(k, key)) big_slot(key, true);
+      }
+      hs[s] = dh;
+      if (chg) atomicOr(&P.chg[(k ? cw1 : 0) + (i >> 5)], 1u << (i & 31));
     }
     __syncthreads();
-  };
-  // the rows formed per sample, and the changed networks counted
-  auto finish = [&]() {
-    for (int s0 = 32 * warp; s0 < n; s0 += nt) {
-      const int s = 1 + s0 + lane;
-      const bool live = s0 + lane < n;
-      const int k = s <= nA ? 0 : 1, sg = live ? sig[s - 1] : 0;
-      unsigned long long dh = live ? hs[s] : 0ull;
-      bool chg = live && cng[sg] > 0;
-      for (int kk = 0; kk < 2; kk++)
-        for (int r = 0; r < SM.nbig[kk]; r++) {
-          if (!live || k != kk) continue;
-          const int t = P.big[k * g + r];
-          unsigned long long key, h;
-          int len;
-          if (!sample_list(sd, P, ent, k, t, sg, key, h, len)) continue;
-          const unsigned long long d = h - P.fh[k * g + t];
-          if (d == 0ull) atomicOr(&SM.status, kUnitHashCollision);
-          dh += d;
-          chg = true;
-          if (differs(k, key)) big_slot(key, true);
-        }
-      if (live) hs[s] = chg ? as_key(dh) : ~0ull;
-      const unsigned nc = __ballot_sync(0xffffffffu, live && chg);
-      const int first0 = __reduce_min_sync(0xffffffffu, (k && live && !chg) ? s : S - 1);
-      if (lane == 0) {
-        if (nc) atomicAdd(&SM.nchg, __popc(nc));
-        if (first0 < S - 1) atomicMin(&SM.firstB0, first0);
-      }
+    // changed networks, the first unchanged one of class 2
+    for (int i = tid; i < cw1 + class_words(nB); i += nt) {
+      const uint32_t x = P.chg[i];
+      if (x) atomicAdd(&SM.nchg, __popc(x));
+      const int at = 32 * (i - cw1), left = nB - at;
+      if (at < 0 || left <= 0) continue;
+      const uint32_t same = ~x & (left >= 32 ? ~0u : (1u << left) - 1u);
+      if (same) atomicMin(&SM.firstB0, 1 + nA + at + __ffs(same) - 1);
     }
-  };
-  if (entries) {
-    uint32_t *tr_sm = (uint32_t *)P.itk;
-    const unsigned long long *gdh = (const unsigned long long *)(scr + L.mdh);
-    if (tcap_sm < kMinTrig) walk((uint32_t *)(scr + L.trig), kTrigScratch, gdh);
-    else if (mdh_sm) walk((uint32_t *)((char *)P.itk + mdhb), tcap_sm, P.itk);
-    else walk(tr_sm, tcap_sm, gdh);
-    finish();
-  } else if (tid == 0) {
-    SM.firstB0 = nA + 1;  // the first class-2 network
+    // the used variants in order
+    for (int w0 = 0; w0 < (nvar + 31) >> 5; w0 += nt) {
+      const int w = w0 + tid;
+      const uint32_t word = w < (nvar + 31) >> 5 ? P.used[w] : 0u;
+      int total;
+      int at = nul + block_scan(__popc(word), total, SM.scan);
+      for (uint32_t x = word; x; x &= x - 1) {
+        const int v = 32 * w + __ffs(x) - 1;
+        uv[at++] = make_uint2((unsigned)v, vinf[v]);
+      }
+      nul += total;
+    }
+    __syncthreads();
+    int hi = nul;  // class 1's
+    while (ulsplit < hi) {
+      const int mid = (ulsplit + hi) >> 1;
+      if ((int)uv[mid].x < vsplit) ulsplit = mid + 1;
+      else hi = mid;
+    }
+  } else {
+    if (tid == 0) SM.firstB0 = nA + 1;  // the first class-2 network
+    __syncthreads();
   }
-  __syncthreads();
   const int firstB0 = SM.firstB0;
 
-  // ---- P4: first-occurrence dedup.  Networks without changed nodes are
+  auto report = [&](int U) {
+    if (tid != 0) return;
+    bd.js[u] = __longlong_as_double(0x7ff8000000000000ll);
+    bd.U[u] = SM.status ? -1 : U;
+    bd.status[u] = SM.status;
+    if (bd.stats) atomicAdd(&bd.stats[4 * (size_t)bd.uslot[u] + 3], (unsigned long long)(S - U));
+  };
+  // one network has no JS (the range of its scores is empty), whatever its
+  // score is
+  if ((SM.nchg == 0 && !SM.ndab && keep < 0) || SM.status) {
+    report(1);
+    return;
+  }
+
+  // ---- P4: BDeu.  The JS takes only differences of the networks' scores,
+  // so the nodes that every network scores alike are left out (unless the
+  // scores themselves are kept): needed are the nodes whose full lists
+  // differ between the classes and those of rows with entries.
+  for (int i = tid; i < g * 3; i += nt) {
+    // state counts per class from the word-major planes: a warp's loads of
+    // a word are 32 consecutive planes
+    const uint64_t *pl = sd.planesT + i;
+    int a = 0, b = 0;
+    for (int w = 0; w < W; w++) {
+      const uint64_t x = pl[(size_t)w * 3 * g];
+      a += __popcll(x & P.mA[w]);
+      b += __popcll(x & P.mB[w]);
+    }
+    P.cnt3[i] = (uint16_t)a;
+    P.cnt3[3 * g + i] = (uint16_t)b;
+  }
+  __syncthreads();
+  for (int i = tid; i < 2 * g; i += nt) {
+    const uint16_t *c3 = P.cnt3 + 3 * i;
+    P.nobs[i] = (uint8_t)((c3[0] > 0) + (c3[1] > 0) + (c3[2] > 0));
+  }
+  for (int t = tid; t < g; t += nt)
+    if (keep >= 0 || P.need[t] || P.phs[t] < P.phe[t] || P.phs[g + t] < P.phe[g + t]) P.need[t] |= 2;
+  for (int i = tid; i < 4 * g; i += nt) P.fsc[i] = 0;
+  __syncthreads();
+  // base scores of the needed nodes in the two full networks; a class-2
+  // node whose first parents equal the class-1 one's copies its scores
+  auto same_as_class1 = [&](int t) -> bool {
+    const int a = P.fcnt[t] < 3 ? P.fcnt[t] : 3, b = P.fcnt[g + t] < 3 ? P.fcnt[g + t] : 3;
+    if (a != b) return false;
+    for (int q = 0; q < a; q++)
+      if (P.fps[t * 3 + q] != P.fps[(g + t) * 3 + q]) return false;
+    return true;
+  };
+  bdeu_items(
+      sd, P, cp, SM.scan, 2 * g,
+      [&](int i) -> unsigned long long {
+        const int k = i >= g ? 1 : 0, t = i - k * g;
+        if (!(P.need[t] & 2) || (k == 1 && same_as_class1(t))) return ~0ull;
+        const int ps[3] = {P.fps[i * 3], P.fps[i * 3 + 1], P.fps[i * 3 + 2]};
+        return list_key(t, P.fcnt[i], ps);
+      },
+      [&](int i, unsigned long long key, long long s1, long long s2) {
+        if (key == ~0ull) return;
+        const int k = i >= g ? 1 : 0, t = i - k * g;
+        P.fsc[(k * 2 + 0) * g + t] = s1;
+        P.fsc[(k * 2 + 1) * g + t] = s2;
+      });
+  for (int t = tid; t < g; t += nt)
+    if ((P.need[t] & 2) && same_as_class1(t)) {
+      P.fsc[(1 * 2 + 0) * g + t] = P.fsc[(0 * 2 + 0) * g + t];
+      P.fsc[(1 * 2 + 1) * g + t] = P.fsc[(0 * 2 + 1) * g + t];
+    }
+  __syncthreads();
+  if (warp < 4) {
+    // warp 2 k + cls: the sum of full network k's scores over class cls
+    long long s = 0;
+    for (int t = lane; t < g; t += 32) s += P.fsc[warp * g + t];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) SM.base[warp & 1][warp >> 1] = s;
+  }
+  // the used variants' distinct keys, and the keys of the lists formed per
+  // sample, scored once each.  A table in the work region (free between the
+  // two rounds of scores) gives each key its first variant: 38 bits of key
+  // (genes below 512) and 16 of the variant a slot.  A variant that finds no
+  // room is scored on its own.
+  longlong2 *msc = (longlong2 *)(scr + L.msc);
+  longlong2 *bsc = (longlong2 *)(scr + L.bsc);
+  uint16_t *vcan = (uint16_t *)(scr + L.vcan), *sel = (uint16_t *)(scr + L.sel);
+  if (SM.nchg) {
+    constexpr int kKeySlots = 2048;
+    static_assert(kKeySlots * sizeof(unsigned long long) <= kWorkBytes, "key table");
+    unsigned long long *kt = P.itk;
+    int slots = 64;
+    while (slots < 2 * nul && slots < kKeySlots) slots <<= 1;
+    for (int i = tid; i < slots; i += nt) kt[i] = ~0ull;
+    __syncthreads();
+    for (int q = tid; q < nul; q += nt) {
+      const int v = (int)uv[q].x;
+      const unsigned long long key = ment[v];
+      if (!differs(v >= vsplit ? 1 : 0, key)) {
+        msc[v] = make_longlong2(0, 0);
+        vcan[v] = (uint16_t)v;
+        continue;
+      }
+      const unsigned long long k38 = (key & 511u) | (((key >> 14) & 3u) << 9) |
+                                     (((key >> 16) & 511u) << 11) | (((key >> 32) & 511u) << 20) |
+                                     (((key >> 48) & 511u) << 29);
+      int can = v;
+      unsigned slot = (unsigned)(mix64(k38) & (slots - 1));
+      for (int pr = 0; pr < 32; pr++, slot = (slot + 1u) & (slots - 1)) {
+        unsigned long long cur = *(volatile unsigned long long *)&kt[slot];
+        if (cur == ~0ull) cur = atomicCAS(&kt[slot], ~0ull, (k38 << 16) | (unsigned)v);
+        if (cur == ~0ull) break;
+        if (cur >> 16 == k38) {
+          can = (int)(cur & 0xFFFFu);
+          break;
+        }
+      }
+      vcan[v] = (uint16_t)can;
+      if (can == v) sel[atomicAdd(&SM.nsel, 1)] = (uint16_t)v;
+    }
+    int *bpos = (int *)(scr + L.bpos);
+    int nbk = 0;
+    if (nbigs) {
+      for (int i0 = 0; i0 < KB; i0 += nt) {
+        const bool has = i0 + tid < KB && bkey[i0 + tid] != ~0ull;
+        int total;
+        const int off = block_scan(has ? 1 : 0, total, SM.scan);
+        if (has) bpos[nbk + off] = i0 + tid;
+        nbk += total;
+      }
+    }
+    __syncthreads();
+    const int nsel = SM.nsel;
+    bdeu_items(
+        sd, P, cp, SM.scan, nsel + nbk,
+        [&](int i) -> unsigned long long { return i < nsel ? ment[sel[i]] : bkey[bpos[i - nsel]]; },
+        [&](int i, unsigned long long key, long long s1, long long s2) {
+          if (i < nsel) {
+            const int v = sel[i], k = v >= vsplit ? 1 : 0, t = (int)(key & 0x3FFF);
+            msc[v] = make_longlong2(s1 - P.fsc[(k * 2 + 0) * g + t], s2 - P.fsc[(k * 2 + 1) * g + t]);
+          } else {
+            bsc[bpos[i - nsel]] = make_longlong2(s1, s2);
+          }
+        });
+    for (int q = tid; q < nul; q += nt) {
+      const int v = (int)uv[q].x, c = vcan[v];
+      if (c == v) continue;
+      // the same list of the same node, in either class
+      const int t = (int)(ment[v] & 0x3FFF), k = v >= vsplit ? 1 : 0, kc = c >= vsplit ? 1 : 0;
+      longlong2 x = msc[c];
+      x.x += P.fsc[(kc * 2 + 0) * g + t] - P.fsc[(k * 2 + 0) * g + t];
+      x.y += P.fsc[(kc * 2 + 1) * g + t] - P.fsc[(k * 2 + 1) * g + t];
+      msc[v] = x;
+    }
+  }
+  __syncthreads();
+  // ---- P5: the networks' hashes and scores, less their class's full one's
+  longlong2 *xs = (longlong2 *)(scr + L.xs);
+  int *dc = (int *)(scr + L.dc);
+  if (SM.nchg)
+    for (int k = 0; k < 2; k++) {
+      const int nk = k ? nB : nA, s1 = 1 + (k ? nA : 0);
+      const uint2 *u = uv + (k ? ulsplit : 0), *planes = cp[k].p;
+      const int nu = k ? nul - ulsplit : ulsplit, kw = kept_words(g);
+      const uint32_t *chg = P.chg + (k ? cw1 : 0);
+      const uint16_t *fc = P.fcnt + k * g;
+      const unsigned long long HF = SM.HF[k];
+      const bool big = nbigs > 0;
+      auto put = [=](int i, const unsigned long long *x) {
+        const int s = s1 + i;
+        const bool c = ((chg[i >> 5] >> (i & 31)) & 1u) != 0u;
+        const unsigned long long h = HF + x[0] + (big ? hs[s] : 0ull);
+        hs[s] = !c ? ~0ull : h == ~0ull ? ~1ull : h;
+        xs[s] = make_longlong2((long long)x[1], (long long)x[2]);
+        if (keep >= 0) dc[s] = (int)x[3];
+      };
+      auto word = [=](int i, int w) -> uint32_t {
+        const uint2 x = u[i];
+        return (int)x.x < kw ? vw[(size_t)x.x * vws + w]
+                             : variant_word(planes + (size_t)w * g, ent, x.y);
+      };
+      auto value = [=](int i, int j) -> unsigned long long {
+        const int v = (int)u[i].x;
+        if (j == 0) return mdh[v];
+        if (j < 3) return (unsigned long long)reinterpret_cast<const long long *>(msc + v)[j - 1];
+        return (unsigned long long)((long long)vcnt[v] - fc[(int)(ment[v] & 0x3FFF)]);
+      };
+      if (nu <= kFewVariants) {
+        // few: a lane per sample adds up its own
+        for (int i = tid; i < nk; i += nt) {
+          unsigned long long x[4] = {0ull, 0ull, 0ull, 0ull};
+          for (int q = 0; q < nu; q++)
+            if ((word(q, i >> 5) >> (i & 31)) & 1u)
+              for (int j = 0; j < (keep < 0 ? 3 : 4); j++) x[j] += value(q, j);
+          put(i, x);
+        }
+      } else if (keep < 0) {
+        unit_walk<3>(P.itk, nk, nu, word, value, put);
+      } else {
+        unit_walk<4>(P.itk, nk, nu, word, value, put);
+      }
+    }
+  __syncthreads();
+
+  // ---- P6: first-occurrence dedup.  Networks without changed nodes are
   // their class's full network: class-1 ones duplicate network 0, class-2
   // ones the first of them (firstB0).  So the unique networks are the
   // candidates -- network 0, firstB0 and the changed networks -- that are
@@ -1722,7 +2104,7 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
           const uint32_t b = 4u * ((cb[t * n16] >> hb) & 3u) + ((cb[j * n16] >> hb) & 3u);
           return (((en.y >> a) ^ (en.y >> b)) & 1u) == 0u;
         };
-        auto row = [&](int t) { return lists_equal(sd, P, ent, t, ks, ss, kr, sr); };
+        auto row = [&](int t) { return lists_equal(sd, SM.P, ent, t, ks, ss, kr, sr); };
         // the class's memo entries in a flat walk (a row that disagrees is
         // compared once: the walk goes on behind it), then the other rows
         const int e1 = ks ? nmemo : SM.split[0];
@@ -1737,228 +2119,52 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
       } else if (ks != kr && ss < 0 && sr < 0) {
         ok = SM.ndab == 0;  // the two full networks
       } else {
-        for (int t = 0; ok && t < g; t++) ok = lists_equal(sd, P, ent, t, ks, ss, kr, sr);
+        for (int t = 0; ok && t < g; t++) ok = lists_equal(sd, SM.P, ent, t, ks, ss, kr, sr);
       }
       if (!ok) atomicOr(&SM.status, kUnitHashCollision);
     }
     __syncthreads();
   }
-  if (tid == 0) {
-    bd.js[u] = __longlong_as_double(0x7ff8000000000000ll);
-    bd.U[u] = SM.status ? -1 : U;
-    bd.status[u] = SM.status;
-    if (bd.stats) atomicAdd(&bd.stats[4 * (size_t)bd.uslot[u] + 3], (unsigned long long)(S - U));
-  }
-  // one network has no JS (the range of its scores is empty), whatever its
-  // score is
+  report(U);
   if ((U == 1 && keep < 0) || SM.status) return;
 
-  // ---- P5: BDeu.  The JS takes only differences of the networks' scores,
-  // so the nodes that every network scores alike are left out (unless the
-  // scores themselves are kept): needed are the nodes whose full lists
-  // differ between the classes and those of rows with entries.
-  for (int i = tid; i < g * 3; i += nt) {
-    // state counts per class from the word-major planes: a warp's loads of
-    // a word are 32 consecutive planes
-    const uint64_t *pl = sd.planesT + i;
-    int a = 0, b = 0;
-    for (int w = 0; w < W; w++) {
-      const uint64_t x = pl[(size_t)w * 3 * g];
-      a += __popcll(x & P.mA[w]);
-      b += __popcll(x & P.mB[w]);
-    }
-    P.cnt3[i] = (uint16_t)a;
-    P.cnt3[3 * g + i] = (uint16_t)b;
-  }
-  uint2 *cpw = (uint2 *)(scr + L.cp);
-  pack_classes(sd, P, (uint32_t *)(scr + L.trig), cpw);
-  const ClassPlanes cp[2] = {{cpw, g, class_words(nA)},
-                             {cpw + (size_t)class_words(nA) * g, g, class_words(nB)}};
-  for (int i = tid; i < 2 * g; i += nt) {
-    const uint16_t *c3 = P.cnt3 + 3 * i;
-    P.nobs[i] = (uint8_t)((c3[0] > 0) + (c3[1] > 0) + (c3[2] > 0));
-  }
-  for (int t = tid; t < g; t += nt)
-    if (keep >= 0 || P.need[t] || P.phs[t] < P.phe[t] || P.phs[g + t] < P.phe[g + t]) P.need[t] |= 2;
-  for (int i = tid; i < 4 * g; i += nt) P.fsc[i] = 0;
-  __syncthreads();
-  // base scores of the needed nodes in the two full networks; a class-2
-  // node whose first parents equal the class-1 one's copies its scores
-  auto same_as_class1 = [&](int t) -> bool {
-    const int a = P.fcnt[t] < 3 ? P.fcnt[t] : 3, b = P.fcnt[g + t] < 3 ? P.fcnt[g + t] : 3;
-    if (a != b) return false;
-    for (int q = 0; q < a; q++)
-      if (P.fps[t * 3 + q] != P.fps[(g + t) * 3 + q]) return false;
-    return true;
-  };
-  bdeu_items(
-      sd, P, cp, SM.scan, 2 * g,
-      [&](int i) -> unsigned long long {
-        const int k = i >= g ? 1 : 0, t = i - k * g;
-        if (!(P.need[t] & 2) || (k == 1 && same_as_class1(t))) return ~0ull;
-        const int ps[3] = {P.fps[i * 3], P.fps[i * 3 + 1], P.fps[i * 3 + 2]};
-        return list_key(t, P.fcnt[i], ps);
-      },
-      [&](int i, unsigned long long key, long long s1, long long s2) {
-        if (key == ~0ull) return;
-        const int k = i >= g ? 1 : 0, t = i - k * g;
-        P.fsc[(k * 2 + 0) * g + t] = s1;
-        P.fsc[(k * 2 + 1) * g + t] = s2;
-      });
-  for (int t = tid; t < g; t += nt)
-    if ((P.need[t] & 2) && same_as_class1(t)) {
-      P.fsc[(1 * 2 + 0) * g + t] = P.fsc[(0 * 2 + 0) * g + t];
-      P.fsc[(1 * 2 + 1) * g + t] = P.fsc[(0 * 2 + 1) * g + t];
-    }
-  __syncthreads();
-  if (warp < 4) {
-    // warp 2 k + cls: the sum of full network k's scores over class cls
-    long long s = 0;
-    for (int t = lane; t < g; t += 32) s += P.fsc[warp * g + t];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) SM.base[warp & 1][warp >> 1] = s;
-  }
-  // the used variants' distinct keys, and the keys of the lists formed per
-  // sample, scored once each.  A table in the work region (free between the
-  // two rounds of scores) gives each key its first variant: 38 bits of key
-  // (genes below 512) and 16 of the variant a slot.  A variant that finds no
-  // room is scored on its own.
-  longlong2 *msc = (longlong2 *)(scr + L.msc);
-  longlong2 *bsc = (longlong2 *)(scr + L.bsc);
-  uint16_t *vcan = (uint16_t *)(scr + L.vcan), *sel = (uint16_t *)(scr + L.sel);
-  const int vsplit = SM.split[1];
-  auto is_used = [&](int v) { return ((P.used[v >> 5] >> (v & 31)) & 1u) != 0u; };
-  if (SM.nchg) {
-    constexpr int kKeySlots = 2048;
-    static_assert(kKeySlots * sizeof(unsigned long long) <= kWorkBytes, "key table");
-    unsigned long long *kt = P.itk;
-    int slots = 64;
-    while (slots < 2 * nvar && slots < kKeySlots) slots <<= 1;
-    for (int i = tid; i < slots; i += nt) kt[i] = ~0ull;
-    __syncthreads();
-    for (int v = tid; v < nvar; v += nt) {
-      if (!is_used(v)) continue;
-      const unsigned long long key = ment[v];
-      if (!differs(v >= vsplit ? 1 : 0, key)) {
-        msc[v] = make_longlong2(0, 0);
-        vcan[v] = (uint16_t)v;
-        continue;
-      }
-      const unsigned long long k38 = (key & 511u) | (((key >> 14) & 3u) << 9) |
-                                     (((key >> 16) & 511u) << 11) | (((key >> 32) & 511u) << 20) |
-                                     (((key >> 48) & 511u) << 29);
-      int can = v;
-      unsigned slot = (unsigned)(mix64(k38) & (slots - 1));
-      for (int pr = 0; pr < 32; pr++, slot = (slot + 1u) & (slots - 1)) {
-        unsigned long long cur = *(volatile unsigned long long *)&kt[slot];
-        if (cur == ~0ull) cur = atomicCAS(&kt[slot], ~0ull, (k38 << 16) | (unsigned)v);
-        if (cur == ~0ull) break;
-        if (cur >> 16 == k38) {
-          can = (int)(cur & 0xFFFFu);
-          break;
+  // unique networks: base of their class plus the differences, and those of
+  // the rows formed per sample
+  for (int uu = tid; uu < U; uu += nt) {
+    const int s = urep[uu], k = s <= nA ? 0 : 1;
+    long long d1 = SM.base[0][k], d2 = SM.base[1][k];
+    int edges = SM.flen[k];
+    if (s != 0 && s != firstB0) {
+      const longlong2 x = xs[s];
+      d1 += x.x;
+      d2 += x.y;
+      if (keep >= 0) edges += dc[s];
+      for (int r = 0; r < SM.nbig[k]; r++) {
+        const int t = P.big[k * g + r];
+        unsigned long long key, h;
+        int len;
+        if (!sample_list(sd, SM.P, ent, k, t, sig[s - 1], key, h, len)) continue;
+        edges += len - P.fcnt[k * g + t];
+        if (!differs(k, key)) continue;
+        const int slot = big_slot(key, false);
+        long long sc[2];
+        if (slot >= 0) {
+          sc[0] = bsc[slot].x;
+          sc[1] = bsc[slot].y;
+        } else {
+          key_scores(sd, SM.P, cp, key, sc);  // the table had no room
         }
-      }
-      vcan[v] = (uint16_t)can;
-      if (can == v) sel[atomicAdd(&SM.nsel, 1)] = (uint16_t)v;
-    }
-    int *bpos = (int *)(scr + L.bpos);
-    int nbk = 0;
-    if (nbigs) {
-      for (int i0 = 0; i0 < KB; i0 += nt) {
-        const bool has = i0 + tid < KB && bkey[i0 + tid] != ~0ull;
-        int total;
-        const int off = block_scan(has ? 1 : 0, total, SM.scan);
-        if (has) bpos[nbk + off] = i0 + tid;
-        nbk += total;
+        d1 += sc[0] - P.fsc[(k * 2 + 0) * g + t];
+        d2 += sc[1] - P.fsc[(k * 2 + 1) * g + t];
       }
     }
-    __syncthreads();
-    const int nsel = SM.nsel;
-    bdeu_items(
-        sd, P, cp, SM.scan, nsel + nbk,
-        [&](int i) -> unsigned long long { return i < nsel ? ment[sel[i]] : bkey[bpos[i - nsel]]; },
-        [&](int i, unsigned long long key, long long s1, long long s2) {
-          if (i < nsel) {
-            const int v = sel[i], k = v >= vsplit ? 1 : 0, t = (int)(key & 0x3FFF);
-            msc[v] = make_longlong2(s1 - P.fsc[(k * 2 + 0) * g + t], s2 - P.fsc[(k * 2 + 1) * g + t]);
-          } else {
-            bsc[bpos[i - nsel]] = make_longlong2(s1, s2);
-          }
-        });
-    for (int v = tid; v < nvar; v += nt) {
-      const int c = is_used(v) ? vcan[v] : v;
-      if (c == v) continue;
-      // the same list of the same node, in either class
-      const int t = (int)(ment[v] & 0x3FFF), k = v >= vsplit ? 1 : 0, kc = c >= vsplit ? 1 : 0;
-      longlong2 x = msc[c];
-      x.x += P.fsc[(kc * 2 + 0) * g + t] - P.fsc[(k * 2 + 0) * g + t];
-      x.y += P.fsc[(kc * 2 + 1) * g + t] - P.fsc[(k * 2 + 1) * g + t];
-      msc[v] = x;
-    }
-  }
-  __syncthreads();
-  // unique networks: base of their class plus the variants' differences, a
-  // lane per network, a warp per 32 networks of one class
-  {
-    int lo = 0, hi = U;  // the class-1 networks among the unique ones
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (urep[mid] <= nA) lo = mid + 1;
-      else hi = mid;
-    }
-    const int U1 = lo, uc0 = (U1 + 31) >> 5, uc = uc0 + ((U - U1 + 31) >> 5);
-    for (int ch = warp; ch < uc; ch += nw) {
-      const int k = ch >= uc0 ? 1 : 0;
-      const int uu = 32 * (k ? ch - uc0 : ch) + (k ? U1 : 0) + lane;
-      const bool live = uu < (k ? U : U1);
-      const int s = live ? urep[uu] : 0;
-      long long d1 = SM.base[0][k], d2 = SM.base[1][k];
-      int dc = 0;  // the network's edges less the full one's
-      const bool plain = !live || s == 0 || s == firstB0;
-      if (!__all_sync(0xffffffffu, plain)) {
-        const int sg = plain ? 0 : sig[s - 1];
-        const int c = plain ? 0 : cng[sg];
-        unsigned at = (unsigned)sg;
-        long long x1 = 0, x2 = 0;
-#pragma unroll 4
-        for (int q = 0; q < c; q++, at += (unsigned)n) {
-          const int v = lst[at];
-          const longlong2 x = msc[v];
-          x1 += x.x;
-          x2 += x.y;
-          if (keep >= 0) dc += (int)vcnt[v] - P.fcnt[k * g + (int)(ment[v] & 0x3FFF)];
-        }
-        for (int r = 0; !plain && r < SM.nbig[k]; r++) {
-          const int t = P.big[k * g + r];
-          unsigned long long key, h;
-          int len;
-          if (!sample_list(sd, P, ent, k, t, sg, key, h, len)) continue;
-          dc += len - P.fcnt[k * g + t];
-          if (!differs(k, key)) continue;
-          const int slot = big_slot(key, false);
-          long long sc[2];
-          if (slot >= 0) {
-            sc[0] = bsc[slot].x;
-            sc[1] = bsc[slot].y;
-          } else {
-            key_scores(sd, P, cp, key, sc);  // the table had no room
-          }
-          x1 += sc[0] - P.fsc[(k * 2 + 0) * g + t];
-          x2 += sc[1] - P.fsc[(k * 2 + 1) * g + t];
-        }
-        d1 += x1;
-        d2 += x2;
-      }
-      if (live) {
-        dist[uu] = d1;
-        dist[S + uu] = d2;
-        if (keep >= 0) wl[uu] = SM.flen[k] + dc;
-      }
-    }
+    dist[uu] = d1;
+    dist[S + uu] = d2;
+    if (keep >= 0) wl[uu] = edges;
   }
 
   __syncthreads();
-  // ---- P6: detailed outputs of kept units, packed: a region of the
+  // ---- P7: detailed outputs of kept units, packed: a region of the
   // batch's buffer, its edge ranges and the full networks' edge lists;
   // k_pack writes the unique networks' lists
   double *pl = nullptr, *ql = nullptr;
@@ -2042,9 +2248,26 @@ __global__ void __maxnreg__(80) k_units(const __grid_constant__ BatchDev bd) {
     __syncthreads();
   }
 
-  // ---- P7: normalisation and JS
+  // ---- P8: normalisation and JS
   const double js = unit_js(dist, S, U, SM, pl, ql);
   if (tid == 0) bd.js[u] = js;
+}
+
+// A block per resident slot of the GPU, each unit taken when a block is free:
+// the blocks' scratch, then, and what it holds of the last units, stays in
+// L2.  (A block and a scratch of its own per unit: @@@)
+__global__ void __maxnreg__(kUnitRegs) k_units(const __grid_constant__ BatchDev bd) {
+  extern __shared__ __align__(16) char smraw[];
+  UnitSmem &SM = *reinterpret_cast<UnitSmem *>(smraw);
+  int turn = 0;
+  for (int u = blockIdx.x; u < bd.B; turn ^= 1) {
+    int next = bd.B;
+    if (threadIdx.x == 0 && (int)gridDim.x < bd.B) next = (int)(gridDim.x + atomicAdd(bd.taken, 1u));
+    run_unit(bd, u, smraw);
+    if (threadIdx.x == 0) SM.next[turn] = next;
+    __syncthreads();
+    u = SM.next[turn];
+  }
 }
 
 // The unique networks' capped parent lists of the kept units (their edge
@@ -2057,8 +2280,8 @@ __global__ void __launch_bounds__(256) k_pack(const __grid_constant__ BatchDev b
   const BatchSet &bs = bd.sets[bd.uslot[u]];
   const SetDev &sd = bs.sd;
   const int g = sd.g, GW = sd.GW;
-  uint8_t *scr = bd.scratch + bs.sc0 + (size_t)(u - bs.u0) * bs.unit_bytes;
-  const UnitLayout L = unit_layout(sd.c, sd.S);
+  uint8_t *scr = bd.scratch + (size_t)(bd.blocks + (int)blockIdx.x) * bd.lay.total;
+  const UnitLayout &L = bd.lay;
   const KeepLayout KL = keep_layout(g, km.U, km.E, km.E2);
   uint8_t *kb = reinterpret_cast<uint8_t *>(bd.kbuf + km.off);
   const int *ids = (const int *)(kb + KL.ids), *epn = (const int *)(kb + KL.epn);
@@ -2145,11 +2368,20 @@ cudaError_t launch_pairs(const BatchSet *sets, const int32_t *uslot, const uint6
   return cudaGetLastError();
 }
 
-cudaError_t launch_units(const BatchDev &bd, int gmax, int W, cudaStream_t st) {
-  const size_t smem = unit_smem_bytes(gmax, W);
-  cudaError_t e = cudaFuncSetAttribute(k_units, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+void plan_units(BatchDev &bd, int gmax, int n, int sms) {
+  bd.lay = unit_layout(gmax * (gmax - 1) / 2, n + 2);
+  bd.sm = unit_slices(gmax, (n + 63) / 64);
+  // a block per place on the GPU (an SM: 227 KB of shared memory, 1 KB a
+  // block of it the system's, and 64 K registers)
+  const int per = std::min((227 << 10) / (int)(bd.sm.total + 1024), 65536 / (kUnitRegs * kUnitThreads));
+  bd.blocks = std::min(bd.B, std::max(1, per) * sms);
+}
+
+cudaError_t launch_units(const BatchDev &bd, cudaStream_t st) {
+  cudaError_t e =
+      cudaFuncSetAttribute(k_units, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bd.sm.total);
   if (e != cudaSuccess) return e;
-  k_units<<<bd.B, 256, smem, st>>>(bd);
+  k_units<<<bd.blocks, kUnitThreads, bd.sm.total, st>>>(bd);
   return cudaGetLastError();
 }
 

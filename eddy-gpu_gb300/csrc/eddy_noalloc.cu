@@ -199,7 +199,6 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
     BatchSet bs{};
     bs.sd = sd;
     bs.nb = 1;
-    bs.unit_bytes = (long long)unit_scratch_bytes(c, S);
     memcpy(g_upload + kOffSets, &bs, sizeof bs);
     const PrepSet ps{(uint64_t *)(base + kOffPlanes), (uint32_t *)(base + kOffCodes),
                      (uint16_t *)(base + kOffCtot), g, c, 0, 0};
@@ -228,12 +227,13 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
     bd.masks = (const uint64_t *)(base + kOffMask);
     bd.dmask = (uint32_t *)(base + kOffDmask);
     bd.scratch = base + kOffUnit;
+    plan_units(bd, g, n, 1);
     bd.js = d_js;
     bd.U = d_U;
     bd.status = d_status;
     bd.keep_slot = nullptr;
     bd.stats = nullptr;
-    if (launch_units(bd, g, W, st) != cudaSuccess) return bail(EDDY_ERR_CUDA);
+    if (launch_units(bd, st) != cudaSuccess) return bail(EDDY_ERR_CUDA);
     unsigned char out[16];
     if (cudaMemcpyAsync(out, base + kOffOut, 16, cudaMemcpyDeviceToHost, st) != cudaSuccess)
       return bail(EDDY_ERR_CUDA);
