@@ -154,7 +154,7 @@ EDDY_HD inline KeepLayout keep_layout(int g, int U, int E, int E2) {
 // memory (eddy_kernels.cu), for the largest set of a batch.
 struct UnitLayout {
   uint32_t phi[2], ent, ment, mdh, msc, vcan, sel, hs, dist, sig, urep, wl, vrep, ubits, htab;
-  uint32_t bkey, bsc, bpos, vcnt, krow, vinf, uv, vw, xs, dc, moves, cp;
+  uint32_t bkey, bsc, bpos, vcnt, krow, vinf, uv, vw, xs, dc, moves, cp, ikey, isc;
   uint32_t total;
 };
 struct UnitSlices {
@@ -176,6 +176,7 @@ struct BatchDev {
                                // unit kernel, then one per kept unit
   UnitLayout lay;
   UnitSlices sm;
+  int words_kept;              // variants whose sample words the scratch keeps
   int blocks;                  // blocks of the unit kernel
   unsigned *taken;             // units taken past the first of every block, 0 before
                                // (not read when every unit has a block)

@@ -440,10 +440,8 @@ __device__ __forceinline__ uint32_t cells16(uint32_t fb) {
 // non-empty subset of its entries (a variant) is formed once per unit.  The
 // other rows' lists are formed per left-out sample.  E is lowered until the
 // unit's variants fit unit_variants(g), which rows of up to five entries
-// always do.
+// always do, and the room for their sample words (BatchDev::words_kept).
 __host__ __device__ constexpr int unit_variants(int g) { return 62 * g + 64; }
-// variants whose sample words (variant_word) the unit's scratch keeps
-__host__ __device__ constexpr int kept_words(int g) { return 8 * g + 64; }
 // slots of the table of the lists formed per sample (in the unit's scratch)
 __host__ __device__ constexpr int big_slots(int g) {
   int s = 256;
@@ -460,7 +458,7 @@ static int genes_of_pairs(int c) {
   return (r + 1) / 2;
 }
 
-static UnitLayout unit_layout(int c, int S) {
+static UnitLayout unit_layout(int c, int S, int words_kept) {
   UnitLayout L;
   size_t o = 0;
   auto take = [&](size_t bytes) {
@@ -491,7 +489,7 @@ static UnitLayout unit_layout(int c, int S) {
   L.krow = take(sizeof(uint32_t) * (2 * (size_t)g * ((g + 31) / 32) + 4 * (size_t)g));
   L.vinf = take(sizeof(uint32_t) * nv);         // variants: entries and subset (variant_info)
   L.uv = take(sizeof(uint2) * nv);              // the used ones: number, info
-  L.vw = take(sizeof(uint32_t) * kept_words(g) * class_words(S - 2));  // words of the first ones
+  L.vw = take(sizeof(uint32_t) * (size_t)words_kept * class_words(S - 2));  // their words
   L.xs = take(2 * sizeof(int64_t) * (size_t)S); // per network: scores less the full one's
   L.dc = take(sizeof(int32_t) * (size_t)S);     // and its lists' edges (kept units)
   L.moves = take(sizeof(uint32_t) * 32 * ((size_t)(S - 2 + 63) / 64));  // pack_classes' masks
@@ -499,13 +497,22 @@ static UnitLayout unit_layout(int c, int S) {
   L.bkey = take(sizeof(uint64_t) * nb);
   L.bsc = take(2 * sizeof(int64_t) * nb);
   L.bpos = take(sizeof(int32_t) * nb);
+  L.ikey = take(sizeof(uint64_t) * (nv + nb));    // the keys to score (nv > 2 g)
+  L.isc = take(2 * sizeof(int64_t) * (nv + nb));  // and their scores
   for (int k = 0; k < 2; k++) L.phi[k] = take(sizeof(uint32_t) * cc);
   L.ent = take(2 * sizeof(uint2) * cc);
   L.total = (uint32_t)o;
   return L;
 }
 
-size_t unit_scratch_bytes(int c, int S) { return unit_layout(c, S).total; }
+// Variants whose sample words take at most `bytes` of a unit's scratch.
+static int words_kept(int c, int S, size_t bytes) {
+  return (int)std::min<size_t>(unit_variants(genes_of_pairs(c)), bytes / (4 * class_words(S - 2)));
+}
+
+size_t unit_scratch_bytes(int c, int S, size_t words) {
+  return unit_layout(c, S, words_kept(c, S, words)).total;
+}
 
 // Block-wide exclusive scan (blockDim multiple of 32, <= 1024).
 template <class T>
@@ -740,12 +747,10 @@ __device__ __noinline__ bool sample_list(const SetDev &sd, const UnitPtrs &P, co
   return true;
 }
 
-// Node scores of `n` items, kItems per round, as a flat task list over the
-// block: task (item, class, parent configuration j).  get(i) -> the item's
-// key (t | np << 14 | p0 << 16 | p1 << 32 | p2 << 48; ~0 = nothing to
-// score); emit(i, key, class-1 score, class-2 score).  Fixed-point terms are
-// summed with atomics: exact, in any order.  Nodes without parents are
-// scored from the state counts.
+// The unit kernel's shared memory.  (Functions that are not inlined reach it by
+// offset: through a pointer the loads would be generic ones.)
+extern __shared__ __align__(16) char unit_smem[];
+
 // divisor rows of a score's terms in one class (false: no observed
 // configuration or child state, the score is 0)
 __device__ __forceinline__ bool bdeu_rows(const SetDev &sd, const UnitPtrs &P, int cls, int t, int np,
@@ -759,14 +764,23 @@ __device__ __forceinline__ bool bdeu_rows(const SetDev &sd, const UnitPtrs &P, i
   return true;
 }
 
-template <class Get, class Emit>
-__device__ void bdeu_items(const SetDev &sd, const UnitPtrs &P, const ClassPlanes *cp, int *scan, int n,
-                           Get get, Emit emit) {
+// Node scores of `n` keys (t | np << 14 | p0 << 16 | p1 << 32 | p2 << 48; ~0:
+// nothing to score, 0), kItems per round, as a flat task list over the block:
+// task (key, class, parent configuration j); out: class-1 score, class-2
+// score.  Fixed-point terms are summed with atomics: exact, in any order.
+// Nodes without parents are scored from the state counts.
+__device__ __noinline__ void bdeu_items(const UnitSlices &o, const ClassPlanes cpA,
+                                        const ClassPlanes cpB, int n, const unsigned long long *keys,
+                                        longlong2 *out) {
+  UnitSmem &SM = *reinterpret_cast<UnitSmem *>(unit_smem);
+  const SetDev &sd = SM.sd;
+  const UnitPtrs P = unit_ptrs(unit_smem, o, sd.g);
   const int tid = threadIdx.x, nt = blockDim.x, g = sd.g;
+#pragma unroll 1
   for (int b0 = 0; b0 < n; b0 += kItems) {
     const int m = n - b0 < kItems ? n - b0 : kItems;
     for (int i = tid; i < m; i += nt) {
-      const unsigned long long key = get(b0 + i);
+      const unsigned long long key = keys[b0 + i];
       P.itk[i] = key;
       const int np = (key == ~0ull) ? 0 : (int)((key >> 14) & 3);
       for (int cls = 0; cls < 2; cls++) {
@@ -782,7 +796,7 @@ __device__ void bdeu_items(const SetDev &sd, const UnitPtrs &P, const ClassPlane
       const int e = c0 + tid;
       const int v = e < 2 * m ? P.tq[e] : 0;
       int total;
-      const int off = block_scan(v, total, scan);
+      const int off = block_scan(v, total, SM.scan);
       if (e < 2 * m) P.tq[e] = running + off;
       running += total;
     }
@@ -809,7 +823,7 @@ __device__ void bdeu_items(const SetDev &sd, const UnitPtrs &P, const ClassPlane
                   p2 = (int)((key >> 48) & 0xFFFF);
         const int64_t *LGq, *LGqr;
         if (bdeu_rows(sd, P, cls, t, np, p0, p1, p2, LGq, LGqr))
-          term = bdeu_config_term(cp[cls], t, np, p0, p1, p2, j, LGq, LGqr);
+          term = bdeu_config_term(cls ? cpB : cpA, t, np, p0, p1, p2, j, LGq, LGqr);
         seg = lo;
       }
 #pragma unroll
@@ -823,7 +837,7 @@ __device__ void bdeu_items(const SetDev &sd, const UnitPtrs &P, const ClassPlane
         atomicAdd((unsigned long long *)&P.acc[seg], (unsigned long long)term);
     }
     __syncthreads();
-    for (int i = tid; i < m; i += nt) emit(b0 + i, P.itk[i], P.acc[2 * i], P.acc[2 * i + 1]);
+    for (int i = tid; i < m; i += nt) out[b0 + i] = make_longlong2(P.acc[2 * i], P.acc[2 * i + 1]);
     __syncthreads();
   }
 }
@@ -924,10 +938,12 @@ __device__ __noinline__ void pack_classes(const SetDev &sd, const UnitPtrs &P, u
 }
 
 // Where a variant comes from: its row's first kept entry, their number and
-// the subset of them that fires.
-__device__ __forceinline__ uint32_t variant_info(int e0, int e, int sub) {
-  return (uint32_t)e0 | ((uint32_t)e << 14) | ((uint32_t)sub << 18);
+// the subset of them that fires; bit 31: it has a list of its own (not the
+// full network's).
+__device__ __forceinline__ uint32_t variant_info(int e0, int e, int sub, bool live) {
+  return (uint32_t)e0 | ((uint32_t)e << 14) | ((uint32_t)sub << 18) | (live ? 1u << 31 : 0u);
 }
+__device__ __forceinline__ uint32_t info_live(uint32_t x) { return (uint32_t)((int32_t)x >> 31); }
 __device__ __forceinline__ int info_first(uint32_t x) { return (int)(x & 0x3FFFu); }
 __device__ __forceinline__ int info_count(uint32_t x) { return (int)((x >> 14) & 15u); }
 __device__ __forceinline__ int info_end(uint32_t x) { return info_first(x) + info_count(x); }
@@ -947,38 +963,35 @@ __device__ __forceinline__ uint32_t trigger_word(const uint2 *cw, uint2 en) {
 constexpr int kFewVariants = 16;
 constexpr int kUnitThreads = 256, kUnitWarps = kUnitThreads / 32, kUnitRegs = 80;
 
-// The samples of class word w that fire exactly the variant's subset of its
-// row's entries, from the class planes.
-__device__ __noinline__ uint32_t variant_word(const uint2 *cw, const uint2 *ent, uint32_t info) {
-  uint32_t x = ~0u, sub = info >> 18;
-  const uint2 *e = ent + info_first(info);
-  for (int j = info_count(info); j > 0; j--, e++, sub >>= 1)
-    x &= trigger_word(cw, *e) ^ ((sub & 1u) - 1u);
-  return x;
-}
-
-// Which of the variants [v0, v1) of a class of nk samples some left-out
+// Which of the unit's nvar variants (class 2's from vsplit on) some left-out
 // sample changes its row to (P.used), which samples have a changed list
-// (chg), and the variants' words (vw[v][stride], the first `keep` variants').
-// 8, 16 or 32 words of the class at a time, a lane per variant and word; the
+// (P.chg), and the variants' words (vw[v][stride]).
+// 8, 16 or 32 words of the classes at a time, a lane per variant and word; the
 // entries' trigger words are formed first, as many as `bytes` of the work
 // region hold, word by word (a warp's 32 entries share their nodes' planes;
-// an odd pitch keeps the lanes' words in different banks).
-__device__ __noinline__ void mark_variants(const UnitPtrs &P, const uint2 *cpw, int g, int nk,
-                                           uint32_t *chg, const uint2 *ent, const uint32_t *vinf,
-                                           const unsigned long long *mdh, int v0, int v1, uint32_t *vw,
-                                           int stride, int keep, int bytes) {
-  uint32_t *T = (uint32_t *)P.itk;
-  const int tid = threadIdx.x, lane = tid & 31, words = (nk + 31) >> 5;
+// an odd pitch keeps the lanes' words in different banks).  Both classes go by
+// together and four variants of a lane at a time: bound by the chain from a
+// variant's number to its words.  (The subsets' products from registers, a
+// lane per row and word, unrolled: more instructions than the instruction
+// cache holds beside the rest, 268k cycles of a block at 200 genes x 1000
+// samples against 131k.)
+__device__ __noinline__ void mark_variants(const UnitSlices &o, const ClassPlanes cpA,
+                                           const ClassPlanes cpB, int nA, int nB,
+                                           const uint2 *ent, const uint32_t *vinf, int vsplit,
+                                           int nvar, uint32_t *vw, int stride, int bytes) {
+  uint32_t *T = (uint32_t *)(unit_smem + o.itk), *used = (uint32_t *)(unit_smem + o.used);
+  uint32_t *chg = (uint32_t *)(unit_smem + o.chg);
+  const int tid = threadIdx.x, lane = tid & 31, g = cpA.g;
+  const int w1 = (nA + 31) >> 5, w2 = (nB + 31) >> 5, words = max(w1, w2);
   const int lw = words <= 8 ? 3 : words <= 16 ? 4 : 5, nw = 1 << lw;
   const int pitch = ((bytes >> (lw + 2)) - 1) | 1, w = tid & (nw - 1);
+  constexpr int kAt = 4;  // loads in flight
   for (int w0 = 0; w0 < words; w0 += nw) {
-    const int live = min(nw, words - w0);
-    uint32_t c = 0u;
-    for (int q = v0, qe; q < v1; q = qe) {
+    uint32_t c1 = 0u, c2 = 0u;
+    for (int q = 0, qe; q < nvar; q = qe) {
       const int e0 = info_first(vinf[q]);
-      qe = v1;
-      if (info_end(vinf[v1 - 1]) - e0 > pitch) {
+      qe = nvar;
+      if (info_end(vinf[nvar - 1]) - e0 > pitch) {
         // the longest run of variants whose rows' entries fit
         int lo = q + 1;
         while (lo < qe) {
@@ -988,34 +1001,70 @@ __device__ __noinline__ void mark_variants(const UnitPtrs &P, const uint2 *cpw, 
         }
       }
       const int ne = info_end(vinf[qe - 1]) - e0;
+      // class 1's entries end where class 2's variants begin
+      const int esplit = vsplit <= q ? 0 : vsplit >= qe ? ne : info_first(vinf[vsplit]) - e0;
       __syncthreads();
-      for (int i = tid, x = tid / ne, e = tid - x * ne; i < live * ne; i += kUnitThreads) {
-        T[x * pitch + e] = trigger_word(cpw + (size_t)(w0 + x) * g, ent[e0 + e]);
-        e += kUnitThreads;
-        while (e >= ne) e -= ne, x++;
+      {
+        const int n = ne * min(nw, words - w0);
+        const int dx = kUnitThreads / ne, de = kUnitThreads - dx * ne;
+        int x = tid / ne, e = tid - x * ne;
+        for (int i = tid; i < n; i += kAt * kUnitThreads) {
+          uint32_t y[kAt];
+          int at[kAt];
+#pragma unroll
+          for (int r = 0; r < kAt; r++) {
+            const bool k1 = e < esplit, in = i + r * kUnitThreads < n && w0 + x < (k1 ? w1 : w2);
+            at[r] = x * pitch + e;
+            y[r] = in ? trigger_word((k1 ? cpA.p : cpB.p) + (size_t)(w0 + x) * g, ent[e0 + e]) : 0u;
+            e += de;
+            x += dx;
+            if (e >= ne) e -= ne, x++;
+          }
+#pragma unroll
+          for (int r = 0; r < kAt; r++)
+            if (i + r * kUnitThreads < n) T[at[r]] = y[r];
+        }
       }
       __syncthreads();
       const uint32_t *t0 = T + w * pitch - e0;
-#pragma unroll 2
-      for (int b = q; b < qe; b += kUnitThreads >> lw) {
-        const int v = b + (tid >> lw);
-        uint32_t x = 0u;
-        if (v < qe && w < live) {
-          const uint32_t info = vinf[v];
-          const uint32_t *t = t0 + info_first(info);
-          uint32_t sub = info >> 18;
-          x = ~0u;
-          for (int j = info_count(info); j > 0; j--, t++, sub >>= 1) x &= *t ^ ((sub & 1u) - 1u);
-          if (mdh[v] == 0ull) x = 0u;  // (0: the full list)
-          if (v < keep) vw[(size_t)v * stride + w0 + w] = x;
+      for (int b = q + (tid >> lw); b - (tid >> lw) < qe; b += kAt * (kUnitThreads >> lw)) {
+        uint32_t info[kAt];
+#pragma unroll
+        for (int r = 0; r < kAt; r++) {
+          const int v = b + r * (kUnitThreads >> lw);
+          info[r] = v < qe && w0 + w < words ? vinf[v] : 0u;
         }
-        c |= x;
-        const uint32_t any = __ballot_sync(0xffffffffu, x != 0u) >> (lane & ~(nw - 1));
-        if (w == 0 && (any & (~0u >> (32 - nw)))) atomicOr(&P.used[v >> 5], 1u << (v & 31));
+        // (all loads before the stores, which might alias them)
+        uint32_t y[kAt];
+#pragma unroll
+        for (int r = 0; r < kAt; r++) {
+          const uint32_t *t = t0 + info_first(info[r]);
+          const uint32_t sub = info[r] >> 18;
+          const int cnt = info_count(info[r]);
+          y[r] = info_live(info[r]);
+#pragma unroll
+          for (int j = 0; j < 4; j++)
+            if (j < cnt) y[r] &= t[j] ^ (((sub >> j) & 1u) - 1u);
+          for (int j = 4; j < cnt; j++) y[r] &= t[j] ^ (((sub >> j) & 1u) - 1u);
+        }
+#pragma unroll
+        for (int r = 0; r < kAt; r++) {
+          const int v = b + r * (kUnitThreads >> lw);
+          const uint32_t x = y[r];
+          if (info[r]) vw[(size_t)v * stride + w0 + w] = x;
+          if (v < vsplit) c1 |= x;
+          else c2 |= x;
+          const uint32_t any = __ballot_sync(0xffffffffu, x != 0u) >> (lane & ~(nw - 1));
+          if (w == 0 && (any & (~0u >> (32 - nw)))) atomicOr(&used[v >> 5], 1u << (v & 31));
+        }
       }
     }
-    for (int o = nw; o < 32; o <<= 1) c |= __shfl_xor_sync(0xffffffffu, c, o);
-    if (lane < nw && c) atomicOr(&chg[w0 + w], c);
+    for (int o = nw; o < 32; o <<= 1) {
+      c1 |= __shfl_xor_sync(0xffffffffu, c1, o);
+      c2 |= __shfl_xor_sync(0xffffffffu, c2, o);
+    }
+    if (lane < nw && c1) atomicOr(&chg[w0 + w], c1);
+    if (lane < nw && c2) atomicOr(&chg[cpA.words + w0 + w], c2);
   }
 }
 
@@ -1047,12 +1096,12 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 // of variants' words is held as its low and its high halves, so that bit r of
 // both variants lands in the exponents' top bits of one register.
 template <int J, class Word, class Value, class Put>
-__device__ __noinline__ void unit_walk(void *region, int nk, int nu, Word word, Value value,
+__device__ __noinline__ void unit_walk(uint32_t region, int nk, int nu, Word word, Value value,
                                        Put put) {
   constexpr int kK = 160;                                  // variants of a block
   constexpr int kB = (kK / 2 * J + kUnitThreads - 1) / kUnitThreads;  // pairs of values
   static_assert(kK * (4 * kUnitWarps + 16 * J) <= (int)kWorkBytes, "work region");
-  uint2 *A = (uint2 *)region;                              // [kK / 16][8 words][4][2]
+  uint2 *A = (uint2 *)(unit_smem + region);                          // [kK / 16][8 words][4][2]
   uint32_t *B = (uint32_t *)(A + kK / 2 * kUnitWarps);     // [kK / 16][J][8][4][2]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, words = (nk + 31) >> 5;
   const int r8 = lane >> 2, t4 = lane & 3, aw = tid & (kUnitWarps - 1), ap = tid / kUnitWarps;
@@ -1086,8 +1135,29 @@ __device__ __noinline__ void unit_walk(void *region, int nk, int nu, Word word, 
           xb[r][h] = j < J && i < nu ? value(i, j) : 0ull;
         }
     };
-    load(0);
-    for (int q = 0; q < nu; q += kK) {
+    // (one copy of each part's code: the next block's loads, this block's
+    // products, then the operands)
+#pragma unroll 1
+    for (int q = 0; q < nu + kK; q += kK) {
+      if (q < nu) load(q);
+      if (q > 0 && w0 + warp < words) {
+        const int steps = (min(kK, nu - (q - kK)) + 15) >> 4;
+        const uint4 *a4 = reinterpret_cast<const uint4 *>(A) + warp * 4 + t4;
+        const uint2 *b2 = reinterpret_cast<const uint2 *>(B) + lane;
+#pragma unroll 2
+        for (int ks = 0; ks < steps; ks++, a4 += 4 * kUnitWarps, b2 += 32 * J) {
+          const uint4 a = *a4;
+          const uint32_t l0 = bits(a.x, sh0), l1 = bits(a.x, sh1), l2 = bits(a.z, sh0), l3 = bits(a.z, sh1);
+          const uint32_t h0 = bits(a.y, sh0), h1 = bits(a.y, sh1), h2 = bits(a.w, sh0), h3 = bits(a.w, sh1);
+#pragma unroll
+          for (int j = 0; j < J; j++) {
+            const uint2 b = b2[32 * j];
+            mma_bf16(acc[0][j], l0, l1, l2, l3, b);
+            mma_bf16(acc[1][j], h0, h1, h2, h3, b);
+          }
+        }
+      }
+      if (q >= nu) break;
       __syncthreads();
 #pragma unroll
       for (int r = 0; r < kAp; r++) {
@@ -1113,23 +1183,6 @@ __device__ __noinline__ void unit_walk(void *region, int nk, int nu, Word word, 
         }
       }
       __syncthreads();
-      if (q + kK < nu) load(q + kK);
-      if (w0 + warp < words) {
-        const int steps = (min(kK, nu - q) + 15) >> 4;
-        const uint4 *a4 = reinterpret_cast<const uint4 *>(A) + warp * 4 + t4;
-        const uint2 *b2 = reinterpret_cast<const uint2 *>(B) + lane;
-        for (int ks = 0; ks < steps; ks++, a4 += 4 * kUnitWarps, b2 += 32 * J) {
-          const uint4 a = *a4;
-          const uint32_t l0 = bits(a.x, sh0), l1 = bits(a.x, sh1), l2 = bits(a.z, sh0), l3 = bits(a.z, sh1);
-          const uint32_t h0 = bits(a.y, sh0), h1 = bits(a.y, sh1), h2 = bits(a.w, sh0), h3 = bits(a.w, sh1);
-#pragma unroll
-          for (int j = 0; j < J; j++) {
-            const uint2 b = b2[32 * j];
-            mma_bf16(acc[0][j], l0, l1, l2, l3, b);
-            mma_bf16(acc[1][j], h0, h1, h2, h3, b);
-          }
-        }
-      }
     }
     if (w0 + warp >= words) continue;
     // a lane's two bytes' sums of samples r8 + 8 x, the four lanes' together
@@ -1158,9 +1211,11 @@ __device__ __noinline__ void unit_walk(void *region, int nk, int nu, Word word, 
 // + U]: per class min, max and mean of the scores (exact integers),
 // likelihoods exp((d - mean) 10 / (max - min)) normalised to sum 1, then the
 // two KL terms of kool() (routines.cu:42-60), zeros skipped, in FP64.  The
-// exponentials replace the scores in dist.  Sums are formed in a fixed
-// order: a thread's networks in turn, then a tree over the warp, then the
-// warps in turn.  pl, ql: the kept normalised likelihoods, or null.
+// exponentials replace the scores in dist.  The even lanes take class 1, the
+// odd ones class 2 (one copy of the code for both, and its latency: FP64's is
+// most of a small unit's JS).  Sums are formed in a fixed order, the same in
+// both classes: a thread's networks in turn, then a tree over the warp, then
+// the warps in turn.  pl, ql: the kept normalised likelihoods, or null.
 //
 // Inside k_units rather than after it: FP64 is slow on this part (about two
 // operations a cycle and SM, ~128 cycles to a dependent one), and here its
@@ -1172,125 +1227,105 @@ static __device__ __noinline__ double unit_js(long long *dist, int S, int U, Uni
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
   // the warps that hold networks, and the lanes of a warp that do (the sums
   // over the others' zeros are left out: each costs a dependent FP64 add)
-  const int nw = min(nt >> 5, (U + 31) >> 5), lanes = min(U, 32);
-  long long mn0 = LLONG_MAX, mx0 = LLONG_MIN, mn1 = LLONG_MAX, mx1 = LLONG_MIN;
-  unsigned long long s0 = 0, s1 = 0;  // modulo 2^64
-  for (int uu = tid; uu < U; uu += nt) {
-    const long long a = dist[uu], b = dist[S + uu];
-    mn0 = min(mn0, a);
-    mx0 = max(mx0, a);
-    mn1 = min(mn1, b);
-    mx1 = max(mx1, b);
-    s0 += (unsigned long long)a;
-    s1 += (unsigned long long)b;
+  const int nw = min(nt >> 5, (2 * U + 31) >> 5), lanes = min(2 * U, 32);
+  const int cls = tid & 1, u0 = tid >> 1, us = nt >> 1;
+  long long *d = dist + (cls ? S : 0);
+  long long mn = LLONG_MAX, mx = LLONG_MIN;
+  unsigned long long sum = 0;  // modulo 2^64
+  for (int uu = u0; uu < U; uu += us) {
+    const long long a = d[uu];
+    mn = min(mn, a);
+    mx = max(mx, a);
+    sum += (unsigned long long)a;
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    mn0 = min(mn0, (long long)__shfl_xor_sync(0xffffffffu, mn0, o));
-    mx0 = max(mx0, (long long)__shfl_xor_sync(0xffffffffu, mx0, o));
-    mn1 = min(mn1, (long long)__shfl_xor_sync(0xffffffffu, mn1, o));
-    mx1 = max(mx1, (long long)__shfl_xor_sync(0xffffffffu, mx1, o));
-    s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+  for (int o = 16; o > 1; o >>= 1) {
+    mn = min(mn, (long long)__shfl_xor_sync(0xffffffffu, mn, o));
+    mx = max(mx, (long long)__shfl_xor_sync(0xffffffffu, mx, o));
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
   }
-  if (lane == 0) {
-    SM.red[0][warp] = mn0;
-    SM.red[1][warp] = mx0;
-    SM.red[2][warp] = mn1;
-    SM.red[3][warp] = mx1;
-    SM.red[4][warp] = (long long)s0;
-    SM.red[5][warp] = (long long)s1;
+  if (lane < 2) {
+    SM.red[3 * lane][warp] = mn;
+    SM.red[3 * lane + 1][warp] = mx;
+    SM.red[3 * lane + 2][warp] = (long long)sum;
   }
   __syncthreads();
-  mn0 = mn1 = LLONG_MAX;
-  mx0 = mx1 = LLONG_MIN;
-  s0 = s1 = 0;
+  mn = LLONG_MAX;
+  mx = LLONG_MIN;
+  sum = 0;
+#pragma unroll 1
   for (int w = 0; w < nw; w++) {
-    mn0 = min(mn0, SM.red[0][w]);
-    mx0 = max(mx0, SM.red[1][w]);
-    mn1 = min(mn1, SM.red[2][w]);
-    mx1 = max(mx1, SM.red[3][w]);
-    s0 += (unsigned long long)SM.red[4][w];
-    s1 += (unsigned long long)SM.red[5][w];
+    mn = min(mn, SM.red[3 * cls][w]);
+    mx = max(mx, SM.red[3 * cls + 1][w]);
+    sum += (unsigned long long)SM.red[3 * cls + 2][w];
   }
   // one score for all networks in a class: no JS
-  if ((mn0 == mx0 || mn1 == mx1) && !pl) return __longlong_as_double(0x7ff8000000000000ll);
+  const bool flat = __any_sync(0xffffffffu, mn == mx) != 0;
+  if (flat && !pl) return __longlong_as_double(0x7ff8000000000000ll);
   // the sums of the scores less the smallest: exact
-  s0 -= (unsigned long long)U * (unsigned long long)mn0;
-  s1 -= (unsigned long long)U * (unsigned long long)mn1;
-  const double m0 = (double)(long long)s0 / (double)U, m1 = (double)(long long)s1 / (double)U;
-  const double sA = 10.0 / (double)(mx0 - mn0), sB = 10.0 / (double)(mx1 - mn1);
+  sum -= (unsigned long long)U * (unsigned long long)mn;
+  const double mean = (double)(long long)sum / (double)U, scale = 10.0 / (double)(mx - mn);
+  auto exponent = [&](int uu) { return ((double)(d[uu] - mn) - mean) * scale; };
   // equal exponents in both classes throughout (two networks ranked alike,
   // above all): equal likelihoods, every term of the JS is log(1)
-  if (U <= 32 && !pl) {
-    bool differ = false;
-    if (tid < U)
-      differ = ((double)(dist[tid] - mn0) - m0) * sA != ((double)(dist[S + tid] - mn1) - m1) * sB;
-    if (!__syncthreads_or(differ)) return 0.0;
+  double x = 0.0;
+  if (U <= us) {
+    if (u0 < U) x = exponent(u0);
+    const bool differ = x != __shfl_xor_sync(0xffffffffu, x, 1);
+    if (!pl && !__syncthreads_or(differ)) return 0.0;
   }
-  double za = 0.0, zb = 0.0;
-  for (int uu = tid; uu < U; uu += nt) {
-    const double ea = exp(((double)(dist[uu] - mn0) - m0) * sA);
-    const double eb = exp(((double)(dist[S + uu] - mn1) - m1) * sB);
-    dist[uu] = __double_as_longlong(ea);
-    dist[S + uu] = __double_as_longlong(eb);
-    za += ea;
-    zb += eb;
+  double z = 0.0;
+#pragma unroll 1
+  for (int uu = u0; uu < U; uu += us) {
+    const double e = exp(U <= us ? x : exponent(uu));
+    d[uu] = __double_as_longlong(e);
+    z += e;
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-    if (o < lanes) {
-      za += __shfl_xor_sync(0xffffffffu, za, o);
-      zb += __shfl_xor_sync(0xffffffffu, zb, o);
-    }
-  if (lane == 0) {
-    SM.redd[0][warp] = za;
-    SM.redd[1][warp] = zb;
-  }
+  for (int o = 16; o > 1; o >>= 1)
+    if (o < lanes) z += __shfl_xor_sync(0xffffffffu, z, o);
+  if (lane < 2) SM.redd[lane][warp] = z;
   __syncthreads();
-  za = SM.redd[0][0];
-  zb = SM.redd[1][0];
-  for (int w = 1; w < nw; w++) {
-    za += SM.redd[0][w];
-    zb += SM.redd[1][w];
-  }
+  z = SM.redd[cls][0];
+#pragma unroll 1
+  for (int w = 1; w < nw; w++) z += SM.redd[cls][w];
+  // a network's likelihoods P and Q in the two lanes, and its two terms
   double t = 0.0;
-  for (int uu = tid; uu < U; uu += nt) {
-    const double Pu = __longlong_as_double(dist[uu]) / za;
-    const double Qu = __longlong_as_double(dist[S + uu]) / zb;
-    const double M = (Pu + Qu) / 2;
-    if (M != 0) {
-      double x = 0.0;
-      if (Pu != 0) x += 0.5 * (Pu * log(Pu / M));
-      if (Qu != 0) x += 0.5 * (Qu * log(Qu / M));
-      t += x;
-    }
-    if (pl) {
-      pl[uu] = Pu;
-      ql[uu] = Qu;
-    }
+#pragma unroll 1
+  for (int b = 0; b < U; b += us) {
+    const int uu = b + u0;
+    const double p = uu < U ? __longlong_as_double(d[uu]) / z : 0.0;
+    const double m = (p + __shfl_xor_sync(0xffffffffu, p, 1)) / 2;
+    double y = 0.0;
+    if (p != 0 && m != 0) y = 0.5 * (p * log(p / m));
+    t += y + __shfl_xor_sync(0xffffffffu, y, 1);
+    if (pl && uu < U) (cls ? ql : pl)[uu] = p;
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
+  for (int o = 16; o > 1; o >>= 1)
     if (o < lanes) t += __shfl_xor_sync(0xffffffffu, t, o);
   if (lane == 0) SM.redd[2][warp] = t;
   __syncthreads();
   t = SM.redd[2][0];
+#pragma unroll 1
   for (int w = 1; w < nw; w++) t += SM.redd[2][w];
-  if (mn0 == mx0 || mn1 == mx1) return __longlong_as_double(0x7ff8000000000000ll);
+  if (flat) return __longlong_as_double(0x7ff8000000000000ll);
   return t / log(2.0);
 }
 
 // One block per unit.  A left-out sample changes only rows whose flip
 // entries it triggers, and both a network's hash and its score are sums over
-// rows, so nothing is kept per network but those sums and the rows it
-// changes: a lane takes one left-out sample, a warp 32 of one class, and walks
-// the class's memo rows.  A warp per network that lists its changed nodes
-// waited on chains of its own: 10000 units of 200 genes x 1000 samples near
-// the threshold took 44.0 ms against 19.5 ms now (with the normalisation and
-// JS, then 6.0 ms more), 301 units of 387 x 600 35.0 against 4.6 ms.  Bound by
-// issue (1.3 million warp instructions a unit at that shape), about half of
-// them in the node scores.
+// rows, so nothing is kept per network but those sums: which samples change a
+// row to which list (variant) is found 32 samples at a time, and the sums are
+// a product of the samples' bits with the variants' values (unit_walk).
+// 10000 units of 200 genes x 1000 samples near the threshold: 44.0 ms with a
+// warp per network that lists its changed nodes, 14.3 with a lane per left-out
+// sample that walks the rows and sums a list of its changes, 12.2 now; 301
+// units of 387 x 600 35.0, 2.8, 2.4 ms (all but the first with the
+// normalisation and JS, then 6.0 ms more).  Bound by issue and the waits
+// between dependent steps (0.68 million warp instructions a unit at the first
+// shape, 45% of the issue slots), a third of the time in the node scores'
+// population counts, whose rate (16 a cycle and SM) they reach.
 __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw) {
   UnitSmem &SM = *reinterpret_cast<UnitSmem *>(smraw);
   const int nw = blockDim.x >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1521,7 +1556,7 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
         running += total;
       }
       nvar = (int)(running >> kV);
-      if (nvar <= unit_variants(g) || E <= 0) break;
+      if (nvar <= min(unit_variants(g), bd.words_kept) || E <= 0) break;
       E--;
       __syncthreads();
     }
@@ -1662,7 +1697,7 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
     }
     ment[v] = key;
     mdh[v] = dh;
-    vinf[v] = variant_info(e0, e1 - e0, sub);
+    vinf[v] = variant_info(e0, e1 - e0, sub, dh != 0ull);
     if (keep >= 0) vcnt[v] = (uint16_t)len;
   }
   // sample lists of both classes in index order (network -> left-out
@@ -1742,12 +1777,9 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
   int nul = 0, ulsplit = 0;
   if (entries) {
     // (the base scores' room behind the work region is free until then)
-    const int room = (int)(kWorkBytes + 4 * sizeof(long long) * (size_t)g);
-    if (vsplit > 0)
-      mark_variants(SM.P, cp[0].p, g, nA, P.chg, ent, vinf, mdh, 0, vsplit, vw, vws, kept_words(g), room);
-    if (nvar > vsplit)
-      mark_variants(SM.P, cp[1].p, g, nB, P.chg + cw1, ent, vinf, mdh, vsplit, nvar, vw, vws,
-                    kept_words(g), room);
+    if (nvar)
+      mark_variants(bd.sm, cp[0], cp[1], nA, nB, ent, vinf, vsplit, nvar, vw, vws,
+                    (int)(kWorkBytes + 4 * sizeof(long long) * (size_t)g));
     // the rows formed per sample: their hash differences, and their keys
     // into the table
     for (int s0 = 32 * warp; nbigs && s0 < n; s0 += nt) {
@@ -1843,7 +1875,6 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
   }
   for (int t = tid; t < g; t += nt)
     if (keep >= 0 || P.need[t] || P.phs[t] < P.phe[t] || P.phs[g + t] < P.phe[g + t]) P.need[t] |= 2;
-  for (int i = tid; i < 4 * g; i += nt) P.fsc[i] = 0;
   __syncthreads();
   // base scores of the needed nodes in the two full networks; a class-2
   // node whose first parents equal the class-1 one's copies its scores
@@ -1854,25 +1885,21 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
       if (P.fps[t * 3 + q] != P.fps[(g + t) * 3 + q]) return false;
     return true;
   };
-  bdeu_items(
-      sd, P, cp, SM.scan, 2 * g,
-      [&](int i) -> unsigned long long {
-        const int k = i >= g ? 1 : 0, t = i - k * g;
-        if (!(P.need[t] & 2) || (k == 1 && same_as_class1(t))) return ~0ull;
-        const int ps[3] = {P.fps[i * 3], P.fps[i * 3 + 1], P.fps[i * 3 + 2]};
-        return list_key(t, P.fcnt[i], ps);
-      },
-      [&](int i, unsigned long long key, long long s1, long long s2) {
-        if (key == ~0ull) return;
-        const int k = i >= g ? 1 : 0, t = i - k * g;
-        P.fsc[(k * 2 + 0) * g + t] = s1;
-        P.fsc[(k * 2 + 1) * g + t] = s2;
-      });
-  for (int t = tid; t < g; t += nt)
-    if ((P.need[t] & 2) && same_as_class1(t)) {
-      P.fsc[(1 * 2 + 0) * g + t] = P.fsc[(0 * 2 + 0) * g + t];
-      P.fsc[(1 * 2 + 1) * g + t] = P.fsc[(0 * 2 + 1) * g + t];
-    }
+  unsigned long long *ikey = (unsigned long long *)(scr + L.ikey);
+  longlong2 *isc = (longlong2 *)(scr + L.isc);
+  for (int i = tid; i < 2 * g; i += nt) {
+    const int k = i >= g ? 1 : 0, t = i - k * g;
+    const int ps[3] = {P.fps[i * 3], P.fps[i * 3 + 1], P.fps[i * 3 + 2]};
+    ikey[i] = (P.need[t] & 2) && !(k == 1 && same_as_class1(t)) ? list_key(t, P.fcnt[i], ps) : ~0ull;
+  }
+  __syncthreads();
+  bdeu_items(bd.sm, cp[0], cp[1], 2 * g, ikey, isc);
+  for (int i = tid; i < 2 * g; i += nt) {
+    const int k = i >= g ? 1 : 0, t = i - k * g;
+    const longlong2 x = isc[k == 1 && same_as_class1(t) ? t : i];
+    P.fsc[(k * 2 + 0) * g + t] = x.x;
+    P.fsc[(k * 2 + 1) * g + t] = x.y;
+  }
   __syncthreads();
   if (warp < 4) {
     // warp 2 k + cls: the sum of full network k's scores over class cls
@@ -1920,8 +1947,14 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
         }
       }
       vcan[v] = (uint16_t)can;
-      if (can == v) sel[atomicAdd(&SM.nsel, 1)] = (uint16_t)v;
+      if (can == v) {
+        const int at = atomicAdd(&SM.nsel, 1);
+        sel[at] = (uint16_t)v;
+        ikey[at] = key;
+      }
     }
+    __syncthreads();
+    const int nsel = SM.nsel;
     int *bpos = (int *)(scr + L.bpos);
     int nbk = 0;
     if (nbigs) {
@@ -1929,23 +1962,25 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
         const bool has = i0 + tid < KB && bkey[i0 + tid] != ~0ull;
         int total;
         const int off = block_scan(has ? 1 : 0, total, SM.scan);
-        if (has) bpos[nbk + off] = i0 + tid;
+        if (has) {
+          bpos[nbk + off] = i0 + tid;
+          ikey[nsel + nbk + off] = bkey[i0 + tid];
+        }
         nbk += total;
+      }
+      __syncthreads();
+    }
+    bdeu_items(bd.sm, cp[0], cp[1], nsel + nbk, ikey, isc);
+    for (int i = tid; i < nsel + nbk; i += nt) {
+      const longlong2 x = isc[i];
+      if (i < nsel) {
+        const int v = sel[i], k = v >= vsplit ? 1 : 0, t = (int)(ikey[i] & 0x3FFF);
+        msc[v] = make_longlong2(x.x - P.fsc[(k * 2 + 0) * g + t], x.y - P.fsc[(k * 2 + 1) * g + t]);
+      } else {
+        bsc[bpos[i - nsel]] = x;
       }
     }
     __syncthreads();
-    const int nsel = SM.nsel;
-    bdeu_items(
-        sd, P, cp, SM.scan, nsel + nbk,
-        [&](int i) -> unsigned long long { return i < nsel ? ment[sel[i]] : bkey[bpos[i - nsel]]; },
-        [&](int i, unsigned long long key, long long s1, long long s2) {
-          if (i < nsel) {
-            const int v = sel[i], k = v >= vsplit ? 1 : 0, t = (int)(key & 0x3FFF);
-            msc[v] = make_longlong2(s1 - P.fsc[(k * 2 + 0) * g + t], s2 - P.fsc[(k * 2 + 1) * g + t]);
-          } else {
-            bsc[bpos[i - nsel]] = make_longlong2(s1, s2);
-          }
-        });
     for (int q = tid; q < nul; q += nt) {
       const int v = (int)uv[q].x, c = vcan[v];
       if (c == v) continue;
@@ -1964,8 +1999,8 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
   if (SM.nchg)
     for (int k = 0; k < 2; k++) {
       const int nk = k ? nB : nA, s1 = 1 + (k ? nA : 0);
-      const uint2 *u = uv + (k ? ulsplit : 0), *planes = cp[k].p;
-      const int nu = k ? nul - ulsplit : ulsplit, kw = kept_words(g);
+      const uint2 *u = uv + (k ? ulsplit : 0);
+      const int nu = k ? nul - ulsplit : ulsplit;
       const uint32_t *chg = P.chg + (k ? cw1 : 0);
       const uint16_t *fc = P.fcnt + k * g;
       const unsigned long long HF = SM.HF[k];
@@ -1979,9 +2014,7 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
         if (keep >= 0) dc[s] = (int)x[3];
       };
       auto word = [=](int i, int w) -> uint32_t {
-        const uint2 x = u[i];
-        return (int)x.x < kw ? vw[(size_t)x.x * vws + w]
-                             : variant_word(planes + (size_t)w * g, ent, x.y);
+        return vw[(size_t)u[i].x * vws + w];
       };
       auto value = [=](int i, int j) -> unsigned long long {
         const int v = (int)u[i].x;
@@ -1999,9 +2032,9 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
           put(i, x);
         }
       } else if (keep < 0) {
-        unit_walk<3>(P.itk, nk, nu, word, value, put);
+        unit_walk<3>(bd.sm.itk, nk, nu, word, value, put);
       } else {
-        unit_walk<4>(P.itk, nk, nu, word, value, put);
+        unit_walk<4>(bd.sm.itk, nk, nu, word, value, put);
       }
     }
   __syncthreads();
@@ -2253,17 +2286,19 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
   if (tid == 0) bd.js[u] = js;
 }
 
-// A block per resident slot of the GPU, each unit taken when a block is free:
-// the blocks' scratch, then, and what it holds of the last units, stays in
-// L2.  (A block and a scratch of its own per unit: @@@)
+// A block per place on the GPU, each unit taken when a block is free, so that
+// a batch holds the scratch of those blocks only (1.5 GB for 33 GB at 10000
+// units of 200 genes x 1000 samples; as fast as a block and a scratch per unit,
+// 14.9 ms for 15.0).  The layouts, computed on the host, come with the
+// parameters: with each block's own (every thread's, before) 14.9 ms against
+// 12.0, 19.7 against 16.6 ms for 2000 small sets.
 __global__ void __maxnreg__(kUnitRegs) k_units(const __grid_constant__ BatchDev bd) {
-  extern __shared__ __align__(16) char smraw[];
-  UnitSmem &SM = *reinterpret_cast<UnitSmem *>(smraw);
+  UnitSmem &SM = *reinterpret_cast<UnitSmem *>(unit_smem);
   int turn = 0;
   for (int u = blockIdx.x; u < bd.B; turn ^= 1) {
     int next = bd.B;
     if (threadIdx.x == 0 && (int)gridDim.x < bd.B) next = (int)(gridDim.x + atomicAdd(bd.taken, 1u));
-    run_unit(bd, u, smraw);
+    run_unit(bd, u, unit_smem);
     if (threadIdx.x == 0) SM.next[turn] = next;
     __syncthreads();
     u = SM.next[turn];
@@ -2368,8 +2403,10 @@ cudaError_t launch_pairs(const BatchSet *sets, const int32_t *uslot, const uint6
   return cudaGetLastError();
 }
 
-void plan_units(BatchDev &bd, int gmax, int n, int sms) {
-  bd.lay = unit_layout(gmax * (gmax - 1) / 2, n + 2);
+void plan_units(BatchDev &bd, int gmax, int n, int sms, size_t words) {
+  const int c = gmax * (gmax - 1) / 2;
+  bd.words_kept = words_kept(c, n + 2, words);
+  bd.lay = unit_layout(c, n + 2, bd.words_kept);
   bd.sm = unit_slices(gmax, (n + 63) / 64);
   // a block per place on the GPU (an SM: 227 KB of shared memory, 1 KB a
   // block of it the system's, and 64 K registers)

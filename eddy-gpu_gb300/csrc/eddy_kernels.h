@@ -7,7 +7,10 @@
 #include "eddy_internal.h"
 
 namespace eddy {
-size_t unit_scratch_bytes(int c, int S);
+// A unit's scratch, with `words` bytes at most of its variants' sample words
+// (4 MB hold all of them up to 387 genes x 900 samples).
+constexpr size_t kVariantWords = (size_t)4 << 20;
+size_t unit_scratch_bytes(int c, int S, size_t words = kVariantWords);
 constexpr int kMemoMax = 8;  // BatchDev::memo_max unless lowered
 // State planes, packed states and full-sample tables of the sets of a table
 // on the device (genes and pair_blocks: of all of them).
@@ -24,7 +27,7 @@ cudaError_t launch_pairs(const BatchSet *sets, const int32_t *uslot, const uint6
                          cudaStream_t st);
 // Network, BDeu and JS kernel of a batch; before, its layouts and blocks (B:
 // bd.B units, the largest set of gmax genes, n samples).
-void plan_units(BatchDev &bd, int gmax, int n, int sms);
+void plan_units(BatchDev &bd, int gmax, int n, int sms, size_t words = kVariantWords);
 cudaError_t launch_units(const BatchDev &bd, cudaStream_t st);
 // Lists of the kept units' unique networks, after launch_units (S: networks).
 cudaError_t launch_pack(const BatchDev &bd, int kept, int S, cudaStream_t st);

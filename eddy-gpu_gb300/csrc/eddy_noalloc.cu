@@ -64,10 +64,9 @@ constexpr size_t kOffUnit = kOffOut + 256;
 
 }  // namespace
 
-// size of the per-unit scratch at the maximum shape (computed at set-up)
-size_t unit_scratch_bytes(int c, int S);
-
 namespace {
+// room for the variants' sample words in the unit scratch
+constexpr size_t kNAWords = 512u << 10;
 constexpr size_t kNoAllocBytes = kOffUnit + (2u << 20);  // unit scratch <= 2 MB (checked)
 
 static __device__ __align__(256) unsigned char g_noalloc[kNoAllocBytes];
@@ -115,7 +114,7 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
   if (g < 2 || n < 2 || opts->max_parents < 1) return EDDY_ERR_ARG;
   if (g > kNAMaxGenes || n > kNAMaxSamples) return EDDY_ERR_CAPACITY;
   const int c = g * (g - 1) / 2, W = (n + 63) / 64, S = n + 2;
-  if (unit_scratch_bytes(c, S) > (2u << 20)) return EDDY_ERR_CAPACITY;
+  if (unit_scratch_bytes(c, S, kNAWords) > (2u << 20)) return EDDY_ERR_CAPACITY;
   int nA = 0;
   for (int s = 0; s < n; s++) {
     if (labels[s] > 1) return EDDY_ERR_ARG;
@@ -227,7 +226,7 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
     bd.masks = (const uint64_t *)(base + kOffMask);
     bd.dmask = (uint32_t *)(base + kOffDmask);
     bd.scratch = base + kOffUnit;
-    plan_units(bd, g, n, 1);
+    plan_units(bd, g, n, 1, kNAWords);
     bd.js = d_js;
     bd.U = d_U;
     bd.status = d_status;

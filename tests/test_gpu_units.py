@@ -85,3 +85,31 @@ def test_entries_past_the_shared_memory_cache(eddy_lib, oracle_lib, monkeypatch)
     ojs, oU = oracle_lib.units(data, labs[:1], None, oracle_lib.params(mp=3))
     assert np.array_equal(out[0][1][:1], oU)
     assert js_close(out[0][0][:1], ojs)
+
+
+# classes of one word of samples to more than 32, of one side only, and units
+# of a few variants (summed by a lane per sample) to several blocks of them
+# (summed on the matrix units)
+WALKS = [
+    # g, n, nA, mp, bonf, loading
+    (8, 40, 3, 3, True, 1.0),
+    (12, 2100, 1056, 3, True, 0.5),
+    (24, 1061, 1029, 3, True, 0.6),
+    (90, 520, 257, 3, True, 0.7),
+    (110, 290, 33, 4, True, 0.8),
+]
+
+
+@pytest.mark.parametrize("case", WALKS, ids=[f"g{c[0]}n{c[1]}a{c[2]}" for c in WALKS])
+def test_sums_over_left_out_samples(case, eddy_lib, oracle_lib):
+    g, n, nA, mp, bonf, loading = case
+    rng = np.random.default_rng(g * 7919 + n)
+    data = factor(rng, g, n, loading, 0.01)
+    labels0 = np.concatenate([np.zeros(nA, np.uint8), np.ones(n - nA, np.uint8)])
+    labs = np.stack([labels0] + [make_labels(rng, n, nA) for _ in range(3)])
+    ctx = eddy_lib.Context(max_parents=mp, bonferroni=bonf, rng=eddy_lib.RNG_EXTERNAL)
+    ctx.load_matrix(data, labels0)
+    js, U = ctx.run_labellings(ctx.add_set(np.arange(g)), labs)
+    ojs, oU = oracle_lib.units(data, labs, None, oracle_lib.params(mp=mp, bonferroni=bonf))
+    assert np.array_equal(U, oU)
+    assert js_close(js, ojs)
