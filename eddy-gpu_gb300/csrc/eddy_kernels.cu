@@ -137,109 +137,117 @@ __device__ __forceinline__ void philox10(uint32_t c[4], uint32_t k0, uint32_t k1
   }
 }
 
-// One block per unit.  key(s) = word s mod 4 of Philox(ctr = (s / 4, perm,
-// set, 0), key = seed); the nA samples with the smallest (key, s) are class 1.
-// Selection: a histogram of the keys' top 11 bits finds the bin that holds
-// the nA-th smallest key; the samples of that bin (about n / 2048 of them)
-// are ranked by (key, s) against each other, which gives the last one in,
-// (T, sT); sample s is in when (key, s) <= (T, sT).  The same set as
-// sorting the pairs and taking the first nA.
-constexpr int kCmBlock = 128, kCmBins = 2048, kCmShift = 21;
-__global__ void __launch_bounds__(kCmBlock) k_counter_masks(int n, int nA, int W, uint64_t seed,
-                                                            const int32_t *unit_set,
-                                                            const int32_t *unit_perm,
-                                                            const uint64_t *mask0,
-                                                            uint64_t *masks) {
-  // keys [n] u32 (padded to 8 bytes), the W mask words, then the bin's
-  // samples [n] u16
-  extern __shared__ uint32_t key[];
-  __shared__ int hist[kCmBins];
-  __shared__ int wsum[kCmBlock / 32];
-  __shared__ int s_bin, s_need, s_cnt;
-  __shared__ uint32_t s_T;
-  __shared__ int s_sT;
-  const int u = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// A warp per unit.  key(s) = word s mod 4 of Philox(ctr = (s / 4, perm, set,
+// 0), key = seed); the nA samples with the smallest (key, s) are class 1.
+// Selection: a histogram of the keys' top 8 bits finds the bin that holds the
+// nA-th smallest key; the samples of that bin (about n / 256 of them) are
+// ranked by (key, s) against each other, which gives the last one in, (T,
+// sT); sample s is in when (key, s) <= (T, sT).  The same set as sorting the
+// pairs and taking the first nA.  (A block of 128 threads per unit, 2048
+// bins, waited at its barriers: 4.5 ms for 339000 units of 300 samples, now
+// 0.9 ms.)
+constexpr int kCmWarps = 4, kCmBins = 256, kCmShift = 24;
+__host__ __device__ constexpr int cm_words(int n) { return ((n + 3) & ~3) + kCmBins; }  // a warp's shared memory
+__global__ void __launch_bounds__(32 * kCmWarps) k_counter_masks(int n, int nA, int W, uint64_t seed,
+                                                                 const int32_t *unit_set,
+                                                                 const int32_t *unit_perm,
+                                                                 const uint64_t *mask0,
+                                                                 uint64_t *masks, int B) {
+  extern __shared__ __align__(16) uint32_t cm_smem[];
+  const int lane = threadIdx.x & 31, u = blockIdx.x * kCmWarps + (threadIdx.x >> 5);
+  if (u >= B) return;
+  // the unit's keys, then the histogram, then (in its place) the bin's samples
+  uint32_t *key = cm_smem + (threadIdx.x >> 5) * cm_words(n), *hist = key + ((n + 3) & ~3);
+  uint16_t *cand = reinterpret_cast<uint16_t *>(hist);
   const int perm = unit_perm[u];
   uint64_t *out = masks + (size_t)u * W;
   if (perm == 0) {
-    for (int w = tid; w < W; w += kCmBlock) out[w] = mask0[w];
+    for (int w = lane; w < W; w += 32) out[w] = mask0[w];
     return;
   }
-  unsigned long long *mw = reinterpret_cast<unsigned long long *>(key + ((n + 1) & ~1));
-  uint16_t *cand = reinterpret_cast<uint16_t *>(mw + W);
-  const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
+#pragma unroll
+  for (int i = 0; i < kCmBins / 32; i++) hist[32 * i + lane] = 0u;
+  __syncwarp();
+  const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32), set = (uint32_t)unit_set[u];
   // one Philox call gives the keys of four samples
-  for (int s4 = tid; 4 * s4 < n; s4 += kCmBlock) {
-    uint32_t c[4] = {(uint32_t)s4, (uint32_t)perm, (uint32_t)unit_set[u], 0u};
+  for (int s4 = lane; 4 * s4 < n; s4 += 32) {
+    uint32_t c[4] = {(uint32_t)s4, (uint32_t)perm, set, 0u};
     philox10(c, k0, k1);
+    *reinterpret_cast<uint4 *>(key + 4 * s4) = make_uint4(c[0], c[1], c[2], c[3]);
 #pragma unroll
     for (int j = 0; j < 4; j++)
-      if (4 * s4 + j < n) key[4 * s4 + j] = c[j];
+      if (4 * s4 + j < n) atomicAdd(&hist[c[j] >> kCmShift], 1u);
   }
-  for (int w = tid; w < W; w += kCmBlock) mw[w] = 0ull;
-  for (int i = tid; i < kCmBins; i += kCmBlock) hist[i] = 0;
-  if (tid == 0) s_cnt = 0;
-  __syncthreads();
-  for (int s = tid; s < n; s += kCmBlock) atomicAdd(&hist[key[s] >> kCmShift], 1);
-  __syncthreads();
-  // the bin of the nA-th smallest key: thread t sums bins [16 t, 16 t + 16),
-  // then a block scan of those sums
-  constexpr int kPer = kCmBins / kCmBlock;
-  int loc = 0;
+  __syncwarp();
+  // the bin of the nA-th smallest key, and the samples it has to give: a lane
+  // sums eight bins, then a scan of the sums
+  constexpr int kPer = kCmBins / 32;
+  int h[kPer], loc = 0;
 #pragma unroll
-  for (int j = 0; j < kPer; j++) loc += hist[tid * kPer + j];
-  int incl = loc;
+  for (int j = 0; j < kPer; j++) loc += h[j] = (int)hist[lane * kPer + j];
+  int before = loc;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
+    const int y = __shfl_up_sync(0xffffffffu, before, o);
+    if (lane >= o) before += y;
   }
-  if (lane == 31) wsum[warp] = incl;
-  __syncthreads();
-  int before = incl - loc;
-  for (int w = 0; w < warp; w++) before += wsum[w];
-  if (before < nA && nA <= before + loc) {
-    for (int j = 0; j < kPer; j++) {
-      const int h = hist[tid * kPer + j];
-      if (before < nA && nA <= before + h) {
-        s_bin = tid * kPer + j;
-        s_need = nA - before;
-      }
-      before += h;
+  before -= loc;
+  __syncwarp();
+  const int owner = 31 - __clz(__ballot_sync(0xffffffffu, before < nA && nA <= before + loc));
+  int bin = 0, need = 0;
+#pragma unroll
+  for (int j = 0; j < kPer; j++) {
+    if (before < nA && nA <= before + h[j]) {
+      bin = lane * kPer + j;
+      need = nA - before;
     }
+    before += h[j];
   }
-  __syncthreads();
-  const uint32_t bin = (uint32_t)s_bin;
-  const int need = s_need;
-  for (int s = tid; s < n; s += kCmBlock)
-    if ((key[s] >> kCmShift) == bin) cand[atomicAdd(&s_cnt, 1)] = (uint16_t)s;
-  __syncthreads();
-  // rank of each of the bin's samples among them by (key, s): the one of
-  // rank need - 1 is the last one in
-  const int cnt = s_cnt;
-  for (int c = tid; c < cnt; c += kCmBlock) {
-    const int s = cand[c];
+  bin = __shfl_sync(0xffffffffu, bin, owner);
+  need = __shfl_sync(0xffffffffu, need, owner);
+  // the bin's samples in order, as many as the histogram's place holds
+  constexpr int kCand = 2 * kCmBins;
+  int cnt = 0;
+  for (int s0 = 0; s0 < n; s0 += 32) {
+    const bool in = s0 + lane < n && (int)(key[s0 + lane] >> kCmShift) == bin;
+    const unsigned bal = __ballot_sync(0xffffffffu, in);
+    const int at = cnt + __popc(bal & ((1u << lane) - 1u));
+    if (in && at < kCand) cand[at] = (uint16_t)(s0 + lane);
+    cnt += __popc(bal);
+  }
+  __syncwarp();
+  // rank of each of them by (key, s): the one of rank need - 1 is the last in
+  const bool listed = cnt <= kCand;
+  uint32_t T = 0u;
+  int sT = -1;
+  for (int c = lane; c < (listed ? cnt : n); c += 32) {
+    const int s = listed ? cand[c] : c;
     const uint32_t k = key[s];
     int rank = 0;
-    for (int d = 0; d < cnt; d++) {
-      const int t = cand[d];
+    if (!listed && (int)(k >> kCmShift) != bin) continue;
+    for (int d = 0; d < (listed ? cnt : n); d++) {
+      const int t = listed ? cand[d] : d;
       const uint32_t kt = key[t];
-      rank += (kt < k || (kt == k && t < s)) ? 1 : 0;
+      rank += ((int)(kt >> kCmShift) == bin && (kt < k || (kt == k && t < s))) ? 1 : 0;
     }
     if (rank == need - 1) {
-      s_T = k;
-      s_sT = s;
+      T = k;
+      sT = s;
     }
   }
-  __syncthreads();
-  const uint32_t T = s_T;
-  const int sT = s_sT;
-  for (int s = tid; s < n; s += kCmBlock) {
-    const uint32_t k = key[s];
-    if (k < T || (k == T && s <= sT)) atomicOr(&mw[s >> 6], 1ull << (s & 63));
+  const int last = 31 - __clz(__ballot_sync(0xffffffffu, sT >= 0));
+  T = __shfl_sync(0xffffffffu, T, last);
+  sT = __shfl_sync(0xffffffffu, sT, last);
+  uint32_t *out32 = reinterpret_cast<uint32_t *>(out);
+  uint32_t mine = 0u;
+  for (int w = 0; w < 2 * W; w++) {
+    const int s = 32 * w + lane;
+    const uint32_t k = s < n ? key[s] : 0u;
+    const uint32_t bal = __ballot_sync(0xffffffffu, s < n && (k < T || (k == T && s <= sT)));
+    if (lane == (w & 31)) mine = bal;
+    if ((w & 31) == 31 || w == 2 * W - 1)
+      if (lane <= (w & 31)) out32[(w & ~31) + lane] = mine;
   }
-  __syncthreads();
-  for (int w = tid; w < W; w += kCmBlock) out[w] = mw[w];
 }
 
 // ------------------------------------------------------------ k_pairs
@@ -2380,16 +2388,14 @@ cudaError_t launch_prep(const PrepSet *sets, int ns, int genes, int pair_blocks,
 cudaError_t launch_counter_masks(int n, int nA, int W, uint64_t seed, const int32_t *unit_set,
                                  const int32_t *unit_perm, const uint64_t *mask0, uint64_t *masks,
                                  int B, cudaStream_t st) {
-  // keys [n] u32 (padded to 8 bytes), the W mask words, then [n] u16
-  // sample indices; 128-thread blocks (more blocks per SM hide the barriers)
-  const size_t smem = sizeof(uint32_t) * (size_t)((n + 1) & ~1) + sizeof(uint64_t) * W +
-                      sizeof(uint16_t) * (size_t)n;
+  const size_t smem = sizeof(uint32_t) * kCmWarps * (size_t)cm_words(n);
   if (smem > 48 * 1024) {
     cudaError_t e =
         cudaFuncSetAttribute(k_counter_masks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  k_counter_masks<<<B, kCmBlock, smem, st>>>(n, nA, W, seed, unit_set, unit_perm, mask0, masks);
+  k_counter_masks<<<(B + kCmWarps - 1) / kCmWarps, 32 * kCmWarps, smem, st>>>(n, nA, W, seed, unit_set,
+                                                                              unit_perm, mask0, masks, B);
   return cudaGetLastError();
 }
 
