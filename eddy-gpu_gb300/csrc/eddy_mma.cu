@@ -920,14 +920,14 @@ __global__ void __launch_bounds__(32) k_exact(const BatchSet *__restrict__ sets,
 }
 
 // -------------------------------------------------------------- operands
-// 16 samples of an indicator row as e4m3 0/1 (1.0 = 0x38)
+// 16 samples of an indicator row as e4m3 0/1 (1.0 = 0x38): four bits at a time
+// spread to the bytes' low bits by a product, then times 0x38
 __device__ __forceinline__ void store_e4m3_16(uint8_t *dst, uint32_t bits) {
-  uint8_t v[16];
+  uint32_t o[4];
 #pragma unroll
-  for (int k = 0; k < 16; k++) v[k] = ((bits >> k) & 1u) ? 0x38 : 0x00;
-  uint4 o;
-  memcpy(&o, v, 16);
-  *reinterpret_cast<uint4 *>(dst) = o;
+  for (int k = 0; k < 4; k++)
+    o[k] = ((((bits >> (4 * k)) & 0xFu) * 0x00204081u) & 0x01010101u) * 0x38u;
+  *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
 }
 // One row of Y for a warp: the indicator over the samples of plane rows x & y
 // (null: a zero row), lanes over its 16-sample chunks.
@@ -983,29 +983,33 @@ __device__ __forceinline__ uint32_t core_group_entry(int k, int g) {
 // group's pairs and three zero words (144 bytes).
 __device__ __forceinline__ void ctot_core_group(const uint16_t *ctot, const uint8_t *prior, int g,
                                                 int grp, float *out) {
+  // (a warp: a lane per pair)
   float4 *o = reinterpret_cast<float4 *>(out + (size_t)grp * (kGroupCtBytes / 4));
   const uint32_t e = core_group_entry(grp, g);
-  const int row = (int)(e >> 16), col0 = (int)(e & 0xFFFFu);
-  uint32_t pb = 0;
-  for (int q = 0; q < kCorePairs; q++) {
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (row != 0xFFFF && col0 + q < row) {
-      const int p = row * (row - 1) / 2 + col0 + q;
-      const uint16_t *t = ctot + (size_t)p * 9;
-      v = make_float4((float)t[0], (float)t[1], (float)t[3], (float)t[4]);
-      if (prior[p]) pb |= 1u << q;
-    }
-    o[q] = v;
+  const int row = (int)(e >> 16), col = (int)(e & 0xFFFFu) + (threadIdx.x & 31);
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  const bool live = (threadIdx.x & 31) < kCorePairs && row != 0xFFFF && col < row;
+  bool pr = false;
+  if (live) {
+    const int p = row * (row - 1) / 2 + col;
+    const uint16_t *t = ctot + (size_t)p * 9;
+    v = make_float4((float)t[0], (float)t[1], (float)t[3], (float)t[4]);
+    pr = prior[p] != 0;
   }
-  o[kCorePairs] = make_float4(__uint_as_float(pb), 0.f, 0.f, 0.f);
+  const uint32_t pb = __ballot_sync(0xffffffffu, pr);
+  if ((threadIdx.x & 31) < kCorePairs) o[threadIdx.x & 31] = v;
+  if ((threadIdx.x & 31) == 0) o[kCorePairs] = make_float4(__uint_as_float(pb), 0.f, 0.f, 0.f);
 }
 
-// Full-sample counts of gene i's states -1, 0, 1 (4-cell layout).
+// Full-sample counts of gene i's states -1, 0, 1 (4-cell layout), by a warp.
 __device__ __forceinline__ void gene_counts(const uint64_t *planes, int W, int i, float4 *out) {
   int cnt[3] = {0, 0, 0};
-  for (int a = 0; a < 3; a++)
-    for (int w = 0; w < W; w++) cnt[a] += __popcll(planes[((size_t)i * 3 + a) * W + w]);
-  out[i] = make_float4((float)cnt[0], (float)cnt[1], (float)cnt[2], 0.f);
+  for (int w = threadIdx.x & 31; w < W; w += 32)
+#pragma unroll
+    for (int a = 0; a < 3; a++) cnt[a] += __popcll(planes[((size_t)i * 3 + a) * W + w]);
+#pragma unroll
+  for (int a = 0; a < 3; a++) cnt[a] = (int)__reduce_add_sync(0xffffffffu, (unsigned)cnt[a]);
+  if ((threadIdx.x & 31) == 0) out[i] = make_float4((float)cnt[0], (float)cnt[1], (float)cnt[2], 0.f);
 }
 
 __host__ __device__ inline int ngroups_of(const SetDev &sd, bool core) {
@@ -1023,7 +1027,10 @@ __host__ __device__ inline int ngroups_pad_of(const SetDev &sd, bool core) {
 // (x_row = a-1, x_col = b-1), rows 27..31 zero; 4-cell rows: 4q + 2a + b, a, b
 // in {0, 1}.  A warp takes whole rows, so a row's genes are found once and
 // its stores are coalesced (found per 16 bytes, with a 64-bit division and a
-// square root each, the same 12 GB of 500 sets took 11.9 ms).
+// square root each, the same 12 GB of 500 sets took 11.9 ms).  A block's time
+// is its chain of loads: 500 sets of a sweep 1.59 ms with a row at a time and
+// one thread for the tables and counts, 0.95 with a warp's eight rows together
+// and warps for the others.
 struct SetupArgs {
   const BatchSet *sets;
   int nsets, W, n_pad, core;
@@ -1046,31 +1053,38 @@ __global__ void __launch_bounds__(128) k_setup(const __grid_constant__ SetupArgs
   uint8_t *Y = a.Y + (size_t)blockIdx.x * 32 * a.n_pad;
   float *ctf = a.ctf + (size_t)bs.grp0 * (kGroupCtBytes / 4);
   const uint32_t e = a.core ? core_group_entry(grp, sd.g) : 0u;
-  for (int r = warp; r < 32; r += 4) {
-    int row = 0xFFFF, col = 0, x = 0, y = 0;
-    if (a.core) {
-      row = (int)(e >> 16);
-      col = (int)(e & 0xFFFFu) + r / 4;
-      x = (r >> 1) & 1;
-      y = r & 1;
-      if (col >= row) row = 0xFFFF;
-    } else {
-      const int p = grp * kPairsPerGroup + r / 9;
-      if (r < kPairsPerGroup * 9 && p < sd.c) pair_rc(p, row, col);
-      x = (r % 9) / 3;
-      y = r % 3;
+  if (a.core) {
+    // rows 4 q + 2 x + y: warp 2 x + y has the row gene's plane x and the
+    // eight column genes' planes y, all loaded before the stores
+    const int row = (int)(e >> 16), col0 = (int)(e & 0xFFFFu), n = row == 0xFFFF ? 0 : row - col0;
+    const uint64_t *px = sd.planes + ((size_t)(n > 0 ? row : 0) * 3 + (warp >> 1)) * W;
+    const uint64_t *py = sd.planes + ((size_t)(n > 0 ? col0 : 0) * 3 + (warp & 1)) * W;
+    for (int ch = lane; ch < a.n_pad / 16; ch += 32) {
+      const int w = ch >> 2, sh = 16 * (ch & 3);
+      const uint64_t x = w < W ? px[w] : 0ull;
+      uint64_t y[kCorePairs];
+#pragma unroll
+      for (int q = 0; q < kCorePairs; q++) y[q] = w < W && q < n ? py[(size_t)3 * W * q + w] : 0ull;
+#pragma unroll
+      for (int q = 0; q < kCorePairs; q++)
+        store_e4m3_16(Y + (size_t)(4 * q + warp) * a.n_pad + 16 * ch, (uint32_t)((x & y[q]) >> sh) & 0xFFFFu);
     }
+  }
+  for (int r = warp; !a.core && r < 32; r += 4) {
+    int row = 0xFFFF, col = 0;
+    const int p = grp * kPairsPerGroup + r / 9, x = (r % 9) / 3, y = r % 3;
+    if (r < kPairsPerGroup * 9 && p < sd.c) pair_rc(p, row, col);
     const bool live = row != 0xFFFF;
     build_y_row(live ? sd.planes + ((size_t)row * 3 + x) * W : nullptr,
                 sd.planes + ((size_t)col * 3 + y) * W, W, a.n_pad, Y + (size_t)r * a.n_pad);
   }
   if (a.core) {
-    if (threadIdx.x == 0) {
+    if (warp == 0) {
       ctot_core_group(sd.ctot, sd.prior, sd.g, grp, ctf);
-      a.gtab[blockIdx.x] = e;
+      if (lane == 0) a.gtab[blockIdx.x] = e;
     }
     // genes grp, grp + ng, ...
-    if (threadIdx.x == 32)
+    if (warp == 1)
       for (int i = grp; i < sd.g; i += ng) gene_counts(sd.planes, W, i, a.gcnt + bs.gc0);
   } else if (lane == 0 && warp < kPairsPerGroup) {
     ctot_f_pair(sd.ctot, sd.prior, sd.c, grp * kPairsPerGroup + warp, ctf);
