@@ -440,7 +440,7 @@ def run_ours(args, rank, world, local):
     # a step's units run as equal batches of at most 2^28 / (2 c) units (the
     # library's general-path queue holds every table of a batch): one launch
     # of each kernel per batch
-    batches = -(-B // min(16384, (1 << 28) // (2 * c)))
+    batches = -(-B // min(32768, (1 << 28) // (2 * c)))
     launches_per_kernel = args.steps * batches
     Bl = B / batches  # units per launch
     traffic_info = {}

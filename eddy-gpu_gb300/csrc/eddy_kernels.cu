@@ -2404,7 +2404,7 @@ cudaError_t launch_pairs(const BatchSet *sets, const int32_t *uslot, const uint6
                          cudaStream_t st) {
   if (gmax < 2) return cudaSuccess;
   const int t = (gmax + kPairTile - 1) / kPairTile;
-  // grid.y holds at most 65535 units (a batch has at most 16384)
+  // grid.y holds at most 65535 units (a batch has at most 32768)
   k_pairs<<<dim3(t * (t + 1) / 2, B), 32 * kPairWarps, 0, st>>>(sets, uslot, masks, W, dmask, stats);
   return cudaGetLastError();
 }
