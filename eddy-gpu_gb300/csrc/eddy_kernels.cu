@@ -505,8 +505,8 @@ static UnitLayout unit_layout(int c, int S, int words_kept) {
   L.bkey = take(sizeof(uint64_t) * nb);
   L.bsc = take(2 * sizeof(int64_t) * nb);
   L.bpos = take(sizeof(int32_t) * nb);
-  L.ikey = take(sizeof(uint64_t) * (nv + nb));    // the keys to score (nv > 2 g)
-  L.isc = take(2 * sizeof(int64_t) * (nv + nb));  // and their scores
+  L.ikey = take(sizeof(uint64_t) * (2 * g + nv + nb));    // the keys to score
+  L.isc = take(2 * sizeof(int64_t) * (2 * g + nv + nb));  // and their scores
   for (int k = 0; k < 2; k++) L.phi[k] = take(sizeof(uint32_t) * cc);
   L.ent = take(2 * sizeof(uint2) * cc);
   L.total = (uint32_t)o;
@@ -1884,8 +1884,15 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
   for (int t = tid; t < g; t += nt)
     if (keep >= 0 || P.need[t] || P.phs[t] < P.phe[t] || P.phs[g + t] < P.phe[g + t]) P.need[t] |= 2;
   __syncthreads();
-  // base scores of the needed nodes in the two full networks; a class-2
-  // node whose first parents equal the class-1 one's copies its scores
+  // the keys to score, all in one list: the needed nodes' lists in the two
+  // full networks (a class-2 node whose first parents equal the class-1
+  // one's has its scores), then the used variants' distinct keys, then the
+  // keys of the lists formed per sample.  A table in the work region (free
+  // until the scores) gives each key its first variant: 38 bits of key (genes
+  // below 512) and 16 of the variant a slot.  A variant that finds no room is
+  // scored on its own.  (Scored in two rounds, the full networks' first, a
+  // small unit's waits came twice: one labelling of 20 genes x 200 samples
+  // 55 us in the unit kernel for 52.)
   auto same_as_class1 = [&](int t) -> bool {
     const int a = P.fcnt[t] < 3 ? P.fcnt[t] : 3, b = P.fcnt[g + t] < 3 ? P.fcnt[g + t] : 3;
     if (a != b) return false;
@@ -1893,37 +1900,18 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
       if (P.fps[t * 3 + q] != P.fps[(g + t) * 3 + q]) return false;
     return true;
   };
+  longlong2 *msc = (longlong2 *)(scr + L.msc);
+  longlong2 *bsc = (longlong2 *)(scr + L.bsc);
+  uint16_t *vcan = (uint16_t *)(scr + L.vcan), *sel = (uint16_t *)(scr + L.sel);
   unsigned long long *ikey = (unsigned long long *)(scr + L.ikey);
   longlong2 *isc = (longlong2 *)(scr + L.isc);
+  int *bpos = (int *)(scr + L.bpos);
+  int nsel = 0, nbk = 0;
   for (int i = tid; i < 2 * g; i += nt) {
     const int k = i >= g ? 1 : 0, t = i - k * g;
     const int ps[3] = {P.fps[i * 3], P.fps[i * 3 + 1], P.fps[i * 3 + 2]};
     ikey[i] = (P.need[t] & 2) && !(k == 1 && same_as_class1(t)) ? list_key(t, P.fcnt[i], ps) : ~0ull;
   }
-  __syncthreads();
-  bdeu_items(bd.sm, cp[0], cp[1], 2 * g, ikey, isc);
-  for (int i = tid; i < 2 * g; i += nt) {
-    const int k = i >= g ? 1 : 0, t = i - k * g;
-    const longlong2 x = isc[k == 1 && same_as_class1(t) ? t : i];
-    P.fsc[(k * 2 + 0) * g + t] = x.x;
-    P.fsc[(k * 2 + 1) * g + t] = x.y;
-  }
-  __syncthreads();
-  if (warp < 4) {
-    // warp 2 k + cls: the sum of full network k's scores over class cls
-    long long s = 0;
-    for (int t = lane; t < g; t += 32) s += P.fsc[warp * g + t];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) SM.base[warp & 1][warp >> 1] = s;
-  }
-  // the used variants' distinct keys, and the keys of the lists formed per
-  // sample, scored once each.  A table in the work region (free between the
-  // two rounds of scores) gives each key its first variant: 38 bits of key
-  // (genes below 512) and 16 of the variant a slot.  A variant that finds no
-  // room is scored on its own.
-  longlong2 *msc = (longlong2 *)(scr + L.msc);
-  longlong2 *bsc = (longlong2 *)(scr + L.bsc);
-  uint16_t *vcan = (uint16_t *)(scr + L.vcan), *sel = (uint16_t *)(scr + L.sel);
   if (SM.nchg) {
     constexpr int kKeySlots = 2048;
     static_assert(kKeySlots * sizeof(unsigned long long) <= kWorkBytes, "key table");
@@ -1958,31 +1946,43 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
       if (can == v) {
         const int at = atomicAdd(&SM.nsel, 1);
         sel[at] = (uint16_t)v;
-        ikey[at] = key;
+        ikey[2 * g + at] = key;
       }
     }
     __syncthreads();
-    const int nsel = SM.nsel;
-    int *bpos = (int *)(scr + L.bpos);
-    int nbk = 0;
-    if (nbigs) {
-      for (int i0 = 0; i0 < KB; i0 += nt) {
-        const bool has = i0 + tid < KB && bkey[i0 + tid] != ~0ull;
-        int total;
-        const int off = block_scan(has ? 1 : 0, total, SM.scan);
-        if (has) {
-          bpos[nbk + off] = i0 + tid;
-          ikey[nsel + nbk + off] = bkey[i0 + tid];
-        }
-        nbk += total;
+    nsel = SM.nsel;
+    for (int i0 = 0; nbigs && i0 < KB; i0 += nt) {
+      const bool has = i0 + tid < KB && bkey[i0 + tid] != ~0ull;
+      int total;
+      const int off = block_scan(has ? 1 : 0, total, SM.scan);
+      if (has) {
+        bpos[nbk + off] = i0 + tid;
+        ikey[2 * g + nsel + nbk + off] = bkey[i0 + tid];
       }
-      __syncthreads();
+      nbk += total;
     }
-    bdeu_items(bd.sm, cp[0], cp[1], nsel + nbk, ikey, isc);
+  }
+  __syncthreads();
+  bdeu_items(bd.sm, cp[0], cp[1], 2 * g + nsel + nbk, ikey, isc);
+  for (int i = tid; i < 2 * g; i += nt) {
+    const int k = i >= g ? 1 : 0, t = i - k * g;
+    const longlong2 x = isc[k == 1 && same_as_class1(t) ? t : i];
+    P.fsc[(k * 2 + 0) * g + t] = x.x;
+    P.fsc[(k * 2 + 1) * g + t] = x.y;
+  }
+  __syncthreads();
+  if (warp < 4) {
+    // warp 2 k + cls: the sum of full network k's scores over class cls
+    long long s = 0;
+    for (int t = lane; t < g; t += 32) s += P.fsc[warp * g + t];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) SM.base[warp & 1][warp >> 1] = s;
+  }
+  if (SM.nchg) {
     for (int i = tid; i < nsel + nbk; i += nt) {
-      const longlong2 x = isc[i];
+      const longlong2 x = isc[2 * g + i];
       if (i < nsel) {
-        const int v = sel[i], k = v >= vsplit ? 1 : 0, t = (int)(ikey[i] & 0x3FFF);
+        const int v = sel[i], k = v >= vsplit ? 1 : 0, t = (int)(ikey[2 * g + i] & 0x3FFF);
         msc[v] = make_longlong2(x.x - P.fsc[(k * 2 + 0) * g + t], x.y - P.fsc[(k * 2 + 1) * g + t]);
       } else {
         bsc[bpos[i - nsel]] = x;
