@@ -908,8 +908,16 @@ __device__ __noinline__ void pack_classes(const SetDev &sd, const UnitPtrs &P, u
     const uint4 *mv4 = reinterpret_cast<const uint4 *>(moves + 8 * (size_t)cls * W32);
     uint32_t a0 = 0u, a1 = 0u;
     int fill = 0;
-    for (int w = 0; w < sd.W; w++, pl += 3 * (size_t)g) {
-      const uint64_t q0 = pl[0], q1 = pl[1], q2 = pl[2];
+    uint64_t n0 = pl[0], n1 = pl[1], n2 = pl[2];  // the next word's planes
+#pragma unroll 1
+    for (int w = 0; w < sd.W; w++) {
+      const uint64_t q0 = n0, q1 = n1, q2 = n2;
+      if (w + 1 < sd.W) {
+        pl += 3 * (size_t)g;
+        n0 = pl[0];
+        n1 = pl[1];
+        n2 = pl[2];
+      }
       const uint64_t mis = ~(q0 | q1 | q2), b0 = q1 | mis, b1 = q2 | mis;
 #pragma unroll
       for (int h = 0; h < 2; h++) {
@@ -2160,7 +2168,14 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
       } else if (ks != kr && ss < 0 && sr < 0) {
         ok = SM.ndab == 0;  // the two full networks
       } else {
-        for (int t = 0; ok && t < g; t++) ok = lists_equal(sd, SM.P, ent, t, ks, ss, kr, sr);
+        // (a row without entries has its class's full list, the same in both
+        // classes but for the nodes marked)
+        for (int t = 0; ok && t < g; t++) {
+          if (P.phs[ks * g + t] >= P.phe[ks * g + t] && P.phs[kr * g + t] >= P.phe[kr * g + t] &&
+              (ks == kr || !(P.need[t] & 1)))
+            continue;
+          ok = lists_equal(sd, SM.P, ent, t, ks, ss, kr, sr);
+        }
       }
       if (!ok) atomicOr(&SM.status, kUnitHashCollision);
     }
