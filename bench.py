@@ -62,20 +62,12 @@ def load_peaks():
     return 6800.0, 1900.0, "fallback"
 
 
-def algorithmic_bytes(g, n, mp, U):
-    """Per-unit algorithmic bytes of the network stages (k_units:
-    network assembly, dedup, BDeu, normalisation and JS) when each stage reads
-    its inputs and writes its outputs once through HBM: the S x c edge bits
-    of the S leave-one-out networks read, S x g x mp 16-bit parent entries and
-    an 8-byte hash per network written, the U unique networks' parent sets
-    (16-bit) and the set's data (2 x g x n bytes) read by BDeu, two 8-byte
-    scores per unique network and node written, and the JS written.  U is
-    the measured mean of unique networks per unit.  The kernel keeps the edge
-    bits and lists on chip, so this is the work it stands for, not the bytes
-    it moves (those are `traffic`)."""
-    c = g * (g - 1) // 2
-    S = n + 2
-    return S * c / 8 + S * g * mp * 2 + 8 * S + U * g * mp * 2 + 2 * g * n + 16 * U * g + 8
+def required_bytes(g, n):
+    """Per-unit bytes the network stages (k_units: networks, dedup, BDeu,
+    normalisation and JS) cannot do without when everything else stays on
+    chip: the decision masks read and cleared, the labelling's mask, and the
+    JS, unique count and status written."""
+    return 2 * 4 * (g * (g - 1) // 2) + 8 * ((n + 63) // 64) + 16
 
 
 class ClockSampler:
@@ -435,7 +427,7 @@ def run_ours(args, rank, world, local):
         return
     hbm, bf16, peak_kind = load_peaks()
     U_mean = float(np.mean(u_mean[-args.steps:]))
-    bu = algorithmic_bytes(g, n, mp, U_mean)
+    bu = required_bytes(g, n)
     c = g * (g - 1) // 2
     # a step's units run as equal batches of at most 2^28 / (2 c) units (the
     # library's general-path queue holds every table of a batch): one launch
@@ -478,24 +470,27 @@ def run_ours(args, rank, world, local):
           "ncu_sm_throughput_pct": traffic_info.get("k_pairs_mma_sm_throughput_pct"),
           "ncu_tensor_pipe_pct": traffic_info.get("k_pairs_mma_tensor_pipe_pct")}
     k1["frac"] = k1["achieved"] / e4m3
-    # network assembly, dedup, BDeu, JS: algorithmic bytes (each stage's
-    # inputs and outputs once through HBM)
+    # networks, dedup, BDeu, JS: bound by the SMs' issue slots, not by bytes
+    # (which are reported beside it): warp instructions per unit as ncu counts
+    # them, against four a cycle and SM at the sampled clock
     k2_ms = acc["ms_networks"] / launches_per_kernel
-    k2 = {"kernel": "k_units", "bound": "hbm", "achieved": bu * Bl / (k2_ms / 1e3) / 1e9,
-          "peak": hbm, "unit": "GB/s", "ms_per_launch": k2_ms,
-          "algorithmic_bytes_per_launch": bu * Bl, "unique_networks_per_unit": U_mean,
-          "units_per_launch": Bl,
+    insts = traffic_info.get("k_units_warp_instructions_per_unit", 0) * Bl
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    issue = 4.0 * sms * (clk.summary().get("sm_mhz") or 2070.0) / 1e3
+    k2 = {"kernel": "k_units", "bound": "issue", "achieved": insts / (k2_ms / 1e3) / 1e9,
+          "peak": issue, "unit": "G warp instructions/s", "ms_per_launch": k2_ms,
+          "warp_instructions_per_launch": insts, "required_bytes_per_launch": bu * Bl,
+          "required_bytes_hbm_frac": bu * Bl / (k2_ms / 1e3) / 1e9 / hbm,
+          "unique_networks_per_unit": U_mean, "units_per_launch": Bl,
           "traffic": traffic_info.get("k_units_bytes_per_unit", 0) * Bl or None,
-          # the kernel is bound by SM issue and latency, not HBM: the SM
-          # throughput share from ncu (2048-unit launch) goes with the HBM one
           "ncu_sm_throughput_pct": traffic_info.get("k_units_sm_throughput_pct"),
           "ncu_issue_active_pct": traffic_info.get("k_units_issue_active_pct")}
-    k2["frac"] = k2["achieved"] / hbm
+    k2["frac"] = k2["achieved"] / issue
     dom = k1 if k1_ms >= k2_ms else k2
     roofline = dict(dom)
     roofline["peak_source"] = (f"2 x MEASURED_PEAKS.json bf16_tflops ({peak_kind}): the GEMM "
                                "runs e4m3 operands, whose dense peak is twice the bf16 one"
-                               if dom is k1 else f"MEASURED_PEAKS.json hbm_gbs ({peak_kind})")
+                               if dom is k1 else "four warp instructions a cycle and SM at the sampled clock")
     cpu = None
     precision = {"tables": int(stats["tables"]), "filtered": int(stats["filtered"]),
                  "exact_rechecks": int(stats["exact_rechecks"])}
@@ -528,7 +523,7 @@ def run_ours(args, rank, world, local):
                                          "within +-20% of 0.05 (p_band), or whose chi-square is within "
                                          "+-20% of the critical chi-square (chi2_band)"},
                        "l2": "per-launch working set (decision masks + per-unit scratch) "
-                             f"~{(Bl * (c * 4 + 1.3e6)) / 1e9:.2f} GB > L2"},
+                             f"~{(Bl * c * 4 + 1.5e9) / 1e9:.2f} GB > L2"},
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h},
             "gpu_launches": acc["launches"],

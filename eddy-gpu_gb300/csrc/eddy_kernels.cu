@@ -144,7 +144,7 @@ __device__ __forceinline__ void philox10(uint32_t c[4], uint32_t k0, uint32_t k1
 // ranked by (key, s) against each other, which gives the last one in, (T,
 // sT); sample s is in when (key, s) <= (T, sT).  The same set as sorting the
 // pairs and taking the first nA.  (A block of 128 threads per unit, 2048
-// bins, waited at its barriers: 4.5 ms for 339000 units of 300 samples, now
+// bins, waited at its barriers: 4.5 ms for 339000 units of 1000 samples, now
 // 0.9 ms.)
 constexpr int kCmWarps = 4, kCmBins = 256, kCmShift = 24;
 __host__ __device__ constexpr int cm_words(int n) { return ((n + 3) & ~3) + kCmBins; }  // a warp's shared memory

@@ -1027,7 +1027,7 @@ __host__ __device__ inline int ngroups_pad_of(const SetDev &sd, bool core) {
 // (x_row = a-1, x_col = b-1), rows 27..31 zero; 4-cell rows: 4q + 2a + b, a, b
 // in {0, 1}.  A warp takes whole rows, so a row's genes are found once and
 // its stores are coalesced (found per 16 bytes, with a 64-bit division and a
-// square root each, the same 12 GB of 500 sets took 11.9 ms).  A block's time
+// square root each, 500 sets took 11.9 ms).  A block's time
 // is its chain of loads: 500 sets of a sweep 1.59 ms with a row at a time and
 // one thread for the tables and counts, 0.95 with a warp's eight rows together
 // and warps for the others.
