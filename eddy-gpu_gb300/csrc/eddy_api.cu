@@ -733,9 +733,13 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
     bp.fp64 = bp.fp64 && use_popc(b.sd);
   }
   const bool masks_host = jobs[units[0].job].masks_host != nullptr;
+  double pairs = 0;
   {
     double words = 0;
-    for (const BatchSet &b : bp.sets) words += (b.sd.core ? 1.0 : 2.25) * b.nb * (double)b.sd.c * W;
+    for (const BatchSet &b : bp.sets) {
+      words += (b.sd.core ? 1.0 : 2.25) * b.nb * (double)b.sd.c * W;
+      pairs += b.nb * (double)b.sd.c;
+    }
     popc_batch = popc_batch || few_units(Bt, ns, words);
   }
   // kept units: unit 0 of a keeping job
@@ -763,7 +767,7 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   }
   BatchDev bd{};
   bd.B = Bt;
-  plan_units(bd, bp.gmax, n, ctx->sms);
+  plan_units(bd, bp.gmax, pairs, n, ctx->sms);
   CK(ctx->d_scratch.ensure(bd.lay.total * (size_t)(bd.blocks + nk)));
   // uploads, in one copy: [set table][slots][kept slots], then the labellings'
   // masks, or the sets and permutations they are drawn from.  (A batch of

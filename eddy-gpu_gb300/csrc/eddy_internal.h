@@ -177,7 +177,7 @@ struct BatchDev {
   UnitLayout lay;
   UnitSlices sm;
   int words_kept;              // variants whose sample words the scratch keeps
-  int blocks;                  // blocks of the unit kernel
+  int blocks, threads;         // of the unit kernel
   unsigned *taken;             // units taken past the first of every block, 0 before
                                // (not read when every unit has a block)
   double *js;                  // [B]

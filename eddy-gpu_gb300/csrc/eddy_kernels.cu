@@ -4,13 +4,13 @@
 //                       samples and the permutation-invariant full-sample
 //                       3x3 table of every pair.
 //   k_counter_masks     counter-based labelling (Philox-4x32-10) -> class-1
-//                       sample masks, one block per unit.
+//                       sample masks, a warp per unit.
 //   k_pairs             contingency counts of class 1 for every (unit, pair)
 //                       (class 2 = full table - class 1), and the 10-bit
 //                       leave-one-out decision mask per class: the reference's
 //                       run2/run2Scalable (kernel1.cu:389-477) over all S
 //                       networks collapsed to <= 10 distinct tables per class.
-//   k_units             one block per unit: full networks, flip lists, the
+//   k_units             a block per unit at a time: full networks, flip lists, the
 //                       capped parent lists that left-out samples change
 //                       (kernel2.cu:114-142, kernel3.cu:134-165), network
 //                       hashing and first-occurrence dedup with exact
@@ -18,6 +18,7 @@
 //                       BDeu over the unique networks in fixed point
 //                       (kernel5.cu:237-257), normalisation and JS
 //                       (main.cu:1293-1428).
+//   k_pack              the networks of the units kept for output files.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -977,7 +978,7 @@ __device__ __forceinline__ uint32_t trigger_word(const uint2 *cw, uint2 en) {
 }
 
 constexpr int kFewVariants = 16;
-constexpr int kUnitThreads = 256, kUnitWarps = kUnitThreads / 32, kUnitRegs = 80;
+constexpr int kUnitRegs = 80;
 
 // Which of the unit's nvar variants (class 2's from vsplit on) some left-out
 // sample changes its row to (P.used), which samples have a changed list
@@ -991,6 +992,7 @@ constexpr int kUnitThreads = 256, kUnitWarps = kUnitThreads / 32, kUnitRegs = 80
 // lane per row and word, unrolled: more instructions than the instruction
 // cache holds beside the rest, 268k cycles of a block at 200 genes x 1000
 // samples against 131k.)
+template <int kThreads>
 __device__ __noinline__ void mark_variants(const UnitSlices &o, const ClassPlanes cpA,
                                            const ClassPlanes cpB, int nA, int nB,
                                            const uint2 *ent, const uint32_t *vinf, int vsplit,
@@ -1022,14 +1024,14 @@ __device__ __noinline__ void mark_variants(const UnitSlices &o, const ClassPlane
       __syncthreads();
       {
         const int n = ne * min(nw, words - w0);
-        const int dx = kUnitThreads / ne, de = kUnitThreads - dx * ne;
+        const int dx = kThreads / ne, de = kThreads - dx * ne;
         int x = tid / ne, e = tid - x * ne;
-        for (int i = tid; i < n; i += kAt * kUnitThreads) {
+        for (int i = tid; i < n; i += kAt * kThreads) {
           uint32_t y[kAt];
           int at[kAt];
 #pragma unroll
           for (int r = 0; r < kAt; r++) {
-            const bool k1 = e < esplit, in = i + r * kUnitThreads < n && w0 + x < (k1 ? w1 : w2);
+            const bool k1 = e < esplit, in = i + r * kThreads < n && w0 + x < (k1 ? w1 : w2);
             at[r] = x * pitch + e;
             y[r] = in ? trigger_word((k1 ? cpA.p : cpB.p) + (size_t)(w0 + x) * g, ent[e0 + e]) : 0u;
             e += de;
@@ -1038,16 +1040,16 @@ __device__ __noinline__ void mark_variants(const UnitSlices &o, const ClassPlane
           }
 #pragma unroll
           for (int r = 0; r < kAt; r++)
-            if (i + r * kUnitThreads < n) T[at[r]] = y[r];
+            if (i + r * kThreads < n) T[at[r]] = y[r];
         }
       }
       __syncthreads();
       const uint32_t *t0 = T + w * pitch - e0;
-      for (int b = q + (tid >> lw); b - (tid >> lw) < qe; b += kAt * (kUnitThreads >> lw)) {
+      for (int b = q + (tid >> lw); b - (tid >> lw) < qe; b += kAt * (kThreads >> lw)) {
         uint32_t info[kAt];
 #pragma unroll
         for (int r = 0; r < kAt; r++) {
-          const int v = b + r * (kUnitThreads >> lw);
+          const int v = b + r * (kThreads >> lw);
           info[r] = v < qe && w0 + w < words ? vinf[v] : 0u;
         }
         // (all loads before the stores, which might alias them)
@@ -1065,7 +1067,7 @@ __device__ __noinline__ void mark_variants(const UnitSlices &o, const ClassPlane
         }
 #pragma unroll
         for (int r = 0; r < kAt; r++) {
-          const int v = b + r * (kUnitThreads >> lw);
+          const int v = b + r * (kThreads >> lw);
           const uint32_t x = y[r];
           if (info[r]) vw[(size_t)v * stride + w0 + w] = x;
           if (v < vsplit) c1 |= x;
@@ -1111,11 +1113,12 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 // warp issues for it.  The bits pass into registers by shift and mask: a pair
 // of variants' words is held as its low and its high halves, so that bit r of
 // both variants lands in the exponents' top bits of one register.
-template <int J, class Word, class Value, class Put>
+template <int kThreads, int J, class Word, class Value, class Put>
 __device__ __noinline__ void unit_walk(uint32_t region, int nk, int nu, Word word, Value value,
                                        Put put) {
+  constexpr int kUnitWarps = 8;                            // words of a step (warps past them help to stage)
   constexpr int kK = 160;                                  // variants of a block
-  constexpr int kB = (kK / 2 * J + kUnitThreads - 1) / kUnitThreads;  // pairs of values
+  constexpr int kB = (kK / 2 * J + kThreads - 1) / kThreads;  // pairs of values
   static_assert(kK * (4 * kUnitWarps + 16 * J) <= (int)kWorkBytes, "work region");
   uint2 *A = (uint2 *)(unit_smem + region);                          // [kK / 16][8 words][4][2]
   uint32_t *B = (uint32_t *)(A + kK / 2 * kUnitWarps);     // [kK / 16][J][8][4][2]
@@ -1123,7 +1126,7 @@ __device__ __noinline__ void unit_walk(uint32_t region, int nk, int nu, Word wor
   const int r8 = lane >> 2, t4 = lane & 3, aw = tid & (kUnitWarps - 1), ap = tid / kUnitWarps;
   const uint32_t sh0 = 14 - r8, sh1 = (6 - r8) & 31;
   auto bits = [](uint32_t x, uint32_t sh) { return __funnelshift_l(x, x, sh) & 0x40004000u; };
-  constexpr int kPairs = kUnitThreads / kUnitWarps;          // pairs of operand A at a time
+  constexpr int kPairs = kThreads / kUnitWarps;          // pairs of operand A at a time
   constexpr int kAp = (kK / 2 + kPairs - 1) / kPairs;
   for (int w0 = 0; w0 < words; w0 += kUnitWarps) {
     float acc[2][J][4];
@@ -1147,7 +1150,7 @@ __device__ __noinline__ void unit_walk(uint32_t region, int nk, int nu, Word wor
       for (int r = 0; r < kB; r++)
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-          const int x = tid + r * kUnitThreads, j = x / (kK / 2), i = q + 2 * (x - j * (kK / 2)) + h;
+          const int x = tid + r * kThreads, j = x / (kK / 2), i = q + 2 * (x - j * (kK / 2)) + h;
           xb[r][h] = j < J && i < nu ? value(i, j) : 0ull;
         }
     };
@@ -1156,7 +1159,7 @@ __device__ __noinline__ void unit_walk(uint32_t region, int nk, int nu, Word wor
 #pragma unroll 1
     for (int q = 0; q < nu + kK; q += kK) {
       if (q < nu) load(q);
-      if (q > 0 && w0 + warp < words) {
+      if (q > 0 && warp < kUnitWarps && w0 + warp < words) {
         const int steps = (min(kK, nu - (q - kK)) + 15) >> 4;
         const uint4 *a4 = reinterpret_cast<const uint4 *>(A) + warp * 4 + t4;
         const uint2 *b2 = reinterpret_cast<const uint2 *>(B) + lane;
@@ -1184,7 +1187,7 @@ __device__ __noinline__ void unit_walk(uint32_t region, int nk, int nu, Word wor
       }
 #pragma unroll
       for (int r = 0; r < kB; r++) {
-        const int x = tid + r * kUnitThreads, j = x / (kK / 2), p = x - j * (kK / 2);
+        const int x = tid + r * kThreads, j = x / (kK / 2), p = x - j * (kK / 2);
         if (j >= J) continue;
         uint32_t *b = B + ((p >> 3) * J + j) * 64 + 2 * (p & 3) + ((p >> 2) & 1);
 #pragma unroll
@@ -1200,7 +1203,7 @@ __device__ __noinline__ void unit_walk(uint32_t region, int nk, int nu, Word wor
       }
       __syncthreads();
     }
-    if (w0 + warp >= words) continue;
+    if (warp >= kUnitWarps || w0 + warp >= words) continue;
     // a lane's two bytes' sums of samples r8 + 8 x, the four lanes' together
     // the value's; lane t4 keeps sample r8 + 8 t4
     unsigned long long sum[J];
@@ -1342,10 +1345,12 @@ static __device__ __noinline__ double unit_js(long long *dist, int S, int U, Uni
 // between dependent steps (0.68 million warp instructions a unit at the first
 // shape, 45% of the issue slots), a third of the time in the node scores'
 // population counts, whose rate (16 a cycle and SM) they reach.
+template <int kThreads>
 __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw) {
   UnitSmem &SM = *reinterpret_cast<UnitSmem *>(smraw);
-  const int nw = blockDim.x >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int tid = threadIdx.x, nt = blockDim.x;
+  // (not a constant: the loops would be unrolled past the instruction cache)
+  const int nt = blockDim.x, nw = nt >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // the unit's set: its descriptor into shared memory, its slices of the
   // batch's masks
   const BatchSet &bs = bd.sets[bd.uslot[u]];
@@ -1794,7 +1799,7 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
   if (entries) {
     // (the base scores' room behind the work region is free until then)
     if (nvar)
-      mark_variants(bd.sm, cp[0], cp[1], nA, nB, ent, vinf, vsplit, nvar, vw, vws,
+      mark_variants<kThreads>(bd.sm, cp[0], cp[1], nA, nB, ent, vinf, vsplit, nvar, vw, vws,
                     (int)(kWorkBytes + 4 * sizeof(long long) * (size_t)g));
     // the rows formed per sample: their hash differences, and their keys
     // into the table
@@ -2048,9 +2053,9 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
           put(i, x);
         }
       } else if (keep < 0) {
-        unit_walk<3>(bd.sm.itk, nk, nu, word, value, put);
+        unit_walk<kThreads, 3>(bd.sm.itk, nk, nu, word, value, put);
       } else {
-        unit_walk<4>(bd.sm.itk, nk, nu, word, value, put);
+        unit_walk<kThreads, 4>(bd.sm.itk, nk, nu, word, value, put);
       }
     }
   __syncthreads();
@@ -2315,13 +2320,14 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
 // 14.9 ms for 15.0).  The layouts, computed on the host, come with the
 // parameters: with each block's own (every thread's, before) 14.9 ms against
 // 12.0, 19.7 against 16.6 ms for 2000 small sets.
+template <int kThreads>
 __global__ void __maxnreg__(kUnitRegs) k_units(const __grid_constant__ BatchDev bd) {
   UnitSmem &SM = *reinterpret_cast<UnitSmem *>(unit_smem);
   int turn = 0;
   for (int u = blockIdx.x; u < bd.B; turn ^= 1) {
     int next = bd.B;
     if (threadIdx.x == 0 && (int)gridDim.x < bd.B) next = (int)(gridDim.x + atomicAdd(bd.taken, 1u));
-    run_unit(bd, u, unit_smem);
+    run_unit<kThreads>(bd, u, unit_smem);
     if (threadIdx.x == 0) SM.next[turn] = next;
     __syncthreads();
     u = SM.next[turn];
@@ -2424,23 +2430,34 @@ cudaError_t launch_pairs(const BatchSet *sets, const int32_t *uslot, const uint6
   return cudaGetLastError();
 }
 
-void plan_units(BatchDev &bd, int gmax, int n, int sms, size_t words) {
+void plan_units(BatchDev &bd, int gmax, double pairs, int n, int sms, size_t words) {
   const int c = gmax * (gmax - 1) / 2;
   bd.words_kept = words_kept(c, n + 2, words);
   bd.lay = unit_layout(c, n + 2, bd.words_kept);
   bd.sm = unit_slices(gmax, (n + 63) / 64);
   // a block per place on the GPU (an SM: 227 KB of shared memory, 1 KB a
   // block of it the system's, and 64 K registers)
-  const int per = std::min((227 << 10) / (int)(bd.sm.total + 1024), 65536 / (kUnitRegs * kUnitThreads));
-  bd.blocks = std::min(bd.B, std::max(1, per) * sms);
+  // Where shared memory leaves room for fewer than three blocks of 256
+  // threads (sets above about 230 genes), blocks of 384 fill the registers:
+  // 387 genes x 600 samples, 301 units 2.45 -> 1.88 ms, 3000 units 22.7 ->
+  // 17.7; with three blocks they are slower (200 x 1000, 12.2 -> 13.4).  A
+  // batch of mostly smaller sets keeps 256, which suits its units (150
+  // co-expressed sets of 8-250 genes 24.8 ms, with 384 25.5).
+  const int fit = (227 << 10) / (int)(bd.sm.total + 1024), warps = 65536 / (kUnitRegs * 32);
+  bd.threads = fit < 3 && 2.0 * pairs >= (double)bd.B * c ? 384 : 256;
+  bd.blocks = std::min(bd.B, std::max(1, std::min(fit, 32 * warps / bd.threads)) * sms);
 }
 
-cudaError_t launch_units(const BatchDev &bd, cudaStream_t st) {
-  cudaError_t e =
-      cudaFuncSetAttribute(k_units, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bd.sm.total);
+template <int kThreads>
+static cudaError_t launch_units_of(const BatchDev &bd, cudaStream_t st) {
+  cudaError_t e = cudaFuncSetAttribute(k_units<kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)bd.sm.total);
   if (e != cudaSuccess) return e;
-  k_units<<<bd.blocks, kUnitThreads, bd.sm.total, st>>>(bd);
+  k_units<kThreads><<<bd.blocks, kThreads, bd.sm.total, st>>>(bd);
   return cudaGetLastError();
+}
+cudaError_t launch_units(const BatchDev &bd, cudaStream_t st) {
+  return bd.threads == 384 ? launch_units_of<384>(bd, st) : launch_units_of<256>(bd, st);
 }
 
 cudaError_t launch_pack(const BatchDev &bd, int kept, int S, cudaStream_t st) {

@@ -25,9 +25,10 @@ cudaError_t launch_counter_masks(int n, int nA, int W, uint64_t seed, const int3
 cudaError_t launch_pairs(const BatchSet *sets, const int32_t *uslot, const uint64_t *masks,
                          uint32_t *dmask, int B, int W, int gmax, unsigned long long *stats,
                          cudaStream_t st);
-// Network, BDeu and JS kernel of a batch; before, its layouts and blocks (B:
-// bd.B units, the largest set of gmax genes, n samples).
-void plan_units(BatchDev &bd, int gmax, int n, int sms, size_t words = kVariantWords);
+// Network, BDeu and JS kernel of a batch; before, its layouts and blocks
+// (bd.B units of `pairs` pairs together, the largest set of gmax genes, n
+// samples).
+void plan_units(BatchDev &bd, int gmax, double pairs, int n, int sms, size_t words = kVariantWords);
 cudaError_t launch_units(const BatchDev &bd, cudaStream_t st);
 // Lists of the kept units' unique networks, after launch_units (S: networks).
 cudaError_t launch_pack(const BatchDev &bd, int kept, int S, cudaStream_t st);

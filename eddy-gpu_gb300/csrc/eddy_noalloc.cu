@@ -226,7 +226,7 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
     bd.masks = (const uint64_t *)(base + kOffMask);
     bd.dmask = (uint32_t *)(base + kOffDmask);
     bd.scratch = base + kOffUnit;
-    plan_units(bd, g, n, 1, kNAWords);
+    plan_units(bd, g, (double)c, n, 1, kNAWords);
     bd.js = d_js;
     bd.U = d_U;
     bd.status = d_status;
