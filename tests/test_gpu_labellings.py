@@ -28,3 +28,23 @@ def test_labellings_on_the_device(n, nA, R, eddy_lib, oracle_lib):
                                oracle_lib.params(mp=3))
     assert np.array_equal(U, oU)
     assert js_close(js, ojs)
+
+
+@pytest.mark.parametrize("units", [32768, 32771])
+def test_largest_batches(units, eddy_lib):
+    """One batch of 32768 units (the queue's largest unit index is used) and
+    one more than a batch holds, against the same labellings in batches of
+    8192."""
+    rng = np.random.default_rng(9)
+    g, n, nA = 40, 96, 40
+    z = rng.standard_normal(n)
+    data = np.digitize(z[None, :] + rng.standard_normal((g, n)), [-0.6, 0.6]).astype(np.int8) - 1
+    labels0 = np.concatenate([np.zeros(nA, np.uint8), np.ones(n - nA, np.uint8)])
+    ctx = eddy_lib.Context(max_parents=2, permutations=units, rng=eddy_lib.RNG_COUNTER, seed=3)
+    ctx.load_matrix(data, labels0)
+    sid = ctx.add_set(np.arange(g))
+    js, U = ctx.run_permutations(sid, 0, units)
+    parts = [ctx.run_permutations(sid, k, min(8192, units - k)) for k in range(0, units, 8192)]
+    ctx.close()
+    assert np.array_equal(U, np.concatenate([p[1] for p in parts]))
+    assert np.array_equal(js, np.concatenate([p[0] for p in parts]), equal_nan=True)
