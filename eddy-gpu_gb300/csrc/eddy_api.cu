@@ -690,11 +690,13 @@ struct UnitRef {
 // Runs the units `units` (in job order: a job's units are consecutive) as
 // one batch: the sets' data resident, the set table, labellings, decisions,
 // networks, normalisation and JS, one synchronisation.  Units whose status
-// asks for a re-run (a hash collision) go to *again; *queue_full: the general-path queue
+// asks for a re-run (a hash collision, no room for kept outputs) go to
+// *again; *queue_full: the general-path queue
 // overflowed (nothing was stored: the batch must be decided another way).
+// rerun: the units' decisions are in the sets' counters already.
 int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> &units,
-              bool popc_batch, std::vector<UnitRef> *again, bool *collision, bool *queue_full,
-              float *t_pairs, float *t_units) {
+              bool popc_batch, bool rerun, std::vector<UnitRef> *again, bool *collision,
+              bool *queue_full, float *t_pairs, float *t_units) {
   const int Bt = (int)units.size(), W = ctx->W, n = ctx->samples, S = n + 2;
   // slots: the jobs of the batch, in order
   std::vector<int> slot_job, ids;
@@ -757,8 +759,11 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   const int nk = (int)kept.size();
   if (nk) {
     // room for what earlier batches took or 128 MB (a batch that needs more
-    // says how much, and its kept units run again)
-    const size_t cap = std::min(kwords, std::max(ctx->d_kbuf.n / 8, (size_t)16 << 20));
+    // says how much, and its kept units run again; EDDY_KEEP_CAP lowers the
+    // 128 MB, to test that)
+    size_t first = (size_t)128 << 20;
+    if (const char *ek = getenv("EDDY_KEEP_CAP")) first = std::min(first, (size_t)std::max(8l, atol(ek)));
+    const size_t cap = std::min(kwords, std::max(ctx->d_kbuf.n, first) / 8);
     CK(ctx->d_kbuf.ensure(8 * cap));
   }
   {
@@ -842,7 +847,9 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   bd.kmeta = (KeepMeta *)(dout + o_km);
   bd.kbuf = ctx->d_kbuf.as<uint64_t>();
   bd.kcap = ctx->d_kbuf.n / 8;
-  bd.stats = (unsigned long long *)(dout + o_cnt);
+  // per set: exact rechecks, tables decided, tables settled by a filter (and a
+  // word of padding)
+  unsigned long long *stats = (unsigned long long *)(dout + o_cnt);
   // the batch's device work: labellings, decisions, networks (events
   // become record nodes when captured)
   auto record = [&](cudaEvent_t e, bool capturing) -> cudaError_t {
@@ -862,7 +869,7 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
     }
     CK(record(ctx->ev[0], capturing));
     {
-      int rc = launch_pairs_any(ctx, bp, bd.masks, bd.dmask, bd.stats, popc_batch,
+      int rc = launch_pairs_any(ctx, bp, bd.masks, bd.dmask, stats, popc_batch,
                                 ctx->ev[4]);
       if (rc) return rc;
     }
@@ -921,7 +928,7 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
                                       ctx->stream));
           cap_ck(record(ctx->ev[0], true));
           cap_ck(launch_pairs_mma(bp.d_sets, ns, mp, bd.masks, bd.uslot, n, W,
-                                  ctx->d_afp8.as<uint8_t>(), ctx->y, bd.dmask, bd.stats, bp.d_err,
+                                  ctx->d_afp8.as<uint8_t>(), ctx->y, bd.dmask, stats, bp.d_err,
                                   ctx->sms, ctx->stream, v,
                                   layout_core(v), ns == 1 ? bp.sets[0].sd.g : 0, ctx->ev[4],
                                   true));
@@ -982,8 +989,9 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
         ctx->ms_stage[q] += m;
     }
   }
-  for (int k = 0; k < ns; k++) {
-    for (int q = 0; q < 4; q++) ctx->last_stats[q] += hst4[4 * k + q];
+  // (a unit that runs again was decided, and counted, the first time)
+  for (int k = 0; k < ns && !rerun; k++) {
+    for (int q = 0; q < 3; q++) ctx->last_stats[q] += hst4[4 * k + q];
     jobs[slot_job[k]].exact += hst4[4 * k];
     jobs[slot_job[k]].tables += hst4[4 * k + 1];
   }
@@ -995,6 +1003,7 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
     } else {
       J.js[units[i].i] = hjs[i];
       J.U[units[i].i] = hU[i];
+      ctx->last_stats[3] += (unsigned long long)(S - hU[i]);
     }
   }
   // the packed outputs of the kept units that finished, in one copy
@@ -1056,12 +1065,12 @@ int run_jobs(eddy_ctx *ctx, std::vector<Job> &jobs) {
   float t_pairs = 0, t_units = 0;
   for (int b0 = 0; b0 < total; b0 += Bmax) {
     std::vector<UnitRef> todo(all.begin() + b0, all.begin() + std::min(total, b0 + Bmax));
-    bool popc_batch = false;
+    bool popc_batch = false, rerun = false;
     for (int attempt = 0; attempt < 4 && !todo.empty(); attempt++) {
       std::vector<UnitRef> again;
       bool collision = false, queue_full = false;
-      int rc = run_batch(ctx, jobs, todo, popc_batch, &again, &collision, &queue_full, &t_pairs,
-                         &t_units);
+      int rc = run_batch(ctx, jobs, todo, popc_batch, rerun, &again, &collision, &queue_full,
+                         &t_pairs, &t_units);
       if (rc) return rc;
       if (queue_full) {
         // a large share of tables near a threshold: decide this batch with
@@ -1069,6 +1078,7 @@ int run_jobs(eddy_ctx *ctx, std::vector<Job> &jobs) {
         popc_batch = true;
         continue;
       }
+      rerun = true;
       if (collision) ctx->salt = ctx->salt * 6364136223846793005ull + 1442695040888963407ull;
       todo.swap(again);
     }

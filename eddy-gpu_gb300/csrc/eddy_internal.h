@@ -188,8 +188,6 @@ struct BatchDev {
                                // entry 1 + slot is a kept unit's
   uint64_t *kbuf;              // the kept units' packed outputs (KeepLayout)
   unsigned long long kcap;     // its 8-byte words
-  unsigned long long *stats;   // [nsets][4] per set: exact rechecks, tables decided,
-                               // tables settled by a filter, duplicate networks
 };
 
 }  // namespace eddy

@@ -1379,7 +1379,6 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
       bd.js[u] = __longlong_as_double(0x7ff8000000000000ll);
       bd.U[u] = 1;
       bd.status[u] = 0u;
-      if (bd.stats) atomicAdd(&bd.stats[4 * (size_t)bd.uslot[u] + 3], (unsigned long long)(S - 1));
     }
     return;
   }
@@ -1863,7 +1862,6 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
     bd.js[u] = __longlong_as_double(0x7ff8000000000000ll);
     bd.U[u] = SM.status ? -1 : U;
     bd.status[u] = SM.status;
-    if (bd.stats) atomicAdd(&bd.stats[4 * (size_t)bd.uslot[u] + 3], (unsigned long long)(S - U));
   };
   // one network has no JS (the range of its scores is empty), whatever its
   // score is

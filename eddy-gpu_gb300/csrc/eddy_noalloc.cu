@@ -231,7 +231,6 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
     bd.U = d_U;
     bd.status = d_status;
     bd.keep_slot = nullptr;
-    bd.stats = nullptr;
     if (launch_units(bd, st) != cudaSuccess) return bail(EDDY_ERR_CUDA);
     unsigned char out[16];
     if (cudaMemcpyAsync(out, base + kOffOut, 16, cudaMemcpyDeviceToHost, st) != cudaSuccess)
