@@ -303,7 +303,8 @@ int prepare_sets(eddy_ctx *ctx, const std::vector<int> &ids) {
     // (a matrix loaded after the set was added may have fewer rows)
     for (int v : ctx->sets[ids[k]].genes)
       if (v >= ctx->genes) return fail(ctx, EDDY_ERR_ARG, "gene index %d out of range", v);
-    if (g > 512) return fail(ctx, EDDY_ERR_CAPACITY, "gene set %d has %d genes (> 512)", ids[k], (int)g);
+    if (g > kMaxSetGenes)
+      return fail(ctx, EDDY_ERR_CAPACITY, "gene set %d has %d genes (> %d)", ids[k], (int)g, kMaxSetGenes);
     genes += g;
   }
   const size_t orows = o;
@@ -1210,7 +1211,8 @@ int eddy_add_set(eddy_ctx *ctx, const int32_t *gene_idx, int g, const uint8_t *p
   if (!ctx) return EDDY_ERR_ARG;
   if (ctx->samples == 0) return fail(ctx, EDDY_ERR_STATE, "load the matrix first");
   if (!gene_idx || g < 0) return fail(ctx, EDDY_ERR_ARG, "bad gene set");
-  if (g > 512) return fail(ctx, EDDY_ERR_CAPACITY, "gene set of %d genes (> 512)", g);
+  if (g > kMaxSetGenes)
+    return fail(ctx, EDDY_ERR_CAPACITY, "gene set of %d genes (> %d)", g, kMaxSetGenes);
   SetHost S;
   S.genes.assign(gene_idx, gene_idx + g);
   for (int v : S.genes)

@@ -12,6 +12,7 @@
 
 namespace eddy {
 
+constexpr int kMaxSetGenes = 512;   // genes of a set at most
 constexpr int kDofSlots = 3;        // dof 1, 2, 4 (dof 0 never gives an edge)
 constexpr int kMaxBdeuParents = 3;  // kernel5.cu:119-130 caps at 1 + 3
 constexpr int kDivisors = 15;       // distinct q and q*r of the BDeu terms

@@ -148,6 +148,7 @@ __device__ __forceinline__ void philox10(uint32_t c[4], uint32_t k0, uint32_t k1
 // bins, waited at its barriers: 4.5 ms for 339000 units of 1000 samples, now
 // 0.9 ms.)
 constexpr int kCmWarps = 4, kCmBins = 256, kCmShift = 24;
+constexpr int kCmMaxSamples = 4096;  // (more: the labellings come from the host)
 __host__ __device__ constexpr int cm_words(int n) { return ((n + 3) & ~3) + kCmBins; }  // a warp's shared memory
 __global__ void __launch_bounds__(32 * kCmWarps) k_counter_masks(int n, int nA, int W, uint64_t seed,
                                                                  const int32_t *unit_set,
@@ -2394,6 +2395,10 @@ __global__ void __launch_bounds__(256) k_pack(const __grid_constant__ BatchDev b
 }
 
 // ------------------------------------------------------------ launchers
+// A kernel's limit of dynamic shared memory belongs to the process: every
+// launcher sets the largest value any of its launches can need, and the same
+// one each time, so a launch of one thread fits whatever another thread
+// launches meanwhile.  (It is a limit only: a launch takes what it asks for.)
 cudaError_t launch_prep(const PrepSet *sets, int ns, int genes, int pair_blocks, const int8_t *vals,
                         const int32_t *rows, int n, int W, uint64_t *valid, cudaStream_t st) {
   if (genes <= 0) return cudaSuccess;
@@ -2408,9 +2413,10 @@ cudaError_t launch_counter_masks(int n, int nA, int W, uint64_t seed, const int3
                                  const int32_t *unit_perm, const uint64_t *mask0, uint64_t *masks,
                                  int B, cudaStream_t st) {
   const size_t smem = sizeof(uint32_t) * kCmWarps * (size_t)cm_words(n);
+  if (n > kCmMaxSamples) return cudaErrorInvalidValue;
   if (smem > 48 * 1024) {
-    cudaError_t e =
-        cudaFuncSetAttribute(k_counter_masks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_counter_masks, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)sizeof(uint32_t) * kCmWarps * cm_words(kCmMaxSamples));
     if (e != cudaSuccess) return e;
   }
   k_counter_masks<<<(B + kCmWarps - 1) / kCmWarps, 32 * kCmWarps, smem, st>>>(n, nA, W, seed, unit_set,
@@ -2428,6 +2434,7 @@ cudaError_t launch_pairs(const BatchSet *sets, const int32_t *uslot, const uint6
   return cudaGetLastError();
 }
 
+constexpr int kSmBytes = 227 << 10;  // a block's most
 void plan_units(BatchDev &bd, int gmax, double pairs, int n, int sms, size_t words) {
   const int c = gmax * (gmax - 1) / 2;
   bd.words_kept = words_kept(c, n + 2, words);
@@ -2441,7 +2448,7 @@ void plan_units(BatchDev &bd, int gmax, double pairs, int n, int sms, size_t wor
   // 17.7; with three blocks they are slower (200 x 1000, 12.2 -> 13.4).  A
   // batch of mostly smaller sets keeps 256, which suits its units (150
   // co-expressed sets of 8-250 genes 24.8 ms, with 384 25.5).
-  const int fit = (227 << 10) / (int)(bd.sm.total + 1024), warps = 65536 / (kUnitRegs * 32);
+  const int fit = kSmBytes / (int)(bd.sm.total + 1024), warps = 65536 / (kUnitRegs * 32);
   bd.threads = fit < 3 && 2.0 * pairs >= (double)bd.B * c ? 384 : 256;
   bd.blocks = std::min(bd.B, std::max(1, std::min(fit, 32 * warps / bd.threads)) * sms);
 }
@@ -2449,7 +2456,7 @@ void plan_units(BatchDev &bd, int gmax, double pairs, int n, int sms, size_t wor
 template <int kThreads>
 static cudaError_t launch_units_of(const BatchDev &bd, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(k_units<kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)bd.sm.total);
+                                       kSmBytes);
   if (e != cudaSuccess) return e;
   k_units<kThreads><<<bd.blocks, kThreads, bd.sm.total, st>>>(bd);
   return cudaGetLastError();

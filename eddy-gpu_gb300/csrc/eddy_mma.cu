@@ -1321,10 +1321,13 @@ static cudaError_t launch_variant(const BatchSet *sets, int nsets, const MmaPlan
     gcnt = reinterpret_cast<const float4 *>(y.base + y_gc_offset(y));
     gtab = reinterpret_cast<const uint32_t *>(y.base + y_gt_offset(y));
   }
-  const size_t smem = 1024 + (size_t)kStages * (kTM + kTN) * kKC + kBarBytes +
-                      (kCore && nsets == 1 ? sizeof(float4) * (size_t)g_single : 0);
+  // (the limit, which all threads' launches share, is the one of the largest
+  // set: a launch never depends on which set another thread launches)
+  constexpr size_t fixed = 1024 + (size_t)kStages * (kTM + kTN) * kKC + kBarBytes;
+  const size_t smem = fixed + (kCore && nsets == 1 ? sizeof(float4) * (size_t)g_single : 0);
   auto kern = k_pairs_mma<kStages, kEpi, kGroups, kCore>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(fixed + (kCore ? sizeof(float4) * kMaxSetGenes : 0)));
   if (e != cudaSuccess) return e;
   const int grid = plan.ntot < sms ? plan.ntot : sms;
   kern<<<grid, 32 * (2 + kEpi), smem, st>>>(ma, mb, sets, nsets, ctotf, np / kKC, plan.ntot,
