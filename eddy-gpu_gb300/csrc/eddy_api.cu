@@ -996,6 +996,7 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
     jobs[slot_job[k]].exact += hst4[4 * k];
     jobs[slot_job[k]].tables += hst4[4 * k + 1];
   }
+  unsigned long long duplicates = 0;
   for (int i = 0; i < Bt; i++) {
     Job &J = jobs[units[i].job];
     if (hst[i]) {
@@ -1004,9 +1005,10 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
     } else {
       J.js[units[i].i] = hjs[i];
       J.U[units[i].i] = hU[i];
-      ctx->last_stats[3] += (unsigned long long)(S - hU[i]);
+      duplicates += (unsigned long long)(S - hU[i]);
     }
   }
+  ctx->last_stats[3] += duplicates;
   // the packed outputs of the kept units that finished, in one copy
   if (nk) {
     const size_t need = (size_t)hkm[0].off, have = std::min(need, ctx->d_kbuf.n / 8);
