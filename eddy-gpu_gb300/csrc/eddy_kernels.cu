@@ -1235,7 +1235,10 @@ __device__ __noinline__ void unit_walk(uint32_t region, int nk, int nu, Word wor
 // odd ones class 2 (one copy of the code for both, and its latency: FP64's is
 // most of a small unit's JS).  Sums are formed in a fixed order, the same in
 // both classes: a thread's networks in turn, then a tree over the warp, then
-// the warps in turn.  pl, ql: the kept normalised likelihoods, or null.
+// the warps in turn.  The first 256 threads take part, whatever the block
+// has, so that a unit's JS is the same bits in every batch (a set's block
+// size depends on the sets beside it).  pl, ql: the kept normalised
+// likelihoods, or null.
 //
 // Inside k_units rather than after it: FP64 is slow on this part (about two
 // operations a cycle and SM, ~128 cycles to a dependent one), and here its
@@ -1244,11 +1247,12 @@ __device__ __noinline__ void unit_walk(uint32_t region, int nk, int nu, Word wor
 // 1000 networks, 18.4 ms for 75000 of 400 and 68 us for one unit of 300.
 static __device__ __noinline__ double unit_js(long long *dist, int S, int U, UnitSmem &SM, double *pl,
                                               double *ql) {
-  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int kJsThreads = 256, us = kJsThreads / 2;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // the warps that hold networks, and the lanes of a warp that do (the sums
   // over the others' zeros are left out: each costs a dependent FP64 add)
-  const int nw = min(nt >> 5, (2 * U + 31) >> 5), lanes = min(2 * U, 32);
-  const int cls = tid & 1, u0 = tid >> 1, us = nt >> 1;
+  const int nw = min(kJsThreads >> 5, (2 * U + 31) >> 5), lanes = min(2 * U, 32);
+  const int cls = tid & 1, u0 = tid < kJsThreads ? tid >> 1 : U;
   long long *d = dist + (cls ? S : 0);
   long long mn = LLONG_MAX, mx = LLONG_MIN;
   unsigned long long sum = 0;  // modulo 2^64
