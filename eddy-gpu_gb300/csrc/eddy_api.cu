@@ -22,6 +22,7 @@
 #include "eddy_internal.h"
 #include "eddy_kernels.h"
 #include "eddy_mma.h"
+#include "eddy_pool.h"
 
 using namespace eddy;
 
@@ -96,40 +97,17 @@ struct KeepView {
   }
 };
 
-// The kept outputs of the sets: page-locked chunks that the batches' packed
-// outputs are copied into, as they are, and that hold them until
-// eddy_clear_sets.  A context's later sets reuse the room (one chunk of all
-// that was taken).
-struct ResultPool {
-  std::vector<PinnedBuf> chunks;
-  size_t used = 0, grow = 0;
-  cudaError_t take(size_t bytes, uint8_t **out) {
-    bytes = (bytes + 255) & ~(size_t)255;
-    if (chunks.empty() || used + bytes > chunks.back().n) {
-      PinnedBuf b;
-      cudaError_t e = b.ensure(std::max(bytes, grow));
-      if (e != cudaSuccess) return e;
-      chunks.push_back(b);
-      used = 0;
-    }
-    *out = chunks.back().as<uint8_t>(used);
-    used += bytes;
-    return cudaSuccess;
+// Page-locked memory of the sets' kept outputs.
+struct PinnedAlloc {
+  static void *alloc(size_t n) {
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, n, cudaHostAllocDefault) == cudaSuccess) return p;
+    cudaGetLastError();
+    return nullptr;
   }
-  void clear() {
-    if (chunks.size() > 1) {
-      grow = 0;
-      for (PinnedBuf &b : chunks) grow += b.n;
-      release();
-    }
-    used = 0;
-  }
-  void release() {
-    for (PinnedBuf &b : chunks) b.release();
-    chunks.clear();
-    used = 0;
-  }
+  static void release(void *p) { cudaFreeHost(p); }
 };
+using ResultPool = ChunkPool<PinnedAlloc>;
 
 struct SetHost {
   std::vector<int32_t> genes;
@@ -1012,8 +990,8 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   // the packed outputs of the kept units that finished, in one copy
   if (nk) {
     const size_t need = (size_t)hkm[0].off, have = std::min(need, ctx->d_kbuf.n / 8);
-    uint8_t *host = nullptr;
-    CK(ctx->results.take(8 * have, &host));
+    uint8_t *host = ctx->results.take(8 * have);
+    if (!host) return fail(ctx, EDDY_ERR_CUDA, "no host memory for %zu bytes of networks", 8 * have);
     CK(cudaMemcpyAsync(host, ctx->d_kbuf.p, 8 * have, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     for (int q = 0; q < nk; q++) {
@@ -1797,11 +1775,11 @@ int eddy_debug_unit(eddy_ctx *ctx, int set_id, const uint8_t *labels, int mpk, i
   KeepView K;
   double j = 0;
   int32_t u = 0;
-  const size_t used = ctx->results.used, chunks = ctx->results.chunks.size();
+  const ResultPool::Mark before = ctx->results.mark();
   int rc = run_units(ctx, set_id, 1, m.data(), nullptr, &j, &u, &K);
-  if (rc) return rc;
   // (this call's outputs are copied out below: their room is free again)
-  if (ctx->results.chunks.size() == chunks) ctx->results.used = used;
+  ctx->results.rewind(before);
+  if (rc) return rc;
   const int g = (int)ctx->sets[set_id].genes.size(), S = n + 2;
   const KeepLayout k = K.at();
   const int32_t *nodes = K.as<int32_t>(k.nodes), *epn = K.as<int32_t>(k.epn);
