@@ -404,6 +404,16 @@ void labels_to_mask(const uint8_t *labels, int n, int W, uint64_t *mask) {
     if (labels[s] == 0) mask[s >> 6] |= 1ull << (s & 63);
 }
 
+// Labellings from the caller keep the class sizes: the unit kernel's arrays
+// (samples in class order, the classes' packed states) are laid out for nA and
+// n - nA samples, and other counts would be written past them.
+int check_labelling(eddy_ctx *ctx, const uint8_t *labels, int index) {
+  int a = 0;
+  for (int s = 0; s < ctx->samples; s++) a += labels[s] == 0;
+  if (a == ctx->nA) return EDDY_OK;
+  return fail(ctx, EDDY_ERR_ARG, "labelling %d has %d class-0 samples, expected %d", index, a, ctx->nA);
+}
+
 // Contingency + decision kernel of a batch: the tcgen05 GEMM path unless
 // EDDY_PAIRS_KERNEL=popc selects the popcount kernel.
 bool use_popc() {
@@ -1339,7 +1349,11 @@ static int run_set(eddy_ctx *ctx, int set_id) {
     // iteration 0 (kept: networks and likelihoods for the output files)
     std::vector<uint64_t> masks((size_t)W);
     std::vector<uint8_t> lab(ctx->labels0);
-    if (ctx->o.rng == EDDY_RNG_EXTERNAL) lab.assign(S.labels.begin(), S.labels.begin() + n);
+    if (ctx->o.rng == EDDY_RNG_EXTERNAL) {
+      lab.assign(S.labels.begin(), S.labels.begin() + n);
+      rc = check_labelling(ctx, lab.data(), 0);
+      if (rc) return rc;
+    }
     if (ctx->o.rng == EDDY_RNG_GLIBC)
       glibc_permutation(ctx->rng, n, ctx->nA, false, lab.data(), ctx->seen, ctx->order);
     labels_to_mask(lab.data(), n, W, masks.data());
@@ -1395,9 +1409,8 @@ static int run_set(eddy_ctx *ctx, int set_id) {
             counter_labels(ctx->o.seed, set_id, i + 1, n, ctx->nA, cur.data());
           } else {
             memcpy(cur.data(), S.labels.data() + (size_t)(i + 1) * n, n);
-            int a = 0;
-            for (int s = 0; s < n; s++) a += cur[s] == 0;
-            if (a != ctx->nA) return fail(ctx, EDDY_ERR_ARG, "labelling %d changes the class sizes", i + 1);
+            rc = check_labelling(ctx, cur.data(), i + 1);
+            if (rc) return rc;
           }
           labels_to_mask(cur.data(), n, W, mh.data() + (size_t)i * W);
         }
@@ -1673,9 +1686,8 @@ int eddy_run_labellings(eddy_ctx *ctx, int set_id, const uint8_t *labels, int R,
     return fail(ctx, EDDY_ERR_ARG, "bad arguments");
   const int n = ctx->samples, W = ctx->W;
   for (int r = 0; r < R; r++) {
-    int a = 0;
-    for (int s = 0; s < n; s++) a += labels[(size_t)r * n + s] == 0;
-    if (a != ctx->nA) return fail(ctx, EDDY_ERR_ARG, "labelling %d has %d class-0 samples, expected %d", r, a, ctx->nA);
+    int rc = check_labelling(ctx, labels + (size_t)r * n, r);
+    if (rc) return rc;
   }
   ctx->ms_total = ctx->ms_pairs = ctx->ms_units = 0;
   for (double &m : ctx->ms_stage) m = 0;
@@ -1696,7 +1708,9 @@ int eddy_debug_edges(eddy_ctx *ctx, int set_id, const uint8_t *labels, uint8_t *
   if (!ctx || !labels || !edges || set_id < 0 || set_id >= (int)ctx->sets.size()) return EDDY_ERR_ARG;
   const int n = ctx->samples, W = ctx->W;
   if (ctx->sets[set_id].genes.size() < 2) return EDDY_OK;  // no pair
-  int rc = prepare_sets(ctx, {set_id});
+  int rc = check_labelling(ctx, labels, 0);
+  if (rc) return rc;
+  rc = prepare_sets(ctx, {set_id});
   if (rc) return rc;
   // a batch of one unit of one set
   BatchPlan bp;
@@ -1770,13 +1784,15 @@ int eddy_debug_unit(eddy_ctx *ctx, int set_id, const uint8_t *labels, int mpk, i
   if (!ctx || !labels || set_id < 0 || set_id >= (int)ctx->sets.size() || mpk < 1) return EDDY_ERR_ARG;
   const int n = ctx->samples, W = ctx->W;
   if (ctx->sets[set_id].genes.size() < 2) return fail(ctx, EDDY_ERR_ARG, "set %d has no pair", set_id);
+  int rc = check_labelling(ctx, labels, 0);
+  if (rc) return rc;
   std::vector<uint64_t> m(W);
   labels_to_mask(labels, n, W, m.data());
   KeepView K;
   double j = 0;
   int32_t u = 0;
   const ResultPool::Mark before = ctx->results.mark();
-  int rc = run_units(ctx, set_id, 1, m.data(), nullptr, &j, &u, &K);
+  rc = run_units(ctx, set_id, 1, m.data(), nullptr, &j, &u, &K);
   // (this call's outputs are copied out below: their room is free again)
   ctx->results.rewind(before);
   if (rc) return rc;
@@ -1837,6 +1853,8 @@ int eddy_run_permutations(eddy_ctx *ctx, int set_id, int first, int count, doubl
     } else {
       if (it >= S.R_ext) return fail(ctx, EDDY_ERR_ARG, "iteration %d has no labelling", it);
       memcpy(cur.data(), S.labels.data() + (size_t)it * n, n);
+      int rc = check_labelling(ctx, cur.data(), it);
+      if (rc) return rc;
     }
     labels_to_mask(cur.data(), n, W, mh.data() + (size_t)i * W);
   }
