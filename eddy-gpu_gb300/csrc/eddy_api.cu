@@ -1021,6 +1021,20 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   return EDDY_OK;
 }
 
+// Device bytes a batch needs for each set of it: the set's part of the arena
+// of prepare_sets and, where the contraction may decide the batch, of the Y
+// arena (in the 9-cell layout, the larger one).
+size_t set_bytes(const eddy_ctx *ctx, int g, bool contraction) {
+  const size_t n = (size_t)ctx->samples, c = (size_t)g * (g - 1) / 2;
+  const size_t inputs = sizeof(PrepSet) + (sizeof(int32_t) + n) * g + 19 * c +
+                        sizeof(uint32_t) * g * code_words((int)n) +
+                        2 * sizeof(uint64_t) * g * 3 * ctx->W + 4 * 256;
+  SetDev sd{};
+  sd.g = g;
+  sd.c = (int)c;
+  return inputs + (contraction ? mma_y_bytes(mma_ngroups_pad(sd, false), g, (int)n) : 0);
+}
+
 // Runs jobs of sets that share a contingency-kernel choice (one tuning key)
 // in equal batches of units across the jobs (a batch may hold the units of
 // several sets), each unit run again until its status is clean.
@@ -1029,8 +1043,13 @@ int run_jobs(eddy_ctx *ctx, std::vector<Job> &jobs) {
   const int n = ctx->samples, S = n + 2, W = ctx->W;
   int cmax = 1, total = 0;
   size_t per_unit_max = 1;
+  // (batches of sets of so few units each never go to the contraction)
+  bool contraction = !use_popc() && !few_units(1, 1, 0.0);
+  for (const Job &J : jobs) contraction = contraction || (J.n_units > kFewUnits && !use_popc());
+  std::vector<BatchJob> parts;
   for (const Job &J : jobs) {
     const int g = (int)ctx->sets[J.set_id].genes.size(), c = g * (g - 1) / 2;
+    parts.push_back({J.n_units, set_bytes(ctx, g, contraction)});
     cmax = std::max(cmax, c);
     total += J.n_units;
     per_unit_max = std::max(per_unit_max, (J.keep ? unit_scratch_bytes(c, S) : 0) + 4 * (size_t)c + 8 * W + 64);
@@ -1040,7 +1059,12 @@ int run_jobs(eddy_ctx *ctx, std::vector<Job> &jobs) {
   // with 16384, 69.4 ms for 67.8 in a sweep of 339000)
   // and by the queue's room for every table of the batch (2^28): the units
   // are then split into batches of equal size (later calls of the same
-  // size replay them)
+  // size replay them).  A batch of many sets ends earlier where the sets' own
+  // data would pass 32 GB: a sweep with few permutations a set holds many sets
+  // a batch (20 permutations of sets of 120 genes x 4096 samples: 989 sets,
+  // 291 GB of operands; 2000 sets of 5-300 genes x 1000 samples with 1000
+  // permutations: 33 sets, 15 GB).
+  constexpr size_t kSetBytes = (size_t)32 << 30;
   int Bmax = (int)std::max<size_t>(1, ((size_t)16 << 30) / per_unit_max);
   Bmax = std::min(Bmax, 32768);
   Bmax = (int)std::min<size_t>((size_t)Bmax, std::max<size_t>(1, ((size_t)1 << 28) / (2 * (size_t)cmax)));
@@ -1054,8 +1078,9 @@ int run_jobs(eddy_ctx *ctx, std::vector<Job> &jobs) {
     for (int i = 0; i < jobs[j].n_units; i++) all.push_back({j, i});
   ctx->last_stats[0] = ctx->last_stats[1] = ctx->last_stats[2] = ctx->last_stats[3] = 0;
   float t_pairs = 0, t_units = 0;
-  for (int b0 = 0; b0 < total; b0 += Bmax) {
-    std::vector<UnitRef> todo(all.begin() + b0, all.begin() + std::min(total, b0 + Bmax));
+  for (int b0 = 0, b1; b0 < total; b0 = b1) {
+    b1 = b0 + batch_units(parts, all[b0].job, all[b0].i, Bmax, kSetBytes);
+    std::vector<UnitRef> todo(all.begin() + b0, all.begin() + b1);
     bool popc_batch = false, rerun = false;
     for (int attempt = 0; attempt < 4 && !todo.empty(); attempt++) {
       std::vector<UnitRef> again;

@@ -270,6 +270,19 @@ bool beta_pddn(const double *js, int R, double &alpha, double &beta, double &pdd
   return true;
 }
 
+// ------------------------------------------------------------ batches
+int batch_units(const std::vector<BatchJob> &jobs, int job, int unit, int max_units,
+                size_t max_bytes) {
+  int n = 0;
+  size_t bytes = 0;
+  for (size_t j = (size_t)job; j < jobs.size() && n < max_units; j++) {
+    if (n > 0 && (bytes > max_bytes || jobs[j].bytes > max_bytes - bytes)) break;
+    bytes += jobs[j].bytes;
+    n += std::min(max_units - n, jobs[j].units - ((int)j == job ? unit : 0));
+  }
+  return n;
+}
+
 // ------------------------------------------------------------ BDeu table
 namespace {
 // an unevaluated sum of two doubles, |lo| <= ulp(hi) / 2

@@ -90,6 +90,18 @@ double ibetac(double a, double b, double x);
 // Returns false when alpha or beta is not positive finite.
 bool beta_pddn(const double *js, int R, double &alpha, double &beta, double &pddn);
 
+// One set's part of a run's batches: its units and the device bytes that a
+// batch holding any of them needs for the set (inputs and operands).
+struct BatchJob {
+  int units;
+  size_t bytes;
+};
+// Units of the batch that starts at unit `unit` of job `job` and goes on
+// through the jobs in order: at most max_units, and no further set once the
+// sets' bytes would pass max_bytes (at least one set's units).
+int batch_units(const std::vector<BatchJob> &jobs, int job, int unit, int max_units,
+                size_t max_bytes);
+
 // Fixed-point BDeu table lg[d][m] = (lgamma(m + 4/d) - lgamma(4/d)) * 2^shift.
 void bdeu_table(int n, std::vector<int64_t> &lg, int &shift, int8_t dmap[82]);
 // The same into a caller array of kDivisors * (n + 1) entries (no allocation).
