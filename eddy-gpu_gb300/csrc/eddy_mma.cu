@@ -567,8 +567,11 @@ __global__ void __maxnreg__(max_regs<kEpi>())
 #pragma unroll 1
       for (int gi = 0; gi < kGpw; gi++) {
         const int grp = wq + gi * kPerQuad;
+        // (tcgen05.ld wants the whole warp; the group before may have ended in
+        // lanes that stored masks of their own)
+        __syncwarp();
         // the group's 32 TMEM columns (the 4-cell layout reads them in two
-        // halves in pass 1, and again in full for pass 2)
+        // halves in pass 1); pass 2 reads a pair's four or nine again
         const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * kTN + grp * 32);
         uint32_t r[kCore ? 1 : 32];
         if constexpr (!kCore) {
