@@ -289,7 +289,7 @@ def run_multiset(args, rank, world, local):
             "wall_units_per_s": units / wall, "units": units, "sets": len(sids),
             "sets_per_s": len(sids) / (ms / 1e3), "ms": ms, "launches": t["launches"],
             "stage_ms": {"k_operands+k_pairs_mma": t["ms_gemm"], "k_general+k_exact": t["ms_decide"],
-                         "k_units": t["ms_networks"]},
+                         "k_units": t["ms_units"], "k_units_js": t["ms_js"]},
             "sets_stopped_at_iteration0": stop0,
             "sets_with_all_iterations": sum(1 for it in iters if it == R),
             "per_set_value": units / (ms_per_set / 1e3),
@@ -473,7 +473,7 @@ def run_ours(args, rank, world, local):
     # networks, dedup, BDeu, JS: bound by the SMs' issue slots, not by bytes
     # (which are reported beside it): warp instructions per unit as ncu counts
     # them, against four a cycle and SM at the sampled clock
-    k2_ms = acc["ms_networks"] / launches_per_kernel
+    k2_ms = acc["ms_units"] / launches_per_kernel
     insts = traffic_info.get("k_units_warp_instructions_per_unit", 0) * Bl
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     issue = 4.0 * sms * (clk.summary().get("sm_mhz") or 2070.0) / 1e3
@@ -528,8 +528,8 @@ def run_ours(args, rank, world, local):
                     "d2h_bytes_per_step": d2h},
             "gpu_launches": acc["launches"],
             "stage_ms": {"k_operands+k_pairs_mma": acc["ms_gemm"],
-                         "k_general+k_exact": acc["ms_decide"], "k_units": acc["ms_networks"],
-                         "steps": args.steps},
+                         "k_general+k_exact": acc["ms_decide"], "k_units": acc["ms_units"],
+                         "k_units_js": acc["ms_js"], "steps": args.steps},
             "roofline": roofline,
             "kernels": {"k_pairs_mma": k1, "k_units": k2},
             "clocks": clk.summary(),

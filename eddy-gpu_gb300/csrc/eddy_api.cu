@@ -180,7 +180,7 @@ struct eddy_ctx {
   // timing of the last run
   double ms_total = 0, ms_pairs = 0, ms_units = 0;
   // the same split by kernel: operands + contraction, general + exact
-  // decisions, networks with normalisation and JS; the last is 0
+  // decisions, networks, normalisation and JS
   double ms_stage[4] = {0, 0, 0, 0};
   long long launches = 0;
   uint64_t salt = 0x5EED5EEDull;
@@ -774,8 +774,10 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   const size_t i_lab = (i_keep + 4 * Bz + 255) & ~(size_t)255;
   const size_t in_bytes = i_lab + (masks_host ? 8 * Bz * W : 8 * Bz);
   // results, in one copy: [JS][U][status], then, 0 before the batch, the error
-  // word, the unit kernel's counter of units taken, the sets' decision counters and the kept units' table
-  const size_t o_U = 8 * Bz, o_st = o_U + 4 * Bz, o_err = o_st + 4 * Bz, o_cnt = o_err + 8;
+  // word, the unit kernel's counter of units taken and its cycles, the sets'
+  // decision counters and the kept units' table
+  const size_t o_U = 8 * Bz, o_st = o_U + 4 * Bz, o_err = o_st + 4 * Bz, o_cyc = o_err + 8;
+  const size_t o_cnt = o_cyc + 16;
   const size_t o_km = o_cnt + 32 * (size_t)ns;
   const size_t out_bytes = o_km + sizeof(KeepMeta) * (size_t)(nk + 1);
   CK(ctx->d_in.ensure(in_bytes));
@@ -836,6 +838,7 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
   bd.kmeta = (KeepMeta *)(dout + o_km);
   bd.kbuf = ctx->d_kbuf.as<uint64_t>();
   bd.kcap = ctx->d_kbuf.n / 8;
+  bd.cycles = (unsigned long long *)(dout + o_cyc);
   // per set: exact rechecks, tables decided, tables settled by a filter (and a
   // word of padding)
   unsigned long long *stats = (unsigned long long *)(dout + o_cnt);
@@ -977,6 +980,11 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
       if (cudaEventElapsedTime(&m, ctx->ev[cut[q]], ctx->ev[cut[q + 1]]) == cudaSuccess)
         ctx->ms_stage[q] += m;
     }
+    // the networks' time by what the unit kernel's blocks spent it on
+    const unsigned long long *cyc = ctx->h_res.as<unsigned long long>(o_cyc);
+    const double js = cyc[0] ? bms * ((double)cyc[1] / (double)cyc[0]) : 0.0;
+    ctx->ms_stage[2] -= js;
+    ctx->ms_stage[3] += js;
   }
   // (a unit that runs again was decided, and counted, the first time)
   for (int k = 0; k < ns && !rerun; k++) {

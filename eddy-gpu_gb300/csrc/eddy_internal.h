@@ -189,6 +189,8 @@ struct BatchDev {
                                // entry 1 + slot is a kept unit's
   uint64_t *kbuf;              // the kept units' packed outputs (KeepLayout)
   unsigned long long kcap;     // its 8-byte words
+  unsigned long long *cycles;  // [2] SM cycles of the unit kernel's blocks, and of their
+                               // normalisation and JS, added up (null: not wanted)
 };
 
 }  // namespace eddy

@@ -591,6 +591,7 @@ struct UnitSmem {
   int nsel;     // variants to score
   int any;
   int next[2];  // the block's next unit (by turns)
+  long long cycles[2];  // BatchDev::cycles of this block
   unsigned status;
   unsigned long long koff;  // a kept unit's region of the packed outputs
   int scan[32];
@@ -2313,8 +2314,12 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
   }
 
   // ---- P8: normalisation and JS
+  if (tid == 0) SM.cycles[1] -= clock64();
   const double js = unit_js(dist, S, U, SM, pl, ql);
-  if (tid == 0) bd.js[u] = js;
+  if (tid == 0) {
+    SM.cycles[1] += clock64();
+    bd.js[u] = js;
+  }
 }
 
 // A block per place on the GPU, each unit taken when a block is free, so that
@@ -2327,6 +2332,10 @@ template <int kThreads>
 __global__ void __maxnreg__(kUnitRegs) k_units(const __grid_constant__ BatchDev bd) {
   UnitSmem &SM = *reinterpret_cast<UnitSmem *>(unit_smem);
   int turn = 0;
+  if (threadIdx.x == 0) {
+    SM.cycles[0] = -clock64();
+    SM.cycles[1] = 0;
+  }
   for (int u = blockIdx.x; u < bd.B; turn ^= 1) {
     int next = bd.B;
     if (threadIdx.x == 0 && (int)gridDim.x < bd.B) next = (int)(gridDim.x + atomicAdd(bd.taken, 1u));
@@ -2334,6 +2343,10 @@ __global__ void __maxnreg__(kUnitRegs) k_units(const __grid_constant__ BatchDev 
     if (threadIdx.x == 0) SM.next[turn] = next;
     __syncthreads();
     u = SM.next[turn];
+  }
+  if (threadIdx.x == 0 && bd.cycles) {
+    atomicAdd(bd.cycles, (unsigned long long)(SM.cycles[0] + clock64()));
+    atomicAdd(bd.cycles + 1, (unsigned long long)SM.cycles[1]);
   }
 }
 

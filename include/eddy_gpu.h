@@ -223,9 +223,9 @@ int eddy_last_timing(const eddy_ctx *ctx, double *ms_kernels, double *ms_pairs, 
 /* The same device time split by kernel, in milliseconds: ms4[0] the
  * operand and contraction kernels (k_operands, k_pairs_mma; k_pairs on the
  * popcount path), ms4[1] the general-path and exact decisions (k_general,
- * k_exact), ms4[2] the network kernel (k_units), which ends with the
- * normalisation and JS, ms4[3] 0 (no kernel of their own).  ms4[0] + ms4[1]
- * = ms_pairs, ms4[2] + ms4[3] = ms_units. */
+ * k_exact), ms4[2] the network kernel (k_units) less ms4[3], the part of it
+ * that its blocks spend in the normalisation and JS at its end (by their SM
+ * cycles).  ms4[0] + ms4[1] = ms_pairs, ms4[2] + ms4[3] = ms_units. */
 int eddy_last_stage_timing(const eddy_ctx *ctx, double *ms4);
 
 #ifdef __cplusplus
