@@ -309,7 +309,7 @@ Two two_of(long double v) {
 // 2 atanh(z), z = 1 / (2 (a + i) + 1) = D / (8 + (2 i + 1) D), whose series
 // 2 (z + z^3 / 3 + ...) needs few terms: z is kept as a pair, the terms from
 // z^3 on, at most z^2 / 3 < 1/26 of z, in double.  The error of a sum of n
-// is below n 2^-58, under 1% of the fixed-point step at n = 1000 (2^-40).
+// is below n 2^-58, under 0.1% of the fixed-point step at n = 1000 (2^-37).
 // lgammal, entry by entry, took 1.1 us each where long double has no
 // hardware (16 ms for a table of 1000 samples); this takes ~20 ns.
 void bdeu_table_into(int n, int64_t *lg, int &shift, int8_t dmap[82]) {

@@ -2460,11 +2460,15 @@ void plan_units(BatchDev &bd, int gmax, double pairs, int n, int sms, size_t wor
   // a block per place on the GPU (an SM: 227 KB of shared memory, 1 KB a
   // block of it the system's, and 64 K registers)
   // Where shared memory leaves room for fewer than three blocks of 256
-  // threads (sets above about 230 genes), blocks of 384 fill the registers:
-  // 387 genes x 600 samples, 301 units 2.45 -> 1.88 ms, 3000 units 22.7 ->
-  // 17.7; with three blocks they are slower (200 x 1000, 12.2 -> 13.4).  A
-  // batch of mostly smaller sets keeps 256, which suits its units (150
-  // co-expressed sets of 8-250 genes 24.8 ms, with 384 25.5).
+  // threads (sets above about 240 genes), blocks of 384 give an SM more
+  // warps: 24 for 16 where two blocks fit (up to about 380 genes), 12 for 8
+  // where one does.  n = 600, 3000 units of 245 / 300 / 378 genes (two
+  // blocks) 5.85 -> 5.07, 9.17 -> 7.73, 14.7 -> 11.9 ms, of 387 / 512 (one)
+  // 22.6 -> 17.6, 38.8 -> 29.8; 301 units of 387 genes 2.43 -> 1.87.  With
+  // three blocks the registers are full already, and blocks of 384 come two
+  // an SM: 230 genes 4.67 -> 4.76, 200 x 1000 12.2 -> 13.4.  A batch of mostly
+  // smaller sets keeps 256, which suits its units (150 co-expressed sets of
+  // 8-250 genes 24.8 ms, with 384 25.5).
   const int fit = kSmBytes / (int)(bd.sm.total + 1024), warps = 65536 / (kUnitRegs * 32);
   bd.threads = fit < 3 && 2.0 * pairs >= (double)bd.B * c ? 384 : 256;
   bd.blocks = std::min(bd.B, std::max(1, std::min(fit, 32 * warps / bd.threads)) * sms);

@@ -83,7 +83,9 @@ int eddy_add_set(eddy_ctx *ctx, const int32_t *gene_idx, int g, const uint8_t *p
 
 /* Caller-supplied labellings for EDDY_RNG_EXTERNAL (replaces the
  * permutation loop's classIDs, main.cu:561-570).  labels: R x samples,
- * row 0 is the unpermuted labelling. */
+ * row 0 is the unpermuted labelling.  As everywhere below, a labelling has
+ * the matrix's class sizes: the call that runs another one refuses it
+ * (EDDY_ERR_ARG). */
 int eddy_set_labellings(eddy_ctx *ctx, int set_id, const uint8_t *labels, int R);
 
 /* Runs every set: all permutations of the hot path (main.cu:538-1460) and
