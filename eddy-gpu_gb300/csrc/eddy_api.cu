@@ -444,6 +444,17 @@ bool few_units(int units, int nsets, double pair_words) {
   return units <= kFewUnits * nsets || (units < 512 && pair_words <= kFewPairWords);
 }
 
+// A class above kFastMaxN samples is decided in FP64 throughout (one class at
+// most, ten decisions a pair): k_exact spreads them over the GPU, where the
+// popcount kernel's blocks take their own pairs' in turn.  One set whose
+// decisions the contraction's list has room for goes there: 65000 samples,
+// 52000 in a class, one labelling of 10 / 30 / 100 genes 0.53 / 0.58 / 0.60
+// ms -> 0.22 / 0.26 / 0.67; 16 labellings of 30 genes (too many for the list:
+// decided twice) 1.78 against 0.61.
+bool exact_class(const eddy_ctx *ctx, int nsets, double pairs) {
+  return nsets == 1 && std::max(ctx->nA, ctx->nB) > kFastMaxN && 10 * pairs <= kQueueMin;
+}
+
 // Contingency-kernel choices for a batch: tile shape v % mma_variants(), in
 // the 4-cell layout when v >= mma_variants() and in the 9-cell layout
 // otherwise.  The 4-cell layout is offered to sets that allow it (sd.core)
@@ -592,7 +603,8 @@ int launch_pairs_any(eddy_ctx *ctx, BatchPlan &bp, const uint64_t *masks, uint32
   }
   const int ns = (int)bp.sets.size();
   if (use_popc() || bp.fp64 || force_popc) {
-    CK(launch_pairs(bp.d_sets, bp.d_uslot, masks, dmask, bp.B, ctx->W, bp.gmax, stats, ctx->stream));
+    CK(launch_pairs(bp.d_sets, bp.d_uslot, masks, dmask, bp.B, ctx->W, bp.gmax, ctx->sms, stats,
+                    ctx->stream));
     CK(mark());
     ctx->launches += 1;
     return EDDY_OK;
@@ -731,7 +743,7 @@ int run_batch(eddy_ctx *ctx, std::vector<Job> &jobs, const std::vector<UnitRef> 
       words += (b.sd.core ? 1.0 : 2.25) * b.nb * (double)b.sd.c * W;
       pairs += b.nb * (double)b.sd.c;
     }
-    popc_batch = popc_batch || few_units(Bt, ns, words);
+    popc_batch = popc_batch || (few_units(Bt, ns, words) && !exact_class(ctx, ns, pairs));
   }
   // kept units: unit 0 of a keeping job
   std::vector<int> kept;  // batch indices of kept units

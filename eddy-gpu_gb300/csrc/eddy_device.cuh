@@ -180,7 +180,6 @@ __device__ __forceinline__ float rcp_approx(float x) {
 // FP32 chi-square of a 3x3 table: (1/N) sum (|N o - R C| - yN)^2 / (R C),
 // numerators exact in 32-bit integers (tables of N <= 32767 samples; larger
 // ones take the exact FP64 path).  Returns the marginals too.
-constexpr int kFastMaxN = 32767;
 __device__ __forceinline__ void table_info(const int *t, TabInfo &ti) {
   ti.R[0] = t[0] + t[1] + t[2];
   ti.R[1] = t[3] + t[4] + t[5];

@@ -12,6 +12,7 @@
 
 namespace eddy {
 
+constexpr int kFastMaxN = 32767;    // samples of a table at most that FP32 decides
 constexpr int kMaxSetGenes = 512;   // genes of a set at most
 constexpr int kDofSlots = 3;        // dof 1, 2, 4 (dof 0 never gives an edge)
 constexpr int kMaxBdeuParents = 3;  // kernel5.cu:119-130 caps at 1 + 3

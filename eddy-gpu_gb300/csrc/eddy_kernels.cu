@@ -261,17 +261,18 @@ __global__ void __launch_bounds__(32 * kCmWarps) k_counter_masks(int n, int nA, 
 // A block takes a 32 x 32 tile of one unit's pairs (rows above columns), a
 // lane one column gene, a warp four row genes, so a lane's three plane words
 // of 64 samples serve four pairs; the masked row planes are staged in shared
-// memory kPairWords words at a time.  A set without missing values counts
+// memory kPairWords words at a time.  Where the tiles are too few for the GPU
+// a block takes half or a quarter of one (launch_pairs).  A set without missing values counts
 // cells (-1,-1), (-1,0), (0,-1), (0,0) and derives the other five from the
 // genes' class-1 counts.  Bound by POPC (32 a word and lane in that case, 72
 // otherwise).
-constexpr int kPairTile = 32, kPairWords = 16, kPairRows = 4, kPairWarps = kPairTile / kPairRows;
-template <bool kCore>
-__device__ __forceinline__ void pairs_tile(const BatchSet &bs, int u, int tr, int tc, int W,
+constexpr int kPairTile = 32, kPairWords = 16, kPairWarps = 8;
+template <bool kCore, int kPairRows>
+__device__ __forceinline__ void pairs_tile(const BatchSet &bs, int u, int row0, int tc, int W,
                                            const uint64_t *__restrict__ mask, uint32_t *dmask,
                                            unsigned &nexact, unsigned &nfilt, unsigned &ntab) {
-  constexpr int kSt = kCore ? 2 : 3, kCells = kSt * kSt;
-  __shared__ uint64_t rowp[kPairTile][kSt][kPairWords + 1];  // (+ 1: fewer bank conflicts)
+  constexpr int kSt = kCore ? 2 : 3, kCells = kSt * kSt, kRows = kPairWarps * kPairRows;
+  __shared__ uint64_t rowp[kRows][kSt][kPairWords + 1];  // (+ 1: fewer bank conflicts)
   __shared__ int n1;  // the unit's class-1 samples
   __shared__ uint64_t mw[kPairWords];
   __shared__ int marg[2][kPairTile][2];  // class-1 counts of states -1, 0: rows, columns
@@ -290,8 +291,8 @@ __device__ __forceinline__ void pairs_tile(const BatchSet &bs, int u, int tr, in
     __syncthreads();
     if (threadIdx.x < nw) mw[threadIdx.x] = mask[w0 + threadIdx.x];
     // the masked row planes, word by word from the gene-major planes
-    for (int i = threadIdx.x; i < kPairTile * kSt * nw; i += blockDim.x) {
-      const int w = i % nw, ra = i / nw, r = ra / kSt, a = ra % kSt, row = tr * kPairTile + r;
+    for (int i = threadIdx.x; i < kRows * kSt * nw; i += blockDim.x) {
+      const int w = i % nw, ra = i / nw, r = ra / kSt, a = ra % kSt, row = row0 + r;
       rowp[r][a][w] = row < g ? sd.planes[((size_t)row * 3 + a) * W + w0 + w] & mask[w0 + w] : 0ull;
     }
     __syncthreads();
@@ -308,8 +309,8 @@ __device__ __forceinline__ void pairs_tile(const BatchSet &bs, int u, int tr, in
           cm[0] += __popcll(c[0] & m);
           cm[1] += __popcll(c[1] & m);
         } else if (warp == 1) {
-          rm[0] += __popcll(rowp[lane][0][w]);
-          rm[1] += __popcll(rowp[lane][1][w]);
+          rm[0] += __popcll(rowp[lane % kRows][0][w]);
+          rm[1] += __popcll(rowp[lane % kRows][1][w]);
         } else if (warp == 2) {
           nc += __popcll(mw[w]);
         }
@@ -339,7 +340,7 @@ __device__ __forceinline__ void pairs_tile(const BatchSet &bs, int u, int tr, in
   uint32_t *udm = unit_dmask(dmask, bs, u), *ucb = unit_chunks(dmask, bs, u);
 #pragma unroll
   for (int i = 0; i < kPairRows; i++) {
-    const int r = warp * kPairRows + i, row = tr * kPairTile + r;
+    const int r = warp * kPairRows + i, row = row0 + r;
     const bool live = row < g && col < row;
     if (!__any_sync(0xffffffffu, live)) continue;
     const int p = live ? row * (row - 1) / 2 + col : 0;
@@ -404,6 +405,7 @@ __device__ __forceinline__ void pairs_tile(const BatchSet &bs, int u, int tr, in
   }
 }
 
+template <int kPairRows>
 __global__ void __launch_bounds__(32 * kPairWarps, 2) k_pairs(const BatchSet *__restrict__ sets,
                                                            const int32_t *__restrict__ uslot,
                                                            const uint64_t *masks, int W,
@@ -416,11 +418,12 @@ __global__ void __launch_bounds__(32 * kPairWarps, 2) k_pairs(const BatchSet *__
   while (tr * (tr + 1) / 2 > (int)blockIdx.x) tr--;
   while ((tr + 1) * (tr + 2) / 2 <= (int)blockIdx.x) tr++;
   const int tc = (int)blockIdx.x - tr * (tr + 1) / 2;
-  if (tr * kPairTile >= bs.sd.g) return;
+  const int row0 = tr * kPairTile + (int)blockIdx.z * kPairWarps * kPairRows;
+  if (row0 >= bs.sd.g) return;
   unsigned nexact = 0, nfilt = 0, ntab = 0;
   const uint64_t *mask = masks + (size_t)u * W;
-  if (bs.sd.core) pairs_tile<true>(bs, u, tr, tc, W, mask, dmask, nexact, nfilt, ntab);
-  else pairs_tile<false>(bs, u, tr, tc, W, mask, dmask, nexact, nfilt, ntab);
+  if (bs.sd.core) pairs_tile<true, kPairRows>(bs, u, row0, tc, W, mask, dmask, nexact, nfilt, ntab);
+  else pairs_tile<false, kPairRows>(bs, u, row0, tc, W, mask, dmask, nexact, nfilt, ntab);
   if (stats) {
     // warp-aggregated counters
     for (int o = 16; o > 0; o >>= 1) {
@@ -2442,12 +2445,26 @@ cudaError_t launch_counter_masks(int n, int nA, int W, uint64_t seed, const int3
 }
 
 cudaError_t launch_pairs(const BatchSet *sets, const int32_t *uslot, const uint64_t *masks,
-                         uint32_t *dmask, int B, int W, int gmax, unsigned long long *stats,
-                         cudaStream_t st) {
+                         uint32_t *dmask, int B, int W, int gmax, int sms,
+                         unsigned long long *stats, cudaStream_t st) {
   if (gmax < 2) return cudaSuccess;
   const int t = (gmax + kPairTile - 1) / kPairTile;
+  const dim3 grid(t * (t + 1) / 2, B);
+  const long long tiles = (long long)grid.x * B;
   // grid.y holds at most 65535 units (a batch has at most 32768)
-  k_pairs<<<dim3(t * (t + 1) / 2, B), 32 * kPairWarps, 0, st>>>(sets, uslot, masks, W, dmask, stats);
+  // A block's time is a chain over the sample words, then over its warps'
+  // rows (their general and exact decisions above all), so while the quarters
+  // or halves of all tiles fit on the GPU together they are quicker: one tile
+  // of 100 samples, most tables on the general path, 0.060 / 0.035 / 0.021 ms
+  // (whole, halves, quarters), of 10000 samples 0.096 / 0.071 / 0.054, of
+  // 65000 with exact decisions 1.71 / 0.96 / 0.59; 112 tiles of 10000 samples
+  // 0.097 / 0.079 / 0.093, 448 0.199 / 0.212 / 0.236.
+  const auto launch = [&](auto *kernel, int parts) {
+    kernel<<<dim3(grid.x, grid.y, parts), 32 * kPairWarps, 0, st>>>(sets, uslot, masks, W, dmask, stats);
+  };
+  if (4 * tiles <= 2 * sms) launch(k_pairs<1>, 4);
+  else if (2 * tiles <= 2 * sms) launch(k_pairs<2>, 2);
+  else launch(k_pairs<4>, 1);
   return cudaGetLastError();
 }
 

@@ -1219,13 +1219,13 @@ size_t mma_y_bytes(int G, int genes, int n) {
 }
 // the A operand, then the general-path queue: a 16-byte counter and room
 // for every table of the batch (near-threshold workloads send half of them
-// or more to the general path), at least 65536 and at most 2^28 items
+// or more to the general path), at least kQueueMin and at most 2^28 items
 // (7.5 GB with the deferred list; the list's entries, item * 10 + slot,
 // stay below 2^32)
 static size_t a_operand_bytes(int rowsA, int n) { return (size_t)rowsA * mma_npad(n); }
 static unsigned queue_cap(long long tables) {
   const long long t = tables < (1ll << 28) ? tables : (1ll << 28);
-  return (unsigned)(t < 65536 ? 65536 : t);
+  return (unsigned)(t < kQueueMin ? kQueueMin : t);
 }
 // EDDY_GENERAL_QUEUE_CAP lowers the queue's capacity (tests of the
 // overflow path: the batch is then decided by the popcount kernel)

@@ -12,6 +12,9 @@ namespace eddy {
 // one row gene x 4 cells), padded for every tile shape
 int mma_ngroups_pad(const SetDev &sd, bool core);
 int mma_npad(int n);
+// Tables the general-path queue, and decisions its list for the exact path,
+// hold at least.
+constexpr int kQueueMin = 65536;
 
 // The Y arena of the sets of a batch: their column groups, G in all, and
 // their genes, `genes` in all, at a sample count n.  Set k's groups start at

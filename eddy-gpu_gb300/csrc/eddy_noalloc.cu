@@ -38,6 +38,7 @@ constexpr int kNAMaxGenes = 64;
 constexpr int kNAMaxSamples = 2048;
 constexpr int kNAPairs = kNAMaxGenes * (kNAMaxGenes - 1) / 2;
 constexpr int kNAW = kNAMaxSamples / 64;
+constexpr int kNASms = 128;  // of any GPU that runs this code, at least
 
 __host__ __device__ constexpr size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -215,7 +216,7 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
       return bail(EDDY_ERR_CUDA);
     if (cudaMemsetAsync(base + kOffDmask, 0, dmask_bytes(1, c), st) != cudaSuccess ||
         launch_pairs(d_sets, d_slot, (const uint64_t *)(base + kOffMask),
-                     (uint32_t *)(base + kOffDmask), 1, W, g, nullptr, st) != cudaSuccess)
+                     (uint32_t *)(base + kOffDmask), 1, W, g, kNASms, nullptr, st) != cudaSuccess)
       return bail(EDDY_ERR_CUDA);
     BatchDev bd{};
     bd.B = 1;
