@@ -880,6 +880,14 @@ __device__ __noinline__ void key_scores(const SetDev &sd, const UnitPtrs &P, con
 // are moved together (Hacker's Delight's compress, its five move masks
 // formed once per word and class) and appended to the gene's current output
 // word; the lanes share the masks, so they fill and store words together.
+//
+// A warp's words are one chain of latencies.  With many of them (kLong) the
+// warps that the genes leave over share the words, eight each at least, and a
+// word's masks are loaded a word ahead as its planes are (cycles of a block:
+// 10 genes x 16000 samples 235k -> 55k, 250 x 4000 133k -> 88k).  With few it
+// costs more than it gives (5025 units of 51 x 66 2.82 -> 2.87 ms).
+constexpr int kLongWords = 16;
+template <bool kLong>
 __device__ __noinline__ void pack_classes(const SetDev &sd, const UnitPtrs &P, uint32_t *moves,
                                           uint2 *out) {
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
@@ -904,30 +912,56 @@ __device__ __noinline__ void pack_classes(const SetDev &sd, const UnitPtrs &P, u
     }
   }
   __syncthreads();
-  const int gb = (g + 31) >> 5;
-  for (int task = warp; task < 2 * gb; task += nw) {
-    const int cls = task >= gb ? 1 : 0, i = 32 * (task - cls * gb) + lane;
+  const int gb = (g + 31) >> 5, segs = kLong ? max(1, min(nw / (2 * gb), sd.W / 8)) : 1;
+  for (int task = warp; task < 2 * gb * segs; task += nw) {
+    const int seg = kLong ? task / (2 * gb) : 0, ct = task - seg * 2 * gb, cls = ct >= gb ? 1 : 0;
+    const int i = 32 * (ct - cls * gb) + lane;
     const bool live = i < g;
-    const uint64_t *pl = sd.planesT + 3 * (size_t)(live ? i : g - 1);
-    uint2 *dst = out + (cls ? (size_t)class_words(sd.nA) * g : 0) + i;
-    const uint2 *end = dst + (size_t)class_words(cls ? sd.nB : sd.nA) * g;
+    // the sample words [ws, we): the class's output words [o0, o1) that start
+    // there, the last of which is filled from the words behind
+    int ws = 0, o0 = 0, o1 = class_words(cls ? sd.nB : sd.nA), fill = 0, at = 0;
+    if (kLong) {
+      const int *pc = cls ? P.pcB : P.pcA;
+      const int we = sd.W * (seg + 1) / segs;
+      ws = sd.W * seg / segs;
+      o0 = (pc[ws] + 31) >> 5;
+      if (we < sd.W) o1 = (pc[we] + 31) >> 5;
+      if (o0 >= o1) continue;
+      fill = pc[ws] & 31;
+      at = pc[ws] >> 5;
+    }
+    const uint64_t *pl = sd.planesT + 3 * ((size_t)ws * g + (live ? i : g - 1));
+    uint2 *dst = out + (cls ? (size_t)class_words(sd.nA) * g : 0) + (size_t)at * g + i;
+    auto store = [&](uint32_t x, uint32_t y) {
+      if (live && (!kLong || at >= o0)) *dst = make_uint2(x, y);
+      dst += g;
+      if (kLong) at++;
+    };
+    const uint2 *end = dst + (size_t)(o1 - at) * g;
     const uint4 *mv4 = reinterpret_cast<const uint4 *>(moves + 8 * (size_t)cls * W32);
     uint32_t a0 = 0u, a1 = 0u;
-    int fill = 0;
     uint64_t n0 = pl[0], n1 = pl[1], n2 = pl[2];  // the next word's planes
+    uint4 mn[4];
+#pragma unroll
+    for (int x = 0; kLong && x < 4; x++) mn[x] = mv4[4 * ws + x];
 #pragma unroll 1
-    for (int w = 0; w < sd.W; w++) {
+    for (int w = ws; w < sd.W && (!kLong || at < o1); w++) {
       const uint64_t q0 = n0, q1 = n1, q2 = n2;
+      uint4 mq[4];
+#pragma unroll
+      for (int x = 0; kLong && x < 4; x++) mq[x] = mn[x];
       if (w + 1 < sd.W) {
         pl += 3 * (size_t)g;
         n0 = pl[0];
         n1 = pl[1];
         n2 = pl[2];
+#pragma unroll
+        for (int x = 0; kLong && x < 4; x++) mn[x] = mv4[4 * (w + 1) + x];
       }
       const uint64_t mis = ~(q0 | q1 | q2), b0 = q1 | mis, b1 = q2 | mis;
 #pragma unroll
       for (int h = 0; h < 2; h++) {
-        const uint4 u = mv4[2 * (2 * w + h)], v = mv4[2 * (2 * w + h) + 1];
+        const uint4 u = kLong ? mq[2 * h] : mv4[4 * w + 2 * h], v = kLong ? mq[2 * h + 1] : mv4[4 * w + 2 * h + 1];
         const uint32_t mv[5] = {u.x, u.y, u.z, u.w, v.x};
         uint32_t x0 = (uint32_t)(b0 >> (32 * h)) & v.y, x1 = (uint32_t)(b1 >> (32 * h)) & v.y;
 #pragma unroll
@@ -940,8 +974,7 @@ __device__ __noinline__ void pack_classes(const SetDev &sd, const UnitPtrs &P, u
         a1 |= x1 << fill;
         const int c = __popc(v.y);
         if (fill + c >= 32) {
-          if (live) *dst = make_uint2(a0, a1);
-          dst += g;
+          if (!kLong || at < o1) store(a0, a1);
           a0 = fill ? x0 >> (32 - fill) : 0u;
           a1 = fill ? x1 >> (32 - fill) : 0u;
           fill -= 32;
@@ -949,12 +982,9 @@ __device__ __noinline__ void pack_classes(const SetDev &sd, const UnitPtrs &P, u
         fill += c;
       }
     }
-    // the rest of the class's words: no value
-    if (fill) {
-      if (live) *dst = make_uint2(a0 | (~0u << fill), a1 | (~0u << fill));
-      dst += g;
-    }
-    if (dst != end && live) *dst = make_uint2(~0u, ~0u);
+    // past the class's last sample: no value
+    if (fill && (!kLong || at < o1)) store(a0 | (~0u << fill), a1 | (~0u << fill));
+    while (kLong ? at < o1 : dst != end) store(~0u, ~0u);
   }
   __syncthreads();
 }
@@ -1799,7 +1829,11 @@ __device__ __forceinline__ void run_unit(const BatchDev &bd, int u, char *smraw)
   uint2 *cpw = (uint2 *)(scr + L.cp);
   const int cw1 = class_words(nA);
   const ClassPlanes cp[2] = {{cpw, g, cw1}, {cpw + (size_t)cw1 * g, g, class_words(nB)}};
-  if (networks || SM.ndab) pack_classes(sd, SM.P, (uint32_t *)(scr + L.moves), cpw);
+  if (networks || SM.ndab) {
+    uint32_t *moves = (uint32_t *)(scr + L.moves);
+    if (W >= kLongWords) pack_classes<true>(sd, SM.P, moves, cpw);
+    else pack_classes<false>(sd, SM.P, moves, cpw);
+  }
   uint2 *uv = (uint2 *)(scr + L.uv);
   uint32_t *vw = (uint32_t *)(scr + L.vw);
   const int vws = max(cw1, class_words(nB));
