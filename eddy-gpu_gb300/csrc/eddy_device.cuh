@@ -244,17 +244,6 @@ __device__ __forceinline__ int fast_decision(const TabInfo &ti, int prior, const
   return 2;
 }
 
-__device__ __forceinline__ int decide(const int *t, int prior, const SetDev &sd, TabInfo &ti,
-                                      unsigned &nexact) {
-  table_info(t, ti);
-  int d = fast_decision(ti, prior, sd);
-  if (d == 2) {
-    nexact++;
-    d = exact_decision(t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], prior, sd);
-  }
-  return d;
-}
-
 // Rigorous leave-one-out filter.  True when every table t - e_ab (one
 // sample of any cell removed) is certain to get the same decision as t.
 // Bound: with u_rc = (|o-e|-y)/sqrt(e), chi = |u|^2 and Minkowski,
@@ -516,52 +505,6 @@ __device__ __forceinline__ unsigned loo_f2(const f32x2 *o, const f32x2 *R, const
   const bool sx = okx && ax == bx && hx < f2_x(qK), sy = oky && ay == by && hy < f2_y(qK);
   mask = (sx ? bx : 0u) | (sy ? by << 16 : 0u);
   return (sx ? 0u : 1u) | (sy ? 0u : 2u);
-}
-
-// The general path: full-table decision, the Minkowski leave-one-out filter
-// and, when that cannot settle them, the nine cell-removed tables one by one.
-// Counts by value and not inlined: it runs for a small share of the tables.
-// Returns the mask in bits 0-9, the number of exact evaluations in bits
-// 32-47 and 1 in bit 48 when the filter settled the table.
-static __device__ __noinline__ uint64_t pair_mask_general(int a0, int a1, int a2, int a3, int a4,
-                                                          int a5, int a6, int a7, int a8,
-                                                          int prior, const SetDev &sd) {
-  int t[9] = {a0, a1, a2, a3, a4, a5, a6, a7, a8};
-  TabInfo ti;
-  unsigned nexact = 0;
-  const int bit0 = decide(t, prior, sd, ti, nexact);
-  if (loo_safe(ti, prior, sd))
-    return (bit0 ? 0x3FFull : 0ull) | ((uint64_t)nexact << 32) | (1ull << 48);
-  uint32_t m = (uint32_t)bit0;
-#pragma unroll 1
-  for (int cell = 0; cell < 9; cell++) {
-    int bit = bit0;
-    if (t[cell] > 0) {
-      t[cell]--;
-      TabInfo tj;
-      bit = decide(t, prior, sd, tj, nexact);
-      t[cell]++;
-    }
-    m |= (uint32_t)bit << (1 + cell);
-  }
-  return m | ((uint64_t)nexact << 32);
-}
-
-// 10-bit decision mask of one (pair, class) table: bit 0 = full table,
-// bit 1+3a+b = table with one sample of cell (a,b) removed.
-__device__ __forceinline__ uint32_t pair_mask(const int *t, int prior, const SetDev &sd,
-                                              unsigned &nexact, unsigned &nfilt) {
-  TabInfo ti;
-  table_info(t, ti);
-  if (quick_zero(ti, prior, sd)) {
-    nfilt++;
-    return 0u;
-  }
-  const uint64_t r =
-      pair_mask_general(t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], prior, sd);
-  nexact += (unsigned)(r >> 32) & 0xFFFFu;
-  nfilt += (unsigned)(r >> 48) & 1u;
-  return (uint32_t)r & 0x3FFu;
 }
 
 // --------------------------------------------------- capped parent lists

@@ -267,12 +267,111 @@ __global__ void __launch_bounds__(32 * kCmWarps) k_counter_masks(int n, int nA, 
 // genes' class-1 counts.  Bound by POPC (32 a word and lane in that case, 72
 // otherwise).
 constexpr int kPairTile = 32, kPairWords = 16, kPairWarps = 8;
+
+// The tables of a tile that the packed forms leave: their decisions are shared
+// out over the block, the FP32 ones a lane per table, the exact FP64 ones a
+// lane per decision.  (With each lane deciding its own tables a warp waited for
+// ten exact decisions one after the other of the few lanes that had any: every
+// decision in FP64, 8 genes x 40 samples, 700 units 3.19 ms a call, now 0.50; 60
+// x 400 at alpha 1e-9, where 5% of the tables needs them, 100 units 1.53, now
+// 0.19.)
+constexpr int kTileThreads = 32 * kPairWarps, kTileStep = 2 * kTileThreads;
+struct TileGeneral {
+  // counts (nine of 16 bits), then prior | class << 1 in the fifth word's high
+  // half, and the pair
+  uint32_t table[2 * kTileStep][6];
+  // of kTileThreads of them at a time: decisions known so far, the bits that
+  // share the full table's, and what is left, item * 10 + slot (0: the full
+  // table)
+  uint32_t bits[kTileThreads];
+  uint16_t shared0[kTileThreads], exact[10 * kTileThreads];
+};
+__device__ __forceinline__ void tile_table(const uint32_t *w, int *t) {
+#pragma unroll
+  for (int k = 0; k < 9; k++) t[k] = (int)((w[k >> 1] >> (16 * (k & 1))) & 0xFFFFu);
+}
+// The masks of the n tables listed in G into the unit's (*left: 0 before and
+// after).  Returns the exact evaluations of this thread, and in the high half
+// the tables a filter settled.
+__device__ __noinline__ uint64_t tile_general(TileGeneral &G, int n, int *left, const SetDev &sd,
+                                              uint32_t *udm, uint32_t *ucb) {
+  unsigned nexact = 0, nfilt = 0;
+  const int tid = threadIdx.x;
+#pragma unroll 1
+  for (int k0 = 0; k0 < n; k0 += kTileThreads) {
+    const uint32_t *w = G.table[k0 + tid];
+    if (k0 + tid < n) {
+      int t[9];
+      tile_table(w, t);
+      const int prior = (w[4] >> 16) & 1;
+      TabInfo ti;
+      table_info(t, ti);
+      uint32_t bits = 0u, shared0 = 1u;
+      if (quick_zero(ti, prior, sd)) {
+        nfilt++;
+      } else {
+        const int bit0 = fast_decision(ti, prior, sd);
+        if (loo_safe(ti, prior, sd)) {
+          shared0 = 0x3FFu;
+          nfilt++;
+        } else {
+#pragma unroll
+          for (int cell = 0; cell < 9; cell++) {
+            if (t[cell] == 0) {
+              shared0 |= 2u << cell;
+              continue;
+            }
+            t[cell]--;
+            TabInfo tj;
+            table_info(t, tj);
+            t[cell]++;
+            const int bit = fast_decision(tj, prior, sd);
+            if (bit == 2) G.exact[atomicAdd(left, 1)] = (uint16_t)(10 * tid + 1 + cell);
+            else bits |= (uint32_t)bit << (1 + cell);
+          }
+        }
+        if (bit0 == 2) G.exact[atomicAdd(left, 1)] = (uint16_t)(10 * tid);
+        else if (bit0) bits |= shared0;
+      }
+      G.bits[tid] = bits;
+      G.shared0[tid] = (uint16_t)shared0;
+    }
+    __syncthreads();
+    const int ne = *left;
+    for (int e = tid; e < ne; e += kTileThreads) {
+      const int k = G.exact[e] / 10, slot = G.exact[e] - 10 * k;
+      const uint32_t *x = G.table[k0 + k];
+      int t[9];
+      tile_table(x, t);
+#pragma unroll
+      for (int c = 0; c < 9; c++) t[c] -= slot == 1 + c ? 1 : 0;
+      nexact++;
+      if (exact_decision(t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], (x[4] >> 16) & 1, sd))
+        atomicOr(&G.bits[k], slot ? 1u << slot : (uint32_t)G.shared0[k]);
+    }
+    __syncthreads();
+    if (tid == 0) *left = 0;
+    if (k0 + tid < n && G.bits[tid]) {
+      atomicOr(&udm[w[5]], G.bits[tid] << ((w[4] >> 17) & 1 ? 16 : 0));
+      mark_chunk(ucb, (int)w[5]);
+    }
+    __syncthreads();
+  }
+  return (uint64_t)nexact | ((uint64_t)nfilt << 32);
+}
+
 template <bool kCore, int kPairRows>
 __device__ __forceinline__ void pairs_tile(const BatchSet &bs, int u, int row0, int tc, int W,
                                            const uint64_t *__restrict__ mask, uint32_t *dmask,
-                                           unsigned &nexact, unsigned &nfilt, unsigned &ntab) {
+                                           TileGeneral &G, int *listed, unsigned &nexact,
+                                           unsigned &nfilt, unsigned &ntab) {
   constexpr int kSt = kCore ? 2 : 3, kCells = kSt * kSt, kRows = kPairWarps * kPairRows;
-  __shared__ uint64_t rowp[kRows][kSt][kPairWords + 1];  // (+ 1: fewer bank conflicts)
+  // the masked row planes (+ 1: fewer bank conflicts), then in their place the
+  // tables the packed forms leave
+  using Rows = uint64_t[kRows][kSt][kPairWords + 1];
+  static_assert(sizeof(Rows) <= sizeof(TileGeneral), "room");
+  Rows &rowp = *reinterpret_cast<Rows *>(&G);
+  int &items = listed[0], &left = listed[1];  // tables; their exact decisions
   __shared__ int n1;  // the unit's class-1 samples
   __shared__ uint64_t mw[kPairWords];
   __shared__ int marg[2][kPairTile][2];  // class-1 counts of states -1, 0: rows, columns
@@ -335,60 +434,57 @@ __device__ __forceinline__ void pairs_tile(const BatchSet &bs, int u, int row0, 
     } else if (warp == 2 && lane == 0) {
       n1 = nc;
     }
-    __syncthreads();
   }
+  if (threadIdx.x == 0) items = left = 0;
+  __syncthreads();
   uint32_t *udm = unit_dmask(dmask, bs, u), *ucb = unit_chunks(dmask, bs, u);
 #pragma unroll
   for (int i = 0; i < kPairRows; i++) {
     const int r = warp * kPairRows + i, row = row0 + r;
     const bool live = row < g && col < row;
-    if (!__any_sync(0xffffffffu, live)) continue;
     const int p = live ? row * (row - 1) / 2 + col : 0;
-    int t[2][9];
-    if (kCore) {
-      t[0][0] = cnt[i][0], t[0][1] = cnt[i][1], t[0][3] = cnt[i][2], t[0][4] = cnt[i][3];
-      t[0][2] = marg[0][r][0] - t[0][0] - t[0][1];
-      t[0][5] = marg[0][r][1] - t[0][3] - t[0][4];
-      t[0][6] = marg[1][lane][0] - t[0][0] - t[0][3];
-      t[0][7] = marg[1][lane][1] - t[0][1] - t[0][4];
-      t[0][8] = n1 - marg[0][r][0] - marg[0][r][1] - t[0][6] - t[0][7];
-    } else {
-#pragma unroll
-      for (int k = 0; k < 9; k++) t[0][k] = cnt[i][k];
-    }
-    const uint16_t *ct = sd.ctot + (size_t)p * 9;
-#pragma unroll
-    for (int k = 0; k < 9; k++) t[1][k] = (int)ct[k] - t[0][k];
-    const int prior = sd.prior[p] ? 1 : 0;
-    const Thr &T = sd.thr[prior][2];
-    f32x2 o[9];
-#pragma unroll
-    for (int k = 0; k < 9; k++) o[k] = f2_pack((float)t[0][k], (float)t[1][k]);
+    int t[2][9], prior = 0;
     uint32_t m = 0u;
-    unsigned want = live ? ~quick_zero_f2(o, sd.exact_all ? -1.f : T.chiA) & 3u : 0u;
-    if (live) {
-      nfilt += 2 - __popc(want);
-      ntab += 2;
-    }
-    if (__any_sync(0xffffffffu, want)) {
-      f32x2 R[3], C[3];
+    unsigned unc = 0u;
+    if (__any_sync(0xffffffffu, live)) {
+      if (kCore) {
+        t[0][0] = cnt[i][0], t[0][1] = cnt[i][1], t[0][3] = cnt[i][2], t[0][4] = cnt[i][3];
+        t[0][2] = marg[0][r][0] - t[0][0] - t[0][1];
+        t[0][5] = marg[0][r][1] - t[0][3] - t[0][4];
+        t[0][6] = marg[1][lane][0] - t[0][0] - t[0][3];
+        t[0][7] = marg[1][lane][1] - t[0][1] - t[0][4];
+        t[0][8] = n1 - marg[0][r][0] - marg[0][r][1] - t[0][6] - t[0][7];
+      } else {
 #pragma unroll
-      for (int a = 0; a < 3; a++) {
-        R[a] = f2_add(f2_add(o[3 * a], o[3 * a + 1]), o[3 * a + 2]);
-        C[a] = f2_add(f2_add(o[a], o[3 + a]), o[6 + a]);
+        for (int k = 0; k < 9; k++) t[0][k] = cnt[i][k];
       }
-      const unsigned unc =
-          want & loo_f2(o, R, C, f2_add(f2_add(R[0], R[1]), R[2]), T, sd.exact_all != 0, m);
-      m = (want & 1u ? m & 0x3FFu : 0u) | (want & 2u ? m & 0x3FF0000u : 0u);
+      const uint16_t *ct = sd.ctot + (size_t)p * 9;
 #pragma unroll
-      for (int cls = 0; cls < 2; cls++) {
-        if (!((want >> cls) & 1u)) continue;
-        uint32_t mm = (m >> (16 * cls)) & 0x3FFu;
-        if ((unc >> cls) & 1u) {
-          mm = pair_mask(t[cls], prior, sd, nexact, nfilt);
-          m |= mm << (16 * cls);
-        } else if (mm == 0u || mm == 0x3FFu) {
-          nfilt++;  // the ten tables agree: settled at once
+      for (int k = 0; k < 9; k++) t[1][k] = (int)ct[k] - t[0][k];
+      prior = sd.prior[p] ? 1 : 0;
+      const Thr &T = sd.thr[prior][2];
+      f32x2 o[9];
+#pragma unroll
+      for (int k = 0; k < 9; k++) o[k] = f2_pack((float)t[0][k], (float)t[1][k]);
+      const unsigned want = live ? ~quick_zero_f2(o, sd.exact_all ? -1.f : T.chiA) & 3u : 0u;
+      if (live) {
+        nfilt += 2 - __popc(want);
+        ntab += 2;
+      }
+      if (__any_sync(0xffffffffu, want)) {
+        f32x2 R[3], C[3];
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+          R[a] = f2_add(f2_add(o[3 * a], o[3 * a + 1]), o[3 * a + 2]);
+          C[a] = f2_add(f2_add(o[a], o[3 + a]), o[6 + a]);
+        }
+        unc = want & loo_f2(o, R, C, f2_add(f2_add(R[0], R[1]), R[2]), T, sd.exact_all != 0, m);
+        m = (want & 1u ? m & 0x3FFu : 0u) | (want & 2u ? m & 0x3FF0000u : 0u);
+#pragma unroll
+        for (int cls = 0; cls < 2; cls++) {
+          const uint32_t mm = (m >> (16 * cls)) & 0x3FFu;
+          // (the ten tables agree: settled at once)
+          nfilt += (((want & ~unc) >> cls) & 1u) && (mm == 0u || mm == 0x3FFu);
         }
       }
     }
@@ -401,6 +497,34 @@ __device__ __forceinline__ void pairs_tile(const BatchSet &bs, int u, int row0, 
       const unsigned first = cut >= 32 ? ~0u : (1u << cut) - 1u;
       if (lane == 0 && (nz & first)) mark_chunk(ucb, p0);
       if (lane == 1 && (nz & ~first)) mark_chunk(ucb, p0 + cut);
+    }
+    // what is left goes into the list, which has room for two steps
+    const unsigned b0 = __ballot_sync(0xffffffffu, unc & 1u);
+    const unsigned b1 = __ballot_sync(0xffffffffu, (unc & 2u) != 0u), below = (1u << lane) - 1u;
+    const int cnt = __popc(b0) + __popc(b1);
+    int at = 0;
+    if (cnt) {
+      if (lane == 0) at = atomicAdd(&items, cnt);
+      at = __shfl_sync(0xffffffffu, at, 0);
+#pragma unroll
+      for (int cls = 0; cls < 2; cls++)
+        if ((unc >> cls) & 1u) {
+          uint32_t *w = G.table[at + (cls ? __popc(b0) + __popc(b1 & below) : __popc(b0 & below))];
+#pragma unroll
+          for (int k = 0; k < 4; k++)
+            w[k] = (uint32_t)t[cls][2 * k] | ((uint32_t)t[cls][2 * k + 1] << 16);
+          w[4] = (uint32_t)t[cls][8] | ((uint32_t)(prior | (cls << 1)) << 16);
+          w[5] = (uint32_t)p;
+        }
+    }
+    // (a barrier: the masks stored above are there before bits are added)
+    if (!__syncthreads_or(i == kPairRows - 1 ? cnt != 0 || items > 0 : at + cnt > kTileStep)) continue;
+    const uint64_t c = tile_general(G, items, &left, sd, udm, ucb);
+    nexact += (unsigned)c;
+    nfilt += (unsigned)(c >> 32);
+    if (i < kPairRows - 1) {
+      if (threadIdx.x == 0) items = 0;
+      __syncthreads();
     }
   }
 }
@@ -420,10 +544,12 @@ __global__ void __launch_bounds__(32 * kPairWarps, 2) k_pairs(const BatchSet *__
   const int tc = (int)blockIdx.x - tr * (tr + 1) / 2;
   const int row0 = tr * kPairTile + (int)blockIdx.z * kPairWarps * kPairRows;
   if (row0 >= bs.sd.g) return;
+  __shared__ __align__(16) TileGeneral G;
+  __shared__ int listed[2];
   unsigned nexact = 0, nfilt = 0, ntab = 0;
   const uint64_t *mask = masks + (size_t)u * W;
-  if (bs.sd.core) pairs_tile<true, kPairRows>(bs, u, row0, tc, W, mask, dmask, nexact, nfilt, ntab);
-  else pairs_tile<false, kPairRows>(bs, u, row0, tc, W, mask, dmask, nexact, nfilt, ntab);
+  if (bs.sd.core) pairs_tile<true, kPairRows>(bs, u, row0, tc, W, mask, dmask, G, listed, nexact, nfilt, ntab);
+  else pairs_tile<false, kPairRows>(bs, u, row0, tc, W, mask, dmask, G, listed, nexact, nfilt, ntab);
   if (stats) {
     // warp-aggregated counters
     for (int o = 16; o > 0; o >>= 1) {
