@@ -662,11 +662,13 @@ int launch_pairs_any(eddy_ctx *ctx, BatchPlan &bp, const uint64_t *masks, uint32
   return run(variant, stats, ev_mid);
 }
 
-int check_mma_error(eddy_ctx *ctx, const BatchPlan &bp) {
+// *full: the general-path queue or its list overflowed.
+int check_mma_error(eddy_ctx *ctx, const BatchPlan &bp, bool *full) {
   unsigned e = 0;
   CK(cudaMemcpyAsync(&e, bp.d_err, sizeof e, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
-  if (e) return fail(ctx, EDDY_ERR_INTERNAL, "tensor-core pipeline wait timed out");
+  if (e & 1u) return fail(ctx, EDDY_ERR_INTERNAL, "tensor-core pipeline wait timed out");
+  *full = (e & 2u) != 0u;
   return EDDY_OK;
 }
 
@@ -1787,11 +1789,21 @@ int eddy_debug_edges(eddy_ctx *ctx, int set_id, const uint8_t *labels, uint8_t *
   memcpy(ctx->h_stage.as<uint8_t>(i_mask), m.data(), 8 * W);
   CK(cudaMemcpyAsync(ctx->d_in.p, ctx->h_stage.p, i_mask + 8 * W, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemsetAsync(ctx->d_out.p, 0, 8, ctx->stream));
-  rc = launch_pairs_any(ctx, bp, (const uint64_t *)(ctx->d_in.as<uint8_t>() + i_mask),
-                        ctx->d_dmask.as<uint32_t>(), nullptr);
-  if (rc) return rc;
-  rc = check_mma_error(ctx, bp);
-  if (rc) return rc;
+  bool full = false;
+  for (int attempt = 0; attempt == 0 || full; attempt++) {
+    if (attempt) {
+      // decided another way, as a batch would be: masks at zero again
+      rc = dmask_ready(ctx, dmask_bytes(1, c));
+      if (rc) return rc;
+      ctx->dmask_clean = nullptr;
+      CK(cudaMemsetAsync(ctx->d_out.p, 0, 8, ctx->stream));
+    }
+    rc = launch_pairs_any(ctx, bp, (const uint64_t *)(ctx->d_in.as<uint8_t>() + i_mask),
+                          ctx->d_dmask.as<uint32_t>(), nullptr, attempt > 0);
+    if (rc) return rc;
+    rc = check_mma_error(ctx, bp, &full);
+    if (rc) return rc;
+  }
   std::vector<uint32_t> dm(c);
   CK(cudaMemcpyAsync(dm.data(), ctx->d_dmask.p, 4 * (size_t)c, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
