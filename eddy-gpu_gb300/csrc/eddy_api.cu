@@ -603,7 +603,7 @@ int launch_pairs_any(eddy_ctx *ctx, BatchPlan &bp, const uint64_t *masks, uint32
   }
   const int ns = (int)bp.sets.size();
   if (use_popc() || bp.fp64 || force_popc) {
-    CK(launch_pairs(bp.d_sets, bp.d_uslot, masks, dmask, bp.B, ctx->W, bp.gmax, ctx->sms, stats,
+    CK(launch_pairs(bp.d_sets, bp.d_uslot, masks, dmask, bp.B, ctx->W, bp.gmax, ctx->sms, bp.fp64, stats,
                     ctx->stream));
     CK(mark());
     ctx->launches += 1;

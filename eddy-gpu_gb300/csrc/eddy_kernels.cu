@@ -2605,7 +2605,7 @@ cudaError_t launch_counter_masks(int n, int nA, int W, uint64_t seed, const int3
 }
 
 cudaError_t launch_pairs(const BatchSet *sets, const int32_t *uslot, const uint64_t *masks,
-                         uint32_t *dmask, int B, int W, int gmax, int sms,
+                         uint32_t *dmask, int B, int W, int gmax, int sms, bool exact_all,
                          unsigned long long *stats, cudaStream_t st) {
   if (gmax < 2) return cudaSuccess;
   const int t = (gmax + kPairTile - 1) / kPairTile;
@@ -2618,11 +2618,15 @@ cudaError_t launch_pairs(const BatchSet *sets, const int32_t *uslot, const uint6
   // of 100 samples, most tables on the general path, 0.060 / 0.035 / 0.021 ms
   // (whole, halves, quarters), of 10000 samples 0.096 / 0.071 / 0.054, of
   // 65000 with exact decisions 1.71 / 0.96 / 0.59; 112 tiles of 10000 samples
-  // 0.097 / 0.079 / 0.093, 448 0.199 / 0.212 / 0.236.
+  // 0.097 / 0.079 / 0.093, 448 0.199 / 0.212 / 0.236.  (The figures of general
+  // and exact decisions are from before the block shared them.)  Where every
+  // decision is exact, a tile is FP64 work for one SM and quarters spread it
+  // better however many there are: 10 units of 120 genes x 150 samples 3.26
+  // -> 2.03 ms a call, 700 of 60 x 400 32.6 -> 30.8, of 200 x 1000 404 -> 402.
   const auto launch = [&](auto *kernel, int parts) {
     kernel<<<dim3(grid.x, grid.y, parts), 32 * kPairWarps, 0, st>>>(sets, uslot, masks, W, dmask, stats);
   };
-  if (4 * tiles <= 2 * sms) launch(k_pairs<1>, 4);
+  if (4 * tiles <= 2 * sms || exact_all) launch(k_pairs<1>, 4);
   else if (2 * tiles <= 2 * sms) launch(k_pairs<2>, 2);
   else launch(k_pairs<4>, 1);
   return cudaGetLastError();

@@ -21,9 +21,10 @@ cudaError_t launch_counter_masks(int n, int nA, int W, uint64_t seed, const int3
                                  const int32_t *unit_perm, const uint64_t *mask0, uint64_t *masks,
                                  int B, cudaStream_t st);
 // Popcount contingency and decision kernel for a batch (sets: its device
-// set table, uslot: each unit's set; gmax: the largest set; sms: the GPU's SMs).
+// set table, uslot: each unit's set; gmax: the largest set; sms: the GPU's SMs;
+// exact_all: every set decides in FP64 throughout).
 cudaError_t launch_pairs(const BatchSet *sets, const int32_t *uslot, const uint64_t *masks,
-                         uint32_t *dmask, int B, int W, int gmax, int sms,
+                         uint32_t *dmask, int B, int W, int gmax, int sms, bool exact_all,
                          unsigned long long *stats, cudaStream_t st);
 // Network, BDeu and JS kernel of a batch; before, its layouts and blocks
 // (bd.B units of `pairs` pairs together, the largest set of gmax genes, n

@@ -216,7 +216,8 @@ extern "C" int eddy_unit_noalloc(const eddy_opts *opts, const int8_t *vals, int 
       return bail(EDDY_ERR_CUDA);
     if (cudaMemsetAsync(base + kOffDmask, 0, dmask_bytes(1, c), st) != cudaSuccess ||
         launch_pairs(d_sets, d_slot, (const uint64_t *)(base + kOffMask),
-                     (uint32_t *)(base + kOffDmask), 1, W, g, kNASms, nullptr, st) != cudaSuccess)
+                     (uint32_t *)(base + kOffDmask), 1, W, g, kNASms, sd.exact_all != 0,
+                     nullptr, st) != cudaSuccess)
       return bail(EDDY_ERR_CUDA);
     BatchDev bd{};
     bd.B = 1;
